@@ -417,7 +417,7 @@ class ElasticBuffer:
                             num_max_tokens_per_rank, expert_alignment, num_sms, previous_event,
                             previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream, handle,
                             do_cpu_sync, do_expand, do_zero_padding, use_tma_aligned_col_major_sf, zero_copy, fused_fp8,
-                            round_scale, num_worst_tokens=0):
+                            round_scale, num_worst_tokens=0, do_handle_copy=True):
         a = _C.DispatchArgs()
         if isinstance(x, tuple):
             a.x, a.sf = x
@@ -448,6 +448,7 @@ class ElasticBuffer:
         assert num_max_tokens_per_rank > 0, 'num_max_tokens_per_rank is unknown'
         a.topk_idx = topk_idx
         a.topk_weights = topk_weights
+        a.copy_topk_idx = do_handle_copy and handle is None
         a.cumulative_stats = cumulative_local_expert_recv_stats
         a.num_experts = num_experts
         a.num_max_tokens = num_max_tokens_per_rank
@@ -471,7 +472,7 @@ class ElasticBuffer:
     def _wrap_dispatch_result(self, r, a, do_handle_copy: bool, handle: Optional[EPHandle]):
         num_local = a.num_experts // self.num_ranks
         if handle is None:
-            topk_idx = a.topk_idx.clone() if do_handle_copy else a.topk_idx
+            topk_idx = r.topk_idx if do_handle_copy else a.topk_idx
             new_handle = EPHandle(a.do_expand, a.num_experts, a.expert_alignment, a.num_max_tokens, r.num_sms, topk_idx,
                                   r.num_recv_tokens, r.num_expanded_tokens, r.num_recv_tokens_per_expert_list,
                                   r.psum_rank, r.psum_expert[:num_local], r.num_unaligned, r.recv_src_metadata,
@@ -515,7 +516,7 @@ class ElasticBuffer:
                                      num_max_tokens_per_rank, expert_alignment, num_sms, previous_event,
                                      previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream,
                                      handle, do_cpu_sync, do_expand, do_zero_padding, use_tma_aligned_col_major_sf,
-                                     zero_copy, fused_fp8, round_scale, num_worst_tokens)
+                                     zero_copy, fused_fp8, round_scale, num_worst_tokens, do_handle_copy)
         r = _C.Runtime.dispatch([self.runtime], [a])[0]
         return self._wrap_dispatch_result(r, a, do_handle_copy, handle)
 

@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 
 #include "../common/layout.hpp"
@@ -17,12 +18,30 @@ namespace ep {
 // shared-memory carve-out as the preferred one. All communication kernels ask for the same carve-out, whatever they
 // use: an SM has to drain and reconfigure when consecutive kernels prefer different ones, which costs microseconds
 // between the back-to-back kernels of a dispatch / combine step.
-template <typename Kernel>
-inline cudaError_t prepare_kernel(Kernel kernel, int dynamic_smem_bytes) {
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic_smem_bytes);
-    if (err != cudaSuccess) return err;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-}
+// One static object per kernel remembers, per device, what the attributes were set to: the two driver calls cost a
+// microsecond or two of host time, which every launch used to pay. (The limit only ever grows; two threads that race
+// set the same attributes twice.)
+class PreparedKernel {
+public:
+    template <typename Kernel>
+    cudaError_t prepare(Kernel kernel, int dynamic_smem_bytes) {
+        int device = 0;
+        cudaError_t err = cudaGetDevice(&device);
+        if (err != cudaSuccess) return err;
+        const bool known = device >= 0 && device < kDevices;
+        if (known && granted_[device].load(std::memory_order_acquire) > dynamic_smem_bytes) return cudaSuccess;
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic_smem_bytes);
+        if (err != cudaSuccess) return err;
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (err != cudaSuccess) return err;
+        if (known) granted_[device].store(dynamic_smem_bytes + 1, std::memory_order_release);
+        return cudaSuccess;
+    }
+
+private:
+    static constexpr int kDevices = 64;
+    std::atomic<int> granted_[kDevices] = {};      // granted bytes + 1, 0 = never set
+};
 
 // ---------------------------------------------------------------- cross-rank barrier
 struct BarrierParams {
@@ -122,6 +141,9 @@ struct DispatchEpilogueParams {
     int* recv_src_metadata;   // [num_idx_rows, K + 2]
     int num_out_rows;         // capacity of recv_x in rows (expand: expanded rows)
     int num_idx_rows;         // rows of the routing outputs; rows past the received count are filled with -1 / 0
+    const void* topk_idx = nullptr;     // this rank's own routing, copied to ...
+    void* topk_idx_copy = nullptr;      // ... the handle's tensor (or null)
+    int64_t topk_idx_bytes = 0;
 };
 cudaError_t launch_dispatch_epilogue(const DispatchEpilogueParams* params, int num_vranks, int num_sms, int smem_optin,
                                      cudaStream_t stream, bool programmatic = false);
@@ -180,10 +202,8 @@ struct CombineParams {
     int fuse_reduce;
     int num_send_warps;       // warps of a block (one staging buffer each); filled in by the launcher
     int num_send_blocks;      // blocks of the grid
-    int direct_out;           // single rank, no bias, one row per token: rows go straight to red.combined_x, no reduce
     int flag_chunks;          // counters per source rank = ceil(ranks * max tokens / kCombineFlagRows)
     uint64_t off_comb_flag;   // [2 parities][R][flag_chunks] uint32 rows-landed counters
-    CombineEpilogueParams red;
 };
 struct CombineLaunch {
     int num_sms;
@@ -196,6 +216,72 @@ cudaError_t launch_combine(const Multi<CombineParams>& m, const CombineLaunch& l
 // `programmatic`: launched as a programmatic dependent of the kernel before it in the stream (the send kernel).
 cudaError_t launch_combine_epilogue(const CombineEpilogueParams* params, int num_vranks, int num_sms, cudaStream_t stream,
                                     bool programmatic = false);
+
+// ---------------------------------------------------------------- dispatch / combine of a group of one rank
+struct LocalPlanParams {
+    int num_tokens, num_topk, num_experts, expert_alignment, do_expand, idx32;
+    const void* topk_idx;     // [T, K]
+    int* token_slot;          // [T]  row of the token among the received tokens, -1 = no valid expert
+    int* pair_row;            // [T, K]  row of the pair in the expanded layout, -1 = unused lane
+    int* psum_rank;           // [1]
+    int* psum_expert;         // [E + 1]
+    int* num_unaligned;       // [E]
+    int* count_matrix;        // [1]
+    int* recv_stats;          // [E] cumulative statistics or null
+    uint64_t* host_counts;    // mapped pinned words (see DispatchParams) or null
+    uint32_t epoch;
+    uint64_t* timeline;       // {start, end} of this kernel and its move kernel (ns)
+    uint64_t* stamps;         // [8] phase stamps of the last dispatch
+};
+cudaError_t launch_local_plan(const LocalPlanParams& p, cudaStream_t stream);
+
+struct LocalMoveParams {
+    int num_tokens, num_topk, num_experts, expert_alignment, do_expand, do_zero_padding, write_metadata, idx32, pow2;
+    int src_row_bytes;
+    int plan_ahead;           // 1: launched behind the plan kernel (waits for its end)
+    int wide_in, wide_out;    // rows start on 32-byte boundaries (filled in by the launcher)
+    const uint8_t* x;
+    int64_t x_stride_bytes;
+    const uint32_t* sf;       // caller-made scale factors (packs of 4 bytes) or null
+    int64_t sf_token_stride, sf_pack_stride;
+    int sf_packs;             // packs per output row (made here or by the caller)
+    const void* topk_idx;     // [T, K]
+    void* topk_idx_copy;      // [T, K] or null: the handle's own copy of the routing
+    const float* topk_weights;
+    const int* token_slot;
+    const int* pair_row;
+    const int* psum_rank;
+    const int* psum_expert;
+    uint8_t* recv_x;
+    int64_t recv_x_pitch;     // bytes between output rows
+    uint32_t* recv_sf;        // or null
+    int64_t recv_sf_row_stride, recv_sf_pack_stride;   // in packs
+    void* recv_topk_idx;      // [num_idx_rows, K] or null
+    float* recv_topk_weights; // [num_idx_rows, K], expanded [rows], or null
+    int* recv_src_metadata;   // [num_idx_rows, K + 2]
+    int num_out_rows, num_idx_rows;
+    uint64_t* timeline;
+};
+// `quant`: bf16 rows are cast to e4m3 with 1x128 scales. `programmatic`: behind the plan kernel, nothing in between.
+cudaError_t launch_local_move(const LocalMoveParams& p, bool quant, int num_sms, bool programmatic, cudaStream_t stream);
+
+struct LocalCombineParams {
+    int num_tokens, num_topk, num_experts, row_bytes, do_expand, weighted, idx32;
+    int round_partial;        // the sum of a token's rows is rounded to bf16 before the biases are added
+    int num_x_rows;
+    const uint8_t* x;
+    int64_t x_stride_bytes;
+    const float* topk_weights;       // [N, K], expanded [rows], or null
+    const int* token_slot;           // [T]
+    const int* recv_src_metadata;    // [N, K + 2]
+    const void* topk_idx;            // [T, K]
+    const uint8_t* bias0;
+    const uint8_t* bias1;
+    uint8_t* combined_x;             // [T, row]
+    float* combined_topk_weights;    // [T, K] or null
+    uint64_t* timeline;              // {start, end} (ns)
+};
+cudaError_t launch_local_combine(const LocalCombineParams& p, int num_sms, cudaStream_t stream);
 
 // ---------------------------------------------------------------- layout (legacy get_dispatch_layout)
 cudaError_t launch_dispatch_layout(const void* topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks, int num_experts,

@@ -421,16 +421,6 @@ __global__ void __launch_bounds__(1024, 1) combine_kernel(const __grid_constant_
     // rows are handed out dynamically (SMs differ in how fast their peer stores drain)
     unsigned long long* work = reinterpret_cast<unsigned long long*>(c.local_ws + kWsWork);
     int64_t g = is_sender ? static_cast<int64_t>(bid) * num_warps + warp : total_steps;
-    if (p.direct_out) {
-        // tokens without any valid expert receive no row: their result is zero
-        const int all_warps = blockDim.x >> 5;
-        for (int t = bid * all_warps + warp; t < p.red.num_tokens; t += nb * all_warps) {
-            if (__any_sync(0xffffffffu, token_expert(p.red, t, lane) >= 0)) continue;
-            for (int v = lane; v < vec_per_row; v += 32)
-                st_na_int4(p.red.combined_x + static_cast<uint64_t>(t) * p.row_bytes + v * 16, make_int4(0, 0, 0, 0));
-            if (p.red.combined_topk_weights != nullptr && lane < K) p.red.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = 0.f;
-        }
-    }
     int64_t next_g = 0;
     bool fatal = false;
     for (; g < total_steps && !fatal; g = next_g) {
@@ -460,13 +450,7 @@ __global__ void __launch_bounds__(1024, 1) combine_kernel(const __grid_constant_
             const int slot_lane = p.use_rank_layout ? c.rank : master_lane;
             const uint64_t dst_row = static_cast<uint64_t>(slot_lane) * p.num_max_tokens + src_token;
             uint8_t* dst_ptr = heap + p.off_comb_x + dst_row * p.row_bytes;
-            if (p.direct_out) {
-                // single rank: the row is the token's only contribution, it goes straight to the result
-                dst_ptr = p.red.combined_x + static_cast<uint64_t>(src_token) * p.row_bytes;
-                if (p.red.combined_topk_weights != nullptr && lane < K)
-                    p.red.combined_topk_weights[static_cast<int64_t>(src_token) * K + lane] =
-                        token_expert(p.red, src_token, lane) >= 0 && p.topk_weights != nullptr ? p.topk_weights[static_cast<int64_t>(i) * K + lane] : 0.f;
-            } else if (p.topk_weights != nullptr && lane < K) {
+            if (p.topk_weights != nullptr && lane < K) {
                 reinterpret_cast<float*>(heap + p.off_comb_w)[dst_row * K + lane] = p.topk_weights[static_cast<int64_t>(i) * K + lane];
             }
             const bool landed = mbar_wait(w, bar, parity, kStatusTmaLoad, i);
@@ -482,9 +466,11 @@ __global__ void __launch_bounds__(1024, 1) combine_kernel(const __grid_constant_
             int my_row = lane < K ? md[2 + lane] : -1;
             const uint32_t valid = __ballot_sync(0xffffffffu, my_row >= 0);
             const uint64_t dst_row = static_cast<uint64_t>(c.rank) * p.num_max_tokens + src_token;
-            uint8_t* dst_ptr = p.direct_out ? p.red.combined_x + static_cast<uint64_t>(src_token) * p.row_bytes
-                                            : heap + p.off_comb_x + dst_row * p.row_bytes;
-            for (int v = lane; v < vec_per_row; v += 32) {
+            uint8_t* dst_ptr = heap + p.off_comb_x + dst_row * p.row_bytes;
+            // (every lane takes part in the shuffles of every pass: rows that are not a multiple of 512 bytes leave some without a column)
+            for (int v0 = 0; v0 < vec_per_row; v0 += 32) {
+                const int v = v0 + lane;
+                const bool in_row = v < vec_per_row;
                 float acc[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) acc[j] = 0.f;
@@ -502,23 +488,19 @@ __global__ void __launch_bounds__(1024, 1) combine_kernel(const __grid_constant_
                     float wt[4];
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
-                        if (rows[r] >= 0) raw[r] = ld_nc_int4(p.x + static_cast<int64_t>(rows[r]) * p.x_stride_bytes + v * 16);
+                        if (rows[r] >= 0 && in_row) raw[r] = ld_nc_int4(p.x + static_cast<int64_t>(rows[r]) * p.x_stride_bytes + v * 16);
                         wt[r] = (p.weighted && rows[r] >= 0) ? p.topk_weights[rows[r]] : 1.f;
                     }
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
-                        if (rows[r] >= 0) {
+                        if (rows[r] >= 0 && in_row) {
                             if (p.weighted) accumulate_bf16x8_scaled(acc, raw[r], wt[r]);
                             else accumulate_bf16x8(acc, raw[r]);
                         }
                 }
-                reinterpret_cast<int4*>(buf)[v] = pack_bf16x8(acc);
+                if (in_row) reinterpret_cast<int4*>(buf)[v] = pack_bf16x8(acc);
             }
-            if (p.direct_out) {
-                if (p.red.combined_topk_weights != nullptr && lane < K)
-                    p.red.combined_topk_weights[static_cast<int64_t>(src_token) * K + lane] =
-                        my_row >= 0 && p.topk_weights != nullptr ? p.topk_weights[my_row] : 0.f;
-            } else if (p.topk_weights != nullptr && my_row >= 0) {
+            if (p.topk_weights != nullptr && my_row >= 0) {
                 reinterpret_cast<float*>(heap + p.off_comb_w)[dst_row * K + lane] = p.topk_weights[my_row];
             }
             fence_proxy_async_smem();
@@ -638,7 +620,8 @@ bool plan_combine(const CombineParams& p, int num_sms, int smem_optin, CombineLa
 
 cudaError_t launch_combine(const Multi<CombineParams>& m, const CombineLaunch& l, cudaStream_t stream) {
     void (*kernel)(const Multi<CombineParams>) = m.r[0].fuse_reduce != 0 ? combine_kernel<true> : combine_kernel<false>;
-    cudaError_t err = prepare_kernel(kernel, l.smem_bytes);
+    static PreparedKernel prepared[2];
+    cudaError_t err = prepared[m.r[0].fuse_reduce != 0 ? 1 : 0].prepare(kernel, l.smem_bytes);
     if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(m.num_vranks * m.blocks_per_rank);
@@ -663,7 +646,8 @@ cudaError_t launch_combine_epilogue(const CombineEpilogueParams* params, int num
     m.num_vranks = num_vranks;
     m.blocks_per_rank = num_sms;
     for (int v = 0; v < num_vranks; ++v) m.r[v] = params[v];
-    cudaError_t err = prepare_kernel(combine_epilogue_kernel, kEpiSmem);
+    static PreparedKernel prepared;
+    cudaError_t err = prepared.prepare(combine_epilogue_kernel, kEpiSmem);
     if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_vranks * num_sms);

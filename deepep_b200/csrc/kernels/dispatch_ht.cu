@@ -618,6 +618,10 @@ __global__ void __launch_bounds__(1024, 1) dispatch_epilogue_kernel(const __grid
     }
     __syncwarp();
 
+    // the handle's own copy of the routing: an input of the call, nothing to wait for
+    for (int64_t i = (static_cast<int64_t>(bid) * nthreads + tid) * 4; p.topk_idx_copy != nullptr && i < p.topk_idx_bytes; i += static_cast<int64_t>(nb) * nthreads * 4)
+        *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(p.topk_idx_copy) + i) = *reinterpret_cast<const uint32_t*>(static_cast<const uint8_t*>(p.topk_idx) + i);
+
     dependency_wait();      // the dispatch kernel of this rank has completed (all its writes are visible)
     if (bid == 0 && tid == 0) timeline[0] = globaltimer_ns();
     const WaitCtx w = make_wait_ctx(p.c);
@@ -786,7 +790,8 @@ bool plan_dispatch(const DispatchParams& p, int num_sms, int smem_optin, Dispatc
 }
 
 cudaError_t launch_dispatch(const Multi<DispatchParams>& m, const DispatchLaunch& l, cudaStream_t stream) {
-    cudaError_t err = prepare_kernel(dispatch_kernel, l.smem_bytes);
+    static PreparedKernel prepared;
+    cudaError_t err = prepared.prepare(dispatch_kernel, l.smem_bytes);
     if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(m.num_vranks * m.blocks_per_rank);
@@ -815,7 +820,8 @@ cudaError_t launch_dispatch_epilogue(const DispatchEpilogueParams* params, int n
     if (warps > (move_rows ? 16 : 32)) warps = move_rows ? 16 : 32;
     if (warps < 1) return cudaErrorInvalidValue;
     const int smem_bytes = move_rows ? warps * stage : 0;
-    cudaError_t err = prepare_kernel(dispatch_epilogue_kernel, smem_bytes);
+    static PreparedKernel prepared;
+    cudaError_t err = prepared.prepare(dispatch_epilogue_kernel, smem_bytes);
     if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_vranks * num_sms);

@@ -777,7 +777,8 @@ cudaError_t launch_ll_dispatch(const Multi<LLDispatchParams>& m, int num_sms, cu
     const LLDispatchParams& p = m.r[0];
     const int msg_stride = align_up(ll_dispatch_msg_bytes(p.hidden, p.use_fp8), 128);
     const int smem_bytes = align_up(p.num_max_tokens * p.num_topk * 4, 128) + 2 * msg_stride;
-    cudaError_t err = prepare_kernel(ll_dispatch_kernel, smem_bytes);
+    static PreparedKernel prepared;
+    cudaError_t err = prepared.prepare(ll_dispatch_kernel, smem_bytes);
     if (err != cudaSuccess) return err;
     Multi<LLDispatchParams> copy = m;
     copy.blocks_per_rank = num_sms;
@@ -793,7 +794,8 @@ cudaError_t launch_ll_combine(const Multi<LLCombineParams>& m, int num_sms, int 
     const int smem_bytes = warps * stage;
     // the receive phase of a LogFMT call keeps three words per (lane, group) in the same shared memory
     if (p.use_logfmt && p.num_topk * (p.hidden / 128) * 12 > smem_bytes) return cudaErrorInvalidValue;
-    cudaError_t err = prepare_kernel(ll_combine_kernel, smem_bytes);
+    static PreparedKernel prepared;
+    cudaError_t err = prepared.prepare(ll_combine_kernel, smem_bytes);
     if (err != cudaSuccess) return err;
     Multi<LLCombineParams> copy = m;
     copy.blocks_per_rank = num_sms;

@@ -64,6 +64,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readwrite("num_worst_tokens", &DispatchArgs::num_worst_tokens)
         .def_readwrite("col_major_sf", &DispatchArgs::col_major_sf)
         .def_readwrite("cached", &DispatchArgs::cached)
+        .def_readwrite("copy_topk_idx", &DispatchArgs::copy_topk_idx)
         .def_readwrite("h_token_slot", &DispatchArgs::h_token_slot)
         .def_readwrite("h_pair_row", &DispatchArgs::h_pair_row)
         .def_readwrite("h_psum_rank", &DispatchArgs::h_psum_rank)
@@ -79,6 +80,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def_readonly("recv_sf", &DispatchResult::recv_sf)
         .def_readonly("recv_topk_idx", &DispatchResult::recv_topk_idx)
         .def_readonly("recv_topk_weights", &DispatchResult::recv_topk_weights)
+        .def_readonly("topk_idx", &DispatchResult::topk_idx)
         .def_readonly("token_slot", &DispatchResult::token_slot)
         .def_readonly("pair_row", &DispatchResult::pair_row)
         .def_readonly("psum_rank", &DispatchResult::psum_rank)

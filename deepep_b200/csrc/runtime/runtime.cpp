@@ -1,5 +1,6 @@
 // Implementation of the per-rank host runtime (see runtime.hpp).
 #include "runtime.hpp"
+#include "stream_scope.hpp"
 
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_strided.h>
@@ -30,55 +31,6 @@ const char* status_name(int code) {
         case kStatusTileFlag: return "fused GEMM tile flag";
         default: return "unknown";
     }
-}
-
-bool env_flag(const char* name) {
-    const char* v = std::getenv(name);
-    return v != nullptr && v[0] != '\0' && v[0] != '0';
-}
-
-// Everything the stream-control arguments ask for before the first launch.
-struct StreamScope {
-    at::cuda::CUDAStream compute, comm;
-    bool switched = false;
-    StreamScope(const StreamControl& sc, const at::cuda::CUDAStream& comm_stream)
-        : compute(at::cuda::getCurrentCUDAStream()), comm(comm_stream) {
-        if (sc.allocate_on_comm_stream) {
-            at::cuda::setCurrentCUDAStream(comm);
-            switched = true;
-        }
-        if (sc.previous_event.has_value()) sc.previous_event->stream_wait(comm);
-        else stream_wait(comm, compute);
-    }
-    // Either hands back an event (async) or makes the compute stream wait for the comm stream.
-    std::optional<EventHandle> finish(const StreamControl& sc, const std::vector<at::Tensor>& tensors) {
-        std::optional<EventHandle> event;
-        if (sc.async_with_compute_stream) {
-            event = EventHandle(comm);
-            // EP_AVOID_RECORD_STREAM=1: the event keeps the tensors alive instead (the caller holds the event until it
-            // has waited on it); record_stream delays the reuse of a block by the caching allocator in a way that is
-            // hard to predict (csrc/elastic/buffer.hpp:556-584 of the reference offers the same switch).
-            static const bool avoid_record_stream = env_flag("EP_AVOID_RECORD_STREAM");
-            for (const auto& t : tensors) {
-                if (!t.defined() || !t.is_cuda()) continue;
-                if (avoid_record_stream) {
-                    event->keep_alive.push_back(t);
-                    continue;
-                }
-                // (views of the heap are not owned by the caching allocator; record_stream ignores them)
-                t.record_stream(comm);
-                if (sc.allocate_on_comm_stream) t.record_stream(compute);
-            }
-        } else {
-            stream_wait(compute, comm);
-        }
-        if (switched) at::cuda::setCurrentCUDAStream(compute);
-        return event;
-    }
-};
-
-at::TensorOptions opts(at::ScalarType dtype, int device) {
-    return at::TensorOptions().dtype(dtype).device(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
 }
 
 }  // namespace
@@ -159,6 +111,19 @@ std::vector<int64_t> Runtime::last_timeline() {
     return out;
 }
 
+// A call's kernels share the workspace and the regions of the calls before it. Calls on one stream are ordered by it;
+// when the stream changes, the new one waits for the old one. Inside a graph capture only streams of the capture can be
+// waited for (and work from before the capture is the caller's to order, as ever).
+void Runtime::order_behind_last_call(const at::cuda::CUDAStream& stream) {
+    if (last_stream_.has_value() && *last_stream_ != stream) {
+        cudaStreamCaptureStatus now = cudaStreamCaptureStatusNone, before = cudaStreamCaptureStatusNone;
+        CUDA_RUNTIME_CHECK(cudaStreamIsCapturing(stream.stream(), &now));
+        CUDA_RUNTIME_CHECK(cudaStreamIsCapturing(last_stream_->stream(), &before));
+        if (now == before) stream_wait(stream, *last_stream_);
+    }
+    last_stream_ = stream;
+}
+
 void Runtime::connect_local(const std::vector<std::shared_ptr<Runtime>>& runtimes) {
     std::vector<SymmetricHeap*> heaps;
     for (const auto& rt : runtimes) heaps.push_back(rt->heap_.get());
@@ -211,6 +176,7 @@ void Runtime::barrier(const std::vector<std::shared_ptr<Runtime>>& rts, bool use
     const auto compute = at::cuda::getCurrentCUDAStream();
     const auto stream = use_comm_stream ? rt0.comm_stream_ : compute;
     if (use_comm_stream) stream_wait(stream, compute);
+    rt0.order_behind_last_call(stream);
     Multi<BarrierParams> m;
     m.num_vranks = static_cast<int>(rts.size());
     m.blocks_per_rank = 1;
@@ -228,6 +194,22 @@ void Runtime::barrier(const std::vector<std::shared_ptr<Runtime>>& rts, bool use
     }
 }
 
+// Every count word carries the epoch of its dispatch: each of them is waited for on its own.
+int Runtime::wait_count(int i, uint32_t epoch) {
+    volatile uint64_t* words = host_words_ + kHostStatusWords;
+    uint64_t v = words[i];
+    if (static_cast<uint32_t>(v >> 32) == epoch) return static_cast<int>(static_cast<uint32_t>(v));
+    const auto start = std::chrono::steady_clock::now();
+    int spins = 0;
+    while (static_cast<uint32_t>((v = words[i]) >> 32) != epoch) {
+        if ((++spins & 1023) != 0) continue;
+        check_status();
+        const double waited = std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
+        if (waited > cpu_timeout_secs_) throw EPTimeoutError("EP host wait for the received token counts timed out", 0);
+    }
+    return static_cast<int>(static_cast<uint32_t>(v));
+}
+
 // ============================================================================ dispatch
 std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<Runtime>>& rts, std::vector<DispatchArgs>& args) {
     const int V = static_cast<int>(rts.size());
@@ -235,7 +217,8 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
     auto& rt0 = *rts[0];
     const int device = rt0.heap_->device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    StreamScope scope(args[0].sc, rt0.comm_stream_);
+    if (rt0.num_ranks_ == 1 && V == 1) return {rt0.dispatch_single(args[0])};
+    StreamScope scope(args[0].sc, rt0);
     const cudaStream_t stream = scope.comm.stream();
 
     const int R = rt0.num_ranks_;
@@ -377,25 +360,11 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
             r.num_recv_tokens = a.h_num_recv_tokens;
             r.num_expanded_tokens = a.h_num_expanded_tokens;
         } else if (a.do_cpu_sync) {
-            // every count word carries the epoch of this dispatch: wait for each of them on its own
-            volatile uint64_t* words = rt.host_words_ + kHostStatusWords;
             const uint32_t epoch = rt.dispatch_epoch;
-            const auto start = std::chrono::steady_clock::now();
-            auto wait_word = [&](int i) -> int {
-                uint64_t v;
-                int spins = 0;
-                while (static_cast<uint32_t>((v = words[i]) >> 32) != epoch) {
-                    if ((++spins & 1023) != 0) continue;
-                    rt.check_status();
-                    const double waited = std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
-                    if (waited > rt.cpu_timeout_secs_) throw EPTimeoutError("EP host wait for the received token counts timed out", 0);
-                }
-                return static_cast<int>(static_cast<uint32_t>(v));
-            };
-            r.num_recv_tokens = wait_word(0);
-            r.num_expanded_tokens = wait_word(1);
+            r.num_recv_tokens = rt.wait_count(0, epoch);
+            r.num_expanded_tokens = rt.wait_count(1, epoch);
             r.num_recv_tokens_per_expert_list.resize(EL);
-            for (int le = 0; le < EL; ++le) r.num_recv_tokens_per_expert_list[le] = wait_word(2 + le);
+            for (int le = 0; le < EL; ++le) r.num_recv_tokens_per_expert_list[le] = rt.wait_count(2 + le, epoch);
         } else {
             r.num_recv_tokens = a.num_worst_tokens > 0 ? a.num_worst_tokens : worst_rows;
             EP_HOST_ASSERT_MSG(r.num_recv_tokens <= worst_rows, "num_worst_tokens exceeds ranks x num_max_tokens_per_rank");
@@ -471,10 +440,16 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
         q.recv_src_metadata = r.recv_src_metadata.data_ptr<int>();
         q.num_out_rows = rows;
         q.num_idx_rows = static_cast<int>(r.recv_src_metadata.size(0));
+        if (a.copy_topk_idx) {
+            r.topk_idx = at::empty({a.x.size(0), K}, opts(idx_dtype, device));
+            q.topk_idx = a.topk_idx->data_ptr();
+            q.topk_idx_copy = r.topk_idx->data_ptr();
+            q.topk_idx_bytes = static_cast<int64_t>(a.topk_idx->nbytes());
+        }
         for (const at::Tensor& t : {r.recv_x, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert, r.num_unaligned, r.recv_src_metadata,
                                     a.x, *a.topk_idx})
             touched.push_back(t);
-        for (const auto& t : {r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, a.sf, a.topk_weights, a.cumulative_stats})
+        for (const auto& t : {r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.topk_idx, a.sf, a.topk_weights, a.cumulative_stats})
             if (t.has_value()) touched.push_back(*t);
     }
     const bool gated = a0.sc.previous_event_before_epilogue.has_value();
@@ -500,7 +475,8 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
     auto& rt0 = *rts[0];
     const int device = rt0.heap_->device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    StreamScope scope(args[0].sc, rt0.comm_stream_);
+    if (rt0.num_ranks_ == 1 && V == 1) return {rt0.combine_single(args[0])};
+    StreamScope scope(args[0].sc, rt0);
     const cudaStream_t stream = scope.comm.stream();
 
     const int R = rt0.num_ranks_;
@@ -520,12 +496,9 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
     if (num_sms * V > rt0.num_device_sms_) num_sms = rt0.num_device_sms_ / V;
     const bool gated = a0.sc.previous_event_before_epilogue.has_value();
     const bool split = rt0.profiling_ == 2;
-    // One rank: every token has at most one row (rank layout), so the send kernel can write the result itself.
-    bool direct = R == 1 && rank_layout && !gated && !(a0.weighted && a0.do_expand);
-    for (const auto& a : args) direct = direct && !a.bias0.has_value() && !a.bias1.has_value();
     // Reduce mode: 1 = arrival counters + the reduce kernel beside the send kernel (default with peers), 0 = the
     // reduce kernel after the send kernel.
-    int mode = (direct || a0.fuse_reduce == 0) ? 0 : 1;
+    int mode = a0.fuse_reduce == 0 ? 0 : 1;
     for (const auto& a : args) if (!a.dst_slot.has_value() || !a.count_matrix.has_value()) mode = 0;
     if (gated) mode = 0;
     const int num_blocks = num_sms;
@@ -612,7 +585,6 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
         q.count_matrix = nullptr;
         q.local_ws = rt.local_ws_;
         p.fuse_reduce = mode;
-        p.direct_out = direct ? 1 : 0;
         p.num_send_warps = 0;        // filled in by the launcher
         p.flag_chunks = lay.combine_flag_chunks;
         p.off_comb_flag = lay.combine_flag;
@@ -627,7 +599,6 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
             q.dst_slot = a.dst_slot->data_ptr<int>();
             q.count_matrix = a.count_matrix->data_ptr<int>();
         }
-        p.red = q;
         for (const at::Tensor& t : {r.combined_x, a.x, a.recv_src_metadata, a.topk_idx, a.psum_rank}) touched.push_back(t);
         for (const auto& t : {r.combined_topk_weights, a.topk_weights, a.bias0, a.bias1})
             if (t.has_value()) touched.push_back(*t);
@@ -643,15 +614,13 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
     ++rt0.num_launches_;
     if (split) rt0.prof_record(4, stream);
     if (gated) a0.sc.previous_event_before_epilogue->stream_wait(scope.comm);
-    if (!direct) {
-        // Arrival-driven: the reduce runs beside the send kernel, on the SMs that kernel leaves free (it is launched as
-        // a programmatic dependent, so all send blocks are resident before the first reduce block starts).
-        const bool beside = mode == 1 && !split && rt0.use_pdl_;
-        const int free_sms = rt0.num_device_sms_ / V - num_sms;
-        const int epi_sms = beside && free_sms >= 8 ? free_sms : std::max(1, rt0.num_device_sms_ / V);
-        CUDA_RUNTIME_CHECK(launch_combine_epilogue(ep.data(), V, epi_sms, stream, beside));
-        ++rt0.num_launches_;
-    }
+    // Arrival-driven: the reduce runs beside the send kernel, on the SMs that kernel leaves free (it is launched as
+    // a programmatic dependent, so all send blocks are resident before the first reduce block starts).
+    const bool beside = mode == 1 && !split && rt0.use_pdl_;
+    const int free_sms = rt0.num_device_sms_ / V - num_sms;
+    const int epi_sms = beside && free_sms >= 8 ? free_sms : std::max(1, rt0.num_device_sms_ / V);
+    CUDA_RUNTIME_CHECK(launch_combine_epilogue(ep.data(), V, epi_sms, stream, beside));
+    ++rt0.num_launches_;
     rt0.prof_record(5, stream);
     rt0.prof_valid_[1] = rt0.profiling_ != 0;
     rt0.prof_split_[1] = split;

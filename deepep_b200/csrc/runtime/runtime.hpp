@@ -60,6 +60,7 @@ struct DispatchArgs {
     // count are filled with -1 / 0 (csrc/legacy/buffer.hpp:571-577 and intranode.cu:536-540 of the reference)
     int num_worst_tokens = 0;
     // cached dispatch: tensors of an earlier handle
+    bool copy_topk_idx = false;     // the result carries a copy of topk_idx (the handle's own)
     bool cached = false;
     std::optional<at::Tensor> h_token_slot, h_pair_row, h_psum_rank, h_psum_expert, h_num_unaligned, h_recv_src_metadata;
     int h_num_recv_tokens = 0, h_num_expanded_tokens = 0;
@@ -68,7 +69,7 @@ struct DispatchArgs {
 
 struct DispatchResult {
     at::Tensor recv_x;
-    std::optional<at::Tensor> recv_sf, recv_topk_idx, recv_topk_weights;
+    std::optional<at::Tensor> recv_sf, recv_topk_idx, recv_topk_weights, topk_idx;
     at::Tensor token_slot, pair_row, psum_rank, psum_expert, num_unaligned, recv_src_metadata;
     at::Tensor count_matrix;   // [R, R] tokens rank i sent to rank j (undefined for cached dispatches)
     int num_recv_tokens = 0, num_expanded_tokens = 0, num_sms = 0;
@@ -156,6 +157,12 @@ public:
     static std::vector<DispatchResult> dispatch(const std::vector<std::shared_ptr<Runtime>>& rts, std::vector<DispatchArgs>& args);
     static std::vector<CombineResult> combine(const std::vector<std::shared_ptr<Runtime>>& rts, std::vector<CombineArgs>& args);
 
+    // the same for a group of one rank (kernels/local_exchange.cu)
+    DispatchResult dispatch_single(DispatchArgs& a);
+    CombineResult combine_single(CombineArgs& a);
+    // orders the kernels of a call on `stream` behind those of this runtime's previous call
+    void order_behind_last_call(const at::cuda::CUDAStream& stream);
+
     // sizing
     static int64_t ht_buffer_size(int num_ranks, int num_max_tokens, int hidden, int num_topk) {
         return static_cast<int64_t>(ht_layout(num_ranks, num_max_tokens, hidden, num_topk).end);
@@ -176,6 +183,7 @@ public:
     static constexpr int kHostCountWords = 2 + kMaxLocalExperts;
 
 private:
+    int wait_count(int i, uint32_t epoch);      // host wait for a count word of the dispatch `epoch`
     int rank_, num_ranks_;
     std::unique_ptr<SymmetricHeap> heap_;
     uint64_t* local_ws_ = nullptr;
@@ -184,6 +192,7 @@ private:
     uint64_t gpu_timeout_ns_;
     double cpu_timeout_secs_;
     at::cuda::CUDAStream comm_stream_;
+    std::optional<at::cuda::CUDAStream> last_stream_;      // of the last call
     int num_device_sms_ = 0, smem_optin_ = 0;
     bool destroyed_ = false;
     int profiling_ = 0;

@@ -85,7 +85,7 @@ class LocalCluster:
             kw = dict(kw)
             do_handle_copy = kw.pop('do_handle_copy', True)
             full = {**defaults, **kw}
-            args.append(buf._make_dispatch_args(**full))
+            args.append(buf._make_dispatch_args(**full, do_handle_copy=do_handle_copy))
             metas.append((do_handle_copy, full['handle']))
         results = self._C.Runtime.dispatch(self.runtimes, args)
         return [buf._wrap_dispatch_result(r, a, copy, handle)

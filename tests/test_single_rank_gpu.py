@@ -1,0 +1,131 @@
+"""Dispatch / combine of a one-rank group (plan, move and combine kernels of their own) against the pure-torch oracle, at
+the sizes where their work is cut: one and several planning blocks, more than one batch per warp, top-k beyond what a lane
+keeps in registers, rows that end inside a warp's slice, alignment gaps."""
+import pytest
+import torch
+
+from conftest import make_routed_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _buffer(T, H, K, **kw):
+    import deepep_b200
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    return deepep_b200.ElasticBuffer(SingleProcessGroup(), num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_gpu_timeout_secs=5, **kw)
+
+
+@pytest.mark.parametrize('T,H,E,K', [
+    (1, 128, 4, 1),          # one token
+    (31, 1152, 8, 3),        # 2304-byte rows: a slice and a quarter, rows not a multiple of 512 bytes
+    (1025, 256, 256, 8),     # two planning blocks, the second with one token more than the first leaves
+    (8300, 128, 64, 2),      # more than one batch of 32 tokens per warp
+    (70, 512, 32, 9),        # more top-k lanes than a planning lane keeps in registers
+])
+@pytest.mark.parametrize('expand', [False, True])
+@pytest.mark.parametrize('mode', ['bf16', 'fused', 'fused_col_major', 'prequantised'])
+def test_dispatch_combine_against_the_oracle(T, H, E, K, expand, mode):
+    from deepep_b200.utils import refs
+    from deepep_b200.utils.math import per_token_cast_to_fp8
+    align = 16
+    buf = _buffer(T, H, K)
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=T, device='cuda', masked_ratio=0.2)
+    idx[::5] = -1                                          # tokens that nobody takes
+    q, sf = per_token_cast_to_fp8(x)
+    xin, kw = {'bf16': (x, {}), 'fused': (x, dict(fused_fp8=True)), 'prequantised': ((q, sf), {}),
+               'fused_col_major': (x, dict(fused_fp8=True, use_tma_aligned_col_major_sf=True))}[mode]
+    raw = x.cpu() if mode == 'bf16' else q.view(torch.uint8).cpu()
+    e = refs.dispatch_local([raw], [idx.cpu()], [w.cpu()], 0, E, T, sfs=[sf.cpu()])
+    ex = refs.expand_local(e, E, align)
+    stats = torch.zeros(E, dtype=torch.int32, device='cuda')
+    for sync in (True, False):
+        recv, ridx, rw, handle, _ = buf.dispatch(xin, topk_idx=idx, topk_weights=w, num_experts=E, do_expand=expand, expert_alignment=align,
+                                                 do_zero_padding=True, do_cpu_sync=sync, cumulative_local_expert_recv_stats=stats, **kw)
+        torch.cuda.synchronize()
+        buf.check_status()
+        rows, scales = recv if isinstance(recv, tuple) else (recv, None)
+        rows = rows.view(torch.uint8).cpu() if mode != 'bf16' else rows.cpu()
+        n = e['recv_x'].size(0)
+        if sync:
+            assert handle.num_recv_tokens == n and rows.size(0) == (ex['num_rows'] if expand else n)
+            assert handle.num_recv_tokens_per_expert_list == [-(-int(c) // align) * align for c in ex['counts']]
+        meta = handle.recv_src_metadata.cpu()
+        assert torch.equal(meta[:n, 0], e['recv_src_token_idx']) and (meta[n:] == -1).all()
+        assert torch.equal(handle.num_unaligned_recv_tokens_per_expert.cpu().long(), ex['counts'])
+        assert torch.equal(handle.topk_idx, idx) and handle.topk_idx.data_ptr() != idx.data_ptr()
+        if not expand:
+            assert torch.equal(rows[:n], e['recv_x']) and torch.equal(ridx[:n].cpu(), e['recv_topk_idx']) and torch.equal(rw[:n].cpu(), e['recv_topk_weights'])
+            assert scales is None or torch.equal(scales[:n].cpu(), e['recv_sf'])
+            assert (ridx[n:] == -1).all() and (rw[n:] == 0).all() and (meta[:n, 2:] == -1).all()
+        else:
+            assert torch.equal(meta[:n, 2:].long(), ex['lane_rows'])
+            for g in range(E):
+                s, c = int(ex['starts'][g]), int(ex['counts'][g])
+                pick = ex['row_of'][g]
+                assert torch.equal(rows[s:s + c], e['recv_x'][pick])
+                lane = (e['recv_topk_idx'][pick] == g).float().argmax(dim=1)
+                assert torch.equal(rw[s:s + c].cpu(), e['recv_topk_weights'][pick, lane])
+                end = -(-(s + c) // align) * align
+                assert (rows[s + c:end] == 0).all() and (rw[s + c:end] == 0).all()
+                assert scales is None or (torch.equal(scales[s:s + c].cpu(), e['recv_sf'][pick]) and (scales[s + c:end] == 0).all())
+        if scales is not None and mode == 'fused_col_major':
+            assert scales.stride(0) == 1 and scales.stride(1) % 4 == 0
+    expect = torch.stack([(idx == g).sum() for g in range(E)]).int() * 2
+    assert torch.equal(stats, expect)
+    # replay of the routing with other payload
+    x2 = (x.float() * 2 + 1).bfloat16()
+    again = buf.dispatch(x2, handle=handle, do_expand=expand, do_zero_padding=True, fused_fp8=False)[0]
+    torch.cuda.synchronize()
+    keep = e['recv_src_token_idx'].long()
+    if not expand:
+        assert torch.equal(again[:n].cpu(), x2.cpu()[keep])
+    else:
+        for g in range(E):
+            s, c = int(ex['starts'][g]), int(ex['counts'][g])
+            assert torch.equal(again[s:s + c].cpu(), x2.cpu()[keep[ex['row_of'][g]]])
+    # combine of what came in
+    y = torch.randn((rows.size(0), H), device='cuda', generator=torch.Generator(device='cuda').manual_seed(T)).bfloat16()
+    bias = torch.randn((T, H), device='cuda', generator=torch.Generator(device='cuda').manual_seed(T + 1)).bfloat16()
+    part = torch.zeros((n, H))
+    wpart = torch.zeros((n, H))
+    yc, lanes = y.cpu().float(), ex['lane_rows'] if expand else torch.arange(n).view(n, 1)
+    for k in range(lanes.size(1)):
+        ok = lanes[:, k] >= 0
+        part[ok] += yc[lanes[ok, k]]
+        if expand:
+            wpart[ok] = torch.addcmul(wpart[ok], yc[lanes[ok, k]], rw.cpu()[lanes[ok, k]].view(-1, 1))
+    out, ow, _ = buf.combine(y, handle, topk_weights=rw)
+    outb, _, _ = buf.combine(y, handle, bias=bias)
+    ref = torch.zeros((T, H))
+    ref[keep] = part.bfloat16().float()
+    assert torch.equal(out.cpu(), ref.bfloat16())
+    assert torch.equal(outb.cpu(), (ref + bias.cpu().float()).bfloat16())
+    assert torch.equal(ow, torch.where(idx >= 0, w, torch.zeros_like(w)))
+    if expand:
+        got = buf.combine(y, handle, topk_weights=rw, weighted=True)[0].cpu().float()
+        wref = torch.zeros((T, H))
+        wref[keep] = wpart
+        # fused multiply-adds against separate roundings, then one bf16 rounding: at most one bf16 step apart
+        assert torch.allclose(got, wref, rtol=2 ** -7, atol=1e-5)
+    torch.cuda.synchronize()
+    buf.check_status()
+    buf.destroy()
+
+
+def test_calls_that_change_streams_stay_in_order():
+    """A synchronous call runs on the caller's stream, an asynchronous one on the communication stream: both use the
+    buffer's regions and must not overtake one another."""
+    T, H, E, K = 512, 2048, 16, 4
+    buf = _buffer(T, H, K)
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=3, device='cuda')
+    side = torch.cuda.Stream()
+    for it in range(8):
+        xi = (x.float() * (it + 1)).bfloat16()
+        recv, _, _, h, ev = buf.dispatch(xi, topk_idx=idx, num_experts=E, zero_copy=True, async_with_compute_stream=True)
+        ev.current_stream_wait()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            out = buf.combine(recv, h)[0]
+        torch.cuda.current_stream().wait_stream(side)
+        assert torch.equal(out, xi)
+    buf.destroy()
