@@ -413,17 +413,17 @@ class ElasticBuffer:
         return 0
 
     # ------------------------------------------------------------------ dispatch
-    def _make_dispatch_args(self, x, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts,
-                            num_max_tokens_per_rank, expert_alignment, num_sms, previous_event,
-                            previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream, handle,
-                            do_cpu_sync, do_expand, do_zero_padding, use_tma_aligned_col_major_sf, zero_copy, fused_fp8,
-                            round_scale, num_worst_tokens=0, do_handle_copy=True):
-        a = _C.DispatchArgs()
+    def _dispatch_call(self, x, topk_idx=None, topk_weights=None, cumulative_local_expert_recv_stats=None, num_experts=None,
+                       num_max_tokens_per_rank=None, expert_alignment=None, num_sms=0, previous_event=None,
+                       previous_event_before_epilogue=None, async_with_compute_stream=False, allocate_on_comm_stream=False, handle=None,
+                       do_cpu_sync=None, do_expand=False, do_zero_padding=False, use_tma_aligned_col_major_sf=False, zero_copy=False,
+                       fused_fp8=False, round_scale=False, num_worst_tokens=0, do_handle_copy=True, mask_weights=False):
+        """One rank's dispatch as the tuple that the native driver takes (order: ``dispatch_args`` in bindings.cpp)."""
+        sf = None
         if isinstance(x, tuple):
-            a.x, a.sf = x
+            x, sf = x
             assert not fused_fp8, 'fused FP8 casting takes a bf16 tensor, not a pre-quantised tuple'
-        else:
-            a.x = x
+        routing = None
         if handle is not None:
             assert topk_idx is None, '`topk_idx` is taken from the handle'
             assert cumulative_local_expert_recv_stats is None
@@ -433,56 +433,36 @@ class ElasticBuffer:
             assert num_experts == handle.num_experts and num_max_tokens_per_rank == handle.num_max_tokens_per_rank
             assert expert_alignment == handle.expert_alignment and do_expand == handle.do_expand
             topk_idx = handle.topk_idx
-            a.cached = True
-            a.h_token_slot = handle.dst_buffer_slot_idx
-            a.h_pair_row = handle.dst_expanded_row_idx
-            a.h_psum_rank = handle.psum_num_recv_tokens_per_scaleup_rank
-            a.h_psum_expert = handle._psum_expert_full
-            a.h_num_unaligned = handle.num_unaligned_recv_tokens_per_expert
-            a.h_recv_src_metadata = handle.recv_src_metadata
-            a.h_num_recv_tokens = handle.num_recv_tokens
-            a.h_num_expanded_tokens = handle.num_expanded_tokens
-            do_cpu_sync = False
+            routing = (handle.dst_buffer_slot_idx, handle.dst_expanded_row_idx, handle.psum_num_recv_tokens_per_scaleup_rank,
+                       handle._psum_expert_full, handle.num_unaligned_recv_tokens_per_expert, handle.recv_src_metadata,
+                       handle.num_recv_tokens, handle.num_expanded_tokens)
+            do_cpu_sync = do_handle_copy = False
         assert num_experts is not None and topk_idx is not None
-        num_max_tokens_per_rank = value_or(num_max_tokens_per_rank, self.num_max_tokens_per_rank)
+        if num_max_tokens_per_rank is None:
+            num_max_tokens_per_rank = self.num_max_tokens_per_rank
         assert num_max_tokens_per_rank > 0, 'num_max_tokens_per_rank is unknown'
-        a.topk_idx = topk_idx
-        a.topk_weights = topk_weights
-        a.copy_topk_idx = do_handle_copy and handle is None
-        a.cumulative_stats = cumulative_local_expert_recv_stats
-        a.num_experts = num_experts
-        a.num_max_tokens = num_max_tokens_per_rank
-        a.expert_alignment = value_or(expert_alignment, 1)
-        a.num_sms = num_sms if num_sms > 0 else self.get_theoretical_num_sms(num_experts, topk_idx.size(1))
-        a.quant_mode = (QUANT_E4M3_POW2 if round_scale else QUANT_E4M3) if fused_fp8 else QUANT_NONE
-        a.do_expand = do_expand
-        a.do_zero_padding = do_zero_padding
-        a.do_cpu_sync = value_or(do_cpu_sync, True)
-        a.zero_copy = zero_copy
-        a.num_worst_tokens = num_worst_tokens
-        a.col_major_sf = use_tma_aligned_col_major_sf
-        sc = a.sc
-        sc.previous_event = previous_event
-        sc.previous_event_before_epilogue = previous_event_before_epilogue
-        sc.async_with_compute_stream = async_with_compute_stream
-        sc.allocate_on_comm_stream = allocate_on_comm_stream
-        a.sc = sc
-        return a
+        if num_sms <= 0:
+            num_sms = self.get_theoretical_num_sms(num_experts, topk_idx.size(1))
+        quant_mode = (QUANT_E4M3_POW2 if round_scale else QUANT_E4M3) if fused_fp8 else QUANT_NONE
+        return (x, sf, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts, num_max_tokens_per_rank,
+                1 if expert_alignment is None else expert_alignment, num_sms, quant_mode, do_expand, do_zero_padding,
+                True if do_cpu_sync is None else do_cpu_sync, zero_copy, num_worst_tokens, use_tma_aligned_col_major_sf, do_handle_copy,
+                previous_event, previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream, routing, mask_weights)
 
-    def _wrap_dispatch_result(self, r, a, do_handle_copy: bool, handle: Optional[EPHandle]):
-        num_local = a.num_experts // self.num_ranks
+    @staticmethod
+    def _dispatch_result(result, call, handle: Optional[EPHandle]):
+        """The public return value from the native result tuple and the call's own tuple."""
+        (recv_x, recv_sf, recv_topk_idx, recv_topk_weights, token_slot, pair_row, psum_rank, psum_expert_full, psum_expert, num_unaligned,
+         recv_src_metadata, count_matrix, topk_idx, num_recv_tokens, num_expanded_tokens, num_sms, per_expert_list, event) = result
         if handle is None:
-            topk_idx = r.topk_idx if do_handle_copy else a.topk_idx
-            new_handle = EPHandle(a.do_expand, a.num_experts, a.expert_alignment, a.num_max_tokens, r.num_sms, topk_idx,
-                                  r.num_recv_tokens, r.num_expanded_tokens, r.num_recv_tokens_per_expert_list,
-                                  r.psum_rank, r.psum_expert[:num_local], r.num_unaligned, r.recv_src_metadata,
-                                  r.token_slot, r.pair_row)
-            new_handle._psum_expert_full = r.psum_expert
-            new_handle.num_tokens_per_rank_matrix = r.count_matrix
-        else:
-            new_handle = handle
-        recv_x = (r.recv_x, r.recv_sf) if r.recv_sf is not None else r.recv_x
-        return recv_x, r.recv_topk_idx, r.recv_topk_weights, new_handle, EventOverlap(r.event)
+            handle = EPHandle(call[10], call[5], call[7], call[6], num_sms, call[2] if topk_idx is None else topk_idx, num_recv_tokens,
+                              num_expanded_tokens, per_expert_list, psum_rank, psum_expert, num_unaligned, recv_src_metadata, token_slot,
+                              pair_row)
+            handle._psum_expert_full = psum_expert_full
+            handle.num_tokens_per_rank_matrix = count_matrix
+        if recv_sf is not None:
+            recv_x = (recv_x, recv_sf)
+        return recv_x, recv_topk_idx, recv_topk_weights, handle, EventOverlap(event)
 
     def dispatch(self, x: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]], topk_idx: Optional[torch.Tensor] = None,
                  topk_weights: Optional[torch.Tensor] = None,
@@ -512,13 +492,11 @@ class ElasticBuffer:
         check_torch_deterministic()
         if fused_fp8 is None:
             fused_fp8 = self.use_fp8_dispatch and not isinstance(x, tuple) and x.dtype == torch.bfloat16
-        a = self._make_dispatch_args(x, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts,
-                                     num_max_tokens_per_rank, expert_alignment, num_sms, previous_event,
-                                     previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream,
-                                     handle, do_cpu_sync, do_expand, do_zero_padding, use_tma_aligned_col_major_sf,
-                                     zero_copy, fused_fp8, round_scale, num_worst_tokens, do_handle_copy)
-        r = _C.Runtime.dispatch([self.runtime], [a])[0]
-        return self._wrap_dispatch_result(r, a, do_handle_copy, handle)
+        call = self._dispatch_call(x, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts, num_max_tokens_per_rank,
+                                   expert_alignment, num_sms, previous_event, previous_event_before_epilogue, async_with_compute_stream,
+                                   allocate_on_comm_stream, handle, do_cpu_sync, do_expand, do_zero_padding, use_tma_aligned_col_major_sf,
+                                   zero_copy, fused_fp8, round_scale, num_worst_tokens, do_handle_copy)
+        return self._dispatch_result(_C.Runtime.dispatch([self.runtime], [call])[0], call, handle)
 
     # ------------------------------------------------------------------ combine
     @staticmethod
@@ -530,31 +508,14 @@ class ElasticBuffer:
         assert len(bias) == 2
         return bias[0], bias[1]
 
-    def _make_combine_args(self, x, handle, topk_weights, bias, num_sms, previous_event, previous_event_before_epilogue,
-                           async_with_compute_stream, allocate_on_comm_stream, weighted=False):
-        a = _C.CombineArgs()
-        a.x = x
-        a.topk_weights = topk_weights
-        a.bias0, a.bias1 = self._unpack_bias(bias)
-        a.recv_src_metadata = handle.recv_src_metadata
-        a.topk_idx = handle.topk_idx
-        a.psum_rank = handle.psum_num_recv_tokens_per_scaleup_rank
-        a.num_experts = handle.num_experts
-        a.num_max_tokens = handle.num_max_tokens_per_rank
-        a.num_sms = num_sms if num_sms > 0 else handle.num_sms
-        a.do_expand = handle.do_expand
-        a.weighted = bool(weighted)
-        a.allow_multiple_reduction = self.allow_multiple_reduction
-        a.dst_slot = handle.dst_buffer_slot_idx
-        a.count_matrix = handle.num_tokens_per_rank_matrix
-        a.fuse_reduce = self.fuse_combine_reduce
-        sc = a.sc
-        sc.previous_event = previous_event
-        sc.previous_event_before_epilogue = previous_event_before_epilogue
-        sc.async_with_compute_stream = async_with_compute_stream
-        sc.allocate_on_comm_stream = allocate_on_comm_stream
-        a.sc = sc
-        return a
+    def _combine_call(self, x, handle, topk_weights=None, bias=None, num_sms=0, previous_event=None, previous_event_before_epilogue=None,
+                      async_with_compute_stream=False, allocate_on_comm_stream=False, weighted=False):
+        """One rank's combine as the tuple that the native driver takes (order: ``combine_calls`` in bindings.cpp)."""
+        bias0, bias1 = self._unpack_bias(bias)
+        return (x, topk_weights, bias0, bias1, handle.recv_src_metadata, handle.topk_idx, handle.psum_num_recv_tokens_per_scaleup_rank,
+                handle.dst_buffer_slot_idx, handle.num_tokens_per_rank_matrix, handle.num_experts, handle.num_max_tokens_per_rank,
+                num_sms if num_sms > 0 else handle.num_sms, handle.do_expand, bool(weighted), self.allow_multiple_reduction,
+                self.fuse_combine_reduce, previous_event, previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream)
 
     def combine(self, x: torch.Tensor, handle: EPHandle, topk_weights: Optional[torch.Tensor] = None,
                 bias: Union[None, torch.Tensor, Tuple[torch.Tensor, torch.Tensor]] = None, num_sms: int = 0,
@@ -573,7 +534,7 @@ class ElasticBuffer:
         Returns ``(combined_x, combined_topk_weights, event)``.
         """
         check_torch_deterministic()
-        a = self._make_combine_args(x, handle, topk_weights, bias, num_sms, previous_event, previous_event_before_epilogue,
-                                    async_with_compute_stream, allocate_on_comm_stream, weighted)
-        r = _C.Runtime.combine([self.runtime], [a])[0]
-        return r.combined_x, r.combined_topk_weights, EventOverlap(r.event)
+        call = self._combine_call(x, handle, topk_weights, bias, num_sms, previous_event, previous_event_before_epilogue,
+                                  async_with_compute_stream, allocate_on_comm_stream, weighted)
+        combined_x, combined_topk_weights, event = _C.Runtime.combine([self.runtime], [call])[0]
+        return combined_x, combined_topk_weights, EventOverlap(event)

@@ -193,47 +193,29 @@ class Buffer:
         # num_worst_tokens > 0: no CPU sync (graph-safe); the outputs have exactly that many rows and the routing
         # rows past the received count hold -1 / 0 (csrc/legacy/buffer.hpp:571-577, intranode.cu:536-540 of the reference)
         assert num_worst_tokens <= self.group_size * t_max, 'num_worst_tokens exceeds what the buffer can receive'
-        recv_x, recv_topk_idx, recv_topk_weights, ep_handle, event = self._elastic.dispatch(
-            x, topk_idx=topk_idx, topk_weights=topk_weights, num_experts=num_experts, num_max_tokens_per_rank=t_max,
-            expert_alignment=expert_alignment, num_sms=config.num_sms, previous_event=prev,
-            async_with_compute_stream=async_finish, allocate_on_comm_stream=allocate_on_comm_stream,
-            do_cpu_sync=num_worst_tokens == 0, fused_fp8=False, num_worst_tokens=num_worst_tokens)
-        if recv_topk_weights is not None:
-            # weights of experts that live elsewhere carry no meaning on this rank
+        # weights of experts that live elsewhere carry no meaning on this rank: they arrive as zeros
+        el = self._elastic
+        call = el._dispatch_call(x, topk_idx, topk_weights, num_experts=num_experts, num_max_tokens_per_rank=t_max, expert_alignment=expert_alignment,
+                                 num_sms=config.num_sms, previous_event=prev, async_with_compute_stream=async_finish,
+                                 allocate_on_comm_stream=allocate_on_comm_stream, do_cpu_sync=num_worst_tokens == 0,
+                                 num_worst_tokens=num_worst_tokens, mask_weights=True)
+        recv_x, recv_topk_idx, recv_topk_weights, ep_handle, event = el._dispatch_result(_C.Runtime.dispatch([self.runtime], [call])[0], call, None)
+        # The six tensors of the reference's intranode handle (deep_ep/buffers/legacy.py:401), filled from what the dispatch
+        # left behind. There is one "channel" here (tokens are not cut into channel ranges):
+        #   rank_prefix_matrix[i, j]          tokens that ranks 0..i sent to rank j (the count exchange of the dispatch kernel
+        #                                     gives every rank the whole matrix of totals)
+        #   channel_prefix_matrix[j, 0]       tokens this rank sent to rank j
+        #   recv_channel_prefix_matrix[i, 0]  tokens this rank received from rank i
+        #   recv_src_idx, is_token_in_rank
+        #   send_head[t, j]                   position of token t among this rank's tokens for rank j (-1 = not sent)
+        with torch.cuda.stream(self.get_comm_stream()) if async_finish else contextlib.nullcontext():
+            rank_prefix, sent, received, send_head, in_rank = _C.legacy_handle(self.runtime, ep_handle.num_tokens_per_rank_matrix,
+                                                                               ep_handle.dst_buffer_slot_idx, is_token_in_rank is None)
             if async_finish:
-                with torch.cuda.stream(self.get_comm_stream()):
-                    recv_topk_weights.masked_fill_(recv_topk_idx < 0, 0)
-                    event = EventOverlap(_C.EventHandle())
-            else:
-                recv_topk_weights.masked_fill_(recv_topk_idx < 0, 0)
-        if is_token_in_rank is None:
-            is_token_in_rank = ep_handle.dst_buffer_slot_idx >= 0
-        legacy = LegacyHandle(self._legacy_handle_tensors(ep_handle, is_token_in_rank, async_finish), ep_handle)
+                event = EventOverlap(_C.EventHandle())
+        legacy = LegacyHandle((rank_prefix, sent, received, ep_handle.recv_src_metadata[:, 0],
+                               in_rank if is_token_in_rank is None else is_token_in_rank, send_head), ep_handle)
         return recv_x, recv_topk_idx, recv_topk_weights, ep_handle.num_recv_tokens_per_expert_list, legacy, event
-
-    def _legacy_handle_tensors(self, ep_handle, is_token_in_rank, on_comm_stream: bool):
-        """The six tensors of the reference's intranode handle (deep_ep/buffers/legacy.py:401), filled from what
-        the dispatch left behind. There is one "channel" here (tokens are not cut into channel ranges):
-
-        * ``rank_prefix_matrix[i, j]``: tokens that ranks ``0..i`` sent to rank ``j`` (the count exchange of the
-          dispatch kernel gives every rank the whole matrix of totals);
-        * ``channel_prefix_matrix[j, 0]``: tokens this rank sent to rank ``j``;
-        * ``recv_channel_prefix_matrix[i, 0]``: tokens this rank received from rank ``i``;
-        * ``recv_src_idx``, ``is_token_in_rank``;
-        * ``send_head[t, j]``: position of token ``t`` among this rank's tokens for rank ``j`` (-1 = not sent).
-        """
-        R = self.group_size
-        ctx = torch.cuda.stream(self.get_comm_stream()) if on_comm_stream else contextlib.nullcontext()
-        with ctx:
-            counts = ep_handle.num_tokens_per_rank_matrix      # [source, destination]
-            rank_prefix_matrix = torch.cumsum(counts, dim=0).int()
-            channel_prefix_matrix = counts[self.rank].clone().view(R, 1)
-            recv_channel_prefix_matrix = counts[:, self.rank].clone().view(R, 1)
-            slot = ep_handle.dst_buffer_slot_idx
-            base = (rank_prefix_matrix[self.rank] - counts[self.rank]).view(1, R)
-            send_head = torch.where(slot >= 0, slot - base, slot)
-        return (rank_prefix_matrix, channel_prefix_matrix, recv_channel_prefix_matrix, ep_handle.recv_src_metadata[:, 0],
-                is_token_in_rank, send_head)
 
     def combine(self, x: torch.Tensor, handle: Tuple, topk_weights: Optional[torch.Tensor] = None,
                 bias: Union[None, torch.Tensor, Tuple[torch.Tensor, torch.Tensor]] = None, config: Optional[Config] = None,
@@ -271,21 +253,25 @@ class Buffer:
         With ``return_recv_hook`` only the sends are issued; ``hook()`` launches the receive part.
         """
         check_torch_deterministic()
-        io = _C.LLDispatchIO()
-        io.x, io.topk_idx = x, topk_idx
-        io.cumulative_stats = cumulative_local_expert_recv_stats
-        io.wait_stats = dispatch_wait_recv_cost_stats[self.rank] if dispatch_wait_recv_cost_stats is not None and \
-            dispatch_wait_recv_cost_stats.dim() == 2 else dispatch_wait_recv_cost_stats
-        phases = _C.LL_SEND if return_recv_hook else (_C.LL_SEND | _C.LL_RECV)
+        wait_stats = dispatch_wait_recv_cost_stats
+        if wait_stats is not None and wait_stats.dim() == 2:
+            wait_stats = wait_stats[self.rank]
         args = (num_max_dispatch_tokens_per_rank, num_experts, use_fp8, round_scale, use_ue8m0)
-        event = _C.ll_dispatch([self.runtime], [io], *args, phases, num_sms, self.enable_shrink, async_finish, return_recv_hook)
         hook: Optional[Callable] = None
-        if return_recv_hook:
+        if not return_recv_hook:
+            packed, sf, count, src_info, layout_range, event = _C.ll_dispatch_one(self.runtime, x, topk_idx, cumulative_local_expert_recv_stats,
+                                                                                  wait_stats, *args, num_sms, self.enable_shrink, async_finish)
+        else:
+            io = _C.LLDispatchIO()
+            io.x, io.topk_idx = x, topk_idx
+            io.cumulative_stats, io.wait_stats = cumulative_local_expert_recv_stats, wait_stats
+            event = _C.ll_dispatch([self.runtime], [io], *args, _C.LL_SEND, num_sms, self.enable_shrink, async_finish, True)
+            packed, sf, count, src_info, layout_range = io.packed_recv_x, io.packed_recv_sf, io.packed_recv_count, io.src_info, io.layout_range
+
             def hook():
                 _C.ll_dispatch([self.runtime], [io], *args, _C.LL_RECV, num_sms, self.enable_shrink, False, True)
-        handle = (io.src_info, io.layout_range, num_max_dispatch_tokens_per_rank, x.size(1), num_experts)
-        recv_x = (io.packed_recv_x, io.packed_recv_sf) if use_fp8 else io.packed_recv_x
-        return recv_x, io.packed_recv_count, handle, EventOverlap(event), hook
+        handle = (src_info, layout_range, num_max_dispatch_tokens_per_rank, x.size(1), num_experts)
+        return (packed, sf) if use_fp8 else packed, count, handle, EventOverlap(event), hook
 
     def low_latency_combine(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor, handle: tuple,
                             use_logfmt: bool = False, zero_copy: bool = False, async_finish: bool = False,
@@ -302,22 +288,25 @@ class Buffer:
         check_torch_deterministic()
         assert not (use_logfmt and zero_copy), 'LogFMT encodes while staging the row: it cannot be combined with zero_copy'
         src_info, layout_range, num_max_dispatch_tokens_per_rank, hidden, num_experts = handle
+        wait_stats = combine_wait_recv_cost_stats
+        if wait_stats is not None and wait_stats.dim() == 2:
+            wait_stats = wait_stats[self.rank]
+        hook: Optional[Callable] = None
+        if not return_recv_hook:
+            out, event = _C.ll_combine_one(self.runtime, x, topk_idx, topk_weights, src_info, layout_range, out, wait_stats,
+                                           num_max_dispatch_tokens_per_rank, num_experts, use_logfmt, num_sms, self.enable_shrink, async_finish)
+            return out, EventOverlap(event), hook
         io = _C.LLCombineIO()
         io.x, io.topk_idx, io.topk_weights = x, topk_idx, topk_weights
         io.src_info, io.layout_range = src_info, layout_range
-        io.use_logfmt = bool(use_logfmt)
+        io.use_logfmt, io.wait_stats = bool(use_logfmt), wait_stats
         if out is not None:
             io.combined_x = out
-        io.wait_stats = combine_wait_recv_cost_stats[self.rank] if combine_wait_recv_cost_stats is not None and \
-            combine_wait_recv_cost_stats.dim() == 2 else combine_wait_recv_cost_stats
-        phases = _C.LL_SEND if return_recv_hook else (_C.LL_SEND | _C.LL_RECV)
-        event = _C.ll_combine([self.runtime], [io], num_max_dispatch_tokens_per_rank, num_experts, phases, num_sms,
-                              self.enable_shrink, async_finish, return_recv_hook)
-        hook: Optional[Callable] = None
-        if return_recv_hook:
-            def hook():
-                _C.ll_combine([self.runtime], [io], num_max_dispatch_tokens_per_rank, num_experts, _C.LL_RECV, num_sms,
-                              self.enable_shrink, False, True)
+        event = _C.ll_combine([self.runtime], [io], num_max_dispatch_tokens_per_rank, num_experts, _C.LL_SEND, num_sms, self.enable_shrink,
+                              async_finish, True)
+
+        def hook():
+            _C.ll_combine([self.runtime], [io], num_max_dispatch_tokens_per_rank, num_experts, _C.LL_RECV, num_sms, self.enable_shrink, False, True)
         return io.combined_x, EventOverlap(event), hook
 
     def low_latency_update_mask_buffer(self, rank_to_mask: int, mask: bool = False):

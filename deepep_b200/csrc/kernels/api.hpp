@@ -141,6 +141,7 @@ struct DispatchEpilogueParams {
     int* recv_src_metadata;   // [num_idx_rows, K + 2]
     int num_out_rows;         // capacity of recv_x in rows (expand: expanded rows)
     int num_idx_rows;         // rows of the routing outputs; rows past the received count are filled with -1 / 0
+    int mask_weights = 0;     // weights of experts that live elsewhere are 0 (else handed on as they are)
     const void* topk_idx = nullptr;     // this rank's own routing, copied to ...
     void* topk_idx_copy = nullptr;      // ... the handle's tensor (or null)
     int64_t topk_idx_bytes = 0;
@@ -237,6 +238,7 @@ cudaError_t launch_local_plan(const LocalPlanParams& p, cudaStream_t stream);
 
 struct LocalMoveParams {
     int num_tokens, num_topk, num_experts, expert_alignment, do_expand, do_zero_padding, write_metadata, idx32, pow2;
+    int mask_weights;         // weights of unused top-k lanes are 0 (else handed on as they are)
     int src_row_bytes;
     int plan_ahead;           // 1: launched behind the plan kernel (waits for its end)
     int wide_in, wide_out;    // rows start on 32-byte boundaries (filled in by the launcher)
@@ -287,6 +289,10 @@ cudaError_t launch_local_combine(const LocalCombineParams& p, int num_sms, cudaS
 cudaError_t launch_dispatch_layout(const void* topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks, int num_experts,
                                    int* num_tokens_per_rank, int* num_tokens_per_expert, bool* is_token_in_rank,
                                    cudaStream_t stream);
+// The tensors of the first-generation handle from what a dispatch left behind: rank_prefix [R, R], sent [R], received [R],
+// send_head [T, R], in_rank [T, R] (or null).
+cudaError_t launch_legacy_handle(const int* count_matrix, const int* token_slot, int rank, int num_ranks, int num_tokens, int* rank_prefix,
+                                 int* sent, int* received, int* send_head, bool* in_rank, cudaStream_t stream);
 
 // ---------------------------------------------------------------- low-latency dispatch / combine
 enum LLPhase : int { kLLSend = 1, kLLRecv = 2 };
@@ -328,6 +334,11 @@ struct LLCombineParams {
     uint64_t off_combine_x[2], off_combine_flag[2];
 };
 cudaError_t launch_ll_combine(const Multi<LLCombineParams>& m, int num_sms, int smem_optin, cudaStream_t stream);
+
+// The same for a group of one rank: both phases in one launch, no messages (ll_local.cu). `limited`: the caller gave
+// num_sms (one block per SM then).
+cudaError_t launch_ll_local_dispatch(const LLDispatchParams& p, int num_sms, bool programmatic, cudaStream_t stream);
+cudaError_t launch_ll_local_combine(const LLCombineParams& p, int num_sms, bool limited, bool programmatic, cudaStream_t stream);
 
 // rank mask (shrink mode) kept in the private workspace
 cudaError_t ll_update_mask(uint64_t* local_ws, int rank, int value, cudaStream_t stream);

@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(1024, 1) dispatch_epilogue_kernel(const __grid
                 if (idx32) reinterpret_cast<int*>(p.recv_topk_idx)[j] = local_e;
                 else reinterpret_cast<int64_t*>(p.recv_topk_idx)[j] = local_e;
             }
-            if (p.recv_topk_weights != nullptr) p.recv_topk_weights[j] = wt;
+            if (p.recv_topk_weights != nullptr) p.recv_topk_weights[j] = p.mask_weights && local_e < 0 ? 0.f : wt;
         } else if (row >= 0 && p.recv_topk_weights != nullptr) {
             p.recv_topk_weights[row] = wt;
         }

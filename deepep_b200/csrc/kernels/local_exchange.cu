@@ -64,12 +64,15 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     const int tpw = align_up(ceil_div(max(t1 - t0, 1), kPlanWarps), 32);        // tokens per warp
     const int a = min(t1, t0 + warp * tpw), b = min(t1, a + tpw);
     const bool in_regs = tpw == 32 && K <= kPlanRegTopk;
+    // In registers a lane holds pairs lane, lane + 32, ... of the warp's 32 x K, so that loads and stores are contiguous
+    // over the warp (a lane per token strides by the row: 16.5 us instead of 9 for 8192 x 8 pairs).
     int e_reg[kPlanRegTopk], pos_reg[kPlanRegTopk];
     int slot_reg = -1;
+    const int pairs = (b - a) * K;
     if (in_regs) {
 #pragma unroll
-        for (int k = 0; k < kPlanRegTopk; ++k)
-            e_reg[k] = (k < K && a + lane < b) ? load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(a + lane) * K + k, E) : -1;
+        for (int i = 0; i < kPlanRegTopk; ++i)
+            e_reg[i] = (i < K && lane + 32 * i < pairs) ? load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(a) * K + lane + 32 * i, E) : -1;
     }
     for (int i = tid; i < kPlanWarps * (E + 1) + kPlanWarps * E; i += kPlanThreads) s_cnt[i] = 0;     // counters and masks
     __syncthreads();
@@ -78,24 +81,25 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     uint32_t* mask_of = s_mask + warp * E;
     int tokens_before = 0;
     if (in_regs) {
-        bool any = false;
+        uint32_t taken = 0;         // tokens of the warp with a valid expert
 #pragma unroll
-        for (int k = 0; k < kPlanRegTopk; ++k)
-            if (e_reg[k] >= 0) {
-                atomicOr(mask_of + e_reg[k], 1u << lane);
-                any = true;
+        for (int i = 0; i < kPlanRegTopk; ++i)
+            if (e_reg[i] >= 0) {
+                const uint32_t bit = 1u << ((lane + 32 * i) / K);
+                atomicOr(mask_of + e_reg[i], bit);
+                taken |= bit;
             }
         __syncwarp();               // the masks of all lanes are in
-        const uint32_t bal = __ballot_sync(0xffffffffu, any);
-        slot_reg = any ? __popc(bal & lanemask_lt()) : -1;
-        tokens_before = __popc(bal);
+        taken = __reduce_or_sync(0xffffffffu, taken);
+        slot_reg = (taken >> lane) & 1u ? __popc(taken & lanemask_lt()) : -1;
+        tokens_before = __popc(taken);
 #pragma unroll
-        for (int k = 0; k < kPlanRegTopk; ++k) {
-            pos_reg[k] = 0;
-            if (e_reg[k] >= 0) {
-                const uint32_t m = mask_of[e_reg[k]];
-                pos_reg[k] = __popc(m & lanemask_lt());
-                if (pos_reg[k] == 0) mine[e_reg[k]] = __popc(m);      // the lowest lane of a mask writes the count
+        for (int i = 0; i < kPlanRegTopk; ++i) {
+            pos_reg[i] = 0;
+            if (e_reg[i] >= 0) {
+                const uint32_t m = mask_of[e_reg[i]];
+                pos_reg[i] = __popc(m & ((1u << ((lane + 32 * i) / K)) - 1u));
+                if (pos_reg[i] == 0) mine[e_reg[i]] = __popc(m);      // the first token of a mask writes the count
             }
         }
     } else {
@@ -221,13 +225,11 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     __syncthreads();
     const int slot_base = s_base[E] + mine[E];
     if (in_regs) {
-        const int t = a + lane;
-        if (t < b) {
-            p.token_slot[t] = slot_reg < 0 ? -1 : slot_base + slot_reg;
+        if (a + lane < b) p.token_slot[a + lane] = slot_reg < 0 ? -1 : slot_base + slot_reg;
 #pragma unroll
-            for (int k = 0; k < kPlanRegTopk; ++k)
-                if (k < K) p.pair_row[static_cast<int64_t>(t) * K + k] = e_reg[k] < 0 ? -1 : s_base[e_reg[k]] + mine[e_reg[k]] + pos_reg[k];
-        }
+        for (int i = 0; i < kPlanRegTopk; ++i)
+            if (i < K && lane + 32 * i < pairs)
+                p.pair_row[static_cast<int64_t>(a) * K + lane + 32 * i] = e_reg[i] < 0 ? -1 : s_base[e_reg[i]] + mine[e_reg[i]] + pos_reg[i];
     } else {
         for (int t = a + lane; t < b; t += 32) {        // (every lane wrote the positions of the same tokens itself)
             if (p.token_slot[t] >= 0) p.token_slot[t] += slot_base;
@@ -316,7 +318,8 @@ __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_c
                         if (p.idx32) reinterpret_cast<int*>(p.recv_topk_idx)[o] = e;
                         else reinterpret_cast<int64_t*>(p.recv_topk_idx)[o] = e;
                     }
-                    if (p.recv_topk_weights != nullptr) p.recv_topk_weights[o] = p.topk_weights[static_cast<int64_t>(t) * K + lane];
+                    if (p.recv_topk_weights != nullptr)
+                        p.recv_topk_weights[o] = p.mask_weights && e < 0 ? 0.f : p.topk_weights[static_cast<int64_t>(t) * K + lane];
                 } else if (row >= 0 && p.recv_topk_weights != nullptr) {
                     p.recv_topk_weights[row] = p.topk_weights[static_cast<int64_t>(t) * K + lane];
                 }

@@ -10,6 +10,117 @@
 namespace py = pybind11;
 using namespace ep;
 
+namespace {
+
+using OptTensor = std::optional<at::Tensor>;
+
+template <typename T>
+T item(const py::tuple& t, int i) { return t[i].cast<T>(); }
+
+// A call of one rank arrives as one tuple and its results leave as one tuple: filling an argument block and reading a
+// result block attribute by attribute from Python cost about 15 us per call, which bounded small calls. The orders are
+// those of ElasticBuffer._dispatch_call / _dispatch_result / _combine_call.
+DispatchArgs dispatch_args(const py::tuple& t) {
+    DispatchArgs a;
+    a.x = item<at::Tensor>(t, 0);
+    a.sf = item<OptTensor>(t, 1);
+    a.topk_idx = item<OptTensor>(t, 2);
+    a.topk_weights = item<OptTensor>(t, 3);
+    a.cumulative_stats = item<OptTensor>(t, 4);
+    a.num_experts = item<int>(t, 5);
+    a.num_max_tokens = item<int>(t, 6);
+    a.expert_alignment = item<int>(t, 7);
+    a.num_sms = item<int>(t, 8);
+    a.quant_mode = item<int>(t, 9);
+    a.do_expand = item<bool>(t, 10);
+    a.do_zero_padding = item<bool>(t, 11);
+    a.do_cpu_sync = item<bool>(t, 12);
+    a.zero_copy = item<bool>(t, 13);
+    a.num_worst_tokens = item<int>(t, 14);
+    a.col_major_sf = item<bool>(t, 15);
+    a.copy_topk_idx = item<bool>(t, 16);
+    a.sc.previous_event = item<std::optional<EventHandle>>(t, 17);
+    a.sc.previous_event_before_epilogue = item<std::optional<EventHandle>>(t, 18);
+    a.sc.async_with_compute_stream = item<bool>(t, 19);
+    a.sc.allocate_on_comm_stream = item<bool>(t, 20);
+    a.mask_weights = item<bool>(t, 22);
+    if (!t[21].is_none()) {        // the routing of an earlier dispatch
+        const auto h = item<py::tuple>(t, 21);
+        a.cached = true;
+        a.h_token_slot = item<OptTensor>(h, 0);
+        a.h_pair_row = item<OptTensor>(h, 1);
+        a.h_psum_rank = item<OptTensor>(h, 2);
+        a.h_psum_expert = item<OptTensor>(h, 3);
+        a.h_num_unaligned = item<OptTensor>(h, 4);
+        a.h_recv_src_metadata = item<OptTensor>(h, 5);
+        a.h_num_recv_tokens = item<int>(h, 6);
+        a.h_num_expanded_tokens = item<int>(h, 7);
+    }
+    return a;
+}
+
+py::list dispatch_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const py::list& calls) {
+    std::vector<DispatchArgs> args;
+    for (const auto& c : calls) args.push_back(dispatch_args(c.cast<py::tuple>()));
+    std::vector<DispatchResult> res;
+    {
+        // The drivers may block on the host for a long time (the wait for the received counts): they run without the GIL
+        // so that Python threads of this process -- the heartbeat of the failure detector among them -- keep running.
+        py::gil_scoped_release release;
+        res = Runtime::dispatch(rts, args);
+    }
+    py::list out;
+    for (size_t v = 0; v < res.size(); ++v) {
+        DispatchResult& r = res[v];
+        py::object count_matrix = py::none(), per_expert = py::none();
+        if (r.count_matrix.defined()) count_matrix = py::cast(r.count_matrix);
+        if (!args[v].cached) per_expert = py::cast(r.psum_expert.narrow(0, 0, r.psum_expert.size(0) - 1));    // the last word is the number of expanded rows
+        out.append(py::make_tuple(r.recv_x, r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert,
+                                  per_expert, r.num_unaligned, r.recv_src_metadata, count_matrix, r.topk_idx, r.num_recv_tokens,
+                                  r.num_expanded_tokens, r.num_sms, r.num_recv_tokens_per_expert_list, r.event));
+    }
+    return out;
+}
+
+py::list combine_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const py::list& calls) {
+    std::vector<CombineArgs> args;
+    for (const auto& c : calls) {
+        const auto t = c.cast<py::tuple>();
+        CombineArgs a;
+        a.x = item<at::Tensor>(t, 0);
+        a.topk_weights = item<OptTensor>(t, 1);
+        a.bias0 = item<OptTensor>(t, 2);
+        a.bias1 = item<OptTensor>(t, 3);
+        a.recv_src_metadata = item<at::Tensor>(t, 4);
+        a.topk_idx = item<at::Tensor>(t, 5);
+        a.psum_rank = item<at::Tensor>(t, 6);
+        a.dst_slot = item<OptTensor>(t, 7);
+        a.count_matrix = item<OptTensor>(t, 8);
+        a.num_experts = item<int>(t, 9);
+        a.num_max_tokens = item<int>(t, 10);
+        a.num_sms = item<int>(t, 11);
+        a.do_expand = item<bool>(t, 12);
+        a.weighted = item<bool>(t, 13);
+        a.allow_multiple_reduction = item<bool>(t, 14);
+        a.fuse_reduce = item<int>(t, 15);
+        a.sc.previous_event = item<std::optional<EventHandle>>(t, 16);
+        a.sc.previous_event_before_epilogue = item<std::optional<EventHandle>>(t, 17);
+        a.sc.async_with_compute_stream = item<bool>(t, 18);
+        a.sc.allocate_on_comm_stream = item<bool>(t, 19);
+        args.push_back(std::move(a));
+    }
+    std::vector<CombineResult> res;
+    {
+        py::gil_scoped_release release;
+        res = Runtime::combine(rts, args);
+    }
+    py::list out;
+    for (auto& r : res) out.append(py::make_tuple(r.combined_x, r.combined_topk_weights, r.event));
+    return out;
+}
+
+}  // namespace
+
 void register_extra_bindings(py::module_& m);   // low latency, AGRS, PP, ops (other translation units)
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -37,87 +148,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     py::class_<EventHandle>(m, "EventHandle")
         .def(py::init<>())
         .def("current_stream_wait", &EventHandle::current_stream_wait);
-
-    py::class_<StreamControl>(m, "StreamControl")
-        .def(py::init<>())
-        .def_readwrite("previous_event", &StreamControl::previous_event)
-        .def_readwrite("previous_event_before_epilogue", &StreamControl::previous_event_before_epilogue)
-        .def_readwrite("async_with_compute_stream", &StreamControl::async_with_compute_stream)
-        .def_readwrite("allocate_on_comm_stream", &StreamControl::allocate_on_comm_stream);
-
-    py::class_<DispatchArgs>(m, "DispatchArgs")
-        .def(py::init<>())
-        .def_readwrite("x", &DispatchArgs::x)
-        .def_readwrite("sf", &DispatchArgs::sf)
-        .def_readwrite("topk_idx", &DispatchArgs::topk_idx)
-        .def_readwrite("topk_weights", &DispatchArgs::topk_weights)
-        .def_readwrite("cumulative_stats", &DispatchArgs::cumulative_stats)
-        .def_readwrite("num_experts", &DispatchArgs::num_experts)
-        .def_readwrite("num_max_tokens", &DispatchArgs::num_max_tokens)
-        .def_readwrite("expert_alignment", &DispatchArgs::expert_alignment)
-        .def_readwrite("num_sms", &DispatchArgs::num_sms)
-        .def_readwrite("quant_mode", &DispatchArgs::quant_mode)
-        .def_readwrite("do_expand", &DispatchArgs::do_expand)
-        .def_readwrite("do_zero_padding", &DispatchArgs::do_zero_padding)
-        .def_readwrite("do_cpu_sync", &DispatchArgs::do_cpu_sync)
-        .def_readwrite("zero_copy", &DispatchArgs::zero_copy)
-        .def_readwrite("num_worst_tokens", &DispatchArgs::num_worst_tokens)
-        .def_readwrite("col_major_sf", &DispatchArgs::col_major_sf)
-        .def_readwrite("cached", &DispatchArgs::cached)
-        .def_readwrite("copy_topk_idx", &DispatchArgs::copy_topk_idx)
-        .def_readwrite("h_token_slot", &DispatchArgs::h_token_slot)
-        .def_readwrite("h_pair_row", &DispatchArgs::h_pair_row)
-        .def_readwrite("h_psum_rank", &DispatchArgs::h_psum_rank)
-        .def_readwrite("h_psum_expert", &DispatchArgs::h_psum_expert)
-        .def_readwrite("h_num_unaligned", &DispatchArgs::h_num_unaligned)
-        .def_readwrite("h_recv_src_metadata", &DispatchArgs::h_recv_src_metadata)
-        .def_readwrite("h_num_recv_tokens", &DispatchArgs::h_num_recv_tokens)
-        .def_readwrite("h_num_expanded_tokens", &DispatchArgs::h_num_expanded_tokens)
-        .def_readwrite("sc", &DispatchArgs::sc);
-
-    py::class_<DispatchResult>(m, "DispatchResult")
-        .def_readonly("recv_x", &DispatchResult::recv_x)
-        .def_readonly("recv_sf", &DispatchResult::recv_sf)
-        .def_readonly("recv_topk_idx", &DispatchResult::recv_topk_idx)
-        .def_readonly("recv_topk_weights", &DispatchResult::recv_topk_weights)
-        .def_readonly("topk_idx", &DispatchResult::topk_idx)
-        .def_readonly("token_slot", &DispatchResult::token_slot)
-        .def_readonly("pair_row", &DispatchResult::pair_row)
-        .def_readonly("psum_rank", &DispatchResult::psum_rank)
-        .def_readonly("psum_expert", &DispatchResult::psum_expert)
-        .def_readonly("num_unaligned", &DispatchResult::num_unaligned)
-        .def_readonly("recv_src_metadata", &DispatchResult::recv_src_metadata)
-        .def_readonly("count_matrix", &DispatchResult::count_matrix)
-        .def_readonly("num_recv_tokens", &DispatchResult::num_recv_tokens)
-        .def_readonly("num_expanded_tokens", &DispatchResult::num_expanded_tokens)
-        .def_readonly("num_sms", &DispatchResult::num_sms)
-        .def_readonly("num_recv_tokens_per_expert_list", &DispatchResult::num_recv_tokens_per_expert_list)
-        .def_readonly("event", &DispatchResult::event);
-
-    py::class_<CombineArgs>(m, "CombineArgs")
-        .def(py::init<>())
-        .def_readwrite("x", &CombineArgs::x)
-        .def_readwrite("topk_weights", &CombineArgs::topk_weights)
-        .def_readwrite("bias0", &CombineArgs::bias0)
-        .def_readwrite("bias1", &CombineArgs::bias1)
-        .def_readwrite("recv_src_metadata", &CombineArgs::recv_src_metadata)
-        .def_readwrite("topk_idx", &CombineArgs::topk_idx)
-        .def_readwrite("psum_rank", &CombineArgs::psum_rank)
-        .def_readwrite("num_experts", &CombineArgs::num_experts)
-        .def_readwrite("num_max_tokens", &CombineArgs::num_max_tokens)
-        .def_readwrite("num_sms", &CombineArgs::num_sms)
-        .def_readwrite("do_expand", &CombineArgs::do_expand)
-        .def_readwrite("allow_multiple_reduction", &CombineArgs::allow_multiple_reduction)
-        .def_readwrite("weighted", &CombineArgs::weighted)
-        .def_readwrite("dst_slot", &CombineArgs::dst_slot)
-        .def_readwrite("count_matrix", &CombineArgs::count_matrix)
-        .def_readwrite("fuse_reduce", &CombineArgs::fuse_reduce)
-        .def_readwrite("sc", &CombineArgs::sc);
-
-    py::class_<CombineResult>(m, "CombineResult")
-        .def_readonly("combined_x", &CombineResult::combined_x)
-        .def_readonly("combined_topk_weights", &CombineResult::combined_topk_weights)
-        .def_readonly("event", &CombineResult::event);
 
     py::class_<Runtime, std::shared_ptr<Runtime>>(m, "Runtime")
         .def(py::init<int, int, int64_t, double, double, int64_t>(), py::arg("rank"), py::arg("num_ranks"), py::arg("num_bytes"),
@@ -153,13 +183,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
             return std::make_tuple(static_cast<int64_t>(s.id()), static_cast<int64_t>(s.device_index()),
                                    static_cast<int64_t>(s.device_type()));
         })
-        // The drivers may block on the host for a long time (the wait for the received counts, a stream
-        // synchronisation): they run without the GIL so that Python threads of this process -- the heartbeat of the
-        // failure detector among them -- keep running meanwhile.
+        // (may synchronise a stream: without the GIL, see dispatch_calls)
         .def_static("barrier", &Runtime::barrier, py::arg("runtimes"), py::arg("use_comm_stream") = true, py::arg("with_cpu_sync") = false,
                     py::call_guard<py::gil_scoped_release>())
-        .def_static("dispatch", &Runtime::dispatch, py::call_guard<py::gil_scoped_release>())
-        .def_static("combine", &Runtime::combine, py::call_guard<py::gil_scoped_release>())
+        .def_static("dispatch", &dispatch_calls)
+        .def_static("combine", &combine_calls)
         .def_static("ht_buffer_size", &Runtime::ht_buffer_size);
 
     // A host-side wait of the given length without the GIL: what a driver does while it spins on the received counts

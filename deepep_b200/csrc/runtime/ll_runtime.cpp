@@ -9,16 +9,13 @@
 #include <torch/extension.h>
 
 #include "runtime.hpp"
+#include "stream_scope.hpp"
 
 namespace py = pybind11;
 
 namespace ep {
 
 namespace {
-
-at::TensorOptions opts(at::ScalarType dtype, int device) {
-    return at::TensorOptions().dtype(dtype).device(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
-}
 
 struct LLDispatchIO {
     at::Tensor x, topk_idx;
@@ -38,17 +35,18 @@ int64_t ll_buffer_size(int num_ranks, int num_max_tokens, int hidden, int num_ex
     return static_cast<int64_t>(ll_layout(num_ranks, num_max_tokens, hidden, num_experts).end);
 }
 
-// Launch-stream policy of the low-latency calls: with a receive hook the kernels run on the caller's
-// stream (the caller overlaps them itself), otherwise on the communication stream.
+// Launch-stream policy of the low-latency calls: a call that hands back an event runs on the communication stream, every
+// other one on the caller's stream (with a receive hook the caller overlaps the kernels itself; a synchronous call would
+// only go over the communication stream and back).
 struct LLStreams {
     at::cuda::CUDAStream compute, launch;
-    bool on_comm;
-    LLStreams(Runtime& rt, bool use_compute) : compute(at::cuda::getCurrentCUDAStream()), launch(use_compute ? compute : rt.comm_stream()), on_comm(!use_compute) {
-        if (on_comm) stream_wait(launch, compute);
+    LLStreams(Runtime& rt, bool async_finish, bool use_compute)
+        : compute(at::cuda::getCurrentCUDAStream()), launch(async_finish && !use_compute ? rt.comm_stream() : compute) {
+        if (launch != compute) stream_wait(launch, compute);
+        rt.order_behind_last_call(launch);
     }
     std::optional<EventHandle> finish(bool async_finish) {
         if (async_finish) return EventHandle(launch);
-        if (on_comm) stream_wait(compute, launch);
         return std::nullopt;
     }
 };
@@ -61,7 +59,7 @@ std::optional<EventHandle> ll_dispatch(const std::vector<std::shared_ptr<Runtime
     auto& rt0 = *rts[0];
     const int device = rt0.heap().device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    LLStreams streams(rt0, on_compute_stream);
+    LLStreams streams(rt0, async_finish, on_compute_stream);
     const int R = rt0.num_ranks();
     const int H = static_cast<int>(ios[0]->x.size(1)), K = static_cast<int>(ios[0]->topk_idx.size(1));
     const int E = num_experts, EL = E / R, Tm = num_max_tokens;
@@ -82,13 +80,13 @@ std::optional<EventHandle> ll_dispatch(const std::vector<std::shared_ptr<Runtime
         EP_HOST_ASSERT(io.x.scalar_type() == at::kBFloat16 && io.x.is_contiguous() && io.x.size(1) == H && io.x.size(0) <= Tm);
         EP_HOST_ASSERT((io.topk_idx.scalar_type() == at::kLong || io.topk_idx.scalar_type() == at::kInt) && io.topk_idx.is_contiguous() && io.topk_idx.size(0) == io.x.size(0) && io.topk_idx.size(1) == K);
         if (!io.packed_recv_x.defined()) {
-            io.packed_recv_x = at::empty({EL, R * Tm, H}, opts(use_fp8 ? at::kFloat8_e4m3fn : at::kBFloat16, device));
-            io.packed_recv_count = at::empty({EL}, opts(at::kInt, device));
-            io.src_info = at::empty({EL, R * Tm}, opts(at::kInt, device));
-            io.layout_range = at::empty({EL, R}, opts(at::kLong, device));
+            io.packed_recv_x = new_tensor({EL, R * Tm, H}, use_fp8 ? at::kFloat8_e4m3fn : at::kBFloat16, device);
+            io.packed_recv_count = new_tensor({EL}, at::kInt, device);
+            io.src_info = new_tensor({EL, R * Tm}, at::kInt, device);
+            io.layout_range = new_tensor({EL, R}, at::kLong, device);
             if (use_fp8) {
-                if (use_ue8m0) io.packed_recv_sf = at::empty({EL, H / 512, R * Tm}, opts(at::kInt, device)).transpose(1, 2);
-                else io.packed_recv_sf = at::empty({EL, H / 128, R * Tm}, opts(at::kFloat, device)).transpose(1, 2);
+                if (use_ue8m0) io.packed_recv_sf = new_tensor({EL, H / 512, R * Tm}, at::kInt, device).transpose(1, 2);
+                else io.packed_recv_sf = new_tensor({EL, H / 128, R * Tm}, at::kFloat, device).transpose(1, 2);
             }
         }
         LLDispatchParams& p = m.r[v];
@@ -119,7 +117,12 @@ std::optional<EventHandle> ll_dispatch(const std::vector<std::shared_ptr<Runtime
             p.off_recv_count[h] = lay.recv_count[h];
         }
     }
-    CUDA_RUNTIME_CHECK(launch_ll_dispatch(m, num_sms, streams.launch.stream()));
+    if (R == 1 && V == 1) {
+        // one rank: both phases are one local kernel, a receive call has nothing left to do
+        if (phases & kLLSend) CUDA_RUNTIME_CHECK(launch_ll_local_dispatch(m.r[0], num_sms, rt0.use_pdl(), streams.launch.stream()));
+    } else {
+        CUDA_RUNTIME_CHECK(launch_ll_dispatch(m, num_sms, streams.launch.stream()));
+    }
     return streams.finish(async_finish);
 }
 
@@ -131,7 +134,7 @@ std::optional<EventHandle> ll_combine(const std::vector<std::shared_ptr<Runtime>
     auto& rt0 = *rts[0];
     const int device = rt0.heap().device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    LLStreams streams(rt0, on_compute_stream);
+    LLStreams streams(rt0, async_finish, on_compute_stream);
     const int R = rt0.num_ranks();
     const int H = static_cast<int>(ios[0]->x.size(2)), K = static_cast<int>(ios[0]->topk_idx.size(1));
     const int E = num_experts, EL = E / R, Tm = num_max_tokens;
@@ -139,6 +142,7 @@ std::optional<EventHandle> ll_combine(const std::vector<std::shared_ptr<Runtime>
     EP_HOST_ASSERT_MSG(!ios[0]->use_logfmt || H % 128 == 0, "LogFMT needs a hidden size that is a multiple of 128");
     const LLLayout lay = ll_layout(R, Tm, H, E);
     EP_HOST_ASSERT_MSG(lay.end <= rt0.heap().num_bytes(), "symmetric buffer too small for low-latency mode");
+    const bool limited = num_sms > 0;
     if (num_sms <= 0) num_sms = rt0.num_device_sms();   // latency-bound: one token / one (expert, source) pair per block
     if (num_sms * V > rt0.num_device_sms()) num_sms = rt0.num_device_sms() / V;
 
@@ -153,7 +157,7 @@ std::optional<EventHandle> ll_combine(const std::vector<std::shared_ptr<Runtime>
         EP_HOST_ASSERT((io.topk_idx.scalar_type() == at::kLong || io.topk_idx.scalar_type() == at::kInt) && io.topk_idx.is_contiguous());
         EP_HOST_ASSERT(io.topk_weights.scalar_type() == at::kFloat && io.topk_weights.is_contiguous() && io.topk_weights.size(1) == K);
         const int T = static_cast<int>(io.topk_idx.size(0));
-        if (!io.combined_x.defined()) io.combined_x = at::empty({T, H}, opts(at::kBFloat16, device));
+        if (!io.combined_x.defined()) io.combined_x = new_tensor({T, H}, at::kBFloat16, device);
         EP_HOST_ASSERT(io.combined_x.scalar_type() == at::kBFloat16 && io.combined_x.is_contiguous() && io.combined_x.size(0) == T && io.combined_x.size(1) == H);
         LLCombineParams& p = m.r[v];
         p.c = rt.ctx();
@@ -179,8 +183,44 @@ std::optional<EventHandle> ll_combine(const std::vector<std::shared_ptr<Runtime>
             p.off_combine_flag[h] = lay.combine_flag[h];
         }
     }
-    CUDA_RUNTIME_CHECK(launch_ll_combine(m, num_sms, rt0.smem_optin(), streams.launch.stream()));
+    if (R == 1 && V == 1 && !ios[0]->use_logfmt) {
+        if (phases & kLLSend) CUDA_RUNTIME_CHECK(launch_ll_local_combine(m.r[0], num_sms, limited, rt0.use_pdl(), streams.launch.stream()));
+    } else {
+        CUDA_RUNTIME_CHECK(launch_ll_combine(m, num_sms, rt0.smem_optin(), streams.launch.stream()));
+    }
     return streams.finish(async_finish);
+}
+
+// The calls of one process (one rank) without an IO object on the Python side: one trip into native code.
+py::tuple ll_dispatch_one(const std::shared_ptr<Runtime>& rt, const at::Tensor& x, const at::Tensor& topk_idx, std::optional<at::Tensor> cumulative_stats,
+                          std::optional<at::Tensor> wait_stats, int num_max_tokens, int num_experts, bool use_fp8, bool round_scale, bool use_ue8m0,
+                          int num_sms, bool shrink, bool async_finish) {
+    LLDispatchIO io;
+    io.x = x;
+    io.topk_idx = topk_idx;
+    io.cumulative_stats = std::move(cumulative_stats);
+    io.wait_stats = std::move(wait_stats);
+    std::vector<LLDispatchIO*> ios = {&io};
+    auto event = ll_dispatch({rt}, ios, num_max_tokens, num_experts, use_fp8, round_scale, use_ue8m0, kLLSend | kLLRecv, num_sms, shrink, async_finish, false);
+    return py::make_tuple(std::move(io.packed_recv_x), std::move(io.packed_recv_sf), std::move(io.packed_recv_count), std::move(io.src_info),
+                          std::move(io.layout_range), std::move(event));
+}
+
+py::tuple ll_combine_one(const std::shared_ptr<Runtime>& rt, const at::Tensor& x, const at::Tensor& topk_idx, const at::Tensor& topk_weights,
+                         const at::Tensor& src_info, const at::Tensor& layout_range, std::optional<at::Tensor> out, std::optional<at::Tensor> wait_stats,
+                         int num_max_tokens, int num_experts, bool use_logfmt, int num_sms, bool shrink, bool async_finish) {
+    LLCombineIO io;
+    io.x = x;
+    io.topk_idx = topk_idx;
+    io.topk_weights = topk_weights;
+    io.src_info = src_info;
+    io.layout_range = layout_range;
+    io.use_logfmt = use_logfmt;
+    if (out.has_value()) io.combined_x = std::move(*out);
+    io.wait_stats = std::move(wait_stats);
+    std::vector<LLCombineIO*> ios = {&io};
+    auto event = ll_combine({rt}, ios, num_max_tokens, num_experts, kLLSend | kLLRecv, num_sms, shrink, async_finish, false);
+    return py::make_tuple(std::move(io.combined_x), std::move(event));
 }
 
 // bf16 [EL, R * T_max, H] view of the staging half that the NEXT combine send may read from
@@ -216,14 +256,17 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, std::optional<EventHandle>> get_d
     const auto compute = at::cuda::getCurrentCUDAStream();
     const auto comm = rt.comm_stream();
     if (allocate_on_comm_stream) at::cuda::setCurrentCUDAStream(comm);
+    // (it touches nothing of the runtime: a synchronous query stays on the caller's stream)
+    const bool stay = !async_finish && !allocate_on_comm_stream && !previous_event.has_value();
+    const auto launch = stay ? compute : comm;
     if (previous_event.has_value()) previous_event->stream_wait(comm);
-    else stream_wait(comm, compute);
+    else if (!stay) stream_wait(comm, compute);
     const int T = static_cast<int>(topk_idx.size(0)), K = static_cast<int>(topk_idx.size(1)), R = rt.num_ranks();
-    auto per_rank = at::empty({R}, opts(at::kInt, device));
-    auto per_expert = at::empty({num_experts}, opts(at::kInt, device));
-    auto in_rank = at::empty({T, R}, opts(at::kBool, device));
+    auto per_rank = new_tensor({R}, at::kInt, device);
+    auto per_expert = new_tensor({num_experts}, at::kInt, device);
+    auto in_rank = new_tensor({T, R}, at::kBool, device);
     CUDA_RUNTIME_CHECK(launch_dispatch_layout(topk_idx.data_ptr(), topk_idx.scalar_type() == at::kInt, T, K, R, num_experts, per_rank.data_ptr<int>(),
-                                              per_expert.data_ptr<int>(), in_rank.data_ptr<bool>(), comm.stream()));
+                                              per_expert.data_ptr<int>(), in_rank.data_ptr<bool>(), launch.stream()));
     std::optional<EventHandle> event;
     if (async_finish) {
         event = EventHandle(comm);
@@ -231,11 +274,28 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, std::optional<EventHandle>> get_d
             t.record_stream(comm);
             if (allocate_on_comm_stream) t.record_stream(compute);
         }
-    } else {
+    } else if (!stay) {
         stream_wait(compute, comm);
     }
     if (allocate_on_comm_stream) at::cuda::setCurrentCUDAStream(compute);
     return {per_rank, per_expert, in_rank, event};
+}
+
+// (rank_prefix_matrix, channel_prefix_matrix, recv_channel_prefix_matrix, send_head, is_token_in_rank) of the
+// first-generation handle, on the current stream
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, std::optional<at::Tensor>> legacy_handle(Runtime& rt, const at::Tensor& count_matrix,
+                                                                                                    const at::Tensor& token_slot, bool with_in_rank) {
+    const int R = rt.num_ranks(), T = static_cast<int>(token_slot.size(0)), device = rt.heap().device();
+    EP_HOST_ASSERT(count_matrix.is_contiguous() && count_matrix.numel() == R * R && token_slot.is_contiguous() && token_slot.size(1) == R);
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    auto prefix = new_tensor({R, R}, at::kInt, device), sent = new_tensor({R, 1}, at::kInt, device), received = new_tensor({R, 1}, at::kInt, device);
+    auto send_head = new_tensor({T, R}, at::kInt, device);
+    std::optional<at::Tensor> in_rank;
+    if (with_in_rank) in_rank = new_tensor({T, R}, at::kBool, device);
+    CUDA_RUNTIME_CHECK(launch_legacy_handle(count_matrix.data_ptr<int>(), token_slot.data_ptr<int>(), rt.rank(), R, T, prefix.data_ptr<int>(),
+                                            sent.data_ptr<int>(), received.data_ptr<int>(), send_head.data_ptr<int>(),
+                                            with_in_rank ? in_rank->data_ptr<bool>() : nullptr, at::cuda::getCurrentCUDAStream().stream()));
+    return {prefix, sent, received, send_head, in_rank};
 }
 
 }  // namespace
@@ -263,9 +323,12 @@ void register_ll_bindings(py::module_& m) {
         .def_readwrite("wait_stats", &LLCombineIO::wait_stats)
         .def_readwrite("use_logfmt", &LLCombineIO::use_logfmt);
     m.def("get_dispatch_layout", &get_dispatch_layout);
+    m.def("legacy_handle", &legacy_handle);
     m.def("ll_buffer_size", &ll_buffer_size);
     m.def("ll_dispatch", &ll_dispatch);
     m.def("ll_combine", &ll_combine);
+    m.def("ll_dispatch_one", &ll_dispatch_one);
+    m.def("ll_combine_one", &ll_combine_one);
     m.def("ll_next_combine_buffer", &ll_next_combine_buffer);
     m.def("ll_mask_update", &ll_mask_update);
     m.def("ll_mask_clean", &ll_mask_clean);

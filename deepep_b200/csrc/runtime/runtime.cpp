@@ -440,6 +440,7 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
         q.recv_src_metadata = r.recv_src_metadata.data_ptr<int>();
         q.num_out_rows = rows;
         q.num_idx_rows = static_cast<int>(r.recv_src_metadata.size(0));
+        q.mask_weights = a.mask_weights ? 1 : 0;
         if (a.copy_topk_idx) {
             r.topk_idx = at::empty({a.x.size(0), K}, opts(idx_dtype, device));
             q.topk_idx = a.topk_idx->data_ptr();

@@ -60,6 +60,7 @@ struct DispatchArgs {
     // count are filled with -1 / 0 (csrc/legacy/buffer.hpp:571-577 and intranode.cu:536-540 of the reference)
     int num_worst_tokens = 0;
     // cached dispatch: tensors of an earlier handle
+    bool mask_weights = false;      // received weights of experts that live elsewhere are 0
     bool copy_topk_idx = false;     // the result carries a copy of topk_idx (the handle's own)
     bool cached = false;
     std::optional<at::Tensor> h_token_slot, h_pair_row, h_psum_rank, h_psum_expert, h_num_unaligned, h_recv_src_metadata;
@@ -127,6 +128,7 @@ public:
     int64_t num_bytes() const { return static_cast<int64_t>(heap_->num_bytes()); }
     int num_device_sms() const { return num_device_sms_; }
     int smem_optin() const { return smem_optin_; }
+    bool use_pdl() const { return use_pdl_; }
     SymmetricHeap& heap() { return *heap_; }
     at::Tensor heap_tensor(int64_t offset, int64_t num_bytes) const;   // uint8 view of the own heap (no ownership)
     void set_gpu_timeout(double secs) { gpu_timeout_ns_ = static_cast<uint64_t>(secs * 1e9); }

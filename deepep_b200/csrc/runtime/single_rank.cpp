@@ -1,6 +1,5 @@
 // Dispatch and combine drivers of a group of one rank (kernels/local_exchange.cu): the same arguments, checks and results
 // as the multi-rank drivers (runtime.cpp), without the heap.
-#include <ATen/ops/empty.h>
 #include <ATen/ops/empty_strided.h>
 #include <ATen/ops/from_blob.h>
 
@@ -71,12 +70,12 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
         r.num_unaligned = *a.h_num_unaligned;
         r.recv_src_metadata = *a.h_recv_src_metadata;
     } else {
-        r.token_slot = at::empty({T, 1}, opts(at::kInt, device));
-        r.pair_row = at::empty({T, K}, opts(at::kInt, device));
-        r.psum_rank = at::empty({1}, opts(at::kInt, device));
-        r.psum_expert = at::empty({E + 1}, opts(at::kInt, device));
-        r.num_unaligned = at::empty({E}, opts(at::kInt, device));
-        r.count_matrix = at::empty({1, 1}, opts(at::kInt, device));
+        r.token_slot = new_tensor({T, 1}, at::kInt, device);
+        r.pair_row = new_tensor({T, K}, at::kInt, device);
+        r.psum_rank = new_tensor({1}, at::kInt, device);
+        r.psum_expert = new_tensor({E + 1}, at::kInt, device);
+        r.num_unaligned = new_tensor({E}, at::kInt, device);
+        r.count_matrix = new_tensor({1, 1}, at::kInt, device);
         LocalPlanParams p = {};
         p.num_tokens = T;
         p.num_topk = K;
@@ -145,7 +144,7 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     const bool zero_copy = a.zero_copy && !a.do_expand;
     uint8_t* region = heap_->base() + lay.dispatch_rec[epoch & 1];
     if (zero_copy) r.recv_x = at::from_blob(region, {rows_bound, H}, {rec_pitch / static_cast<int64_t>(c10::elementSize(out_dtype)), 1}, opts(out_dtype, device));
-    else r.recv_x = at::empty({rows_bound, H}, opts(out_dtype, device));
+    else r.recv_x = new_tensor({rows_bound, H}, out_dtype, device);
     if (has_sf) {
         const at::ScalarType sf_dtype = (!quant && a.sf->scalar_type() == at::kInt) ? at::kInt : at::kFloat;
         if (a.col_major_sf) {
@@ -153,17 +152,17 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
         } else if (zero_copy) {
             r.recv_sf = at::from_blob(region + x_row_bytes, {rows_bound, sf_packs}, {rec_pitch / 4, 1}, opts(sf_dtype, device));
         } else {
-            r.recv_sf = at::empty({rows_bound, sf_packs}, opts(sf_dtype, device));
+            r.recv_sf = new_tensor({rows_bound, sf_packs}, sf_dtype, device);
         }
     }
     if (!a.do_expand) {
-        r.recv_topk_idx = at::empty({idx_bound, K}, opts(idx_dtype, device));
-        if (a.topk_weights.has_value()) r.recv_topk_weights = at::empty({idx_bound, K}, opts(at::kFloat, device));
+        r.recv_topk_idx = new_tensor({idx_bound, K}, idx_dtype, device);
+        if (a.topk_weights.has_value()) r.recv_topk_weights = new_tensor({idx_bound, K}, at::kFloat, device);
     } else if (a.topk_weights.has_value()) {
-        r.recv_topk_weights = at::empty({rows_bound}, opts(at::kFloat, device));
+        r.recv_topk_weights = new_tensor({rows_bound}, at::kFloat, device);
     }
-    if (!cached) r.recv_src_metadata = at::empty({idx_bound, K + 2}, opts(at::kInt, device));
-    if (a.copy_topk_idx && !cached) r.topk_idx = at::empty({T, K}, opts(idx_dtype, device));
+    if (!cached) r.recv_src_metadata = new_tensor({idx_bound, K + 2}, at::kInt, device);
+    if (a.copy_topk_idx && !cached) r.topk_idx = new_tensor({T, K}, idx_dtype, device);
 
     LocalMoveParams q = {};
     q.num_tokens = T;
@@ -174,6 +173,7 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     q.do_zero_padding = a.do_zero_padding;
     q.write_metadata = cached ? 0 : 1;
     q.idx32 = idx_dtype == at::kInt ? 1 : 0;
+    q.mask_weights = a.mask_weights ? 1 : 0;
     q.pow2 = a.quant_mode == kQuantE4M3Pow2;
     q.src_row_bytes = src_row_bytes;
     q.x = static_cast<const uint8_t*>(a.x.data_ptr());
@@ -258,8 +258,8 @@ CombineResult Runtime::combine_single(CombineArgs& a) {
         else EP_HOST_ASSERT(a.topk_weights->dim() == 2 && a.topk_weights->size(1) == K);
     }
     CombineResult r;
-    r.combined_x = at::empty({T, H}, opts(at::kBFloat16, device));
-    if (a.topk_weights.has_value()) r.combined_topk_weights = at::empty({T, K}, opts(at::kFloat, device));
+    r.combined_x = new_tensor({T, H}, at::kBFloat16, device);
+    if (a.topk_weights.has_value()) r.combined_topk_weights = new_tensor({T, K}, at::kFloat, device);
     LocalCombineParams p = {};
     p.num_tokens = T;
     p.num_topk = K;

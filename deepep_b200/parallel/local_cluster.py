@@ -74,29 +74,13 @@ class LocalCluster:
 
     def dispatch(self, per_rank_kwargs: Sequence[dict]):
         """``per_rank_kwargs[r]`` holds the keyword arguments of ``ElasticBuffer.dispatch`` for rank r."""
-        defaults = dict(topk_idx=None, topk_weights=None, cumulative_local_expert_recv_stats=None, num_experts=None,
-                        num_max_tokens_per_rank=None, expert_alignment=None, num_sms=0, previous_event=None,
-                        previous_event_before_epilogue=None, async_with_compute_stream=False,
-                        allocate_on_comm_stream=False, handle=None, do_cpu_sync=None, do_expand=False,
-                        do_zero_padding=False, use_tma_aligned_col_major_sf=False, zero_copy=False, fused_fp8=False,
-                        round_scale=False, num_worst_tokens=0)
-        args, metas = [], []
-        for buf, kw in zip(self.buffers, per_rank_kwargs):
-            kw = dict(kw)
-            do_handle_copy = kw.pop('do_handle_copy', True)
-            full = {**defaults, **kw}
-            args.append(buf._make_dispatch_args(**full, do_handle_copy=do_handle_copy))
-            metas.append((do_handle_copy, full['handle']))
-        results = self._C.Runtime.dispatch(self.runtimes, args)
-        return [buf._wrap_dispatch_result(r, a, copy, handle)
-                for buf, r, a, (copy, handle) in zip(self.buffers, results, args, metas)]
+        calls = [buf._dispatch_call(**kw) for buf, kw in zip(self.buffers, per_rank_kwargs)]
+        results = self._C.Runtime.dispatch(self.runtimes, calls)
+        return [buf._dispatch_result(r, call, kw.get('handle')) for buf, r, call, kw in zip(self.buffers, results, calls, per_rank_kwargs)]
 
     def combine(self, per_rank_kwargs: Sequence[dict]):
-        defaults = dict(topk_weights=None, bias=None, num_sms=0, previous_event=None, previous_event_before_epilogue=None,
-                        async_with_compute_stream=False, allocate_on_comm_stream=False, weighted=False)
-        args = [buf._make_combine_args(**{**defaults, **kw}) for buf, kw in zip(self.buffers, per_rank_kwargs)]
-        results = self._C.Runtime.combine(self.runtimes, args)
-        return [(r.combined_x, r.combined_topk_weights, EventOverlap(r.event)) for r in results]
+        calls = [buf._combine_call(**kw) for buf, kw in zip(self.buffers, per_rank_kwargs)]
+        return [(x, w, EventOverlap(event)) for x, w, event in self._C.Runtime.combine(self.runtimes, calls)]
 
     # ------------------------------------------------------------------ low-latency mode
     def low_latency_dispatch(self, xs, topk_idxs, num_max_dispatch_tokens_per_rank: int, num_experts: int, use_fp8: bool = True,

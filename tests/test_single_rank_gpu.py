@@ -129,3 +129,69 @@ def test_calls_that_change_streams_stay_in_order():
         torch.cuda.current_stream().wait_stream(side)
         assert torch.equal(out, xi)
     buf.destroy()
+
+
+@pytest.mark.parametrize('T,H,E,K', [
+    (1, 1024, 8, 2),         # one token: the extra blocks only count
+    (33, 1152, 256, 9),      # a row that ends inside a warp's slice, more top-k lanes than four warps look up in one round
+    (128, 7168, 32, 16),     # the largest top-k, experts that hold more rows than a warp has lanes
+])
+@pytest.mark.parametrize('mode', ['bf16', 'fp8', 'pow2', 'ue8m0'])
+@pytest.mark.parametrize('hook', [False, True])
+def test_low_latency_against_the_oracle(T, H, E, K, mode, hook):
+    import deepep_b200
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    from deepep_b200.utils.math import per_token_cast_back, per_token_cast_to_fp8, unpack_ue8m0
+    if mode == 'ue8m0' and H % 512 != 0:
+        pytest.skip('UE8M0 scales need hidden % 512 == 0')
+    Tm = 128
+    buf = deepep_b200.Buffer(SingleProcessGroup(), num_rdma_bytes=deepep_b200.Buffer.get_low_latency_rdma_size_hint(Tm, H, 1, E),
+                             low_latency_mode=True, num_gpu_timeout_secs=5)
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=T + K, device='cuda', masked_ratio=0.2)
+    stats = torch.zeros(E, dtype=torch.int32, device='cuda')
+    fp8 = mode != 'bf16'
+    q, sc = per_token_cast_to_fp8(x, round_scale=mode in ('pow2', 'ue8m0'))
+    for _ in range(2):
+        recv, count, handle, _, h = buf.low_latency_dispatch(x, idx, Tm, E, cumulative_local_expert_recv_stats=stats, use_fp8=fp8,
+                                                             round_scale=mode in ('pow2', 'ue8m0'), use_ue8m0=mode == 'ue8m0', return_recv_hook=hook)
+        if hook:
+            h()
+        torch.cuda.synchronize()
+        buf.check_status()
+        rows = torch.zeros((E, Tm, H), device='cuda', dtype=torch.bfloat16)
+        for e in range(E):
+            tok, lane = (idx == e).nonzero(as_tuple=True)
+            n = tok.numel()
+            assert int(count[e]) == n and int(handle[1][e, 0]) == n
+            assert torch.equal(handle[0][e, :n], (tok | (lane << 16)).int())
+            if n == 0:
+                continue
+            if not fp8:
+                assert torch.equal(recv[e, :n], x[tok])
+                rows[e, :n] = x[tok]
+                continue
+            assert torch.equal(recv[0][e, :n].view(torch.uint8), q[tok].view(torch.uint8)) and recv[1].stride(1) == 1
+            sf = recv[1][e, :n]
+            sf = unpack_ue8m0(sf.contiguous()).view(n, -1) if mode == 'ue8m0' else sf
+            assert torch.equal(sf.float(), sc[tok])
+            rows[e, :n] = per_token_cast_back(q[tok], sc[tok].contiguous())
+        ref = torch.zeros((T, H), device='cuda')
+        for k in range(K):
+            for t in range(T):
+                e = int(idx[t, k])
+                if e >= 0:
+                    j = int(((idx[:t] == e).any(dim=1)).sum())
+                    ref[t] += w[t, k] * rows[e, j].float()
+        for logfmt in (False, True):        # LogFMT takes the message path of the multi-rank kernels, on the same handle
+            if logfmt and H % 128 != 0:
+                continue
+            out, _, h = buf.low_latency_combine(rows, idx, w, handle, use_logfmt=logfmt, return_recv_hook=hook)
+            if hook:
+                h()
+            torch.cuda.synchronize()
+            buf.check_status()
+            # one bf16 rounding of an fp32 sum; a 10-bit log code is within 2 % of a value
+            tol = 3e-2 if logfmt else 2 ** -8
+            assert (out.float() - ref).norm() <= tol * ref.norm() + 1e-6
+    assert torch.equal(stats, torch.stack([(idx == e).sum() for e in range(E)]).int() * 2)
+    buf.destroy()
