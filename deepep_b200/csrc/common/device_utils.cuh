@@ -145,6 +145,28 @@ __device__ __forceinline__ void st_na_int4(void* p, const int4& v) {
                  ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
+// 32 consecutive bytes of one lane (256-bit accesses where the row allows them, `wide`; else twice 16 bytes). Past the end
+// of the row the load gives zeros and the store does nothing.
+__device__ __forceinline__ void load_32(const uint8_t* src, int bytes_left, bool wide, int4& lo, int4& hi) {
+    lo = hi = make_int4(0, 0, 0, 0);
+    if (wide && bytes_left >= 32) {
+        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "l"(src));
+        return;
+    }
+    if (bytes_left >= 16) lo = *reinterpret_cast<const int4*>(src);
+    if (bytes_left >= 32) hi = *reinterpret_cast<const int4*>(src + 16);
+}
+__device__ __forceinline__ void store_32(uint8_t* dst, int bytes_left, bool wide, const int4& lo, const int4& hi) {
+    if (wide && bytes_left >= 32) {
+        asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                     ::"l"(dst), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w) : "memory");
+        return;
+    }
+    if (bytes_left >= 16) st_na_int4(dst, lo);
+    if (bytes_left >= 32) st_na_int4(dst + 16, hi);
+}
+
 // ---------------------------------------------------------------- status / bounded waits
 struct WaitCtx {
     uint64_t deadline_ns;   // absolute %globaltimer value after which waits give up
@@ -312,6 +334,26 @@ __device__ __forceinline__ uint32_t pack4_e4m3(float a, float b, float c, float 
     const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
     const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
     return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+}
+
+// Sixteen bf16 channels per lane -> e4m3, eight neighbouring lanes share a scale group of 128. Warp-collective.
+__device__ __forceinline__ int4 cast16_e4m3(const int4& lo, const int4& hi, bool round_pow2, float& scale) {
+    float amax = fmaxf(amax_bf16x8(lo), amax_bf16x8(hi));
+    amax = warp_reduce_max_width(amax, 8);
+    float inv;
+    fp8_scale_from_amax(amax, round_pow2, scale, inv);
+    int4 q;
+    uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(h == 0 ? &lo : &hi);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float2 f0 = __bfloat1622float2(h2[2 * j]), f1 = __bfloat1622float2(h2[2 * j + 1]);
+            qw[2 * h + j] = pack4_e4m3(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
+        }
+    }
+    return q;
 }
 
 }  // namespace ep

@@ -242,6 +242,7 @@ struct LocalMoveParams {
     int src_row_bytes;
     int plan_ahead;           // 1: launched behind the plan kernel (waits for its end)
     int wide_in, wide_out;    // rows start on 32-byte boundaries (filled in by the launcher)
+    int columns;              // 1 KB slices of a row (filled in by the launcher)
     const uint8_t* x;
     int64_t x_stride_bytes;
     const uint32_t* sf;       // caller-made scale factors (packs of 4 bytes) or null
@@ -271,6 +272,7 @@ struct LocalCombineParams {
     int num_tokens, num_topk, num_experts, row_bytes, do_expand, weighted, idx32;
     int round_partial;        // the sum of a token's rows is rounded to bf16 before the biases are added
     int num_x_rows;
+    int columns, warps;       // columns of a row, warps (filled in by the launcher)
     const uint8_t* x;
     int64_t x_stride_bytes;
     const float* topk_weights;       // [N, K], expanded [rows], or null

@@ -79,21 +79,8 @@ __global__ void __launch_bounds__(kLLLocalThreads) ll_local_dispatch_kernel(cons
                 continue;
             }
             // 16 channels per lane, eight lanes per scale group
-            float amax = fmaxf(amax_bf16x8(lo), amax_bf16x8(hi));
-            amax = warp_reduce_max_width(amax, 8);
-            float scale, inv;
-            fp8_scale_from_amax(amax, p.round_scale != 0, scale, inv);
-            int4 q;
-            uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(h == 0 ? &lo : &hi);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const float2 f0 = __bfloat1622float2(h2[2 * j]), f1 = __bfloat1622float2(h2[2 * j + 1]);
-                    qw[2 * h + j] = pack4_e4m3(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
-                }
-            }
+            float scale;
+            const int4 q = cast16_e4m3(lo, hi, p.round_scale != 0, scale);
             if (off < row_bytes) {
                 const int g = off >> 8;
                 for (int k = 0; k < K; ++k) {

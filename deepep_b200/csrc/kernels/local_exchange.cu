@@ -17,6 +17,8 @@
 // Results (row order, metadata, rounding) are those of the multi-rank kernels with one rank.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "api.hpp"
 #include "../common/device_utils.cuh"
 
@@ -173,48 +175,44 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     } else {
         __syncthreads();
     }
-    // first row of every expert (alignment applied): one warp scans; the column of the tokens has no start to add
-    if (warp == 0) {
-        int carry = 0;
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + lane;
-            int total = 0, before = 0;
-            if (e < E)
-                for (int c = 0; c < num_ctas; ++c) {
-                    const int v = s_all[c * (E + 1) + e];
-                    total += v;
-                    if (c < cta) before += v;
-                }
-            const int aligned = align_up(total, p.expert_alignment);
-            int incl = aligned;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += up;
-            }
-            const int start = carry + incl - aligned;
-            if (e < E) {
-                s_base[e] = start + before;
-                if (cta == 0) {
-                    if (p.host_counts != nullptr) p.host_counts[2 + e] = pack_epoch(p.epoch, static_cast<uint32_t>(aligned));
-                    p.num_unaligned[e] = total;
-                    p.psum_expert[e] = p.do_expand ? start + total : start + aligned;
-                    if (p.recv_stats != nullptr) p.recv_stats[e] += total;
-                }
-            }
-            carry += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0 && cta == 0) {
-            p.psum_expert[E] = carry;
-            if (p.host_counts != nullptr) p.host_counts[1] = pack_epoch(p.epoch, static_cast<uint32_t>(carry));
-        }
-    } else if (tid == 32) {
-        int total = 0, before = 0;
+    // first row of every expert (alignment applied): a thread per expert, prefix over the warps' sums; the column of the
+    // tokens has no start to add
+    __shared__ int s_warp_sum[kMaxLocalExperts / 32];
+    static_assert(kMaxLocalExperts < kPlanThreads, "a thread per expert and one for the tokens");
+    int total = 0, before = 0;
+    if (tid <= E)
         for (int c = 0; c < num_ctas; ++c) {
-            const int v = s_all[c * (E + 1) + E];
+            const int v = s_all[c * (E + 1) + tid];
             total += v;
             if (c < cta) before += v;
         }
+    const int aligned = tid < E ? align_up(total, p.expert_alignment) : 0;
+    int incl = aligned;
+    if (warp < kMaxLocalExperts / 32) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) s_warp_sum[warp] = incl;
+    }
+    __syncthreads();
+    if (tid < E) {
+        int start = incl - aligned;
+#pragma unroll
+        for (int w = 0; w < kMaxLocalExperts / 32; ++w) start += w < warp ? s_warp_sum[w] : 0;
+        s_base[tid] = start + before;
+        if (cta == 0) {
+            if (p.host_counts != nullptr) {
+                p.host_counts[2 + tid] = pack_epoch(p.epoch, static_cast<uint32_t>(aligned));
+                if (tid == E - 1) p.host_counts[1] = pack_epoch(p.epoch, static_cast<uint32_t>(start + aligned));
+            }
+            p.num_unaligned[tid] = total;
+            p.psum_expert[tid] = p.do_expand ? start + total : start + aligned;
+            if (tid == E - 1) p.psum_expert[E] = start + aligned;
+            if (p.recv_stats != nullptr) p.recv_stats[tid] += total;
+        }
+    } else if (tid == E) {
         s_base[E] = before;
         if (cta == 0) {
             if (p.host_counts != nullptr) p.host_counts[0] = pack_epoch(p.epoch, static_cast<uint32_t>(total));
@@ -244,62 +242,33 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
 }
 
 // ==================================================================== move
-// Sixteen bytes twice (or 32 bytes at once when the row allows it): a lane owns 32 consecutive bytes of the row.
-__device__ __forceinline__ void load_32(const uint8_t* src, int bytes_left, bool wide, int4& lo, int4& hi) {
-    lo = hi = make_int4(0, 0, 0, 0);
-    if (wide && bytes_left >= 32) {
-        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "l"(src));
-        return;
-    }
-    if (bytes_left >= 16) lo = *reinterpret_cast<const int4*>(src);
-    if (bytes_left >= 32) hi = *reinterpret_cast<const int4*>(src + 16);
-}
-__device__ __forceinline__ void store_32(uint8_t* dst, int bytes_left, bool wide, const int4& lo, const int4& hi) {
-    if (wide && bytes_left >= 32) {
-        asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                     ::"l"(dst), "r"(lo.x), "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w) : "memory");
-        return;
-    }
-    if (bytes_left >= 16) st_na_int4(dst, lo);
-    if (bytes_left >= 32) st_na_int4(dst + 16, hi);
-}
-
 constexpr int kMoveThreads = 256;
-constexpr int kMoveSlice = 1024;            // input bytes of a row that a warp takes at once (32 per lane)
-constexpr int kMoveUnroll = 2;              // slices in flight per warp
+constexpr int kMoveSlice = 1024;            // input bytes of a row that a warp moves (32 per lane)
 constexpr int kPadRows = 4;                 // padding rows per zeroing work item
 
-// Work item = (token, kMoveUnroll slices of its row), one warp each: whatever the number of tokens, the row is cut so
-// that all SMs take part (64 tokens of hidden 7168 are 448 items). The item of the first slices also writes the token's
-// routing words. Rows are streamed: every byte is read once and written once per destination row, 32 bytes per lane.
-template <bool kQuant>
+// One warp per (token, 1 KB slice of its row) and nothing else: neighbouring warps have neighbouring slices, and a grid of
+// many short blocks keeps the memory system busier than a resident grid that loops (8192 x 7168 bf16: copy 38 against
+// 41-43 us, cast to e4m3 29 against 31-34 us, whatever the unrolling or prefetching inside the loop). The warps of column 0
+// also write the tokens' routing words. The slice is requested before the plan is awaited (the input was there before the
+// plan kernel started).
+template <bool kQuant, bool kExpand>
 __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_constant__ LocalMoveParams p) {
     const int lane = lane_id();
     const int K = p.num_topk, T = p.num_tokens;
-    const int slices = ceil_div(p.src_row_bytes, kMoveSlice * kMoveUnroll);
-    const int64_t items = static_cast<int64_t>(T) * slices;
-    const int warp_global = blockIdx.x * (kMoveThreads / 32) + warp_id(), num_warps = gridDim.x * (kMoveThreads / 32);
+    const uint32_t warp_global = blockIdx.x * (kMoveThreads / 32) + warp_id(), num_warps = gridDim.x * (kMoveThreads / 32);
     const bool wide_in = p.wide_in != 0, wide_out = p.wide_out != 0;
+    const int t = static_cast<int>(warp_global / static_cast<uint32_t>(p.columns)), col = static_cast<int>(warp_global % static_cast<uint32_t>(p.columns));
+    const int off = col * kMoveSlice + lane * 32;
+    int4 lo, hi;
+    if (t < T) load_32(p.x + static_cast<int64_t>(t) * p.x_stride_bytes + off, p.src_row_bytes - off, wide_in, lo, hi);
     if (p.plan_ahead) dependency_wait();
+    if (t < T) {
+        // expanded: the row of top-k lane `lane`; else the token's row
+        int row = kExpand ? (lane < K ? p.pair_row[static_cast<int64_t>(t) * K + lane] : -1) : p.token_slot[t];
+        if (row >= p.num_out_rows) row = -1;
+        const uint32_t rows = kExpand ? __ballot_sync(0xffffffffu, row >= 0) : (row >= 0 ? 1u : 0u);
 
-    for (int64_t it = warp_global; it < items; it += num_warps) {
-        const int t = static_cast<int>(it / slices), s = static_cast<int>(it % slices);
-        const uint8_t* src = p.x + static_cast<int64_t>(t) * p.x_stride_bytes;
-        const int off = s * kMoveSlice * kMoveUnroll + lane * 32;
-        int4 lo[kMoveUnroll], hi[kMoveUnroll];
-#pragma unroll
-        for (int u = 0; u < kMoveUnroll; ++u) load_32(src + off + u * kMoveSlice, p.src_row_bytes - off - u * kMoveSlice, wide_in, lo[u], hi[u]);
-        const int slot = p.token_slot[t];
-        int row = -1;                                   // expanded layout: the row of top-k lane `lane`
-        if (p.do_expand && lane < K) {
-            row = p.pair_row[static_cast<int64_t>(t) * K + lane];
-            if (row >= p.num_out_rows) row = -1;
-        }
-        uint32_t rows = p.do_expand ? __ballot_sync(0xffffffffu, row >= 0) : (slot >= 0 && slot < p.num_out_rows ? 1u : 0u);
-        if (!p.do_expand) row = slot;                   // the same on every lane
-
-        if (s == 0) {
+        if (col == 0) {
             // ---- routing words
             int e = -1;
             if (lane < K) {
@@ -311,9 +280,10 @@ __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_c
                 }
             }
             const uint32_t valid = __ballot_sync(0xffffffffu, e >= 0);
+            const int slot = p.token_slot[t];
             if (slot >= 0 && slot < p.num_idx_rows && lane < K) {
                 const int64_t o = static_cast<int64_t>(slot) * K + lane;
-                if (!p.do_expand) {
+                if (!kExpand) {
                     if (p.recv_topk_idx != nullptr) {
                         if (p.idx32) reinterpret_cast<int*>(p.recv_topk_idx)[o] = e;
                         else reinterpret_cast<int64_t*>(p.recv_topk_idx)[o] = e;
@@ -325,7 +295,7 @@ __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_c
                 }
                 if (p.write_metadata) {
                     int* md = p.recv_src_metadata + static_cast<int64_t>(slot) * (K + 2);
-                    md[2 + lane] = p.do_expand ? row : -1;
+                    md[2 + lane] = kExpand ? row : -1;
                     if (lane == 0) {
                         md[0] = t;
                         md[1] = valid != 0 ? __ffs(valid) - 1 : 0;
@@ -338,7 +308,7 @@ __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_c
                     const bool in = i < p.sf_packs;
                     const uint32_t v = in ? p.sf[static_cast<int64_t>(t) * p.sf_token_stride + static_cast<int64_t>(i) * p.sf_pack_stride] : 0u;
                     for (uint32_t todo = rows; todo != 0; todo &= todo - 1) {
-                        const int r = __shfl_sync(0xffffffffu, row, __ffs(todo) - 1);
+                        const int r = kExpand ? __shfl_sync(0xffffffffu, row, __ffs(todo) - 1) : row;
                         if (in) p.recv_sf[static_cast<int64_t>(r) * p.recv_sf_row_stride + static_cast<int64_t>(i) * p.recv_sf_pack_stride] = v;
                     }
                 }
@@ -348,54 +318,28 @@ __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_c
         // ---- payload
         if constexpr (!kQuant) {
             for (uint32_t todo = rows; todo != 0; todo &= todo - 1) {
-                const int r = __shfl_sync(0xffffffffu, row, __ffs(todo) - 1);
-                uint8_t* dst = p.recv_x + static_cast<int64_t>(r) * p.recv_x_pitch;
-#pragma unroll
-                for (int u = 0; u < kMoveUnroll; ++u)
-                    store_32(dst + off + u * kMoveSlice, p.src_row_bytes - off - u * kMoveSlice, wide_out, lo[u], hi[u]);
+                const int r = kExpand ? __shfl_sync(0xffffffffu, row, __ffs(todo) - 1) : row;
+                store_32(p.recv_x + static_cast<int64_t>(r) * p.recv_x_pitch + off, p.src_row_bytes - off, wide_out, lo, hi);
             }
         } else {
             // a lane holds 16 channels, eight lanes a scale group of 128 (hidden is a multiple of 128: a group is all in or all out)
-            float scale[kMoveUnroll];
-            int4 q[kMoveUnroll];
-#pragma unroll
-            for (int u = 0; u < kMoveUnroll; ++u) {
-                float amax = fmaxf(amax_bf16x8(lo[u]), amax_bf16x8(hi[u]));
-                amax = warp_reduce_max_width(amax, 8);
-                float inv;
-                fp8_scale_from_amax(amax, p.pow2 != 0, scale[u], inv);
-                uint32_t* qw = reinterpret_cast<uint32_t*>(&q[u]);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(h == 0 ? &lo[u] : &hi[u]);
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const float2 f0 = __bfloat1622float2(h2[2 * j]), f1 = __bfloat1622float2(h2[2 * j + 1]);
-                        qw[2 * h + j] = pack4_e4m3(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
-                    }
-                }
-            }
+            float scale;
+            const int4 q = cast16_e4m3(lo, hi, p.pow2 != 0, scale);
             for (uint32_t todo = rows; todo != 0; todo &= todo - 1) {
-                const int r = __shfl_sync(0xffffffffu, row, __ffs(todo) - 1);
-                uint8_t* dst = p.recv_x + static_cast<int64_t>(r) * p.recv_x_pitch;
-                float* sf = reinterpret_cast<float*>(p.recv_sf) + static_cast<int64_t>(r) * p.recv_sf_row_stride;
-#pragma unroll
-                for (int u = 0; u < kMoveUnroll; ++u) {
-                    const int o = off + u * kMoveSlice;
-                    if (o < p.src_row_bytes) {
-                        st_na_int4(dst + o / 2, q[u]);
-                        if ((lane & 7) == 0) sf[static_cast<int64_t>(o >> 8) * p.recv_sf_pack_stride] = scale[u];
-                    }
-                }
+                const int r = kExpand ? __shfl_sync(0xffffffffu, row, __ffs(todo) - 1) : row;
+                if (off >= p.src_row_bytes) continue;
+                st_na_int4(p.recv_x + static_cast<int64_t>(r) * p.recv_x_pitch + off / 2, q);
+                if ((lane & 7) == 0)
+                    reinterpret_cast<float*>(p.recv_sf)[static_cast<int64_t>(r) * p.recv_sf_row_stride + (off >> 8) * p.recv_sf_pack_stride] = scale;
             }
         }
     }
 
     // ---- routing rows past the received count
     const int n = p.psum_rank[0];
-    for (int64_t j = static_cast<int64_t>(n) * K + warp_global * 32 + lane; j < static_cast<int64_t>(p.num_idx_rows) * K; j += static_cast<int64_t>(num_warps) * 32) {
+    for (int64_t j = static_cast<int64_t>(n) * K + static_cast<int64_t>(warp_global) * 32 + lane; j < static_cast<int64_t>(p.num_idx_rows) * K; j += static_cast<int64_t>(num_warps) * 32) {
         const int i = static_cast<int>(j / K), k = static_cast<int>(j % K);
-        if (!p.do_expand) {
+        if (!kExpand) {
             if (p.recv_topk_idx != nullptr) {
                 if (p.idx32) reinterpret_cast<int*>(p.recv_topk_idx)[j] = -1;
                 else reinterpret_cast<int64_t*>(p.recv_topk_idx)[j] = -1;
@@ -410,7 +354,7 @@ __global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_c
     }
 
     // ---- alignment gaps of the expanded layout, kPadRows rows per item so that the few experts keep every SM busy
-    if (p.do_expand && p.do_zero_padding) {
+    if (kExpand && p.do_zero_padding) {
         const int out_row_bytes = kQuant ? p.src_row_bytes / 2 : p.src_row_bytes;
         const int per_expert = ceil_div(p.expert_alignment, kPadRows);
         for (int64_t it = warp_global; it < static_cast<int64_t>(p.num_experts) * per_expert; it += num_warps) {
@@ -452,86 +396,98 @@ __device__ __forceinline__ void fma_bf16x8(float (&acc)[8], const int4& raw, flo
     }
 }
 
-constexpr int kCombineThreads = 256;
+constexpr int kCombineThreads = 128;
 
-// Work item = (token, NV columns of 16 bytes per lane), a warp takes a run of consecutive items, so that the rows of a
-// token are looked up once per token and not once per column. NR rows x NV columns = 128 bytes are in flight per lane
-// before the first add; the adds run in ascending top-k order.
-template <int NV, int NR, bool kWeighted>
+// Like the move kernel: a warp owns a column (NV x 512 bytes) of the rows and walks over tokens, so that neighbouring warps
+// read neighbouring bytes of the same rows (a warp that walked along its own token's rows left every DRAM page after 512
+// bytes: 121 us for 32768 rows of hidden 7168 against 81 us that the bytes take). NR rows x NV vectors = up to 128 bytes are
+// in flight per lane before the first add; the rows of the next token are looked up meanwhile. The adds run in ascending
+// top-k order.
+template <int NV, int NR, bool kExpand, bool kWeighted>
 __global__ void __launch_bounds__(kCombineThreads) local_combine_kernel(const __grid_constant__ LocalCombineParams p) {
     const int lane = lane_id();
-    const int K = p.num_topk;
+    const int K = p.num_topk, T = p.num_tokens;
     const int vec_per_row = p.row_bytes / 16;
-    const int cols = ceil_div(vec_per_row, 32 * NV);
-    const int64_t items = static_cast<int64_t>(p.num_tokens) * cols;
-    const int64_t num_warps = static_cast<int64_t>(gridDim.x) * (kCombineThreads / 32);
-    const int64_t w = static_cast<int64_t>(blockIdx.x) * (kCombineThreads / 32) + warp_id();
-    const int64_t first = items * w / num_warps, last = items * (w + 1) / num_warps;
+    const int warp_global = blockIdx.x * (kCombineThreads / 32) + warp_id();
+    const int col = warp_global % p.columns, step = p.warps / p.columns;
+    const int v0 = col * 32 * NV + lane;
     if (blockIdx.x == 0 && threadIdx.x == 0) p.timeline[0] = globaltimer_ns();
-    int cur = -1, row = -1;         // token whose rows are held, this lane's row
-    float wt = 1.f;
-    uint32_t rows = 0;
-    for (int64_t it = first; it < last; ++it) {
-        const int t = static_cast<int>(it / cols), c = static_cast<int>(it % cols);
-        if (t != cur) {
-            cur = t;
-            const int slot = p.token_slot[t];
-            row = -1;
-            if (lane < K && slot >= 0) row = p.do_expand ? p.recv_src_metadata[static_cast<int64_t>(slot) * (K + 2) + 2 + lane] : (lane == 0 ? slot : -1);
-            if (row >= p.num_x_rows) row = -1;
-            rows = __ballot_sync(0xffffffffu, row >= 0);
-            if (kWeighted) wt = row >= 0 ? p.topk_weights[row] : 0.f;
-            if (c == 0 && p.combined_topk_weights != nullptr && lane < K) {
-                float v = 0.f;
-                if (p.topk_weights != nullptr) {
-                    if (p.do_expand) v = row >= 0 ? p.topk_weights[row] : 0.f;
-                    else if (slot >= 0 && load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + lane, p.num_experts) >= 0)
-                        v = p.topk_weights[static_cast<int64_t>(slot) * K + lane];
-                }
-                p.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = v;
+    int t = warp_global < p.warps ? warp_global / p.columns : T;
+    int next_row = -1, later_slot = -1;     // row of the next token (this lane's, when expanded), slot of the one after it
+    auto request_row = [&](int slot) {
+        if (kExpand) next_row = lane < K && slot >= 0 ? p.recv_src_metadata[static_cast<int64_t>(slot) * (K + 2) + 2 + lane] : -1;
+        else next_row = slot;
+    };
+    if (t < T) request_row(p.token_slot[t]);
+    if (t + step < T) later_slot = p.token_slot[t + step];
+    for (; t < T; t += step) {
+        const int row = next_row < p.num_x_rows ? next_row : -1;
+        if (t + step < T) request_row(later_slot);
+        if (t + 2 * step < T) later_slot = p.token_slot[t + 2 * step];
+        uint8_t* dst = p.combined_x + static_cast<int64_t>(t) * p.row_bytes;
+        if (col == 0 && p.combined_topk_weights != nullptr && lane < K) {
+            float v = 0.f;
+            if (p.topk_weights != nullptr && row >= 0) {
+                if (kExpand) v = p.topk_weights[row];
+                else if (load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + lane, p.num_experts) >= 0)
+                    v = p.topk_weights[static_cast<int64_t>(row) * K + lane];
             }
+            p.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = v;
         }
+        if (!kExpand && p.bias0 == nullptr && p.bias1 == nullptr) {
+            // one row per token and nothing to add: the row is the result
+            const uint8_t* src = p.x + static_cast<int64_t>(row) * p.x_stride_bytes;
+            int4 raw[NV];
+#pragma unroll
+            for (int j = 0; j < NV; ++j) raw[j] = row >= 0 && v0 + 32 * j < vec_per_row ? ld_nc_int4(src + (v0 + 32 * j) * 16) : make_int4(0, 0, 0, 0);
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+                if (v0 + 32 * j < vec_per_row) st_na_int4(dst + (v0 + 32 * j) * 16, raw[j]);
+            continue;
+        }
+        const uint32_t rows = kExpand ? __ballot_sync(0xffffffffu, row >= 0) : (row >= 0 ? 1u : 0u);
+        const float wt = kWeighted && row >= 0 ? p.topk_weights[row] : 0.f;
         float acc[NV][8];
 #pragma unroll
         for (int j = 0; j < NV; ++j)
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
-        const int v0 = c * 32 * NV + lane;
         for (uint32_t todo = rows; todo != 0;) {        // (uniform over the warp: lanes past the row's end take part in the shuffles)
             int4 raw[NR][NV];
-            int rr[NR];
-            float ww[NR];
+            const uint32_t batch = todo;
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                const int k = todo != 0 ? __ffs(todo) - 1 : 0;
-                const int got = __shfl_sync(0xffffffffu, row, k);
-                rr[r] = todo != 0 ? got : -1;
-                if (kWeighted) ww[r] = __shfl_sync(0xffffffffu, wt, k);
+                const int rr = kExpand ? __shfl_sync(0xffffffffu, row, todo != 0 ? __ffs(todo) - 1 : 0) : row;
+                const uint8_t* src = p.x + static_cast<int64_t>(rr) * p.x_stride_bytes;
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    if (todo != 0 && v0 + 32 * j < vec_per_row) raw[r][j] = ld_nc_int4(src + (v0 + 32 * j) * 16);
                 todo &= todo - 1;       // 0 stays 0
-#pragma unroll
-                for (int j = 0; j < NV; ++j)
-                    if (rr[r] >= 0 && v0 + 32 * j < vec_per_row) raw[r][j] = ld_nc_int4(p.x + static_cast<int64_t>(rr[r]) * p.x_stride_bytes + (v0 + 32 * j) * 16);
             }
+            uint32_t now = batch;
 #pragma unroll
-            for (int r = 0; r < NR; ++r)
+            for (int r = 0; r < NR; ++r) {
+                const float wr = kWeighted ? __shfl_sync(0xffffffffu, wt, now != 0 ? __ffs(now) - 1 : 0) : 1.f;
 #pragma unroll
                 for (int j = 0; j < NV; ++j)
-                    if (rr[r] >= 0 && v0 + 32 * j < vec_per_row) {
-                        if (kWeighted) fma_bf16x8(acc[j], raw[r][j], ww[r]);
+                    if (now != 0 && v0 + 32 * j < vec_per_row) {
+                        if (kWeighted) fma_bf16x8(acc[j], raw[r][j], wr);
                         else add_bf16x8(acc[j], raw[r][j]);
                     }
+                now &= now - 1;
+            }
         }
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
             const int v = v0 + 32 * j;
             if (v >= vec_per_row) continue;
-            const int64_t off = static_cast<int64_t>(t) * p.row_bytes + v * 16;
             if (p.bias0 != nullptr || p.bias1 != nullptr) {
                 if (p.round_partial) {
                     // a rank's partial sum is rounded once before it leaves the rank, then the biases are added
 #pragma unroll
                     for (int i = 0; i < 8; ++i) acc[j][i] = __bfloat162float(__float2bfloat16_rn(acc[j][i]));
                 }
+                const int64_t off = static_cast<int64_t>(t) * p.row_bytes + v * 16;
                 if (p.bias0 != nullptr) add_bf16x8(acc[j], ld_nc_int4(p.bias0 + off));
                 if (p.bias1 != nullptr) add_bf16x8(acc[j], ld_nc_int4(p.bias1 + off));
             }
@@ -539,11 +495,31 @@ __global__ void __launch_bounds__(kCombineThreads) local_combine_kernel(const __
             __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
 #pragma unroll
             for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(acc[j][2 * i], acc[j][2 * i + 1]);
-            st_na_int4(p.combined_x + off, out);
+            st_na_int4(dst + v * 16, out);
         }
     }
     if (threadIdx.x == 0 && (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1))
         atomicMax(reinterpret_cast<unsigned long long*>(p.timeline + 1), static_cast<unsigned long long>(globaltimer_ns()));
+}
+
+// Blocks that fit an SM at once, looked up once per kernel.
+template <typename Kernel>
+int resident_blocks(Kernel kernel, int threads, std::atomic<int>& known) {
+    int n = known.load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess || n < 1) n = 1;
+        known.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// Warps for `tokens` x `columns` items on at most `most` resident warps: a multiple of the columns, such that every warp
+// takes the same number of tokens (give or take one).
+int balanced_warps(int tokens, int columns, int most) {
+    const int64_t items = static_cast<int64_t>(tokens) * columns;
+    const int rounds = static_cast<int>(ceil_div<int64_t>(items, most));
+    int per_column = ceil_div(tokens, rounds < 1 ? 1 : rounds);
+    return (per_column < 1 ? 1 : per_column) * columns;
 }
 
 template <typename Kernel, typename Params>
@@ -584,46 +560,53 @@ cudaError_t launch_local_plan(const LocalPlanParams& p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, local_plan_kernel, p);
 }
 
+template <bool kQuant, bool kExpand>
+static cudaError_t launch_move_cfg(LocalMoveParams& p, int num_sms, bool programmatic, cudaStream_t stream) {
+    static PreparedKernel prepared;
+    cudaError_t err = prepared.prepare(local_move_kernel<kQuant, kExpand>, 0);
+    if (err != cudaSuccess) return err;
+    p.columns = ceil_div(p.src_row_bytes, kMoveSlice);
+    int64_t warps = static_cast<int64_t>(p.num_tokens) * p.columns;
+    if (warps >= (1ll << 31)) return cudaErrorInvalidValue;
+    // (a few tokens can leave more padding rows to clear than there are slices to move)
+    if (kExpand && p.do_zero_padding)
+        warps = std::max<int64_t>(warps, std::min<int64_t>(num_sms * 32, static_cast<int64_t>(p.num_experts) * ceil_div(p.expert_alignment, kPadRows)));
+    const int grid = std::max(1, static_cast<int>(ceil_div<int64_t>(warps, kMoveThreads / 32)));
+    return launch_plain(local_move_kernel<kQuant, kExpand>, p, grid, kMoveThreads, stream, programmatic);
+}
+
 cudaError_t launch_local_move(const LocalMoveParams& params, bool quant, int num_sms, bool programmatic, cudaStream_t stream) {
     LocalMoveParams p = params;
-    static PreparedKernel prepared[2];
-    cudaError_t err = quant ? prepared[1].prepare(local_move_kernel<true>, 0) : prepared[0].prepare(local_move_kernel<false>, 0);
-    if (err != cudaSuccess) return err;
     const uint64_t in_bits = reinterpret_cast<uintptr_t>(p.x) | static_cast<uint64_t>(p.x_stride_bytes);
     const uint64_t out_bits = reinterpret_cast<uintptr_t>(p.recv_x) | static_cast<uint64_t>(p.recv_x_pitch);
     p.wide_in = in_bits % 32 == 0;
     p.wide_out = out_bits % 32 == 0;
-    const int64_t items = static_cast<int64_t>(p.num_tokens) * ceil_div(p.src_row_bytes, kMoveSlice * kMoveUnroll) +
-                          (p.do_expand && p.do_zero_padding ? static_cast<int64_t>(p.num_experts) * ceil_div(p.expert_alignment, kPadRows) : 0);
-    const int64_t want = ceil_div<int64_t>(items, kMoveThreads / 32), most = static_cast<int64_t>(num_sms) * 8;
-    const int grid = static_cast<int>(want < 1 ? 1 : (want > most ? most : want));
-    return quant ? launch_plain(local_move_kernel<true>, p, grid, kMoveThreads, stream, programmatic)
-                 : launch_plain(local_move_kernel<false>, p, grid, kMoveThreads, stream, programmatic);
+    if (quant) return p.do_expand ? launch_move_cfg<true, true>(p, num_sms, programmatic, stream) : launch_move_cfg<true, false>(p, num_sms, programmatic, stream);
+    return p.do_expand ? launch_move_cfg<false, true>(p, num_sms, programmatic, stream) : launch_move_cfg<false, false>(p, num_sms, programmatic, stream);
 }
 
-template <int NV, int NR, bool kWeighted>
-static cudaError_t launch_combine_cfg(const LocalCombineParams& p, int num_sms, cudaStream_t stream) {
+template <int NV, int NR, bool kExpand, bool kWeighted>
+static cudaError_t launch_combine_cfg(LocalCombineParams& p, int num_sms, cudaStream_t stream) {
     static PreparedKernel prepared;
-    static int per_sm = 0;
-    cudaError_t err = prepared.prepare(local_combine_kernel<NV, NR, kWeighted>, 0);
+    static std::atomic<int> per_sm{0};
+    auto kernel = local_combine_kernel<NV, NR, kExpand, kWeighted>;
+    cudaError_t err = prepared.prepare(kernel, 0);
     if (err != cudaSuccess) return err;
-    if (per_sm == 0) {
-        int n = 0;
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, local_combine_kernel<NV, NR, kWeighted>, kCombineThreads, 0);
-        if (err != cudaSuccess) return err;
-        per_sm = n < 1 ? 1 : n;
-    }
-    const int64_t items = static_cast<int64_t>(p.num_tokens) * ceil_div(p.row_bytes / 16, 32 * NV);
-    const int64_t want = ceil_div<int64_t>(items, kCombineThreads / 32), most = static_cast<int64_t>(num_sms) * per_sm;
-    return launch_plain(local_combine_kernel<NV, NR, kWeighted>, p, static_cast<int>(want > most ? most : want), kCombineThreads, stream, false);
+    const int warps_per_block = kCombineThreads / 32, most = num_sms * resident_blocks(kernel, kCombineThreads, per_sm) * warps_per_block;
+    p.columns = ceil_div(p.row_bytes / 16, 32 * NV);
+    p.warps = kExpand ? balanced_warps(p.num_tokens, p.columns, most) : p.num_tokens * p.columns;
+    return launch_plain(kernel, p, ceil_div(p.warps, warps_per_block), kCombineThreads, stream, false);
 }
 
-cudaError_t launch_local_combine(const LocalCombineParams& p, int num_sms, cudaStream_t stream) {
-    if (p.num_tokens == 0) return cudaSuccess;
-    // one row per token: four columns of it; up to four rows: two columns; more: eight rows of one column (128 bytes per lane or less)
-    if (!p.do_expand) return launch_combine_cfg<4, 1, false>(p, num_sms, stream);
-    if (p.num_topk <= 4) return p.weighted ? launch_combine_cfg<2, 4, true>(p, num_sms, stream) : launch_combine_cfg<2, 4, false>(p, num_sms, stream);
-    return p.weighted ? launch_combine_cfg<1, 8, true>(p, num_sms, stream) : launch_combine_cfg<1, 8, false>(p, num_sms, stream);
+cudaError_t launch_local_combine(const LocalCombineParams& params, int num_sms, cudaStream_t stream) {
+    if (params.num_tokens == 0) return cudaSuccess;
+    LocalCombineParams p = params;
+    // One row per token: one warp per KB of a row, each does it once (see the move kernel). Several rows: a resident grid,
+    // since looking up the rows of a token is a chain of two loads that the loop hides; up to four rows two vectors at a
+    // time, more than four one (128 bytes in flight per lane either way).
+    if (!p.do_expand) return launch_combine_cfg<2, 1, false, false>(p, num_sms, stream);
+    if (p.num_topk <= 4) return p.weighted ? launch_combine_cfg<2, 4, true, true>(p, num_sms, stream) : launch_combine_cfg<2, 4, true, false>(p, num_sms, stream);
+    return p.weighted ? launch_combine_cfg<1, 8, true, true>(p, num_sms, stream) : launch_combine_cfg<1, 8, true, false>(p, num_sms, stream);
 }
 
 }  // namespace ep

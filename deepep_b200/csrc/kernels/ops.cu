@@ -1,11 +1,14 @@
 // Small memory-bound operators of the MoE layer (sm_100a): router top-k + softmax, SwiGLU (with an
 // optional fused 1x128 e4m3 cast for the second expert GEMM), 1x128 block quantisation and
 // dequantisation, and a 2-D bf16 transpose for weight-gradient GEMMs.
-// All of them stream each byte once (16-byte accesses, no shared-memory staging except the
+// All of them stream each byte once (32-byte accesses, no shared-memory staging except the
 // transpose) and are bound by HBM bandwidth.
 //
 // The reference has none of these as kernels; its test helpers (deep_ep/utils/math.py:30-56) are
 // the arithmetic these follow.
+#include <algorithm>
+#include <initializer_list>
+
 #include "ops_api.hpp"
 #include "../common/device_utils.cuh"
 
@@ -63,174 +66,201 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
     }
 }
 
-// ---------------------------------------------------------------- 1x128 quantisation
-// thread = 8 channels, 16 threads = one scale group; rows * (hidden / 8) threads in total
-__global__ void __launch_bounds__(256) quant_kernel(const uint8_t* __restrict__ x, int64_t x_stride_bytes, int rows, int hidden, int pow2,
-                                                    uint8_t* __restrict__ out, float* __restrict__ scales, int64_t sf_row_stride,
-                                                    int64_t sf_col_stride) {
-    const int vec_per_row = hidden / 8;
-    const int64_t total = static_cast<int64_t>(rows) * vec_per_row;
-    for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x; base < total; base += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        const bool active = i < total;
-        const int row = active ? static_cast<int>(i / vec_per_row) : 0, ch = active ? static_cast<int>(i % vec_per_row) * 8 : 0;
-        int4 raw = make_int4(0, 0, 0, 0);
-        if (active) raw = ld_nc_int4(x + row * x_stride_bytes + ch * 2);
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-        float f[8];
+// ---------------------------------------------------------------- streaming kernels
+// One warp per (row, 512 channels) and nothing else, sixteen channels per lane: neighbouring warps have neighbouring bytes,
+// and a grid of many short blocks streams faster than a resident grid that loops over the same work (cast of 8192 x 7168:
+// 29 against 31-34 us). All of them are bound by HBM once the arithmetic per channel is short enough to hide.
+constexpr int kSpan = 512;
+
+struct RowCol {
+    int row, ch;        // first channel of this lane
+};
+__device__ __forceinline__ RowCol row_col(int columns) {
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + warp_id();
+    const uint32_t row = w / static_cast<uint32_t>(columns);
+    return {static_cast<int>(row), static_cast<int>(w - row * static_cast<uint32_t>(columns)) * kSpan + lane_id() * 16};
+}
+
+// Is the row in an alignment gap of the expanded layout (behind the rows of its expert)? Warp-collective, the same row on
+// every lane: the row belongs to the first group whose aligned end lies behind it.
+__device__ __forceinline__ bool in_gap(const RowGroups& g, int row) {
+    if (g.ends == nullptr) return false;
+    for (int base = 0; base < g.num; base += 32) {
+        const int i = base + lane_id();
+        const int end = i < g.num ? g.ends[i] : 0x3fffffff;
+        const uint32_t behind = __ballot_sync(0xffffffffu, align_up(end, g.alignment) > row);
+        if (behind != 0) {
+            const int src = __ffs(behind) - 1;
+            return base + src >= g.num || row >= __shfl_sync(0xffffffffu, end, src);
+        }
+    }
+    return true;
+}
+
+// 1 / (1 + e^-x) with the hardware's exponential and reciprocal (a few units in the last place of fp32, where the results
+// are rounded to bf16): with a correctly rounded division the forward kernel issued 40 instructions per value and ran at
+// 45 % of the memory rate.
+__device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+
+__device__ __forceinline__ void unpack16(const int4& lo, const int4& hi, float (&f)[16]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(h == 0 ? &lo : &hi);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float2 t = __bfloat1622float2(h2[j]);
-            f[2 * j] = t.x;
-            f[2 * j + 1] = t.y;
+            f[8 * h + 2 * j] = t.x;
+            f[8 * h + 2 * j + 1] = t.y;
         }
-        float amax = 0.f;
+    }
+}
+__device__ __forceinline__ void pack16(const float (&f)[16], int4& lo, int4& hi) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(f[j]));
-        amax = warp_reduce_max_width(amax, 16);   // hidden % 128 == 0: a 16-lane group never straddles rows
-        float scale, inv;
-        fp8_scale_from_amax(amax, pow2 != 0, scale, inv);
-        uint2 packed;
-        packed.x = pack4_e4m3(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
-        packed.y = pack4_e4m3(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
-        if (active) {
-            *reinterpret_cast<uint2*>(out + static_cast<int64_t>(row) * hidden + ch) = packed;
-            if ((threadIdx.x & 15) == 0) scales[row * sf_row_stride + (ch >> 7) * sf_col_stride] = scale;
-        }
+    for (int h = 0; h < 2; ++h) {
+        __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(h == 0 ? &lo : &hi);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(f[8 * h + 2 * j], f[8 * h + 2 * j + 1]);
+    }
+}
+
+// ---------------------------------------------------------------- 1x128 quantisation
+__global__ void __launch_bounds__(256) quant_kernel(const uint8_t* __restrict__ x, int64_t x_stride_bytes, int rows, int hidden, int columns, int wide, int pow2,
+                                                    uint8_t* __restrict__ out, float* __restrict__ scales, int64_t sf_row_stride,
+                                                    int64_t sf_col_stride) {
+    const RowCol rc = row_col(columns);
+    if (rc.row >= rows) return;
+    int4 lo, hi;
+    load_32(x + rc.row * x_stride_bytes + rc.ch * 2, (hidden - rc.ch) * 2, wide != 0, lo, hi);
+    float scale;
+    const int4 q = cast16_e4m3(lo, hi, pow2 != 0, scale);       // hidden % 128 == 0: a scale group is all in or all out
+    if (rc.ch < hidden) {
+        st_na_int4(out + static_cast<int64_t>(rc.row) * hidden + rc.ch, q);
+        if ((lane_id() & 7) == 0) scales[rc.row * sf_row_stride + (rc.ch >> 7) * sf_col_stride] = scale;
     }
 }
 
 __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scales, int64_t sf_row_stride,
-                                                      int64_t sf_col_stride, int rows, int hidden, uint8_t* __restrict__ out) {
-    const int vec_per_row = hidden / 8;
-    const int64_t total = static_cast<int64_t>(rows) * vec_per_row;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int row = static_cast<int>(i / vec_per_row), ch = static_cast<int>(i % vec_per_row) * 8;
-        const uint2 raw = *reinterpret_cast<const uint2*>(q + static_cast<int64_t>(row) * hidden + ch);
-        const float s = scales[row * sf_row_stride + (ch >> 7) * sf_col_stride];
-        const __nv_fp8x2_storage_t* p2 = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
-        int4 o;
-        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(p2[j], __NV_E4M3);
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-            o2[j] = __floats2bfloat162_rn(f.x * s, f.y * s);
-        }
-        *reinterpret_cast<int4*>(out + (static_cast<int64_t>(row) * hidden + ch) * 2) = o;
+                                                      int64_t sf_col_stride, int rows, int hidden, int columns, int wide, const RowGroups groups, uint8_t* __restrict__ out) {
+    const RowCol rc = row_col(columns);
+    if (rc.row >= rows) return;
+    const bool in = rc.ch < hidden;
+    int4 raw = make_int4(0, 0, 0, 0);
+    float s = 0.f;
+    if (in) {
+        raw = ld_nc_int4(q + static_cast<int64_t>(rc.row) * hidden + rc.ch);
+        s = scales[rc.row * sf_row_stride + (rc.ch >> 7) * sf_col_stride];
     }
+    const bool gap = in_gap(groups, rc.row);
+    const __nv_fp8x2_storage_t* p2 = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
+    float f[16];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(p2[j], __NV_E4M3);
+        const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&h));
+        f[2 * j] = gap ? 0.f : t.x * s;
+        f[2 * j + 1] = gap ? 0.f : t.y * s;
+    }
+    int4 lo, hi;
+    pack16(f, lo, hi);
+    store_32(out + (static_cast<int64_t>(rc.row) * hidden + rc.ch) * 2, (hidden - rc.ch) * 2, wide != 0, lo, hi);
 }
 
 // ---------------------------------------------------------------- SwiGLU: out = silu(gate) * up (* row weight), optional fused 1x128 cast
+// Rows in alignment gaps are left alone (a decode batch over 32 experts has 4096 rows, of which 512 mean something).
 template <bool kQuant>
-__global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__ x, int rows, int inter, const float* __restrict__ row_weight,
-                                                     const int* __restrict__ num_valid_rows, uint8_t* __restrict__ out,
+__global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__ x, int rows, int inter, int columns, int wide, const float* __restrict__ row_weight,
+                                                     const int* __restrict__ num_valid_rows, const RowGroups groups, uint8_t* __restrict__ out,
                                                      float* __restrict__ scales, int64_t sf_row_stride, int64_t sf_col_stride, int pow2) {
-    const int vec_per_row = inter / 8;
-    const int valid = num_valid_rows != nullptr ? min(*num_valid_rows, rows) : rows;
-    const int64_t total = static_cast<int64_t>(valid) * vec_per_row;
-    for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x; base < total; base += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t i = base + threadIdx.x;
-        const bool active = i < total;
-        const int row = active ? static_cast<int>(i / vec_per_row) : 0, ch = active ? static_cast<int>(i % vec_per_row) * 8 : 0;
-        int4 g = make_int4(0, 0, 0, 0), u = make_int4(0, 0, 0, 0);
-        if (active) {
-            const uint8_t* src = x + (static_cast<int64_t>(row) * 2 * inter + ch) * 2;
-            g = ld_nc_int4(src);
-            u = ld_nc_int4(src + static_cast<int64_t>(inter) * 2);
-        }
-        const float wr = (active && row_weight != nullptr) ? row_weight[row] : 1.f;
-        const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&g);
-        const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&u);
-        float f[8];
+    const RowCol rc = row_col(columns);
+    if (rc.row >= (num_valid_rows != nullptr ? min(*num_valid_rows, rows) : rows)) return;
+    if (in_gap(groups, rc.row)) return;
+    const int left = (inter - rc.ch) * 2;
+    const uint8_t* src = x + (static_cast<int64_t>(rc.row) * 2 * inter + rc.ch) * 2;
+    int4 glo, ghi, ulo, uhi;
+    load_32(src, left, wide != 0, glo, ghi);
+    load_32(src + static_cast<int64_t>(inter) * 2, left, wide != 0, ulo, uhi);
+    const float wr = row_weight != nullptr ? row_weight[rc.row] : 1.f;
+    float g[16], u[16];
+    unpack16(glo, ghi, g);
+    unpack16(ulo, uhi, u);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 gv = __bfloat1622float2(g2[j]), uv = __bfloat1622float2(u2[j]);
-            f[2 * j] = gv.x / (1.f + __expf(-gv.x)) * uv.x * wr;
-            f[2 * j + 1] = gv.y / (1.f + __expf(-gv.y)) * uv.y * wr;
-        }
-        if constexpr (!kQuant) {
-            if (active) {
-                int4 o;
-                __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) o2[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-                *reinterpret_cast<int4*>(out + (static_cast<int64_t>(row) * inter + ch) * 2) = o;
-            }
-        } else {
-            // the cast sees what a bf16 round trip would see, so fused and unfused paths agree bit for bit
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = __bfloat162float(__float2bfloat16_rn(f[j]));
-            float amax = 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(f[j]));
-            amax = warp_reduce_max_width(amax, 16);
-            float scale, inv;
-            fp8_scale_from_amax(amax, pow2 != 0, scale, inv);
-            uint2 packed;
-            packed.x = pack4_e4m3(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv);
-            packed.y = pack4_e4m3(f[4] * inv, f[5] * inv, f[6] * inv, f[7] * inv);
-            if (active) {
-                *reinterpret_cast<uint2*>(out + static_cast<int64_t>(row) * inter + ch) = packed;
-                if ((threadIdx.x & 15) == 0) scales[row * sf_row_stride + (ch >> 7) * sf_col_stride] = scale;
-            }
+    for (int j = 0; j < 16; ++j) g[j] = g[j] * sigmoid_fast(g[j]) * u[j] * wr;
+    int4 lo, hi;
+    pack16(g, lo, hi);
+    if constexpr (!kQuant) {
+        store_32(out + (static_cast<int64_t>(rc.row) * inter + rc.ch) * 2, left, wide != 0, lo, hi);
+    } else {
+        // the cast sees the bf16 values, so fused and unfused paths agree bit for bit
+        float scale;
+        const int4 q = cast16_e4m3(lo, hi, pow2 != 0, scale);
+        if (left > 0) {
+            st_na_int4(out + static_cast<int64_t>(rc.row) * inter + rc.ch, q);
+            if ((lane_id() & 7) == 0) scales[rc.row * sf_row_stride + (rc.ch >> 7) * sf_col_stride] = scale;
         }
     }
 }
 
 // d(gate|up) from d(out): dgate = dout * up * sig * (1 + gate * (1 - sig)), dup = dout * silu(gate), both times the
-// row's gate weight. One block per row (grid-strided), so that the two by-products of the MoE backward pass come out
-// of the same read of (gate, up, dout): the weighted activation silu(gate) * up * w (the operand of the W2 weight
-// gradient) and the gradient of the gate weight, sum_i dout_i * silu(gate_i) * up_i (a row dot product).
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ dout, int rows, int inter,
-                                                         const float* __restrict__ row_weight, uint8_t* __restrict__ dx,
+// row's gate weight. One block per row, so that the two by-products of the MoE backward pass come out of the same read of
+// (gate, up, dout): the weighted activation silu(gate) * up * w (the operand of the W2 weight gradient) and the gradient
+// of the gate weight, sum_i dout_i * silu(gate_i) * up_i (a row dot product). Rows in alignment gaps give zeros.
+__global__ void __launch_bounds__(128) swiglu_bwd_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ dout, int inter, int wide,
+                                                         const float* __restrict__ row_weight, const RowGroups groups, uint8_t* __restrict__ dx,
                                                          uint8_t* __restrict__ act_out, float* __restrict__ dweight) {
-    __shared__ float s_part[8];
-    const int vec_per_row = inter / 8;
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-        const float wr = row_weight != nullptr ? row_weight[row] : 1.f;
-        float dot = 0.f;
-        for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
-            const int ch = v * 8;
-            const uint8_t* src = x + (static_cast<int64_t>(row) * 2 * inter + ch) * 2;
-            const int4 g = ld_nc_int4(src), u = ld_nc_int4(src + static_cast<int64_t>(inter) * 2);
-            const int4 d = ld_nc_int4(dout + (static_cast<int64_t>(row) * inter + ch) * 2);
-            const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&g);
-            const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&u);
-            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d);
-            int4 og, ou, oa;
-            __nv_bfloat162* og2 = reinterpret_cast<__nv_bfloat162*>(&og);
-            __nv_bfloat162* ou2 = reinterpret_cast<__nv_bfloat162*>(&ou);
-            __nv_bfloat162* oa2 = reinterpret_cast<__nv_bfloat162*>(&oa);
+    __shared__ float s_part[4];
+    const int row = blockIdx.x;
+    const bool gap = in_gap(groups, row);
+    const float wr = row_weight != nullptr && !gap ? row_weight[row] : 1.f;
+    float dot = 0.f;
+    for (int ch = threadIdx.x * 16; ch < inter; ch += blockDim.x * 16) {
+        const int left = (inter - ch) * 2;
+        const uint8_t* src = x + (static_cast<int64_t>(row) * 2 * inter + ch) * 2;
+        int4 lo = make_int4(0, 0, 0, 0), hi = lo;
+        float g[16], u[16], d[16];
+        if (!gap) {
+            int4 ulo, uhi, dlo, dhi;
+            load_32(src, left, wide != 0, lo, hi);
+            load_32(src + static_cast<int64_t>(inter) * 2, left, wide != 0, ulo, uhi);
+            load_32(dout + (static_cast<int64_t>(row) * inter + ch) * 2, left, wide != 0, dlo, dhi);
+            unpack16(lo, hi, g);
+            unpack16(ulo, uhi, u);
+            unpack16(dlo, dhi, d);
+        } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 gv = __bfloat1622float2(g2[j]), uv = __bfloat1622float2(u2[j]), dv = __bfloat1622float2(d2[j]);
-                const float sx = 1.f / (1.f + __expf(-gv.x)), sy = 1.f / (1.f + __expf(-gv.y));
-                const float dx_ = dv.x * wr, dy_ = dv.y * wr;
-                og2[j] = __floats2bfloat162_rn(dx_ * uv.x * sx * (1.f + gv.x * (1.f - sx)), dy_ * uv.y * sy * (1.f + gv.y * (1.f - sy)));
-                ou2[j] = __floats2bfloat162_rn(dx_ * gv.x * sx, dy_ * gv.y * sy);
-                // the activation as the forward pass rounded it (bf16), before the weight
-                const __nv_bfloat162 a = __floats2bfloat162_rn(gv.x * sx * uv.x, gv.y * sy * uv.y);
-                const float2 af = __bfloat1622float2(a);
-                dot = fmaf(dv.x, af.x, fmaf(dv.y, af.y, dot));
-                oa2[j] = __floats2bfloat162_rn(af.x * wr, af.y * wr);
-            }
-            uint8_t* dst = dx + (static_cast<int64_t>(row) * 2 * inter + ch) * 2;
-            *reinterpret_cast<int4*>(dst) = og;
-            *reinterpret_cast<int4*>(dst + static_cast<int64_t>(inter) * 2) = ou;
-            if (act_out != nullptr) *reinterpret_cast<int4*>(act_out + (static_cast<int64_t>(row) * inter + ch) * 2) = oa;
+            for (int j = 0; j < 16; ++j) g[j] = u[j] = d[j] = 0.f;
         }
-        if (dweight != nullptr) {
+        float a[16];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            __syncthreads();
-            if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = dot;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                float acc = 0.f;
-                for (int i = 0; i < 8; ++i) acc += s_part[i];      // fixed order: the result does not depend on timing
-                dweight[row] = acc;
-            }
+        for (int j = 0; j < 16; ++j) {
+            const float s = sigmoid_fast(g[j]);
+            const float silu = g[j] * s;
+            // the activation as the forward pass rounded it (bf16), before the weight
+            const float act = __bfloat162float(__float2bfloat16_rn(silu * u[j]));
+            dot = fmaf(d[j], act, dot);
+            a[j] = act * wr;
+            const float dw = d[j] * wr;
+            g[j] = dw * u[j] * s * (1.f + g[j] * (1.f - s));
+            u[j] = dw * silu;
+        }
+        uint8_t* dst = dx + (static_cast<int64_t>(row) * 2 * inter + ch) * 2;
+        pack16(g, lo, hi);
+        store_32(dst, left, wide != 0, lo, hi);
+        pack16(u, lo, hi);
+        store_32(dst + static_cast<int64_t>(inter) * 2, left, wide != 0, lo, hi);
+        if (act_out != nullptr) {
+            pack16(a, lo, hi);
+            store_32(act_out + (static_cast<int64_t>(row) * inter + ch) * 2, left, wide != 0, lo, hi);
+        }
+    }
+    if (dweight != nullptr) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = dot;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float acc = 0.f;
+            for (int i = 0; i < (static_cast<int>(blockDim.x) >> 5); ++i) acc += s_part[i];      // fixed order: the result does not depend on timing
+            dweight[row] = acc;
         }
     }
 }
@@ -282,11 +312,17 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __nv_bfloat16* __r
     }
 }
 
-int grid_for(int64_t threads_needed) {
-    int64_t blocks = (threads_needed + 255) / 256;
-    const int64_t cap = 148 * 16;
-    return static_cast<int>(blocks < 1 ? 1 : (blocks > cap ? cap : blocks));
+// blocks of eight warps for one warp per (row, kSpan channels); 0 = too many for one grid
+int span_blocks(int rows, int columns) {
+    const int64_t warps = static_cast<int64_t>(rows) * columns;
+    return warps < (1ll << 32) - 8 ? static_cast<int>((warps + 7) / 8) : 0;
 }
+int is_wide(std::initializer_list<uint64_t> parts) {
+    uint64_t bits = 0;
+    for (uint64_t v : parts) bits |= v;
+    return bits % 32 == 0 ? 1 : 0;
+}
+uint64_t addr(const void* p) { return reinterpret_cast<uintptr_t>(p); }
 
 }  // namespace
 
@@ -306,42 +342,47 @@ cudaError_t router_topk(const float* logits, int num_tokens, int num_experts, in
 cudaError_t quant_1x128(const void* x, int64_t x_stride_bytes, int rows, int hidden, bool pow2, void* out, float* scales,
                         int64_t sf_row_stride, int64_t sf_col_stride, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
-    if (hidden % 128 != 0) return cudaErrorInvalidValue;
-    quant_kernel<<<grid_for(static_cast<int64_t>(rows) * hidden / 8), 256, 0, stream>>>(
-        static_cast<const uint8_t*>(x), x_stride_bytes, rows, hidden, pow2, static_cast<uint8_t*>(out), scales, sf_row_stride, sf_col_stride);
+    const int columns = ceil_div(hidden, kSpan), blocks = span_blocks(rows, columns);
+    if (hidden % 128 != 0 || blocks == 0) return cudaErrorInvalidValue;
+    quant_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(x), x_stride_bytes, rows, hidden, columns,
+                                             is_wide({addr(x), static_cast<uint64_t>(x_stride_bytes)}), pow2, static_cast<uint8_t*>(out), scales,
+                                             sf_row_stride, sf_col_stride);
     return cudaGetLastError();
 }
 
-cudaError_t dequant_1x128(const void* q, const float* scales, int64_t sf_row_stride, int64_t sf_col_stride, int rows, int hidden, void* out,
-                          cudaStream_t stream) {
+cudaError_t dequant_1x128(const void* q, const float* scales, int64_t sf_row_stride, int64_t sf_col_stride, int rows, int hidden,
+                          const RowGroups& groups, void* out, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
-    if (hidden % 128 != 0) return cudaErrorInvalidValue;
-    dequant_kernel<<<grid_for(static_cast<int64_t>(rows) * hidden / 8), 256, 0, stream>>>(
-        static_cast<const uint8_t*>(q), scales, sf_row_stride, sf_col_stride, rows, hidden, static_cast<uint8_t*>(out));
+    const int columns = ceil_div(hidden, kSpan), blocks = span_blocks(rows, columns);
+    if (hidden % 128 != 0 || blocks == 0) return cudaErrorInvalidValue;
+    dequant_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(q), scales, sf_row_stride, sf_col_stride, rows, hidden, columns,
+                                               is_wide({addr(out)}), groups, static_cast<uint8_t*>(out));
     return cudaGetLastError();
 }
 
-cudaError_t swiglu(const void* x, int rows, int inter, const float* row_weight, const int* num_valid_rows, void* out, bool quant,
+cudaError_t swiglu(const void* x, int rows, int inter, const float* row_weight, const int* num_valid_rows, const RowGroups& groups, void* out, bool quant,
                    float* scales, int64_t sf_row_stride, int64_t sf_col_stride, bool pow2, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
-    if (inter % 8 != 0 || (quant && inter % 128 != 0)) return cudaErrorInvalidValue;
-    const int grid = grid_for(static_cast<int64_t>(rows) * inter / 8);
+    const int columns = ceil_div(inter, kSpan), blocks = span_blocks(rows, columns);
+    if (inter % 8 != 0 || (quant && inter % 128 != 0) || blocks == 0) return cudaErrorInvalidValue;
+    const int wide = is_wide({addr(x), addr(out), static_cast<uint64_t>(inter) * 2});
     if (quant)
-        swiglu_kernel<true><<<grid, 256, 0, stream>>>(static_cast<const uint8_t*>(x), rows, inter, row_weight, num_valid_rows,
-                                                      static_cast<uint8_t*>(out), scales, sf_row_stride, sf_col_stride, pow2 ? 1 : 0);
+        swiglu_kernel<true><<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
+                                                        static_cast<uint8_t*>(out), scales, sf_row_stride, sf_col_stride, pow2 ? 1 : 0);
     else
-        swiglu_kernel<false><<<grid, 256, 0, stream>>>(static_cast<const uint8_t*>(x), rows, inter, row_weight, num_valid_rows,
-                                                       static_cast<uint8_t*>(out), nullptr, 0, 0, 0);
+        swiglu_kernel<false><<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
+                                                         static_cast<uint8_t*>(out), nullptr, 0, 0, 0);
     return cudaGetLastError();
 }
 
-cudaError_t swiglu_backward(const void* x, const void* dout, int rows, int inter, const float* row_weight, void* dx, void* act_out,
+cudaError_t swiglu_backward(const void* x, const void* dout, int rows, int inter, const float* row_weight, const RowGroups& groups, void* dx, void* act_out,
                             float* dweight, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
     if (inter % 8 != 0) return cudaErrorInvalidValue;
-    swiglu_bwd_kernel<<<min(rows, 148 * 8), 256, 0, stream>>>(
-        static_cast<const uint8_t*>(x), static_cast<const uint8_t*>(dout), rows, inter, row_weight, static_cast<uint8_t*>(dx),
-        static_cast<uint8_t*>(act_out), dweight);
+    const int threads = std::min(128, align_up(ceil_div(inter, 16), 32));
+    const int wide = is_wide({addr(x), addr(dout), addr(dx), addr(act_out), static_cast<uint64_t>(inter) * 2});
+    swiglu_bwd_kernel<<<rows, threads, 0, stream>>>(static_cast<const uint8_t*>(x), static_cast<const uint8_t*>(dout), inter, wide, row_weight, groups,
+                                                    static_cast<uint8_t*>(dx), static_cast<uint8_t*>(act_out), dweight);
     return cudaGetLastError();
 }
 

@@ -39,7 +39,7 @@ int gemm_check_status() {
 
 at::Tensor gemm_impl(const at::Tensor& a, const at::Tensor& b, const std::optional<at::Tensor>& sfa, const std::optional<at::Tensor>& sfb,
                      const std::optional<at::Tensor>& group_end, int group_alignment, std::optional<at::Tensor> out, int num_sms,
-                     bool pow2_scales) {
+                     bool pow2_scales, bool zero_gap) {
     EP_HOST_ASSERT(a.is_cuda() && b.is_cuda() && a.dim() == 2 && a.stride(1) == 1 && b.stride(-1) == 1);
     EP_HOST_ASSERT(b.dim() == 2 || b.is_contiguous());
     const bool fp8 = a.scalar_type() == at::kFloat8_e4m3fn;
@@ -68,7 +68,7 @@ at::Tensor gemm_impl(const at::Tensor& a, const at::Tensor& b, const std::option
     p.num_groups = G;
     p.group_end = nullptr;
     p.group_alignment = std::max(group_alignment, 1);
-    p.zero_gap = (grouped && p.group_alignment % 128 == 0) ? 1 : 0;
+    p.zero_gap = (zero_gap && grouped && p.group_alignment % 128 == 0) ? 1 : 0;
     if (grouped) {
         EP_HOST_ASSERT(group_end.has_value() && group_end->scalar_type() == at::kInt && group_end->is_contiguous() && group_end->numel() >= G);
         p.group_end = group_end->data_ptr<int>();
@@ -154,19 +154,32 @@ std::tuple<at::Tensor, at::Tensor> quant_1x128(const at::Tensor& x, bool pow2, b
     return {q, sf};
 }
 
-at::Tensor dequant_1x128(const at::Tensor& q, const at::Tensor& sf) {
+// the row groups of an expanded dispatch (null = none)
+ops::RowGroups row_groups(const std::optional<at::Tensor>& group_end, int group_alignment) {
+    ops::RowGroups g;
+    if (!group_end.has_value()) return g;
+    EP_HOST_ASSERT(group_end->is_cuda() && group_end->scalar_type() == at::kInt && group_end->is_contiguous() && group_alignment >= 1);
+    g.ends = group_end->data_ptr<int>();
+    g.num = static_cast<int>(group_end->numel());
+    g.alignment = group_alignment;
+    return g;
+}
+
+at::Tensor dequant_1x128(const at::Tensor& q, const at::Tensor& sf, const std::optional<at::Tensor>& group_end, int group_alignment) {
     EP_HOST_ASSERT(q.is_cuda() && q.dim() == 2 && q.scalar_type() == at::kFloat8_e4m3fn && q.is_contiguous() && sf.scalar_type() == at::kFloat);
     c10::cuda::CUDAGuard guard(q.device());
     const int M = static_cast<int>(q.size(0)), H = static_cast<int>(q.size(1));
     EP_HOST_ASSERT(H % 128 == 0 && sf.size(0) == M && sf.size(1) == H / 128);
     auto out = at::empty({M, H}, q.options().dtype(at::kBFloat16));
-    CUDA_RUNTIME_CHECK(ops::dequant_1x128(q.data_ptr(), sf.data_ptr<float>(), sf.stride(0), sf.stride(1), M, H, out.data_ptr(), cur_stream()));
+    CUDA_RUNTIME_CHECK(ops::dequant_1x128(q.data_ptr(), sf.data_ptr<float>(), sf.stride(0), sf.stride(1), M, H, row_groups(group_end, group_alignment),
+                                          out.data_ptr(), cur_stream()));
     return out;
 }
 
 // returns (out, scales or None)
 std::tuple<at::Tensor, std::optional<at::Tensor>> swiglu(const at::Tensor& x, const std::optional<at::Tensor>& row_weight,
-                                                          const std::optional<at::Tensor>& num_valid_rows, bool quant, bool pow2) {
+                                                          const std::optional<at::Tensor>& num_valid_rows, bool quant, bool pow2,
+                                                          const std::optional<at::Tensor>& group_end, int group_alignment) {
     EP_HOST_ASSERT(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.size(1) % 16 == 0);
     c10::cuda::CUDAGuard guard(x.device());
     const int M = static_cast<int>(x.size(0)), I = static_cast<int>(x.size(1) / 2);
@@ -179,13 +192,14 @@ std::tuple<at::Tensor, std::optional<at::Tensor>> swiglu(const at::Tensor& x, co
     at::Tensor out = at::empty({M, I}, x.options().dtype(quant ? at::kFloat8_e4m3fn : at::kBFloat16));
     std::optional<at::Tensor> sf;
     if (quant) sf = at::empty({M, I / 128}, x.options().dtype(at::kFloat));
-    CUDA_RUNTIME_CHECK(ops::swiglu(x.data_ptr(), M, I, rw, nv, out.data_ptr(), quant, quant ? sf->data_ptr<float>() : nullptr,
+    CUDA_RUNTIME_CHECK(ops::swiglu(x.data_ptr(), M, I, rw, nv, row_groups(group_end, group_alignment), out.data_ptr(), quant, quant ? sf->data_ptr<float>() : nullptr,
                                    quant ? sf->stride(0) : 0, quant ? sf->stride(1) : 0, pow2, cur_stream()));
     return {out, sf};
 }
 
 // returns dx, or with `with_byproducts` (dx, weighted activation [rows, inter] bf16, gradient of the row weight [rows] fp32)
-py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const std::optional<at::Tensor>& row_weight, bool with_byproducts) {
+py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const std::optional<at::Tensor>& row_weight, bool with_byproducts,
+                           const std::optional<at::Tensor>& group_end, int group_alignment) {
     EP_HOST_ASSERT(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && dout.scalar_type() == at::kBFloat16 && dout.is_contiguous());
     c10::cuda::CUDAGuard guard(x.device());
     const int M = static_cast<int>(x.size(0)), I = static_cast<int>(x.size(1) / 2);
@@ -198,7 +212,7 @@ py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const st
         dweight = at::empty({M}, x.options().dtype(at::kFloat));
     }
     CUDA_RUNTIME_CHECK(ops::swiglu_backward(x.data_ptr(), dout.data_ptr(), M, I, row_weight.has_value() ? row_weight->data_ptr<float>() : nullptr,
-                                            dx.data_ptr(), with_byproducts ? act.data_ptr() : nullptr,
+                                            row_groups(group_end, group_alignment), dx.data_ptr(), with_byproducts ? act.data_ptr() : nullptr,
                                             with_byproducts ? dweight.data_ptr<float>() : nullptr, cur_stream()));
     if (with_byproducts) return py::make_tuple(dx, act, dweight);
     return py::cast(dx);
@@ -218,18 +232,19 @@ at::Tensor transpose_bf16(const at::Tensor& x) {
 void register_ops_bindings(py::module_& m) {
     m.def("router_topk", &router_topk);
     m.def("quant_1x128", &quant_1x128, py::arg("x"), py::arg("pow2") = false, py::arg("col_major_sf") = false);
-    m.def("dequant_1x128", &dequant_1x128);
+    m.def("dequant_1x128", &dequant_1x128, py::arg("q"), py::arg("sf"), py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
     m.def("swiglu", &swiglu, py::arg("x"), py::arg("row_weight") = py::none(), py::arg("num_valid_rows") = py::none(), py::arg("quant") = false,
-          py::arg("pow2") = false);
+          py::arg("pow2") = false, py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
     m.def("swiglu_backward", &swiglu_backward, py::arg("x"), py::arg("dout"), py::arg("row_weight") = py::none(),
-          py::arg("with_byproducts") = false);
+          py::arg("with_byproducts") = false, py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
     m.def("transpose_bf16", &transpose_bf16);
     m.def("gemm", &gemm_impl, py::arg("a"), py::arg("b"), py::arg("sfa") = py::none(), py::arg("sfb") = py::none(),
           py::arg("group_end") = py::none(), py::arg("group_alignment") = 1, py::arg("out") = py::none(), py::arg("num_sms") = 0,
-          py::arg("pow2_scales") = false,
+          py::arg("pow2_scales") = false, py::arg("zero_gap") = true,
           "C = A @ B^T on the tcgen05 tensor cores (bf16, or e4m3 with 1x128 / 128x128 block scales); 3-D B = grouped. "
           "pow2_scales: every scale is an exact power of two (round_scale quantisation), which lets the tensor core apply "
-          "them itself (kind::mxf8f6f4.block_scale) when N is a multiple of 256 and K at most 8192");
+          "them itself (kind::mxf8f6f4.block_scale) when N is a multiple of 256 and K at most 8192. "
+          "zero_gap: rows in the alignment gaps of a grouped problem are written as zeros (alignment a multiple of 128), else left alone");
     m.def("gemm_k_grouped", &gemm_k_grouped, py::arg("a"), py::arg("b"), py::arg("group_end"), py::arg("num_groups"),
           py::arg("group_alignment") = 128, py::arg("out") = py::none(), py::arg("num_sms") = 0,
           "C[g] = A[:, k range g] @ B[:, k range g]^T for all groups in one launch (bf16; the ranges come from a device array)");

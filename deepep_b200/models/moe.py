@@ -95,24 +95,26 @@ def moe_forward(comm, weights: Sequence[ExpertWeights], xs: Sequence[torch.Tenso
                 topk_weights: Sequence[torch.Tensor], cfg: MoEConfig):
     """Expert part of the layer for all ranks of ``comm``. Returns ``(ys, contexts)``."""
     R = len(xs)
+    # Rows in the alignment gaps between the experts mean nothing on the way forward: nobody reads their results, so nobody
+    # writes them. The backward pass contracts over rows and makes its own zeros there (for bf16 the dispatch does).
     out = comm.dispatch([dict(x=xs[r], topk_idx=topk_idx[r], topk_weights=topk_weights[r], num_experts=cfg.num_experts,
-                              expert_alignment=cfg.expert_alignment, do_expand=True, do_zero_padding=True, num_sms=cfg.num_sms,
+                              expert_alignment=cfg.expert_alignment, do_expand=True, do_zero_padding=not cfg.use_fp8, num_sms=cfg.num_sms,
                               fused_fp8=cfg.use_fp8, round_scale=cfg.use_fp8 and cfg.pow2_scales) for r in range(R)])
     ctxs, h2s = [], []
     for r in range(R):
         recv_x, _, recv_w, handle, _ = out[r]
         w = weights[r]
-        ends = handle.psum_num_recv_tokens_per_expert
+        groups = dict(group_end=handle.psum_num_recv_tokens_per_expert, group_alignment=cfg.expert_alignment)
         if cfg.use_fp8:
             xq, xsf = recv_x
             pow2 = cfg.pow2_scales and w.pow2_scales
-            h1 = _C.gemm(xq, w.w13_q, sfa=xsf, sfb=w.w13_sf, group_end=ends, group_alignment=cfg.expert_alignment, pow2_scales=pow2)
-            aq, asf = _C.swiglu(h1, recv_w, None, True, pow2)
-            h2 = _C.gemm(aq, w.w2_q, sfa=asf, sfb=w.w2_sf, group_end=ends, group_alignment=cfg.expert_alignment, pow2_scales=pow2)
+            h1 = _C.gemm(xq, w.w13_q, sfa=xsf, sfb=w.w13_sf, pow2_scales=pow2, zero_gap=False, **groups)
+            aq, asf = _C.swiglu(h1, recv_w, None, True, pow2, **groups)
+            h2 = _C.gemm(aq, w.w2_q, sfa=asf, sfb=w.w2_sf, pow2_scales=pow2, zero_gap=False, **groups)
         else:
-            h1 = _C.gemm(recv_x, w.w13, group_end=ends, group_alignment=cfg.expert_alignment)
-            a, _ = _C.swiglu(h1, recv_w)
-            h2 = _C.gemm(a, w.w2, group_end=ends, group_alignment=cfg.expert_alignment)
+            h1 = _C.gemm(recv_x, w.w13, zero_gap=False, **groups)
+            a, _ = _C.swiglu(h1, recv_w, **groups)
+            h2 = _C.gemm(a, w.w2, zero_gap=False, **groups)
         h2s.append(h2)
         ctxs.append(dict(recv_x=recv_x, recv_w=recv_w, handle=handle, h1=h1))
     comb = comm.combine([dict(x=h2s[r], handle=ctxs[r]['handle']) for r in range(R)])
@@ -137,15 +139,16 @@ def moe_backward(comm, weights: Sequence[ExpertWeights], ctxs, dys: Sequence[tor
         c, w = ctxs[r], weights[r]
         handle, h1, recv_w = c['handle'], c['h1'], c['recv_w']
         ends = handle.psum_num_recv_tokens_per_expert
+        groups = dict(group_end=ends, group_alignment=cfg.expert_alignment)
         el = w.w13.size(0)
         x_rows = c['recv_x']
         if cfg.use_fp8:
-            x_rows = _C.dequant_1x128(x_rows[0], x_rows[1].contiguous())
-        # data gradients
-        da = _C.gemm(dh2, w.w2_t, group_end=ends, group_alignment=cfg.expert_alignment)           # [rows, I]
-        dh1, a_w, dw_row = _C.swiglu_backward(h1, da, recv_w, True)                                 # [rows, 2I], [rows, I], [rows]
+            x_rows = _C.dequant_1x128(x_rows[0], x_rows[1], **groups)
+        # data gradients (zeros in the gaps come from the SwiGLU backward: the contractions below run over the rows)
+        da = _C.gemm(dh2, w.w2_t, zero_gap=False, **groups)                                         # [rows, I]
+        dh1, a_w, dw_row = _C.swiglu_backward(h1, da, recv_w, True, **groups)                       # [rows, 2I], [rows, I], [rows]
         dw_rows.append(dw_row)
-        dx_rows.append(_C.gemm(dh1, w.w13_t, group_end=ends, group_alignment=cfg.expert_alignment))
+        dx_rows.append(_C.gemm(dh1, w.w13_t, zero_gap=False, **groups))
         # weight gradients: contraction over every expert's (zero padded) rows, all experts in one launch each
         dh2_t, a_t = _C.transpose_bf16(dh2), _C.transpose_bf16(a_w)
         dh1_t, x_t = _C.transpose_bf16(dh1), _C.transpose_bf16(x_rows)

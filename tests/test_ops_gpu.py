@@ -93,3 +93,37 @@ def test_transpose_interior_edge_and_unaligned(rows, cols):
     if cols > 8:     # a view whose rows start 2 bytes off a 16-byte boundary
         v = x[:, 1:]
         assert torch.equal(C.transpose_bf16(v), v.t().contiguous())
+
+
+@pytest.mark.parametrize('I', [24, 384, 640])       # one lane with half its channels, a partial column, a column and a quarter
+def test_streaming_ops_skip_or_zero_alignment_gaps(I):
+    """Rows of the expanded layout behind their expert's end: the forward kernel leaves them alone, the backward kernels
+    write zeros there, whatever the inputs hold in them."""
+    import deepep_b200
+    C = deepep_b200._C
+    g = torch.Generator(device='cuda').manual_seed(5)
+    align, ends_list = 16, [5, 16, 16, 49]          # a ragged group, a full one, an empty one, one that ends behind a full tile
+    ends = torch.tensor(ends_list, dtype=torch.int32, device='cuda')
+    M = 80                                           # rows past the last group's aligned end as well
+    valid = torch.zeros(M, dtype=torch.bool, device='cuda')
+    start = 0
+    for e in ends_list:
+        valid[start:e] = True
+        start = -(-e // align) * align
+    x = torch.randn((M, 2 * I), device='cuda', generator=g).bfloat16()
+    dout = torch.randn((M, I), device='cuda', generator=g).bfloat16()
+    rw = torch.rand(M, device='cuda', generator=g)
+    full, _ = C.swiglu(x, rw)
+    dx0, act0, dw0 = C.swiglu_backward(x, dout, rw, True)
+    bad = x.clone()
+    bad[~valid] = float('nan')
+    out, _ = C.swiglu(bad, rw, group_end=ends, group_alignment=align)
+    assert torch.equal(out[valid], full[valid])
+    dx, act, dw = C.swiglu_backward(bad, dout, rw, True, group_end=ends, group_alignment=align)
+    assert torch.equal(dx[valid], dx0[valid]) and torch.equal(act[valid], act0[valid]) and torch.equal(dw[valid], dw0[valid])
+    assert (dx[~valid] == 0).all() and (act[~valid] == 0).all() and (dw[~valid] == 0).all()
+    if I % 128 == 0:
+        q, sf = C.quant_1x128(dout)
+        q.view(torch.uint8)[~valid] = 0x7f          # NaN
+        back = C.dequant_1x128(q, sf, group_end=ends, group_alignment=align)
+        assert torch.equal(back[valid], C.dequant_1x128(*C.quant_1x128(dout))[valid]) and (back[~valid] == 0).all()
