@@ -252,7 +252,7 @@ constexpr int kPadRows = 4;                 // padding rows per zeroing work ite
 // also write the tokens' routing words. The slice is requested before the plan is awaited (the input was there before the
 // plan kernel started).
 template <bool kQuant, bool kExpand>
-__global__ void __launch_bounds__(kMoveThreads) local_move_kernel(const __grid_constant__ LocalMoveParams p) {
+__global__ void __launch_bounds__(kMoveThreads, kExpand ? 6 : 8) local_move_kernel(const __grid_constant__ LocalMoveParams p) {
     const int lane = lane_id();
     const int K = p.num_topk, T = p.num_tokens;
     const uint32_t warp_global = blockIdx.x * (kMoveThreads / 32) + warp_id(), num_warps = gridDim.x * (kMoveThreads / 32);
@@ -403,6 +403,31 @@ constexpr int kCombineThreads = 128;
 // bytes: 121 us for 32768 rows of hidden 7168 against 81 us that the bytes take). NR rows x NV vectors = up to 128 bytes are
 // in flight per lane before the first add; the rows of the next token are looked up meanwhile. The adds run in ascending
 // top-k order.
+// One row per token and nothing to add: the row is the result. One warp per KB of a row, as in the move kernel (in the
+// kernel below, whose registers leave a third of the warps resident, the same copy took 45 instead of 39 us).
+__global__ void __launch_bounds__(256, 8) local_return_kernel(const __grid_constant__ LocalCombineParams p) {
+    const int lane = lane_id(), K = p.num_topk;
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.timeline[0] = globaltimer_ns();
+    const uint32_t warp_global = blockIdx.x * 8 + warp_id();
+    const int t = static_cast<int>(warp_global / static_cast<uint32_t>(p.columns)), col = static_cast<int>(warp_global % static_cast<uint32_t>(p.columns));
+    if (t < p.num_tokens) {
+        int row = p.token_slot[t];
+        if (row >= p.num_x_rows) row = -1;
+        const int off = col * 1024 + lane * 32;
+        int4 lo = make_int4(0, 0, 0, 0), hi = lo;
+        if (row >= 0) load_32(p.x + static_cast<int64_t>(row) * p.x_stride_bytes + off, p.row_bytes - off, p.wide != 0, lo, hi);
+        store_32(p.combined_x + static_cast<int64_t>(t) * p.row_bytes + off, p.row_bytes - off, p.wide != 0, lo, hi);
+        if (col == 0 && p.combined_topk_weights != nullptr && lane < K) {
+            float v = 0.f;
+            if (p.topk_weights != nullptr && row >= 0 && load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + lane, p.num_experts) >= 0)
+                v = p.topk_weights[static_cast<int64_t>(row) * K + lane];
+            p.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = v;
+        }
+    }
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1)
+        atomicMax(reinterpret_cast<unsigned long long*>(p.timeline + 1), static_cast<unsigned long long>(globaltimer_ns()));
+}
+
 template <int NV, int NR, bool kExpand, bool kWeighted>
 __global__ void __launch_bounds__(kCombineThreads) local_combine_kernel(const __grid_constant__ LocalCombineParams p) {
     const int lane = lane_id();
@@ -433,17 +458,6 @@ __global__ void __launch_bounds__(kCombineThreads) local_combine_kernel(const __
                     v = p.topk_weights[static_cast<int64_t>(row) * K + lane];
             }
             p.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = v;
-        }
-        if (!kExpand && p.bias0 == nullptr && p.bias1 == nullptr) {
-            // one row per token and nothing to add: the row is the result
-            const uint8_t* src = p.x + static_cast<int64_t>(row) * p.x_stride_bytes;
-            int4 raw[NV];
-#pragma unroll
-            for (int j = 0; j < NV; ++j) raw[j] = row >= 0 && v0 + 32 * j < vec_per_row ? ld_nc_int4(src + (v0 + 32 * j) * 16) : make_int4(0, 0, 0, 0);
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (v0 + 32 * j < vec_per_row) st_na_int4(dst + (v0 + 32 * j) * 16, raw[j]);
-            continue;
         }
         const uint32_t rows = kExpand ? __ballot_sync(0xffffffffu, row >= 0) : (row >= 0 ? 1u : 0u);
         const float wt = kWeighted && row >= 0 ? p.topk_weights[row] : 0.f;
@@ -594,16 +608,25 @@ static cudaError_t launch_combine_cfg(LocalCombineParams& p, int num_sms, cudaSt
     if (err != cudaSuccess) return err;
     const int warps_per_block = kCombineThreads / 32, most = num_sms * resident_blocks(kernel, kCombineThreads, per_sm) * warps_per_block;
     p.columns = ceil_div(p.row_bytes / 16, 32 * NV);
-    p.warps = kExpand ? balanced_warps(p.num_tokens, p.columns, most) : p.num_tokens * p.columns;
+    p.warps = balanced_warps(p.num_tokens, p.columns, most);
     return launch_plain(kernel, p, ceil_div(p.warps, warps_per_block), kCombineThreads, stream, false);
 }
 
 cudaError_t launch_local_combine(const LocalCombineParams& params, int num_sms, cudaStream_t stream) {
     if (params.num_tokens == 0) return cudaSuccess;
     LocalCombineParams p = params;
-    // One row per token: one warp per KB of a row, each does it once (see the move kernel). Several rows: a resident grid,
-    // since looking up the rows of a token is a chain of two loads that the loop hides; up to four rows two vectors at a
-    // time, more than four one (128 bytes in flight per lane either way).
+    if (!p.do_expand && p.bias0 == nullptr && p.bias1 == nullptr) {
+        static PreparedKernel prepared;
+        const cudaError_t err = prepared.prepare(local_return_kernel, 0);
+        if (err != cudaSuccess) return err;
+        p.columns = ceil_div(p.row_bytes, 1024);
+        p.wide = (reinterpret_cast<uintptr_t>(p.x) | static_cast<uint64_t>(p.x_stride_bytes) | reinterpret_cast<uintptr_t>(p.combined_x) | static_cast<uint64_t>(p.row_bytes)) % 32 == 0;
+        const int64_t warps = static_cast<int64_t>(p.num_tokens) * p.columns;
+        if (warps >= (1ll << 31)) return cudaErrorInvalidValue;
+        return launch_plain(local_return_kernel, p, static_cast<int>(ceil_div<int64_t>(warps, 8)), 256, stream, false);
+    }
+    // Otherwise a resident grid, since looking up the rows of a token is a chain of two loads that the loop hides; up to four
+    // rows two vectors at a time, more than four one (128 bytes in flight per lane either way).
     if (!p.do_expand) return launch_combine_cfg<2, 1, false, false>(p, num_sms, stream);
     if (p.num_topk <= 4) return p.weighted ? launch_combine_cfg<2, 4, true, true>(p, num_sms, stream) : launch_combine_cfg<2, 4, true, false>(p, num_sms, stream);
     return p.weighted ? launch_combine_cfg<1, 8, true, true>(p, num_sms, stream) : launch_combine_cfg<1, 8, true, false>(p, num_sms, stream);
