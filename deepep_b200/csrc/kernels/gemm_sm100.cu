@@ -8,6 +8,7 @@
 // the all-gather -> GEMM / GEMM -> reduce-scatter operators (tp_fused.cu).
 #include <cstdlib>
 
+#include "api.hpp"
 #include "gemm_api.hpp"
 #include "gemm_sm100.cuh"
 
@@ -51,7 +52,7 @@ struct Scheduler {
             return true;
         }
         out.kb0 = 0;
-        out.kb1 = p.K / BK;
+        out.kb1 = ceil_div(p.K, BK);      // (only an MN-major problem may end inside a k-block: its missing rows load as zeros)
         while (g < p.num_groups) {
             const int rows = max(end - start, 0);
             const int tiles_m = ceil_div(rows, BM);
@@ -95,7 +96,25 @@ struct Cfg {
     static constexpr int kTmemCols = kAccStages * BN;
 };
 
-template <int BN, bool kFp8>
+// Loads one operand tile of `rows` rows (K-major: one box) or `rows` columns of a [K, MN] matrix (MN-major: boxes of 64 x 64).
+template <bool kMN>
+__device__ __forceinline__ void load_operand(uint8_t* dst, const CUtensorMap* map, int k, int mn, int rows, uint64_t* bar) {
+    if constexpr (!kMN) {
+        tma_load_2d(dst, map, k, mn, bar);
+    } else {
+        for (int i = 0; i < rows / 64; ++i) tma_load_2d(dst + i * 8192, map, mn + i * 64, k, bar);
+    }
+}
+template <bool kMN>
+__device__ __forceinline__ void load_operand_pair(uint8_t* dst, const CUtensorMap* map, int k, int mn, int rows, uint32_t bar) {
+    if constexpr (!kMN) {
+        tma_load_2d_pair(dst, map, k, mn, bar);
+    } else {
+        for (int i = 0; i < rows / 64; ++i) tma_load_2d_pair(dst + i * 8192, map, mn + i * 64, k, bar);
+    }
+}
+
+template <int BN, bool kFp8, bool kAMN = false, bool kBMN = false>
 __global__ void __launch_bounds__(Cfg<BN, kFp8>::kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
     using C = Cfg<BN, kFp8>;
@@ -144,13 +163,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             uint32_t ph = 0;
             bool ok = true;
             for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
-                const int b_row = (p.k_grouped ? 0 : t.g * p.N) + t.n0;
+                // (an MN-major B of a plain problem; group g of a grouped one starts at row g * K of the stacked [K, N] matrices)
+                const int b_row = (p.k_grouped || kBMN ? 0 : t.g * p.N) + t.n0, b_k = kBMN && !p.k_grouped ? t.g * p.K : 0;
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
                     if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
                     uint8_t* sa = smem + s * C::STAGE;
                     mbar_arrive_expect_tx(full + s, C::STAGE);
-                    tma_load_2d(sa, &map_a, kb * C::BK, t.m0, full + s);
-                    tma_load_2d(sa + C::A_BYTES, &map_b, kb * C::BK, b_row, full + s);
+                    load_operand<kAMN>(sa, &map_a, kb * C::BK, t.m0, BM, full + s);
+                    load_operand<kBMN>(sa + C::A_BYTES, &map_b, b_k + kb * C::BK, b_row, BN, full + s);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
             }
@@ -160,7 +180,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (lane == 0) {
             Scheduler sched(p, BN, BM, C::BK);
             Tile t;
-            constexpr uint32_t idesc = make_idesc<kFp8>(BM, BN);
+            constexpr uint32_t idesc = make_idesc<kFp8>(BM, BN, kAMN, kBMN);
             int s = 0, acc = 0;
             uint32_t ph = 0, acc_ph = 0;
             bool ok = true;
@@ -176,12 +196,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     if (!(ok = pipe_wait(pc, full + s, ph))) break;
                     tc_fence_after();
                     const uint8_t* sa = smem + s * C::STAGE;
-                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + C::A_BYTES);
+                    const uint64_t da = kAMN ? make_smem_desc_mn(sa) : make_smem_desc(sa);
+                    const uint64_t db = kBMN ? make_smem_desc_mn(sa + C::A_BYTES) : make_smem_desc(sa + C::A_BYTES);
                     const uint32_t d_addr = tmem_base + acc * BN;
 #pragma unroll
                     for (int k = 0; k < C::BK / C::UMMA_K; ++k) {
                         const uint32_t accumulate = kFp8 ? (k != 0) : (kb != t.kb0 || k != 0);
-                        umma<kFp8>(d_addr, da + 2 * k, db + 2 * k, idesc, accumulate);
+                        umma<kFp8>(d_addr, da + (kAMN ? 128 : 2) * k, db + (kBMN ? 128 : 2) * k, idesc, accumulate);
                     }
                     umma_commit(empty + s);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
@@ -228,20 +249,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
                         for (int i = 0; i < 32; ++i) r[i] = 0u;
                     }
-                    if (row_ok) {
+                    if (zero_row) {
 #pragma unroll
-                        for (int v = 0; v < 4; ++v) {
-                            int4 out;
-                            __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                o2[i] = __floats2bfloat162_rn(__uint_as_float(r[v * 8 + 2 * i]), __uint_as_float(r[v * 8 + 2 * i + 1]));
-                            *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = out;
-                        }
-                    } else if (zero_row) {
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = make_int4(0, 0, 0, 0);
+                        for (int i = 0; i < 32; ++i) r[i] = 0u;
                     }
+                    if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
                 }
                 tc_fence_before();
                 mbar_arrive(tmem_empty + acc);
@@ -315,6 +327,7 @@ struct PairCfg {
     static constexpr int kTmemCols = kAccStages * BN;
 };
 
+template <bool kAMN, bool kBMN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
     using C = PairCfg;
@@ -364,14 +377,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             uint32_t ph = 0;
             bool ok = true;
             for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
-                const int b_row = (p.k_grouped ? 0 : t.g * p.N) + t.n0 + static_cast<int>(cta) * (C::BN / 2);
+                const int b_row = (p.k_grouped || kBMN ? 0 : t.g * p.N) + t.n0 + static_cast<int>(cta) * (C::BN / 2);
+                const int b_k = kBMN && !p.k_grouped ? t.g * p.K : 0;
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
                     if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
                     uint8_t* sa = smem + s * C::STAGE;
                     if (leader) mbar_arrive_expect_tx(full + s, 2 * C::STAGE);
                     const uint32_t bar = map_to_cta(smem_u32(full + s), 0);
-                    tma_load_2d_pair(sa, &map_a, kb * C::BK, t.m0 + static_cast<int>(cta) * BM, bar);
-                    tma_load_2d_pair(sa + C::A_BYTES, &map_b, kb * C::BK, b_row, bar);
+                    load_operand_pair<kAMN>(sa, &map_a, kb * C::BK, t.m0 + static_cast<int>(cta) * BM, BM, bar);
+                    load_operand_pair<kBMN>(sa + C::A_BYTES, &map_b, b_k + kb * C::BK, b_row, C::BN / 2, bar);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
             }
@@ -381,7 +395,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (leader && lane == 0) {
             Scheduler sched(p, C::BN, 2 * BM, C::BK);
             Tile t;
-            constexpr uint32_t idesc = make_idesc<false>(2 * BM, C::BN);
+            constexpr uint32_t idesc = make_idesc<false>(2 * BM, C::BN, kAMN, kBMN);
             int s = 0, acc = 0;
             uint32_t ph = 0, acc_ph = 0;
             bool ok = true;
@@ -392,10 +406,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     if (!(ok = pipe_wait(pc, full + s, ph))) break;
                     tc_fence_after();
                     const uint8_t* sa = smem + s * C::STAGE;
-                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + C::A_BYTES);
+                    const uint64_t da = kAMN ? make_smem_desc_mn(sa) : make_smem_desc(sa);
+                    const uint64_t db = kBMN ? make_smem_desc_mn(sa + C::A_BYTES) : make_smem_desc(sa + C::A_BYTES);
                     const uint32_t d_addr = tmem_base + acc * C::BN;
 #pragma unroll
-                    for (int k = 0; k < C::BK / C::UMMA_K; ++k) umma_pair_bf16(d_addr, da + 2 * k, db + 2 * k, idesc, kb != t.kb0 || k != 0);
+                    for (int k = 0; k < C::BK / C::UMMA_K; ++k)
+                        umma_pair_bf16(d_addr, da + (kAMN ? 128 : 2) * k, db + (kBMN ? 128 : 2) * k, idesc, kb != t.kb0 || k != 0);
                     umma_commit_pair(empty + s);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
@@ -435,20 +451,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                     for (int i = 0; i < 32; ++i) r[i] = 0u;
                 }
-                if (row_ok) {
+                if (zero_row) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        int4 out;
-                        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            o2[i] = __floats2bfloat162_rn(__uint_as_float(r[v * 8 + 2 * i]), __uint_as_float(r[v * 8 + 2 * i + 1]));
-                        *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = out;
-                    }
-                } else if (zero_row) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = make_int4(0, 0, 0, 0);
+                    for (int i = 0; i < 32; ++i) r[i] = 0u;
                 }
+                if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
             }
             tc_fence_before();
             mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty + acc), 0));
@@ -770,20 +777,11 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 uint32_t r[32];
                 tmem_ld_32x32(lane_addr + c * 32, r);
                 tmem_ld_wait();
-                if (row_ok) {
+                if (zero_row) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        int4 out;
-                        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            o2[i] = __floats2bfloat162_rn(__uint_as_float(r[v * 8 + 2 * i]), __uint_as_float(r[v * 8 + 2 * i + 1]));
-                        *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = out;
-                    }
-                } else if (zero_row) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = make_int4(0, 0, 0, 0);
+                    for (int i = 0; i < 32; ++i) r[i] = 0u;
                 }
+                if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
             }
             tc_fence_before();
             __syncwarp();
@@ -1002,20 +1000,11 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 uint32_t r[32];
                 tmem_ld_32x32(lane_addr + c * 32, r);
                 tmem_ld_wait();
-                if (row_ok) {
+                if (zero_row) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        int4 out;
-                        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            o2[i] = __floats2bfloat162_rn(__uint_as_float(r[v * 8 + 2 * i]), __uint_as_float(r[v * 8 + 2 * i + 1]));
-                        *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = out;
-                    }
-                } else if (zero_row) {
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) *reinterpret_cast<int4*>(c_row + c * 32 + v * 8) = make_int4(0, 0, 0, 0);
+                    for (int i = 0; i < 32; ++i) r[i] = 0u;
                 }
+                if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
             }
             tc_fence_before();
             __syncwarp();
@@ -1138,80 +1127,78 @@ bool make_kmajor_map(CUtensorMap* map, const void* base, int elem_bytes, uint64_
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool kFp8>
-static cudaError_t launch_cfg(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int num_sms, cudaStream_t stream) {
-    using C = Cfg<BN, kFp8>;
-    cudaError_t err = cudaFuncSetAttribute(gemm_kernel<BN, kFp8>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+namespace {
+
+template <auto kKernel, typename C>
+cudaError_t launch_tiles(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int grid, cudaStream_t stream) {
+    static PreparedKernel prepared;
+    const cudaError_t err = prepared.prepare(kKernel, C::kSmem);
     if (err != cudaSuccess) return err;
-    gemm_kernel<BN, kFp8><<<num_sms, C::kThreads, C::kSmem, stream>>>(map_a, map_b, p);
+    kKernel<<<grid, C::kThreads, C::kSmem, stream>>>(map_a, map_b, p);
     return cudaGetLastError();
 }
 
-cudaError_t launch_gemm(const GemmParams& p, const void* a, int64_t a_row_stride_bytes, const void* b, int64_t b_row_stride_bytes,
+bool env_is(const char* name, char value) {
+    const char* v = std::getenv(name);
+    return v != nullptr && v[0] == value;
+}
+
+}  // namespace
+
+cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_stride_bytes, const void* b, int64_t b_row_stride_bytes,
                         bool fp8, int num_sms, cudaStream_t stream) {
+    GemmParams p = params;
     const int elem = fp8 ? 1 : 2;
+    p.c_wide = (reinterpret_cast<uintptr_t>(p.C) | static_cast<uint64_t>(p.ldc) * 2 | static_cast<uint64_t>(p.c_group_stride) * 2) % 32 == 0;
     // bf16 with 256-wide tiles runs on CTA pairs (EP_GEMM_CTA_PAIR=0 keeps one CTA per tile); a pair needs two SMs.
     // e4m3 on CTA pairs is opt-in (EP_GEMM_FP8_PAIR=1): with software block scaling the 256 x 256 tile halves the
     // shared-memory fill per flop, but only two accumulator passes fit into tensor memory and the drain of a pass
     // (64 columns per epilogue thread) then sets the pace: 0.94 PFLOP/s measured against 1.3 with 128 x 128 tiles and
     // four passes in flight.
-    const char* pair_env = std::getenv("EP_GEMM_CTA_PAIR");
-    const char* fp8_pair_env = std::getenv("EP_GEMM_FP8_PAIR");
-    const bool pair_enabled = fp8 ? (fp8_pair_env != nullptr && fp8_pair_env[0] == '1') : (pair_env == nullptr || pair_env[0] != '0');
+    const bool pair_enabled = fp8 ? env_is("EP_GEMM_FP8_PAIR", '1') : !env_is("EP_GEMM_CTA_PAIR", '0');
     const bool use_pair = p.N % 256 == 0 && pair_enabled && num_sms >= 2;
     const int bn = fp8 ? (use_pair ? 256 : 128) : ((p.N % 256 == 0) ? 256 : 128);
     const int bk = fp8 ? 128 : 64;
-    if (p.N % bn != 0 || p.K % bk != 0 || p.M <= 0) return cudaErrorInvalidValue;
+    const bool k_tail_ok = p.a_mn && p.b_mn && !p.k_grouped && p.num_groups == 1;     // rows past the end load as zeros
+    if (p.N % bn != 0 || (p.K % bk != 0 && !k_tail_ok) || p.M <= 0) return cudaErrorInvalidValue;
     if (p.k_grouped && (fp8 || p.group_end == nullptr || p.group_alignment % bk != 0)) return cudaErrorInvalidValue;
+    if ((p.a_mn || p.b_mn) && (fp8 || (p.a_mn && !p.b_mn))) return cudaErrorInvalidValue;
+    const uint64_t K = static_cast<uint64_t>(p.K), a_stride = static_cast<uint64_t>(a_row_stride_bytes), b_stride = static_cast<uint64_t>(b_row_stride_bytes);
+    const uint64_t b_mats = p.k_grouped ? 1 : static_cast<uint64_t>(p.num_groups);
+    // operand maps: K-major [rows, K] in boxes of `box` rows, or MN-major [K, columns] in boxes of 64 x 64
+    auto map_of = [&](CUtensorMap* map, const void* base, bool mn, uint64_t rows, uint64_t mats, uint64_t stride, uint32_t box) {
+        return mn ? make_kmajor_map(map, base, elem, mats * K, rows, stride, 64) : make_kmajor_map(map, base, elem, mats * rows, K, stride, box);
+    };
     CUtensorMap map_a, map_b;
-    if (!make_kmajor_map(&map_a, a, elem, static_cast<uint64_t>(p.M), static_cast<uint64_t>(p.K), static_cast<uint64_t>(a_row_stride_bytes), BM) ||
-        !make_kmajor_map(&map_b, b, elem, static_cast<uint64_t>(p.num_groups) * p.N, static_cast<uint64_t>(p.K),
-                         static_cast<uint64_t>(b_row_stride_bytes), static_cast<uint32_t>(use_pair ? bn / 2 : bn)))
-        return cudaErrorInvalidValue;
+    if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM)) return cudaErrorInvalidValue;
     // e4m3 with power-of-two scales: the block-scaled instruction kind (EP_GEMM_FP8_MX=0 keeps the software scaling)
-    const char* mx_env = std::getenv("EP_GEMM_FP8_MX");
-    const bool mx_enabled = mx_env == nullptr || mx_env[0] != '0';
-    if (fp8 && p.scales_pow2 && mx_enabled && !use_pair && p.N % 256 == 0 && p.K / 128 <= MxCfg::kMaxKb && !p.k_grouped) {
+    if (fp8 && p.scales_pow2 && !env_is("EP_GEMM_FP8_MX", '0') && !use_pair && p.N % 256 == 0 && p.K / 128 <= MxCfg::kMaxKb && !p.k_grouped) {
         // CTA pairs (EP_GEMM_FP8_MX_PAIR=1): 256 x 256 tiles, each CTA loads 128 rows of A and 128 of B. Opt-in: measured
         // no faster than lone CTAs (2.21 against 2.16 PFLOP/s), so the fill of shared memory from L2 is not what limits
         // the lone-CTA kernel; per k-block a CTA's shared memory takes 48 KB from TMA and hands 48 KB to the tensor
         // core in 541 tensor-pipe cycles either way, more than its 128 bytes per cycle.
-        const char* mx_pair_env = std::getenv("EP_GEMM_FP8_MX_PAIR");
-        const bool mx_pair = mx_pair_env != nullptr && mx_pair_env[0] == '1';
-        if (mx_pair && num_sms >= 2) {
-            CUtensorMap map_b128;
-            if (!make_kmajor_map(&map_b128, b, elem, static_cast<uint64_t>(p.num_groups) * p.N, static_cast<uint64_t>(p.K),
-                                 static_cast<uint64_t>(b_row_stride_bytes), 128))
-                return cudaErrorInvalidValue;
-            cudaError_t err = cudaFuncSetAttribute(gemm_mx_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MxPairCfg::kSmem);
-            if (err != cudaSuccess) return err;
-            gemm_mx_pair_kernel<<<num_sms & ~1, MxPairCfg::kThreads, MxPairCfg::kSmem, stream>>>(map_a, map_b128, p);
-            return cudaGetLastError();
-        }
-        CUtensorMap map_b256;
-        if (!make_kmajor_map(&map_b256, b, elem, static_cast<uint64_t>(p.num_groups) * p.N, static_cast<uint64_t>(p.K),
-                             static_cast<uint64_t>(b_row_stride_bytes), 256))
-            return cudaErrorInvalidValue;
-        cudaError_t err = cudaFuncSetAttribute(gemm_mx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MxCfg::kSmem);
-        if (err != cudaSuccess) return err;
-        gemm_mx_kernel<<<num_sms, MxCfg::kThreads, MxCfg::kSmem, stream>>>(map_a, map_b256, p);
-        return cudaGetLastError();
+        const bool mx_pair = env_is("EP_GEMM_FP8_MX_PAIR", '1') && num_sms >= 2;
+        if (!map_of(&map_b, b, false, static_cast<uint64_t>(p.N), b_mats, b_stride, mx_pair ? 128 : 256)) return cudaErrorInvalidValue;
+        return mx_pair ? launch_tiles<gemm_mx_pair_kernel, MxPairCfg>(map_a, map_b, p, num_sms & ~1, stream)
+                       : launch_tiles<gemm_mx_kernel, MxCfg>(map_a, map_b, p, num_sms, stream);
     }
-    if (fp8 && use_pair) {
-        cudaError_t err = cudaFuncSetAttribute(gemm_pair_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairFp8Cfg::kSmem);
-        if (err != cudaSuccess) return err;
-        gemm_pair_fp8_kernel<<<num_sms & ~1, PairFp8Cfg::kThreads, PairFp8Cfg::kSmem, stream>>>(map_a, map_b, p);
-        return cudaGetLastError();
-    }
-    if (fp8) return launch_cfg<128, true>(map_a, map_b, p, num_sms, stream);
+    if (!map_of(&map_b, b, p.b_mn != 0, static_cast<uint64_t>(p.N), b_mats, b_stride, static_cast<uint32_t>(use_pair ? bn / 2 : bn))) return cudaErrorInvalidValue;
+    if (fp8 && use_pair) return launch_tiles<gemm_pair_fp8_kernel, PairFp8Cfg>(map_a, map_b, p, num_sms & ~1, stream);
+    if (fp8) return launch_tiles<gemm_kernel<128, true>, Cfg<128, true>>(map_a, map_b, p, num_sms, stream);
     if (bn == 256 && use_pair) {
-        cudaError_t err = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kSmem);
-        if (err != cudaSuccess) return err;
-        gemm_pair_kernel<<<num_sms & ~1, PairCfg::kThreads, PairCfg::kSmem, stream>>>(map_a, map_b, p);
-        return cudaGetLastError();
+        const int grid = num_sms & ~1;
+        if (p.a_mn) return launch_tiles<gemm_pair_kernel<true, true>, PairCfg>(map_a, map_b, p, grid, stream);
+        return p.b_mn ? launch_tiles<gemm_pair_kernel<false, true>, PairCfg>(map_a, map_b, p, grid, stream)
+                      : launch_tiles<gemm_pair_kernel<false, false>, PairCfg>(map_a, map_b, p, grid, stream);
     }
-    if (bn == 256) return launch_cfg<256, false>(map_a, map_b, p, num_sms, stream);
-    return launch_cfg<128, false>(map_a, map_b, p, num_sms, stream);
+    if (bn == 256) {
+        if (p.a_mn) return launch_tiles<gemm_kernel<256, false, true, true>, Cfg<256, false>>(map_a, map_b, p, num_sms, stream);
+        return p.b_mn ? launch_tiles<gemm_kernel<256, false, false, true>, Cfg<256, false>>(map_a, map_b, p, num_sms, stream)
+                      : launch_tiles<gemm_kernel<256, false>, Cfg<256, false>>(map_a, map_b, p, num_sms, stream);
+    }
+    if (p.a_mn) return launch_tiles<gemm_kernel<128, false, true, true>, Cfg<128, false>>(map_a, map_b, p, num_sms, stream);
+    return p.b_mn ? launch_tiles<gemm_kernel<128, false, false, true>, Cfg<128, false>>(map_a, map_b, p, num_sms, stream)
+                  : launch_tiles<gemm_kernel<128, false>, Cfg<128, false>>(map_a, map_b, p, num_sms, stream);
 }
 
 }  // namespace gemm

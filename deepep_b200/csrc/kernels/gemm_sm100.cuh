@@ -243,16 +243,54 @@ __device__ __forceinline__ uint64_t make_smem_desc(const void* smem_tile) {
     return desc;
 }
 
-// Instruction descriptor: D fp32, A/B bf16 (kind::f16) or e4m3 (kind::f8f6f4), both K-major.
+// The same for an MN-major bf16 tile, which is what a row-major [K, MN] matrix gives: boxes of 64 (MN) x 64 (K) elements, a
+// row of a box is one swizzle span of 64 consecutive MN elements, eight rows of K make a 1024-byte atom. Atoms along K are
+// 1024 bytes apart (stride byte offset), the boxes of the next 64 MN elements 8192 bytes (leading byte offset). One K step of
+// 16 is two atoms.
+__device__ __forceinline__ uint64_t make_smem_desc_mn(const void* smem_tile) {
+    const uint32_t addr = smem_u32(smem_tile);
+    uint64_t desc = 0;
+    desc |= static_cast<uint64_t>((addr & 0x3ffff) >> 4);
+    desc |= static_cast<uint64_t>(8192 >> 4) << 16;
+    desc |= static_cast<uint64_t>(1024 >> 4) << 32;
+    desc |= static_cast<uint64_t>(1) << 46;
+    desc |= static_cast<uint64_t>(2) << 61;
+    return desc;
+}
+
+// Instruction descriptor: D fp32, A/B bf16 (kind::f16) or e4m3 (kind::f8f6f4), both K-major unless said otherwise (bf16).
 template <bool kFp8>
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
+__host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool a_mn = false, bool b_mn = false) {
     uint32_t d = 0;
     d |= 1u << 4;                                   // D format: F32
     d |= (kFp8 ? 0u : 1u) << 7;                     // A format: E4M3 (0) / BF16 (1)
     d |= (kFp8 ? 0u : 1u) << 10;                    // B format
+    d |= (a_mn ? 1u : 0u) << 15;                    // A is MN-major
+    d |= (b_mn ? 1u : 0u) << 16;                    // B is MN-major
     d |= static_cast<uint32_t>(n >> 3) << 17;       // N / 8
     d |= static_cast<uint32_t>(m >> 4) << 24;       // M / 16
     return d;
+}
+
+// ---------------------------------------------------------------- epilogue stores
+// 32 fp32 accumulators of one row -> 64 bytes of bf16, as two 256-bit stores (full sectors) where the row allows it
+__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&r)[32], bool wide) {
+    int4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&v[q]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(__uint_as_float(r[q * 8 + 2 * i]), __uint_as_float(r[q * 8 + 2 * i + 1]));
+    }
+    if (wide) {
+#pragma unroll
+        for (int q = 0; q < 4; q += 2)
+            asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                         ::"l"(dst + q * 8), "r"(v[q].x), "r"(v[q].y), "r"(v[q].z), "r"(v[q].w), "r"(v[q + 1].x), "r"(v[q + 1].y), "r"(v[q + 1].z), "r"(v[q + 1].w) : "memory");
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) *reinterpret_cast<int4*>(dst + q * 8) = v[q];
+    }
 }
 
 // ---------------------------------------------------------------- bounded mbarrier wait shared by the roles

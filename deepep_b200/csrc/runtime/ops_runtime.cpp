@@ -2,6 +2,7 @@
 // The reference library has no compute kernels; these exist for the fused MoE layer and the
 // tensor-parallel fused operators built on the same runtime.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -21,6 +22,11 @@ namespace py = pybind11;
 namespace ep {
 
 namespace {
+
+// A new tensor from the caching allocator, without the trip through the operator dispatcher (as long as the allocation).
+at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, int device) {
+    return at::detail::empty_cuda(sizes, dtype, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)), std::nullopt);
+}
 
 // one status word per device for the GEMM pipelines (0 = healthy)
 at::Tensor& gemm_status(int device) {
@@ -56,7 +62,7 @@ at::Tensor gemm_impl(const at::Tensor& a, const at::Tensor& b, const std::option
     EP_HOST_ASSERT_MSG(N % 128 == 0 && K % (fp8 ? 128 : 64) == 0, "N must be a multiple of 128 and K of 64 (bf16) / 128 (fp8)");
     const int device = a.get_device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    if (!out.has_value()) out = at::empty({M, N}, a.options().dtype(at::kBFloat16));
+    if (!out.has_value()) out = new_tensor({M, N}, at::kBFloat16, device);
     EP_HOST_ASSERT(out->scalar_type() == at::kBFloat16 && out->size(0) == M && out->size(1) == N && out->stride(1) == 1 &&
                    (out->stride(0) * 2) % 16 == 0);
     if (M == 0) return *out;
@@ -99,18 +105,21 @@ cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // out[g] = a[:, range g] @ b[:, range g]^T for all groups in one launch (bf16): the k range of group g is
 // [align(group_end[g-1], group_alignment), group_end[g]), read from the device array, no host synchronisation.
+// mn_major: the operands are given as [K, M] and [K, N] (the rows of an expert are the contraction dimension and lie in
+// memory as the forward pass left them): no transposed copies.
 at::Tensor gemm_k_grouped(const at::Tensor& a, const at::Tensor& b, const at::Tensor& group_end, int num_groups, int group_alignment,
-                          std::optional<at::Tensor> out, int num_sms) {
+                          std::optional<at::Tensor> out, int num_sms, bool mn_major) {
     EP_HOST_ASSERT(a.is_cuda() && b.is_cuda() && a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1);
-    EP_HOST_ASSERT(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.size(1) == b.size(1));
-    const int M = static_cast<int>(a.size(0)), N = static_cast<int>(b.size(0)), K = static_cast<int>(a.size(1));
+    const int kd = mn_major ? 0 : 1;
+    EP_HOST_ASSERT(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.size(kd) == b.size(kd));
+    const int M = static_cast<int>(a.size(1 - kd)), N = static_cast<int>(b.size(1 - kd)), K = static_cast<int>(a.size(kd));
     EP_HOST_ASSERT_MSG(N % 128 == 0 && K % 64 == 0 && group_alignment % 64 == 0, "N must be a multiple of 128, K and the group alignment of 64");
     EP_HOST_ASSERT((a.stride(0) * 2) % 16 == 0 && (b.stride(0) * 2) % 16 == 0 && reinterpret_cast<uintptr_t>(a.data_ptr()) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(b.data_ptr()) % 16 == 0);
     EP_HOST_ASSERT(group_end.scalar_type() == at::kInt && group_end.is_contiguous() && group_end.numel() >= num_groups && num_groups >= 1);
     const int device = a.get_device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    if (!out.has_value()) out = at::empty({num_groups, M, N}, a.options());
+    if (!out.has_value()) out = new_tensor({num_groups, M, N}, at::kBFloat16, device);
     EP_HOST_ASSERT(out->scalar_type() == at::kBFloat16 && out->is_contiguous() && out->numel() == static_cast<int64_t>(num_groups) * M * N);
     gemm::GemmParams p = {};
     p.M = M;
@@ -121,6 +130,7 @@ at::Tensor gemm_k_grouped(const at::Tensor& a, const at::Tensor& b, const at::Te
     p.group_alignment = group_alignment;
     p.zero_gap = 0;
     p.k_grouped = 1;
+    p.a_mn = p.b_mn = mn_major ? 1 : 0;
     p.c_group_stride = static_cast<int64_t>(M) * N;
     p.C = reinterpret_cast<__nv_bfloat16*>(out->data_ptr());
     p.ldc = N;
@@ -129,6 +139,38 @@ at::Tensor gemm_k_grouped(const at::Tensor& a, const at::Tensor& b, const at::Te
     const int sms = num_sms > 0 ? num_sms : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     CUDA_RUNTIME_CHECK(gemm::launch_gemm(p, a.data_ptr(), a.stride(0) * 2, b.data_ptr(), b.stride(0) * 2, false, sms, cur_stream()));
     return *out;
+}
+
+// bf16 a @ b with b as it lies in memory: b [K, N]; a [M, K], or a^T @ b with a [K, M] (any K then: the weight gradient of a
+// linear layer, rows of both being the tokens).
+at::Tensor gemm_mn(const at::Tensor& a, const at::Tensor& b, bool a_transposed) {
+    EP_HOST_ASSERT(a.is_cuda() && b.is_cuda() && a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1);
+    EP_HOST_ASSERT(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16);
+    const int M = static_cast<int>(a.size(a_transposed ? 1 : 0)), K = static_cast<int>(a.size(a_transposed ? 0 : 1)), N = static_cast<int>(b.size(1));
+    EP_HOST_ASSERT(b.size(0) == K);
+    EP_HOST_ASSERT_MSG(N % 128 == 0 && (a_transposed || K % 64 == 0), "N must be a multiple of 128, K of 64 unless a is transposed");
+    EP_HOST_ASSERT((a.stride(0) * 2) % 16 == 0 && (b.stride(0) * 2) % 16 == 0 && reinterpret_cast<uintptr_t>(a.data_ptr()) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(b.data_ptr()) % 16 == 0);
+    const int device = a.get_device();
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+    at::Tensor out = new_tensor({M, N}, at::kBFloat16, device);
+    if (M == 0) return out;
+    if (K == 0) return out.zero_();
+    gemm::GemmParams p = {};
+    p.M = M;
+    p.N = N;
+    p.K = K;
+    p.num_groups = 1;
+    p.group_alignment = 1;
+    p.a_mn = a_transposed ? 1 : 0;
+    p.b_mn = 1;
+    p.C = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
+    p.ldc = N;
+    p.error = gemm_status(device).data_ptr<int>();
+    p.timeout_ns = 10ull * 1000 * 1000 * 1000;
+    CUDA_RUNTIME_CHECK(gemm::launch_gemm(p, a.data_ptr(), a.stride(0) * 2, b.data_ptr(), b.stride(0) * 2, false,
+                                         at::cuda::getCurrentDeviceProperties()->multiProcessorCount, cur_stream()));
+    return out;
 }
 
 std::tuple<at::Tensor, at::Tensor> router_topk(const at::Tensor& logits, int num_topk) {
@@ -246,8 +288,10 @@ void register_ops_bindings(py::module_& m) {
           "them itself (kind::mxf8f6f4.block_scale) when N is a multiple of 256 and K at most 8192. "
           "zero_gap: rows in the alignment gaps of a grouped problem are written as zeros (alignment a multiple of 128), else left alone");
     m.def("gemm_k_grouped", &gemm_k_grouped, py::arg("a"), py::arg("b"), py::arg("group_end"), py::arg("num_groups"),
-          py::arg("group_alignment") = 128, py::arg("out") = py::none(), py::arg("num_sms") = 0,
+          py::arg("group_alignment") = 128, py::arg("out") = py::none(), py::arg("num_sms") = 0, py::arg("mn_major") = false,
           "C[g] = A[:, k range g] @ B[:, k range g]^T for all groups in one launch (bf16; the ranges come from a device array)");
+    m.def("gemm_mn", &gemm_mn, py::arg("a"), py::arg("b"), py::arg("a_transposed") = false,
+          "a @ b, or a^T @ b, with b [K, N] row-major (bf16)");
     m.def("gemm_check_status", &gemm_check_status);
 }
 

@@ -149,11 +149,10 @@ def moe_backward(comm, weights: Sequence[ExpertWeights], ctxs, dys: Sequence[tor
         dh1, a_w, dw_row = _C.swiglu_backward(h1, da, recv_w, True, **groups)                       # [rows, 2I], [rows, I], [rows]
         dw_rows.append(dw_row)
         dx_rows.append(_C.gemm(dh1, w.w13_t, zero_gap=False, **groups))
-        # weight gradients: contraction over every expert's (zero padded) rows, all experts in one launch each
-        dh2_t, a_t = _C.transpose_bf16(dh2), _C.transpose_bf16(a_w)
-        dh1_t, x_t = _C.transpose_bf16(dh1), _C.transpose_bf16(x_rows)
-        dW2s.append(_C.gemm_k_grouped(dh2_t, a_t, ends, el, cfg.expert_alignment))               # [EL, hidden, I]
-        dW13s.append(_C.gemm_k_grouped(dh1_t, x_t, ends, el, cfg.expert_alignment))              # [EL, 2I, hidden]
+        # weight gradients: contraction over every expert's (zero padded) rows, all experts in one launch each, the operands
+        # read as they lie in memory (rows outermost)
+        dW2s.append(_C.gemm_k_grouped(dh2, a_w, ends, el, cfg.expert_alignment, mn_major=True))          # [EL, hidden, I]
+        dW13s.append(_C.gemm_k_grouped(dh1, x_rows, ends, el, cfg.expert_alignment, mn_major=True))      # [EL, 2I, hidden]
     # gradient of the dispatch: a combine that also carries the gate-weight gradients back
     comb = comm.combine([dict(x=dx_rows[r], handle=ctxs[r]['handle'], topk_weights=dw_rows[r].contiguous()) for r in range(R)])
     return [c[0] for c in comb], [c[1] for c in comb], dW13s, dW2s

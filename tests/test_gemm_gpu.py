@@ -160,3 +160,55 @@ def test_gemm_k_grouped_weight_gradients():
             assert out[i].float().abs().max().item() == 0
         else:
             assert ((out[i].float() - ref).norm() / ref.norm()).item() < 1e-2
+
+
+@pytest.mark.parametrize('pair', ['1', '0'])
+@pytest.mark.parametrize('M,N,K', [(128, 128, 64), (72, 256, 100), (304, 384, 1), (520, 512, 1001), (256, 1024, 4096)])
+def test_gemm_mn_major(M, N, K, pair, monkeypatch):
+    """Operands with the contraction dimension outermost: a^T @ b (any K, M not a multiple of a tile) and a @ b."""
+    import deepep_b200
+    C = deepep_b200._C
+    monkeypatch.setenv('EP_GEMM_CTA_PAIR', pair)
+    g = torch.Generator(device='cuda').manual_seed(7)
+    a = torch.randn((K, M), device='cuda', generator=g).bfloat16()
+    b = (torch.randn((K, N), device='cuda', generator=g) * 0.05).bfloat16()
+    out = C.gemm_mn(a, b, True)
+    assert _rel_err(out, a.float().t() @ b.float()) < 1e-2
+    if K % 64 == 0:
+        out = C.gemm_mn(a.t().contiguous(), b)
+        assert _rel_err(out, a.float().t() @ b.float()) < 1e-2
+    torch.cuda.synchronize()
+    assert C.gemm_check_status() == 0
+
+
+@pytest.mark.parametrize('N', [128, 512])
+@pytest.mark.parametrize('counts', [[200, 0, 130, 57], [64, 128, 1]])
+def test_gemm_k_grouped_mn_major(counts, N):
+    """Weight gradients from row-major operands, against the K-major form on transposed copies (same tiles, same order of
+    accumulation: identical) and against fp32."""
+    import deepep_b200
+    C = deepep_b200._C
+    align, M = 128, 320
+    g = torch.Generator(device='cuda').manual_seed(8)
+    ends, start = [], 0
+    for c in counts:
+        ends.append(start + c)
+        start = -(-(start + c) // align) * align
+    a = torch.zeros((start, M), device='cuda', dtype=torch.bfloat16)
+    b = torch.zeros((start, N), device='cuda', dtype=torch.bfloat16)
+    s0 = 0
+    for e in ends:
+        a[s0:e] = torch.randn((e - s0, M), device='cuda', generator=g).bfloat16()
+        b[s0:e] = torch.randn((e - s0, N), device='cuda', generator=g).bfloat16()
+        s0 = -(-e // align) * align
+    ends_t = torch.tensor(ends, dtype=torch.int32, device='cuda')
+    out = C.gemm_k_grouped(a, b, ends_t, len(counts), align, mn_major=True)
+    ref = C.gemm_k_grouped(a.t().contiguous(), b.t().contiguous(), ends_t, len(counts), align)
+    torch.cuda.synchronize()
+    assert C.gemm_check_status() == 0
+    assert torch.equal(out, ref)
+    s0 = 0
+    for i, e in enumerate(ends):
+        want = a[s0:e].float().t() @ b[s0:e].float()
+        assert torch.equal(out[i], torch.zeros_like(out[i])) if e == s0 else _rel_err(out[i], want) < 1e-2
+        s0 = -(-e // align) * align
