@@ -93,6 +93,7 @@ class EPHandle:
         # single tier: the hybrid-mode members of the reference handle stay empty
         self.token_metadata_at_forward = token_metadata_at_forward
         self.channel_linked_list = channel_linked_list
+        self._counts_pending = False         # the host has not read the counts yet (ElasticBuffer._finish_counts)
         self._psum_expert_full: Optional[torch.Tensor] = None   # [local experts + 1], last = expanded rows
         # [ranks, ranks] tokens that rank i sent to rank j in this dispatch (every rank gets the whole matrix)
         self.num_tokens_per_rank_matrix: Optional[torch.Tensor] = None
@@ -417,7 +418,7 @@ class ElasticBuffer:
                        num_max_tokens_per_rank=None, expert_alignment=None, num_sms=0, previous_event=None,
                        previous_event_before_epilogue=None, async_with_compute_stream=False, allocate_on_comm_stream=False, handle=None,
                        do_cpu_sync=None, do_expand=False, do_zero_padding=False, use_tma_aligned_col_major_sf=False, zero_copy=False,
-                       fused_fp8=False, round_scale=False, num_worst_tokens=0, do_handle_copy=True, mask_weights=False):
+                       fused_fp8=False, round_scale=False, num_worst_tokens=0, do_handle_copy=True, mask_weights=False, defer_counts=False):
         """One rank's dispatch as the tuple that the native driver takes (order: ``dispatch_args`` in bindings.cpp)."""
         sf = None
         if isinstance(x, tuple):
@@ -447,22 +448,31 @@ class ElasticBuffer:
         return (x, sf, topk_idx, topk_weights, cumulative_local_expert_recv_stats, num_experts, num_max_tokens_per_rank,
                 1 if expert_alignment is None else expert_alignment, num_sms, quant_mode, do_expand, do_zero_padding,
                 True if do_cpu_sync is None else do_cpu_sync, zero_copy, num_worst_tokens, use_tma_aligned_col_major_sf, do_handle_copy,
-                previous_event, previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream, routing, mask_weights)
+                previous_event, previous_event_before_epilogue, async_with_compute_stream, allocate_on_comm_stream, routing, mask_weights, defer_counts)
 
     @staticmethod
     def _dispatch_result(result, call, handle: Optional[EPHandle]):
         """The public return value from the native result tuple and the call's own tuple."""
         (recv_x, recv_sf, recv_topk_idx, recv_topk_weights, token_slot, pair_row, psum_rank, psum_expert_full, psum_expert, num_unaligned,
-         recv_src_metadata, count_matrix, topk_idx, num_recv_tokens, num_expanded_tokens, num_sms, per_expert_list, event) = result
+         recv_src_metadata, count_matrix, topk_idx, num_recv_tokens, num_expanded_tokens, num_sms, per_expert_list, event, pending) = result
         if handle is None:
             handle = EPHandle(call[10], call[5], call[7], call[6], num_sms, call[2] if topk_idx is None else topk_idx, num_recv_tokens,
                               num_expanded_tokens, per_expert_list, psum_rank, psum_expert, num_unaligned, recv_src_metadata, token_slot,
                               pair_row)
             handle._psum_expert_full = psum_expert_full
             handle.num_tokens_per_rank_matrix = count_matrix
+            handle._counts_pending = pending
         if recv_sf is not None:
             recv_x = (recv_x, recv_sf)
         return recv_x, recv_topk_idx, recv_topk_weights, handle, EventOverlap(event)
+
+    def _finish_counts(self, handle: EPHandle) -> None:
+        """Completes the handle of a dispatch with ``defer_counts`` (before the next dispatch on this buffer): waits for the
+        counts and cuts the handle's own tensor to them; the caller cuts the outputs."""
+        tokens, rows, per_expert = self.runtime.take_counts(handle.num_experts // self.num_ranks)
+        handle.num_recv_tokens, handle.num_expanded_tokens, handle.num_recv_tokens_per_expert_list = tokens, rows, per_expert
+        handle.recv_src_metadata = handle.recv_src_metadata[:tokens]
+        handle._counts_pending = False
 
     def dispatch(self, x: Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]], topk_idx: Optional[torch.Tensor] = None,
                  topk_weights: Optional[torch.Tensor] = None,

@@ -48,6 +48,8 @@ struct EngramParams {
     int64_t out_sf_token_stride, out_sf_pack_stride;   // in packs; a token owns entries_per_token consecutive indices
     int entries_per_token;
 };
+// the same for one rank whose table lies in its own GPU's memory
+cudaError_t launch_engram_local(const EngramParams& p, cudaStream_t stream);
 cudaError_t launch_engram_gather(const EngramParams* params, int num_vranks, int num_sms, int smem_optin, cudaStream_t stream);
 
 }  // namespace aux

@@ -19,17 +19,20 @@ namespace {
 
 // ---------------------------------------------------------------- router: top-k over experts, softmax over the selection
 // one warp per token; the warp keeps the row in registers (experts <= 2048 -> 64 values per lane)
-template <int kPerLane>
-__global__ void __launch_bounds__(256) router_topk_kernel(const float* __restrict__ logits, int num_tokens, int num_experts, int num_topk,
+__device__ __forceinline__ float to_float(float v) { return v; }
+__device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+template <int kPerLane, typename Logit>
+__global__ void __launch_bounds__(256) router_topk_kernel(const Logit* __restrict__ logits, int64_t row_stride, int num_tokens, int num_experts, int num_topk,
                                                           int64_t* __restrict__ topk_idx, float* __restrict__ topk_weights) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = lane_id();
     if (warp >= num_tokens) return;
-    const float* row = logits + static_cast<int64_t>(warp) * num_experts;
+    const Logit* row = logits + static_cast<int64_t>(warp) * row_stride;
     float v[kPerLane];
 #pragma unroll
     for (int i = 0; i < kPerLane; ++i) {
         const int e = i * 32 + lane;
-        v[i] = e < num_experts ? row[e] : -INFINITY;
+        v[i] = e < num_experts ? to_float(row[e]) : -INFINITY;
     }
     float sel_val = 0.f;
     int sel_idx = -1;
@@ -63,6 +66,44 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
     if (lane < num_topk) {
         topk_idx[static_cast<int64_t>(warp) * num_topk + lane] = sel_idx;
         topk_weights[static_cast<int64_t>(warp) * num_topk + lane] = ex / sum;
+    }
+}
+
+// Router weights fp32 [experts, hidden] -> bf16 [padded experts, hidden], zero rows behind the last expert (the GEMM tiles
+// its columns in multiples of 128).
+__global__ void __launch_bounds__(256) router_weights_kernel(const float* __restrict__ w, int num_experts, int padded, int hidden, __nv_bfloat16* __restrict__ out) {
+    const int64_t n = static_cast<int64_t>(padded) * hidden / 8, real = static_cast<int64_t>(num_experts) * hidden / 8;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        int4 v = make_int4(0, 0, 0, 0);
+        if (i < real) {
+            const float4 a = reinterpret_cast<const float4*>(w)[2 * i], b = reinterpret_cast<const float4*>(w)[2 * i + 1];
+            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+            h[0] = __floats2bfloat162_rn(a.x, a.y);
+            h[1] = __floats2bfloat162_rn(a.z, a.w);
+            h[2] = __floats2bfloat162_rn(b.x, b.y);
+            h[3] = __floats2bfloat162_rn(b.z, b.w);
+        }
+        reinterpret_cast<int4*>(out)[i] = v;
+    }
+}
+
+// Gradient of the logits from the gradient of the top-k weights, one warp per token: the softmax Jacobian over the selected
+// experts, d logit_k = w_k (dw_k - sum_j w_j dw_j), zeros elsewhere (ten elementwise launches otherwise, bound by the host).
+__global__ void __launch_bounds__(256) router_backward_kernel(const int64_t* __restrict__ topk_idx, const float* __restrict__ w, const float* __restrict__ dw,
+                                                              int num_tokens, int num_topk, int num_experts, int padded, __nv_bfloat16* __restrict__ dlogits) {
+    const int t = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = lane_id();
+    if (t >= num_tokens) return;
+    __nv_bfloat16* row = dlogits + static_cast<int64_t>(t) * padded;
+    for (int i = lane * 8; i < padded; i += 256) *reinterpret_cast<int4*>(row + i) = make_int4(0, 0, 0, 0);
+    const int64_t o = static_cast<int64_t>(t) * num_topk + lane;
+    const float wv = lane < num_topk ? w[o] : 0.f, dv = lane < num_topk ? dw[o] : 0.f;
+    float inner = wv * dv;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) inner += __shfl_xor_sync(0xffffffffu, inner, s);
+    __syncwarp();           // the zeros of all lanes are in place
+    if (lane < num_topk) {
+        const int64_t e = topk_idx[o];
+        if (e >= 0 && e < num_experts) row[e] = __float2bfloat16_rn(wv * (dv - inner));
     }
 }
 
@@ -120,6 +161,46 @@ __device__ __forceinline__ void pack16(const float (&f)[16], int4& lo, int4& hi)
         __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(h == 0 ? &lo : &hi);
 #pragma unroll
         for (int j = 0; j < 4; ++j) h2[j] = __floats2bfloat162_rn(f[8 * h + 2 * j], f[8 * h + 2 * j + 1]);
+    }
+}
+
+// ---------------------------------------------------------------- 128x128 weight quantisation: one block per weight block
+// The arithmetic is that of the elementwise definition (scale = max(amax, 1e-4) / 448, correctly rounded divisions); the block
+// is read once and held in registers between the two passes, instead of five passes over fp32 copies of the weights.
+__global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* __restrict__ w, int rows, int cols, int pow2, uint8_t* __restrict__ q,
+                                                           float* __restrict__ scales) {
+    __shared__ float s_max[8];
+    const int64_t base = (static_cast<int64_t>(blockIdx.z) * rows + blockIdx.y * 128) * cols + blockIdx.x * 128;
+    const int r0 = threadIdx.x >> 3, c = (threadIdx.x & 7) * 16;        // 32 rows per pass, 16 channels per thread
+    int4 lo[4], hi[4];
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(w + base + static_cast<int64_t>(r0 + 32 * i) * cols + c);
+        lo[i] = ld_nc_int4(src);
+        hi[i] = ld_nc_int4(src + 16);
+        amax = fmaxf(amax, fmaxf(amax_bf16x8(lo[i]), amax_bf16x8(hi[i])));
+    }
+    amax = warp_reduce_max_width(amax, 32);
+    if (lane_id() == 0) s_max[warp_id()] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, s_max[i]);
+    float scale = __fdiv_rn(fmaxf(amax, 1e-4f), 448.f);
+    if (pow2) scale = exp2f(ceilf(log2f(scale)));
+    if (threadIdx.x == 0) scales[(static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = scale;
+    const float inv = pow2 ? 1.f / scale : 0.f;                         // exact for a power of two
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float f[16];
+        unpack16(lo[i], hi[i], f);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) f[j] = pow2 ? f[j] * inv : __fdiv_rn(f[j], scale);
+        int4 o;
+        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ow[j] = pack4_e4m3(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+        st_na_int4(q + base + static_cast<int64_t>(r0 + 32 * i) * cols + c, o);
     }
 }
 
@@ -270,10 +351,12 @@ __global__ void __launch_bounds__(128) swiglu_bwd_kernel(const uint8_t* __restri
 // consecutive rows, pairs them up column by column (one 32-bit word = the same column of both rows) and stores the
 // words transposed into shared memory (pitch 33 words); the write side reads four words = eight rows of one column
 // and stores them as one 16-byte vector. Edge tiles and unaligned tensors take the element-wise path.
-__global__ void __launch_bounds__(256) transpose_kernel(const __nv_bfloat16* __restrict__ in, int64_t in_stride, int rows, int cols,
-                                                        __nv_bfloat16* __restrict__ out, int64_t out_stride, int aligned) {
+__global__ void __launch_bounds__(256) transpose_kernel(const __nv_bfloat16* __restrict__ in, int64_t in_stride, int64_t in_batch, int rows, int cols,
+                                                        __nv_bfloat16* __restrict__ out, int64_t out_stride, int64_t out_batch, int aligned) {
     __shared__ uint32_t tile_t[64 * 33];      // [column][row pair]
     const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+    in += blockIdx.z * in_batch;
+    out += blockIdx.z * out_batch;
     if (aligned && r0 + 64 <= rows && c0 + 64 <= cols) {
         const int rp = threadIdx.x >> 3, cv = threadIdx.x & 7;
         const int4 a = ld_nc_int4(reinterpret_cast<const uint8_t*>(in + (r0 + 2 * rp) * in_stride + c0 + cv * 8));
@@ -326,16 +409,48 @@ uint64_t addr(const void* p) { return reinterpret_cast<uintptr_t>(p); }
 
 }  // namespace
 
-cudaError_t router_topk(const float* logits, int num_tokens, int num_experts, int num_topk, int64_t* topk_idx, float* topk_weights,
-                        cudaStream_t stream) {
+template <typename Logit>
+static cudaError_t router_topk_any(const Logit* logits, int64_t row_stride, int num_tokens, int num_experts, int num_topk, int64_t* topk_idx,
+                                   float* topk_weights, cudaStream_t stream) {
     if (num_tokens == 0) return cudaSuccess;
     if (num_experts > 2048 || num_topk > 32 || num_topk > num_experts) return cudaErrorInvalidValue;
     const int blocks = (num_tokens * 32 + 255) / 256;
     const int per_lane = (num_experts + 31) / 32;
-    if (per_lane <= 2) router_topk_kernel<2><<<blocks, 256, 0, stream>>>(logits, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    else if (per_lane <= 8) router_topk_kernel<8><<<blocks, 256, 0, stream>>>(logits, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    else if (per_lane <= 16) router_topk_kernel<16><<<blocks, 256, 0, stream>>>(logits, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    else router_topk_kernel<64><<<blocks, 256, 0, stream>>>(logits, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    if (per_lane <= 2) router_topk_kernel<2><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    else if (per_lane <= 8) router_topk_kernel<8><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    else if (per_lane <= 16) router_topk_kernel<16><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    else router_topk_kernel<64><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    return cudaGetLastError();
+}
+
+cudaError_t router_topk(const void* logits, bool bf16, int64_t row_stride, int num_tokens, int num_experts, int num_topk, int64_t* topk_idx,
+                        float* topk_weights, cudaStream_t stream) {
+    return bf16 ? router_topk_any(static_cast<const __nv_bfloat16*>(logits), row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights, stream)
+                : router_topk_any(static_cast<const float*>(logits), row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights, stream);
+}
+
+cudaError_t router_weights(const float* w, int num_experts, int padded_experts, int hidden, void* out, cudaStream_t stream) {
+    if (hidden % 8 != 0) return cudaErrorInvalidValue;
+    const int64_t want = (static_cast<int64_t>(padded_experts) * hidden / 8 + 255) / 256;
+    router_weights_kernel<<<static_cast<int>(std::min<int64_t>(std::max<int64_t>(want, 1), 148 * 16)), 256, 0, stream>>>(
+        w, num_experts, padded_experts, hidden, static_cast<__nv_bfloat16*>(out));
+    return cudaGetLastError();
+}
+
+cudaError_t router_backward(const int64_t* topk_idx, const float* w, const float* dw, int num_tokens, int num_topk, int num_experts, int padded_experts,
+                            void* dlogits, cudaStream_t stream) {
+    if (num_tokens == 0) return cudaSuccess;
+    if (num_topk > 32 || padded_experts % 8 != 0) return cudaErrorInvalidValue;
+    router_backward_kernel<<<(num_tokens + 7) / 8, 256, 0, stream>>>(topk_idx, w, dw, num_tokens, num_topk, num_experts, padded_experts,
+                                                                     static_cast<__nv_bfloat16*>(dlogits));
+    return cudaGetLastError();
+}
+
+cudaError_t quant_weights_128x128(const void* w, int groups, int rows, int cols, bool pow2, void* q, float* scales, cudaStream_t stream) {
+    if (groups == 0 || rows == 0 || cols == 0) return cudaSuccess;
+    if (rows % 128 != 0 || cols % 128 != 0 || groups > 65535 || rows / 128 > 65535) return cudaErrorInvalidValue;
+    weight_quant_kernel<<<dim3(cols / 128, rows / 128, groups), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w), rows, cols, pow2 ? 1 : 0,
+                                                                                  static_cast<uint8_t*>(q), scales);
     return cudaGetLastError();
 }
 
@@ -386,13 +501,13 @@ cudaError_t swiglu_backward(const void* x, const void* dout, int rows, int inter
     return cudaGetLastError();
 }
 
-cudaError_t transpose_bf16(const void* in, int64_t in_stride, int rows, int cols, void* out, int64_t out_stride, cudaStream_t stream) {
-    if (rows == 0 || cols == 0) return cudaSuccess;
-    dim3 grid((cols + 63) / 64, (rows + 63) / 64);
-    const int aligned = in_stride % 8 == 0 && out_stride % 8 == 0 && reinterpret_cast<uintptr_t>(in) % 16 == 0 &&
-                        reinterpret_cast<uintptr_t>(out) % 16 == 0;
-    transpose_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(in), in_stride, rows, cols,
-                                               static_cast<__nv_bfloat16*>(out), out_stride, aligned);
+cudaError_t transpose_bf16(const void* in, int64_t in_stride, int64_t in_batch, int batch, int rows, int cols, void* out, int64_t out_stride,
+                           int64_t out_batch, cudaStream_t stream) {
+    if (rows == 0 || cols == 0 || batch == 0) return cudaSuccess;
+    dim3 grid((cols + 63) / 64, (rows + 63) / 64, batch);
+    const int aligned = in_stride % 8 == 0 && out_stride % 8 == 0 && in_batch % 8 == 0 && out_batch % 8 == 0 && addr(in) % 16 == 0 && addr(out) % 16 == 0;
+    transpose_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(in), in_stride, in_batch, rows, cols, static_cast<__nv_bfloat16*>(out),
+                                               out_stride, out_batch, aligned);
     return cudaGetLastError();
 }
 

@@ -12,6 +12,7 @@
 #include "../kernels/aux_api.hpp"
 #include "host_segment.hpp"
 #include "runtime.hpp"
+#include "stream_scope.hpp"
 #include "stream_tools.hpp"
 
 namespace py = pybind11;
@@ -148,6 +149,7 @@ std::vector<std::tuple<at::Tensor, std::optional<at::Tensor>>> engram_gather(
     const int elem = static_cast<int>(c10::elementSize(dtype));
     const int row_bytes = hidden * elem;
     EP_HOST_ASSERT(row_bytes % 16 == 0 && table_offset % 16 == 0 && table_offset >= static_cast<int64_t>(kCtlBytes));
+    const bool local = V == 1 && rt0.num_ranks() == 1 && host_tables.empty() && num_sms <= 0;
     if (num_sms <= 0) num_sms = std::max(1, rt0.num_device_sms() / V / 4);
     std::vector<aux::EngramParams> params(V);
     std::vector<std::tuple<at::Tensor, std::optional<at::Tensor>>> out(V);
@@ -157,7 +159,7 @@ std::vector<std::tuple<at::Tensor, std::optional<at::Tensor>>> engram_gather(
         EP_HOST_ASSERT(idx.is_cuda() && idx.dim() == 2 && idx.scalar_type() == at::kInt && idx.is_contiguous());
         EP_HOST_ASSERT(!host_tables.empty() || table_offset + static_cast<int64_t>(entries_per_rank) * row_bytes <= rt.num_bytes());
         const int tokens = static_cast<int>(idx.size(0)), per_token = static_cast<int>(idx.size(1));
-        auto data = at::empty({static_cast<int64_t>(tokens) * per_token, hidden}, idx.options().dtype(dtype));
+        auto data = new_tensor({static_cast<int64_t>(tokens) * per_token, hidden}, dtype, device);
         std::optional<at::Tensor> sf_out;
         aux::EngramParams& p = params[v];
         p.c = rt.ctx();
@@ -198,8 +200,32 @@ std::vector<std::tuple<at::Tensor, std::optional<at::Tensor>>> engram_gather(
         }
         out[v] = {data, sf_out};
     }
-    CUDA_RUNTIME_CHECK(aux::launch_engram_gather(params.data(), V, num_sms, rt0.smem_optin(), cur_stream()));
+    if (local) CUDA_RUNTIME_CHECK(aux::launch_engram_local(params[0], cur_stream()));
+    else CUDA_RUNTIME_CHECK(aux::launch_engram_gather(params.data(), V, num_sms, rt0.smem_optin(), cur_stream()));
     return out;
+}
+
+// A fetch of this process' rank in one trip: on the communication stream, behind the caller's work so far; returns the rows,
+// the scales and the event that says they are there.
+std::tuple<at::Tensor, std::optional<at::Tensor>, EventHandle> engram_fetch_one(const std::shared_ptr<Runtime>& rt, const at::Tensor& indices, int64_t table_offset,
+                                                                               int entries_per_rank, int hidden, at::ScalarType dtype,
+                                                                               const std::optional<at::Tensor>& sf_table, bool col_major_sf,
+                                                                               const std::vector<std::shared_ptr<HostSegment>>& host_tables) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(rt->heap().device()));
+    const auto compute = at::cuda::getCurrentCUDAStream(), comm = rt->comm_stream();
+    stream_wait(comm, compute);
+    at::cuda::setCurrentCUDAStream(comm);
+    std::vector<std::tuple<at::Tensor, std::optional<at::Tensor>>> out;
+    try {
+        out = engram_gather({rt}, {indices}, table_offset, entries_per_rank, hidden, dtype, {sf_table}, col_major_sf, 0,
+                            host_tables.empty() ? std::vector<std::vector<std::shared_ptr<HostSegment>>>{} : std::vector<std::vector<std::shared_ptr<HostSegment>>>{host_tables});
+    } catch (...) {
+        at::cuda::setCurrentCUDAStream(compute);
+        throw;
+    }
+    EventHandle done(comm);
+    at::cuda::setCurrentCUDAStream(compute);
+    return {std::get<0>(out[0]), std::get<1>(out[0]), std::move(done)};
 }
 
 }  // namespace
@@ -220,6 +246,7 @@ void register_aux_bindings(py::module_& m) {
     m.def("copy_from_heap", &copy_from_heap);
     m.def("reduce_slots", &reduce_slots);
     m.def("engram_gather", &engram_gather);
+    m.def("engram_fetch_one", &engram_fetch_one);
     py::class_<HostSegment, std::shared_ptr<HostSegment>>(m, "HostSegment")
         .def_static("create", &HostSegment::create)
         .def_static("open", &HostSegment::open)

@@ -44,6 +44,7 @@ DispatchArgs dispatch_args(const py::tuple& t) {
     a.sc.async_with_compute_stream = item<bool>(t, 19);
     a.sc.allocate_on_comm_stream = item<bool>(t, 20);
     a.mask_weights = item<bool>(t, 22);
+    a.defer_counts = item<bool>(t, 23);
     if (!t[21].is_none()) {        // the routing of an earlier dispatch
         const auto h = item<py::tuple>(t, 21);
         a.cached = true;
@@ -77,7 +78,7 @@ py::list dispatch_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const 
         if (!args[v].cached) per_expert = py::cast(r.psum_expert.narrow(0, 0, r.psum_expert.size(0) - 1));    // the last word is the number of expanded rows
         out.append(py::make_tuple(r.recv_x, r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert,
                                   per_expert, r.num_unaligned, r.recv_src_metadata, count_matrix, r.topk_idx, r.num_recv_tokens,
-                                  r.num_expanded_tokens, r.num_sms, r.num_recv_tokens_per_expert_list, r.event));
+                                  r.num_expanded_tokens, r.num_sms, r.num_recv_tokens_per_expert_list, r.event, r.counts_pending));
     }
     return out;
 }
@@ -186,6 +187,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         // (may synchronise a stream: without the GIL, see dispatch_calls)
         .def_static("barrier", &Runtime::barrier, py::arg("runtimes"), py::arg("use_comm_stream") = true, py::arg("with_cpu_sync") = false,
                     py::call_guard<py::gil_scoped_release>())
+        .def("take_counts", &Runtime::take_counts, py::call_guard<py::gil_scoped_release>())
         .def_static("dispatch", &dispatch_calls)
         .def_static("combine", &combine_calls)
         .def_static("ht_buffer_size", &Runtime::ht_buffer_size);

@@ -174,13 +174,55 @@ at::Tensor gemm_mn(const at::Tensor& a, const at::Tensor& b, bool a_transposed) 
 }
 
 std::tuple<at::Tensor, at::Tensor> router_topk(const at::Tensor& logits, int num_topk) {
-    EP_HOST_ASSERT(logits.is_cuda() && logits.dim() == 2 && logits.scalar_type() == at::kFloat && logits.is_contiguous());
+    const bool bf16 = logits.scalar_type() == at::kBFloat16;
+    EP_HOST_ASSERT(logits.is_cuda() && logits.dim() == 2 && (bf16 || logits.scalar_type() == at::kFloat) && logits.stride(1) == 1);
     c10::cuda::CUDAGuard guard(logits.device());
-    const int T = static_cast<int>(logits.size(0)), E = static_cast<int>(logits.size(1));
-    auto idx = at::empty({T, num_topk}, logits.options().dtype(at::kLong));
-    auto w = at::empty({T, num_topk}, logits.options());
-    CUDA_RUNTIME_CHECK(ops::router_topk(logits.data_ptr<float>(), T, E, num_topk, idx.data_ptr<int64_t>(), w.data_ptr<float>(), cur_stream()));
+    const int T = static_cast<int>(logits.size(0)), E = static_cast<int>(logits.size(1)), device = logits.get_device();
+    auto idx = new_tensor({T, num_topk}, at::kLong, device), w = new_tensor({T, num_topk}, at::kFloat, device);
+    CUDA_RUNTIME_CHECK(ops::router_topk(logits.data_ptr(), bf16, logits.stride(0), T, E, num_topk, idx.data_ptr<int64_t>(), w.data_ptr<float>(), cur_stream()));
     return {idx, w};
+}
+
+// Router of the MoE layer: (topk_idx, topk_weights, bf16 weights padded to a multiple of 128 experts) from x [T, hidden] and
+// the fp32 or bf16 router weights [experts, hidden]
+std::tuple<at::Tensor, at::Tensor, at::Tensor> router_forward(const at::Tensor& x, const at::Tensor& router, int num_topk) {
+    EP_HOST_ASSERT(router.is_cuda() && router.dim() == 2 && router.is_contiguous() && router.size(1) == x.size(1) && router.size(1) % 8 == 0);
+    c10::cuda::CUDAGuard guard(x.device());
+    const int E = static_cast<int>(router.size(0)), H = static_cast<int>(router.size(1)), padded = align_up(E, 128), device = x.get_device();
+    at::Tensor w = router;
+    if (router.scalar_type() != at::kBFloat16 || padded != E) {
+        w = new_tensor({padded, H}, at::kBFloat16, device);
+        const at::Tensor f = router.scalar_type() == at::kFloat ? router : router.to(at::kFloat);
+        CUDA_RUNTIME_CHECK(ops::router_weights(f.data_ptr<float>(), E, padded, H, w.data_ptr(), cur_stream()));
+    }
+    const at::Tensor logits = gemm_impl(x, w, std::nullopt, std::nullopt, std::nullopt, 1, std::nullopt, 0, false, true);
+    const int T = static_cast<int>(x.size(0));
+    auto idx = new_tensor({T, num_topk}, at::kLong, device), tw = new_tensor({T, num_topk}, at::kFloat, device);
+    CUDA_RUNTIME_CHECK(ops::router_topk(logits.data_ptr(), true, logits.stride(0), T, E, num_topk, idx.data_ptr<int64_t>(), tw.data_ptr<float>(), cur_stream()));
+    return {idx, tw, w};
+}
+
+// (dx [T, hidden], d_router [experts, hidden] bf16) from the gradient of the top-k weights
+std::tuple<at::Tensor, at::Tensor> router_backward(const at::Tensor& x, const at::Tensor& router_padded, const at::Tensor& topk_idx, const at::Tensor& w,
+                                                   const at::Tensor& dw, int num_experts) {
+    EP_HOST_ASSERT(topk_idx.scalar_type() == at::kLong && topk_idx.is_contiguous() && w.is_contiguous() && w.scalar_type() == at::kFloat &&
+                   dw.scalar_type() == at::kFloat && dw.is_contiguous() && dw.numel() == w.numel());
+    c10::cuda::CUDAGuard guard(x.device());
+    const int T = static_cast<int>(topk_idx.size(0)), K = static_cast<int>(topk_idx.size(1)), padded = static_cast<int>(router_padded.size(0));
+    at::Tensor dlogits = new_tensor({T, padded}, at::kBFloat16, x.get_device());
+    CUDA_RUNTIME_CHECK(ops::router_backward(topk_idx.data_ptr<int64_t>(), w.data_ptr<float>(), dw.data_ptr<float>(), T, K, num_experts, padded,
+                                            dlogits.data_ptr(), cur_stream()));
+    return {gemm_mn(dlogits, router_padded, false), gemm_mn(dlogits, x, true).narrow(0, 0, num_experts)};
+}
+
+// bf16 [G, N, K] -> (e4m3 [G, N, K], fp32 scales [G, N / 128, K / 128])
+std::tuple<at::Tensor, at::Tensor> quant_weights_128x128(const at::Tensor& w, bool pow2) {
+    EP_HOST_ASSERT(w.is_cuda() && w.dim() == 3 && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.size(1) % 128 == 0 && w.size(2) % 128 == 0);
+    c10::cuda::CUDAGuard guard(w.device());
+    const int G = static_cast<int>(w.size(0)), N = static_cast<int>(w.size(1)), K = static_cast<int>(w.size(2)), device = w.get_device();
+    auto q = new_tensor({G, N, K}, at::kFloat8_e4m3fn, device), sf = new_tensor({G, N / 128, K / 128}, at::kFloat, device);
+    CUDA_RUNTIME_CHECK(ops::quant_weights_128x128(w.data_ptr(), G, N, K, pow2, q.data_ptr(), sf.data_ptr<float>(), cur_stream()));
+    return {q, sf};
 }
 
 std::tuple<at::Tensor, at::Tensor> quant_1x128(const at::Tensor& x, bool pow2, bool col_major_sf) {
@@ -188,9 +230,9 @@ std::tuple<at::Tensor, at::Tensor> quant_1x128(const at::Tensor& x, bool pow2, b
     c10::cuda::CUDAGuard guard(x.device());
     const int M = static_cast<int>(x.size(0)), H = static_cast<int>(x.size(1));
     EP_HOST_ASSERT(H % 128 == 0);
-    auto q = at::empty({M, H}, x.options().dtype(at::kFloat8_e4m3fn));
+    auto q = new_tensor({M, H}, at::kFloat8_e4m3fn, x.get_device());
     at::Tensor sf = col_major_sf ? at::empty({H / 128, align_up(std::max(M, 1), 4)}, x.options().dtype(at::kFloat)).t().slice(0, 0, M)
-                                 : at::empty({M, H / 128}, x.options().dtype(at::kFloat));
+                                 : new_tensor({M, H / 128}, at::kFloat, x.get_device());
     CUDA_RUNTIME_CHECK(ops::quant_1x128(x.data_ptr(), x.stride(0) * 2, M, H, pow2, q.data_ptr(), sf.data_ptr<float>(), sf.stride(0),
                                         sf.stride(1), cur_stream()));
     return {q, sf};
@@ -212,7 +254,7 @@ at::Tensor dequant_1x128(const at::Tensor& q, const at::Tensor& sf, const std::o
     c10::cuda::CUDAGuard guard(q.device());
     const int M = static_cast<int>(q.size(0)), H = static_cast<int>(q.size(1));
     EP_HOST_ASSERT(H % 128 == 0 && sf.size(0) == M && sf.size(1) == H / 128);
-    auto out = at::empty({M, H}, q.options().dtype(at::kBFloat16));
+    auto out = new_tensor({M, H}, at::kBFloat16, q.get_device());
     CUDA_RUNTIME_CHECK(ops::dequant_1x128(q.data_ptr(), sf.data_ptr<float>(), sf.stride(0), sf.stride(1), M, H, row_groups(group_end, group_alignment),
                                           out.data_ptr(), cur_stream()));
     return out;
@@ -231,9 +273,9 @@ std::tuple<at::Tensor, std::optional<at::Tensor>> swiglu(const at::Tensor& x, co
         rw = row_weight->data_ptr<float>();
     }
     const int* nv = num_valid_rows.has_value() ? num_valid_rows->data_ptr<int>() : nullptr;
-    at::Tensor out = at::empty({M, I}, x.options().dtype(quant ? at::kFloat8_e4m3fn : at::kBFloat16));
+    at::Tensor out = new_tensor({M, I}, quant ? at::kFloat8_e4m3fn : at::kBFloat16, x.get_device());
     std::optional<at::Tensor> sf;
-    if (quant) sf = at::empty({M, I / 128}, x.options().dtype(at::kFloat));
+    if (quant) sf = new_tensor({M, I / 128}, at::kFloat, x.get_device());
     CUDA_RUNTIME_CHECK(ops::swiglu(x.data_ptr(), M, I, rw, nv, row_groups(group_end, group_alignment), out.data_ptr(), quant, quant ? sf->data_ptr<float>() : nullptr,
                                    quant ? sf->stride(0) : 0, quant ? sf->stride(1) : 0, pow2, cur_stream()));
     return {out, sf};
@@ -247,11 +289,11 @@ py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const st
     const int M = static_cast<int>(x.size(0)), I = static_cast<int>(x.size(1) / 2);
     EP_HOST_ASSERT(dout.size(0) == M && dout.size(1) == I);
     if (row_weight.has_value()) EP_HOST_ASSERT(row_weight->scalar_type() == at::kFloat && row_weight->is_contiguous() && row_weight->numel() >= M);
-    auto dx = at::empty_like(x);
+    auto dx = new_tensor({M, 2 * I}, at::kBFloat16, x.get_device());
     at::Tensor act, dweight;
     if (with_byproducts) {
-        act = at::empty({M, I}, x.options());
-        dweight = at::empty({M}, x.options().dtype(at::kFloat));
+        act = new_tensor({M, I}, at::kBFloat16, x.get_device());
+        dweight = new_tensor({M}, at::kFloat, x.get_device());
     }
     CUDA_RUNTIME_CHECK(ops::swiglu_backward(x.data_ptr(), dout.data_ptr(), M, I, row_weight.has_value() ? row_weight->data_ptr<float>() : nullptr,
                                             row_groups(group_end, group_alignment), dx.data_ptr(), with_byproducts ? act.data_ptr() : nullptr,
@@ -260,12 +302,16 @@ py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const st
     return py::cast(dx);
 }
 
+// [rows, cols] -> [cols, rows], or the same for every matrix of a batch [n, rows, cols]
 at::Tensor transpose_bf16(const at::Tensor& x) {
-    EP_HOST_ASSERT(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1);
+    EP_HOST_ASSERT(x.is_cuda() && (x.dim() == 2 || x.dim() == 3) && x.scalar_type() == at::kBFloat16 && x.stride(-1) == 1);
     c10::cuda::CUDAGuard guard(x.device());
-    auto out = at::empty({x.size(1), x.size(0)}, x.options());
-    CUDA_RUNTIME_CHECK(ops::transpose_bf16(x.data_ptr(), x.stride(0), static_cast<int>(x.size(0)), static_cast<int>(x.size(1)), out.data_ptr(),
-                                           out.stride(0), cur_stream()));
+    const bool batched = x.dim() == 3;
+    const int n = batched ? static_cast<int>(x.size(0)) : 1, rows = static_cast<int>(x.size(-2)), cols = static_cast<int>(x.size(-1));
+    EP_HOST_ASSERT(n <= 65535);
+    auto out = batched ? new_tensor({n, cols, rows}, at::kBFloat16, x.get_device()) : new_tensor({cols, rows}, at::kBFloat16, x.get_device());
+    CUDA_RUNTIME_CHECK(ops::transpose_bf16(x.data_ptr(), x.stride(-2), batched ? x.stride(0) : 0, n, rows, cols, out.data_ptr(), rows,
+                                           static_cast<int64_t>(rows) * cols, cur_stream()));
     return out;
 }
 
@@ -273,6 +319,9 @@ at::Tensor transpose_bf16(const at::Tensor& x) {
 
 void register_ops_bindings(py::module_& m) {
     m.def("router_topk", &router_topk);
+    m.def("router_forward", &router_forward);
+    m.def("router_backward", &router_backward);
+    m.def("quant_weights_128x128", &quant_weights_128x128, py::arg("w"), py::arg("pow2") = false);
     m.def("quant_1x128", &quant_1x128, py::arg("x"), py::arg("pow2") = false, py::arg("col_major_sf") = false);
     m.def("dequant_1x128", &dequant_1x128, py::arg("q"), py::arg("sf"), py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
     m.def("swiglu", &swiglu, py::arg("x"), py::arg("row_weight") = py::none(), py::arg("num_valid_rows") = py::none(), py::arg("quant") = false,

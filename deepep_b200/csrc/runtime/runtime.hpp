@@ -61,6 +61,9 @@ struct DispatchArgs {
     int num_worst_tokens = 0;
     // cached dispatch: tensors of an earlier handle
     bool mask_weights = false;      // received weights of experts that live elsewhere are 0
+    // One rank with CPU sync: hand back outputs of the largest possible size at once; take_counts() delivers the counts (the
+    // caller asks for them before the next dispatch). Lets a driver queue the work behind the dispatch without waiting.
+    bool defer_counts = false;
     bool copy_topk_idx = false;     // the result carries a copy of topk_idx (the handle's own)
     bool cached = false;
     std::optional<at::Tensor> h_token_slot, h_pair_row, h_psum_rank, h_psum_expert, h_num_unaligned, h_recv_src_metadata;
@@ -74,6 +77,7 @@ struct DispatchResult {
     at::Tensor token_slot, pair_row, psum_rank, psum_expert, num_unaligned, recv_src_metadata;
     at::Tensor count_matrix;   // [R, R] tokens rank i sent to rank j (undefined for cached dispatches)
     int num_recv_tokens = 0, num_expanded_tokens = 0, num_sms = 0;
+    bool counts_pending = false;       // take_counts() has them
     std::vector<int> num_recv_tokens_per_expert_list;
     std::optional<EventHandle> event;
 };
@@ -162,6 +166,8 @@ public:
     // the same for a group of one rank (kernels/local_exchange.cu)
     DispatchResult dispatch_single(DispatchArgs& a);
     CombineResult combine_single(CombineArgs& a);
+    // (received tokens, expanded rows, aligned counts per expert) of the last dispatch with host counts
+    std::tuple<int, int, std::vector<int>> take_counts(int num_local_experts);
     // orders the kernels of a call on `stream` behind those of this runtime's previous call
     void order_behind_last_call(const at::cuda::CUDAStream& stream);
 

@@ -105,12 +105,7 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
 
     // ---- sizes of the outputs
     const int worst_expanded = align_up(T_max * std::min(K, E) + E * (a.expert_alignment - 1), a.expert_alignment);
-    auto read_counts = [&]() {
-        r.num_recv_tokens = wait_count(0, epoch);
-        r.num_expanded_tokens = wait_count(1, epoch);
-        r.num_recv_tokens_per_expert_list.resize(E);
-        for (int e = 0; e < E; ++e) r.num_recv_tokens_per_expert_list[e] = wait_count(2 + e, epoch);
-    };
+    auto read_counts = [&]() { std::tie(r.num_recv_tokens, r.num_expanded_tokens, r.num_recv_tokens_per_expert_list) = take_counts(E); };
     // The exact sizes are known when the plan kernel has run. The move kernel does not wait for the host to learn them:
     // it gets outputs that hold the most rows these tokens can have (every token, every pair plus the alignment gaps),
     // which are cut to their real length afterwards. Only where the row count is part of a stride (column-major scales) or
@@ -217,7 +212,11 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     std::vector<at::Tensor> touched = {r.recv_x, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert, r.num_unaligned, r.recv_src_metadata, a.x, topk_idx};
     for (const auto& t : {r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.topk_idx, a.sf, a.topk_weights, a.cumulative_stats})
         if (t.has_value()) touched.push_back(*t);
-    if (cut) {
+    if (cut && a.defer_counts) {
+        r.counts_pending = true;
+        r.num_recv_tokens = idx_bound;
+        r.num_expanded_tokens = rows_bound;
+    } else if (cut) {
         read_counts();
         const int rows = a.do_expand ? r.num_expanded_tokens : r.num_recv_tokens;
         auto shorten = [](at::Tensor& t, int n) { if (t.size(0) != n) t = t.narrow(0, 0, n); };
@@ -229,6 +228,13 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     }
     r.event = scope.finish(a.sc, touched);
     return r;
+}
+
+std::tuple<int, int, std::vector<int>> Runtime::take_counts(int num_local_experts) {
+    std::vector<int> per_expert(num_local_experts);
+    const int tokens = wait_count(0, dispatch_epoch), rows = wait_count(1, dispatch_epoch);
+    for (int e = 0; e < num_local_experts; ++e) per_expert[e] = wait_count(2 + e, dispatch_epoch);
+    return {tokens, rows, std::move(per_expert)};
 }
 
 CombineResult Runtime::combine_single(CombineArgs& a) {

@@ -45,6 +45,8 @@ class MoEConfig:
 def quantize_weight_128x128(w: torch.Tensor, pow2: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
     """``[G, N, K]`` -> (e4m3 ``[G, N, K]``, fp32 scales ``[G, N / 128, K / 128]``); ``pow2`` rounds the scales up to
     powers of two."""
+    if w.is_cuda and w.dtype == torch.bfloat16 and _C is not None:
+        return _C.quant_weights_128x128(w.contiguous(), pow2)
     G, N, K = w.shape
     blocks = w.float().view(G, N // 128, 128, K // 128, 128)
     amax = blocks.abs().amax(dim=(2, 4)).clamp(1e-4)
@@ -65,8 +67,8 @@ class ExpertWeights:
 
     def refresh(self) -> None:
         """Rebuilds the transposed (for data gradients) and quantised (for FP8 forward) copies after an update."""
-        self.w13_t = self.w13.transpose(1, 2).contiguous()     # [EL, hidden, 2I]
-        self.w2_t = self.w2.transpose(1, 2).contiguous()       # [EL, I, hidden]
+        self.w13_t = _C.transpose_bf16(self.w13)               # [EL, hidden, 2I]
+        self.w2_t = _C.transpose_bf16(self.w2)                 # [EL, I, hidden]
         if self.use_fp8:
             self.w13_q, self.w13_sf = quantize_weight_128x128(self.w13, self.pow2_scales)
             self.w2_q, self.w2_sf = quantize_weight_128x128(self.w2, self.pow2_scales)
@@ -79,7 +81,9 @@ class _SingleRankComm:
         self.buffers = [buffer]
 
     def dispatch(self, per_rank_kwargs):
-        return [self.buffers[0].dispatch(**per_rank_kwargs[0])]
+        buf, kw = self.buffers[0], per_rank_kwargs[0]
+        call = buf._dispatch_call(**kw)
+        return [buf._dispatch_result(_C.Runtime.dispatch([buf.runtime], [call])[0], call, kw.get('handle'))]
 
     def combine(self, per_rank_kwargs):
         return [self.buffers[0].combine(**per_rank_kwargs[0])]
@@ -88,7 +92,9 @@ class _SingleRankComm:
 def route(logits: torch.Tensor, num_topk: int) -> Tuple[torch.Tensor, torch.Tensor]:
     """Top-k experts and softmax weights over the selected logits (hand-written kernel)."""
     require_native()
-    return _C.router_topk(logits.float().contiguous(), num_topk)
+    if logits.dtype not in (torch.float32, torch.bfloat16) or logits.stride(1) != 1:
+        logits = logits.float().contiguous()
+    return _C.router_topk(logits, num_topk)
 
 
 def moe_forward(comm, weights: Sequence[ExpertWeights], xs: Sequence[torch.Tensor], topk_idx: Sequence[torch.Tensor],
@@ -99,7 +105,7 @@ def moe_forward(comm, weights: Sequence[ExpertWeights], xs: Sequence[torch.Tenso
     # writes them. The backward pass contracts over rows and makes its own zeros there (for bf16 the dispatch does).
     out = comm.dispatch([dict(x=xs[r], topk_idx=topk_idx[r], topk_weights=topk_weights[r], num_experts=cfg.num_experts,
                               expert_alignment=cfg.expert_alignment, do_expand=True, do_zero_padding=not cfg.use_fp8, num_sms=cfg.num_sms,
-                              fused_fp8=cfg.use_fp8, round_scale=cfg.use_fp8 and cfg.pow2_scales) for r in range(R)])
+                              fused_fp8=cfg.use_fp8, round_scale=cfg.use_fp8 and cfg.pow2_scales, defer_counts=True) for r in range(R)])
     ctxs, h2s = [], []
     for r in range(R):
         recv_x, _, recv_w, handle, _ = out[r]
@@ -118,6 +124,13 @@ def moe_forward(comm, weights: Sequence[ExpertWeights], xs: Sequence[torch.Tenso
         h2s.append(h2)
         ctxs.append(dict(recv_x=recv_x, recv_w=recv_w, handle=handle, h1=h1))
     comb = comm.combine([dict(x=h2s[r], handle=ctxs[r]['handle']) for r in range(R)])
+    # With one rank nothing above waited for the host to learn the row counts: the whole layer is queued by now.
+    for r, c in enumerate(ctxs):
+        if c['handle']._counts_pending:
+            comm.buffers[r]._finish_counts(c['handle'])
+            rows = c['handle'].num_expanded_tokens
+            c['recv_x'] = tuple(t[:rows] for t in c['recv_x']) if isinstance(c['recv_x'], tuple) else c['recv_x'][:rows]
+            c['recv_w'], c['h1'] = c['recv_w'][:rows], c['h1'][:rows]
     return [c[0] for c in comb], ctxs
 
 
@@ -166,36 +179,18 @@ class _RouterFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, router, num_topk):
-        E = router.size(0)
-        router_bf16 = router.detach().to(torch.bfloat16)
-        if E % 128 != 0:                                                        # the GEMM tiles N in multiples of 128: zero rows
-            router_bf16 = torch.nn.functional.pad(router_bf16, (0, 0, 0, -(-E // 128) * 128 - E))
-        router_bf16 = router_bf16.contiguous()
-        logits = _C.gemm(x.detach().contiguous(), router_bf16)[:, :E]          # [T, E] bf16
-        topk_idx, topk_weights = _C.router_topk(logits.float().contiguous(), num_topk)
+        topk_idx, topk_weights, router_bf16 = _C.router_forward(x.detach().contiguous(), router.detach().contiguous(), num_topk)
         ctx.save_for_backward(x, router_bf16, topk_idx, topk_weights)
-        ctx.router_dtype, ctx.num_experts = router.dtype, E
+        ctx.router_dtype, ctx.num_experts = router.dtype, router.size(0)
         ctx.mark_non_differentiable(topk_idx)
         return topk_idx, topk_weights
 
     @staticmethod
     def backward(ctx, _d_idx, d_weights):
+        # d logit_k = w_k * (dw_k - sum_j w_j dw_j) on the selected experts; dx = dlogits @ W_r, dW_r = dlogits^T @ x
         x, router_bf16, topk_idx, w = ctx.saved_tensors
-        T, E = x.size(0), router_bf16.size(0)                                  # E: padded to a multiple of 128
-        # d logit_k = w_k * (dw_k - sum_j w_j dw_j) on the selected experts
-        inner = (w * d_weights).sum(dim=1, keepdim=True)
-        d_sel = (w * (d_weights - inner)).to(torch.bfloat16)
-        d_logits = torch.zeros((T, E), dtype=torch.bfloat16, device=x.device)
-        d_logits.scatter_(1, topk_idx.clamp(min=0), torch.where(topk_idx >= 0, d_sel, torch.zeros_like(d_sel)))
-        pad_t = -(-T // 64) * 64                                               # the GEMM wants K (here: tokens) in multiples of 64
-        if pad_t != T:
-            d_logits = torch.nn.functional.pad(d_logits, (0, 0, 0, pad_t - T))
-            x_p = torch.nn.functional.pad(x.detach(), (0, 0, 0, pad_t - T))
-        else:
-            x_p = x.detach()
-        dx = _C.gemm(d_logits[:T].contiguous(), _C.transpose_bf16(router_bf16))                         # [T, H] = dlogits @ W_r
-        d_router = _C.gemm(_C.transpose_bf16(d_logits), _C.transpose_bf16(x_p.contiguous()))             # [E, H] = dlogits^T @ x
-        return dx, d_router[:ctx.num_experts].to(ctx.router_dtype), None
+        dx, d_router = _C.router_backward(x.detach().contiguous(), router_bf16, topk_idx, w, d_weights.contiguous(), ctx.num_experts)
+        return dx, d_router.to(ctx.router_dtype), None
 
 
 class _MoEFunction(torch.autograd.Function):

@@ -53,7 +53,15 @@ class EngramStore:
             self.buffer.barrier()
 
     def fetch(self, indices: torch.Tensor, use_tma_aligned_col_major_sf: bool = False, num_sms: int = 0) -> Callable:
-        return EngramStore.multi_fetch([self], [indices], use_tma_aligned_col_major_sf, num_sms)[0]
+        if num_sms > 0:
+            return EngramStore.multi_fetch([self], [indices], use_tma_aligned_col_major_sf, num_sms)[0]
+        data, sf, done = _C.engram_fetch_one(self.rt, indices.contiguous(), self.table_offset, self.entries_per_rank, self.hidden, self.dtype,
+                                             self.sf, use_tma_aligned_col_major_sf, list(self.buffer.host_segments) if self.on_host else [])
+
+        def hook():
+            done.current_stream_wait()
+            return data, sf
+        return hook
 
     @staticmethod
     def multi_fetch(stores: List['EngramStore'], indices: Sequence[torch.Tensor], col_major_sf: bool = False,

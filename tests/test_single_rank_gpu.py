@@ -195,3 +195,31 @@ def test_low_latency_against_the_oracle(T, H, E, K, mode, hook):
             assert (out.float() - ref).norm() <= tol * ref.norm() + 1e-6
     assert torch.equal(stats, torch.stack([(idx == e).sum() for e in range(E)]).int() * 2)
     buf.destroy()
+
+
+@pytest.mark.parametrize('hidden,fp8', [(8, False), (520, False), (2048, False), (48, True), (1040, True)])
+def test_engram_fetch_from_local_memory(hidden, fp8):
+    """Rows that end inside a warp's kilobyte, on and off 32-byte boundaries; indices outside the table fetch nothing."""
+    import deepep_b200
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    entries = 300
+    dtype = torch.float8_e4m3fn if fp8 else torch.bfloat16
+    buf = deepep_b200.ElasticBuffer(SingleProcessGroup(), num_bytes=deepep_b200.ElasticBuffer.get_engram_storage_size_hint(entries, hidden), num_gpu_timeout_secs=5)
+    g = torch.Generator(device='cuda').manual_seed(hidden)
+    table = torch.randn((entries, hidden), device='cuda', generator=g).to(dtype)
+    sf = torch.rand((entries, 3), device='cuda', generator=g) if fp8 else None
+    buf.engram_write(table, sf)
+    idx = torch.randint(0, entries, (37, 3), device='cuda', generator=g, dtype=torch.int32)
+    flat = idx.flatten().long()
+    for _ in range(2):
+        data, got = buf.engram_fetch(idx, use_tma_aligned_col_major_sf=fp8)()
+        assert torch.equal(data.view(torch.uint8), table.view(torch.uint8)[flat])
+        assert got is None or torch.equal(got, sf[flat].view(37, 9))
+    bad = idx.clone()
+    bad[5, 1], bad[6, 2] = -1, entries
+    data, _ = buf.engram_fetch(bad)()
+    keep = (bad.flatten() >= 0) & (bad.flatten() < entries)
+    assert torch.equal(data.view(torch.uint8)[keep], table.view(torch.uint8)[flat[keep]])
+    torch.cuda.synchronize()
+    buf.check_status()
+    buf.destroy()
