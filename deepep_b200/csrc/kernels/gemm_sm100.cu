@@ -6,6 +6,7 @@
 //
 // The reference library contains no GEMM; this is the compute half of the fused MoE layer and of
 // the all-gather -> GEMM / GEMM -> reduce-scatter operators (tp_fused.cu).
+#include <algorithm>
 #include <cstdlib>
 
 #include "api.hpp"
@@ -17,6 +18,10 @@ namespace gemm {
 
 namespace {
 
+// How the MMA issuers work: the whole warp walks the pipeline and one elected lane issues, the next barriers are tested before
+// this k-block's instructions go out, and with an accumulator pass per k-block (software-scaled e4m3) one commit frees the
+// stage and announces the pass. With one lane walking, testing and committing twice, a k-block cost the issuer 950 cycles,
+// twice what the tensor pipe needs for it. (The bf16 pair kernel, whose k-block is longer, keeps the plain form: 1 % faster.)
 struct Tile {
     int g, m0, m_end, n0;
     int kb0, kb1;       // k-blocks [kb0, kb1) of this tile (all of K unless the problem is grouped along K)
@@ -96,6 +101,34 @@ struct Cfg {
     static constexpr int kTmemCols = kAccStages * BN;
 };
 
+// Sums of accumulator passes, two per 64-bit register: fma.rn.f32x2 rounds each half like fmaf and takes half the issue slots,
+// which is what the epilogue warps of the software-scaled kernels are short of.
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+    return v;
+}
+template <int N>
+__device__ __forceinline__ void fold(uint64_t* sum, const uint32_t (&r)[N], float scale) {
+    const uint64_t s2 = pack2(__float_as_uint(scale), __float_as_uint(scale));
+#pragma unroll
+    for (int i = 0; i < N; i += 2) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[i / 2]) : "l"(pack2(r[i], r[i + 1])), "l"(s2));
+}
+__device__ __forceinline__ void unpack_sums(const uint64_t* sum, bool zero, uint32_t (&r)[32]) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = zero ? 0u : static_cast<uint32_t>(sum[i / 2] >> (32 * (i & 1)));
+}
+
+// Rows of a K-major A tile that the problem has (rows past the group's end give outputs that nobody stores): a tile with few
+// of them is loaded in boxes of 32 rows. A decode batch has a handful of rows per expert, and the full box doubled what its
+// tiles pull out of L2 (32 experts of 16 rows, 4096 x 7168 e4m3: 185 us with full boxes).
+constexpr int kSmallBox = 32, kMaxSmallRows = 96;
+__device__ __forceinline__ int small_boxes(int rows) { return rows <= kMaxSmallRows ? ceil_div(rows, kSmallBox) : 0; }
+__device__ __forceinline__ void load_rows(uint8_t* dst, const CUtensorMap* map, const CUtensorMap* map_small, int boxes, int k, int row, uint64_t* bar) {
+    if (boxes == 0) tma_load_2d(dst, map, k, row, bar);
+    else for (int i = 0; i < boxes; ++i) tma_load_2d(dst + i * (kSmallBox * 128), map_small, k, row + i * kSmallBox, bar);
+}
+
 // Loads one operand tile of `rows` rows (K-major: one box) or `rows` columns of a [K, MN] matrix (MN-major: boxes of 64 x 64).
 template <bool kMN>
 __device__ __forceinline__ void load_operand(uint8_t* dst, const CUtensorMap* map, int k, int mn, int rows, uint64_t* bar) {
@@ -116,7 +149,8 @@ __device__ __forceinline__ void load_operand_pair(uint8_t* dst, const CUtensorMa
 
 template <int BN, bool kFp8, bool kAMN = false, bool kBMN = false>
 __global__ void __launch_bounds__(Cfg<BN, kFp8>::kThreads, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a32,
+            const GemmParams p) {
     using C = Cfg<BN, kFp8>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -165,58 +199,71 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
                 // (an MN-major B of a plain problem; group g of a grouped one starts at row g * K of the stacked [K, N] matrices)
                 const int b_row = (p.k_grouped || kBMN ? 0 : t.g * p.N) + t.n0, b_k = kBMN && !p.k_grouped ? t.g * p.K : 0;
+                const int boxes = kAMN ? 0 : small_boxes(t.m_end - t.m0);
+                const uint32_t bytes = boxes == 0 ? C::STAGE : boxes * (kSmallBox * 128) + C::B_BYTES;
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
                     if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
                     uint8_t* sa = smem + s * C::STAGE;
-                    mbar_arrive_expect_tx(full + s, C::STAGE);
-                    load_operand<kAMN>(sa, &map_a, kb * C::BK, t.m0, BM, full + s);
+                    mbar_arrive_expect_tx(full + s, bytes);
+                    if constexpr (kAMN) load_operand<kAMN>(sa, &map_a, kb * C::BK, t.m0, BM, full + s);
+                    else load_rows(sa, &map_a, &map_a32, boxes, kb * C::BK, t.m0, full + s);
                     load_operand<kBMN>(sa + C::A_BYTES, &map_b, b_k + kb * C::BK, b_row, BN, full + s);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            Scheduler sched(p, BN, BM, C::BK);
-            Tile t;
-            constexpr uint32_t idesc = make_idesc<kFp8>(BM, BN, kAMN, kBMN);
-            int s = 0, acc = 0;
-            uint32_t ph = 0, acc_ph = 0;
-            bool ok = true;
-            for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
-                if constexpr (!kFp8) {
-                    if (!(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
-                    tc_fence_after();
+        // ------------------------------------------------------------ MMA issuer (see the note at the top)
+        Scheduler sched(p, BN, BM, C::BK);
+        Tile t;
+        constexpr uint32_t idesc = make_idesc<kFp8>(BM, BN, kAMN, kBMN);
+        const uint64_t da0 = kAMN ? make_smem_desc_mn(smem) : make_smem_desc(smem);
+        const uint64_t db0 = kBMN ? make_smem_desc_mn(smem + C::A_BYTES) : make_smem_desc(smem + C::A_BYTES);
+        int s = 0, acc = 0;
+        uint32_t ph = 0, acc_ph = 0;
+        bool ok = true, full_seen = false, empty_seen = false;
+        for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
+            if constexpr (!kFp8) {
+                if (!(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
+            }
+            for (int kb = t.kb0; kb < t.kb1; ++kb) {
+                if constexpr (kFp8) {
+                    if (!empty_seen && !(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
                 }
-                for (int kb = t.kb0; kb < t.kb1; ++kb) {
-                    if constexpr (kFp8) {
-                        if (!(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
-                    }
-                    if (!(ok = pipe_wait(pc, full + s, ph))) break;
-                    tc_fence_after();
-                    const uint8_t* sa = smem + s * C::STAGE;
-                    const uint64_t da = kAMN ? make_smem_desc_mn(sa) : make_smem_desc(sa);
-                    const uint64_t db = kBMN ? make_smem_desc_mn(sa + C::A_BYTES) : make_smem_desc(sa + C::A_BYTES);
-                    const uint32_t d_addr = tmem_base + acc * BN;
+                if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
+                tc_fence_after();
+                const int s1 = s + 1 == C::kStages ? 0 : s + 1;
+                const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
+                full_seen = mbar_test_wait(full + s1, ph1);
+                int acc1 = acc;
+                uint32_t acc_ph1 = acc_ph;
+                if constexpr (kFp8) {
+                    acc1 = acc + 1 == C::kAccStages ? 0 : acc + 1;
+                    acc_ph1 = acc1 == 0 ? acc_ph ^ 1 : acc_ph;
+                    empty_seen = mbar_test_wait(tmem_empty + acc1, acc_ph1 ^ 1);
+                }
+                const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
+                const uint32_t d_addr = tmem_base + acc * BN;
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < C::BK / C::UMMA_K; ++k) {
                         const uint32_t accumulate = kFp8 ? (k != 0) : (kb != t.kb0 || k != 0);
                         umma<kFp8>(d_addr, da + (kAMN ? 128 : 2) * k, db + (kBMN ? 128 : 2) * k, idesc, accumulate);
                     }
-                    umma_commit(empty + s);
-                    if (++s == C::kStages) { s = 0; ph ^= 1; }
-                    if constexpr (kFp8) {
-                        umma_commit(tmem_full + acc);
-                        if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
-                    }
+                    umma_commit(empty + s);         // (FP8: also tells the epilogue that this pass is complete)
                 }
-                if constexpr (!kFp8) {
-                    if (!ok) break;
+                s = s1;
+                ph = ph1;
+                acc = acc1;
+                acc_ph = acc_ph1;
+            }
+            if constexpr (!kFp8) {
+                if (!ok) break;
+                if (elect_one()) {
                     if (t.kb1 > t.kb0) umma_commit(tmem_full + acc);
                     else mbar_arrive(tmem_full + acc);        // an empty k range: nothing was issued, the epilogue writes zeros
-                    if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
                 }
+                if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
             }
         }
     } else {
@@ -226,9 +273,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         constexpr int kCols = kFp8 ? BN / 4 : BN;      // columns per thread
         Scheduler sched(p, BN, BM, C::BK);
         Tile t;
-        int acc = 0;
-        uint32_t acc_ph = 0;
-        bool ok = true;
+        int acc = 0, s = 0;
+        uint32_t acc_ph = 0, ph = 0;
+        bool ok = true, seen = false;
         for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
             const int row = t.m0 + quarter * 32 + lane;
             const bool row_ok = row < t.m_end && row < p.M;
@@ -259,19 +306,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 mbar_arrive(tmem_empty + acc);
                 if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
             } else {
-                float sum[kCols];
+                static_assert(kCols == 32, "the FP8 epilogue is written for 32 columns per thread");
+                uint64_t sum[kCols / 2];
 #pragma unroll
-                for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
-                const int kblocks_b = p.K / 128;
-                const float* sfb = p.sfb + (static_cast<int64_t>(t.g) * (p.N / 128) + t.n0 / 128) * kblocks_b;
+                for (int i = 0; i < kCols / 2; ++i) sum[i] = 0ull;
+                const float* sfb = p.sfb + (static_cast<int64_t>(t.g) * (p.N / 128) + t.n0 / 128) * num_kb;
                 const float* sfa = p.sfa + static_cast<int64_t>(row_ok ? row : 0) * p.sfa_row_stride;
                 float next_scale = sfa[0] * sfb[0];
                 for (int kb = 0; kb < num_kb; ++kb) {
                     const float scale = next_scale;
                     if (kb + 1 < num_kb) next_scale = sfa[static_cast<int64_t>(kb + 1) * p.sfa_k_stride] * sfb[kb + 1];
-                    if (!(ok = pipe_wait(pc, tmem_full + acc, acc_ph))) break;
+                    // The commit that frees stage s of the ring. (At most kAccStages <= kStages passes are ahead of this warp: the
+                    // barrier cannot have completed another phase meanwhile.)
+                    static_assert(C::kAccStages <= C::kStages, "the stage barrier would lap the epilogue");
+                    if (!seen && !(ok = pipe_wait(pc, empty + s, ph))) break;
+                    if (++s == C::kStages) { s = 0; ph ^= 1; }
                     tc_fence_after();
-                    static_assert(kCols == 32, "the FP8 epilogue is written for 32 columns per thread");
                     uint32_t r0[32];
                     tmem_ld_32x32(lane_addr + acc * BN + part * kCols, r0);
                     tmem_ld_wait();
@@ -279,22 +329,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tmem_empty + acc);      // the values are in registers: the accumulator can be reused
                     if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) sum[i] = fmaf(scale, __uint_as_float(r0[i]), sum[i]);
+                    seen = mbar_test_wait(empty + s, ph);              // (asked before the sums, needed after them)
+                    fold(sum, r0, scale);
                 }
-                if (ok && zero_row) {
-#pragma unroll
-                    for (int v = 0; v < kCols / 8; ++v) *reinterpret_cast<int4*>(c_row + v * 8) = make_int4(0, 0, 0, 0);
-                }
-                if (ok && row_ok) {
-#pragma unroll
-                    for (int v = 0; v < kCols / 8; ++v) {
-                        int4 out;
-                        __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(sum[v * 8 + 2 * i], sum[v * 8 + 2 * i + 1]);
-                        *reinterpret_cast<int4*>(c_row + v * 8) = out;
-                    }
+                if (ok && (row_ok || zero_row)) {
+                    uint32_t r[32];
+                    unpack_sums(sum, zero_row, r);
+                    store_row32(c_row, r, p.c_wide != 0);
                 }
             }
         }
@@ -314,7 +355,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 // per flop), the leader's MMA warp issues tcgen05.mma.cta_group::2 (M = 256), each CTA's epilogue warps drain the
 // 128 accumulator rows in their own tensor memory. Barriers: `full` lives in the leader and counts the bytes of both
 // CTAs; `empty` and `tmem_full` are signalled in both CTAs by one multicast commit; the leader's `tmem_empty`
-// collects the epilogue threads of both CTAs.
+// collects the epilogue warps of both CTAs.
 struct PairCfg {
     static constexpr int BN = 256, BK = 64, UMMA_K = 16;
     static constexpr int A_BYTES = BM * 128, B_BYTES = (BN / 2) * 128, STAGE = A_BYTES + B_BYTES;
@@ -343,7 +384,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t cta = cluster_ctarank();
     const bool leader = cta == 0;
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    const int num_kb = p.K / C::BK;
     PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
 
     if (warp == 0 && lane == 0) {
@@ -355,7 +395,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         for (int a = 0; a < C::kAccStages; ++a) {
             mbar_init(tmem_full + a, 1);
-            mbar_init(tmem_empty + a, 2 * C::kEpiWarps * 32);
+            mbar_init(tmem_empty + a, 2 * C::kEpiWarps);
         }
         fence_mbar_init();
     }
@@ -458,7 +498,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
             }
             tc_fence_before();
-            mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty + acc), 0));
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(tmem_empty + acc), 0));     // (the loads have completed: tcgen05.wait::ld)
             if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
         }
     }
@@ -472,23 +513,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 }
 
 // ==================================================================== CTA-pair kernel, e4m3 with software block scaling (256 x 256 tiles)
-// Same division of labour as gemm_pair_kernel; a stage holds a 128-wide k-block (128 bytes per row), and every
-// k-block is an accumulator pass of its own (two passes fit into the 512 columns of tensor memory): the leader
-// commits the pass, the sixteen epilogue warps of each CTA -- four lane quarters x four column quarters of 64 --
-// drain it sixteen columns at a time and add it, times the product of the 1x128 scale of the row and the 128x128
-// scale of the weight block, to fp32 sums in registers. Per flop a pair loads a third less than two lone CTAs with
-// 128 x 128 tiles would, which is what the FP8 rate needs: the main loop is bound by the fill of shared memory.
+// Same division of labour as gemm_pair_kernel; a stage holds a 128-wide k-block (128 bytes per row), and every k-block is an
+// accumulator pass of its own (two passes fit into the 512 columns of tensor memory): the leader commits the pass, the
+// sixteen epilogue warps of each CTA -- four lane quarters x four column quarters of 64 -- take it into registers sixteen
+// columns at a time and add it, times the product of the 1x128 scale of the row and the 128x128 scale of the weight block,
+// to fp32 sums.
+// What bounds it: the chain of one epilogue warp per pass (wait, four tensor-memory loads, the sums), 1300 cycles against 512
+// of the tensor pipe at first. Hence: paired FMAs; the next barrier and scale asked for before the sums that precede their
+// use; loads and sums alternate; scales come through a shared-memory ring that two warps of their own fill (read by the
+// epilogue warps, one row per lane, they took 512 L1 cycles per pass); the second CTA's sixteen arrivals per pass travel as
+// one. Passes of 128 columns, four in flight, were slower (619 against 525 us for 8 x 2048 x 4096 x 7168): the chain has the
+// same length and there are twice as many.
 struct PairFp8Cfg {
     static constexpr int BN = 256, BK = 128, UMMA_K = 32;
     static constexpr int A_BYTES = BM * 128, B_BYTES = (BN / 2) * 128, STAGE = A_BYTES + B_BYTES;
     static constexpr int kStages = 6;
     static constexpr int kAccStages = 2;
-    static constexpr int kEpiWarps = 16;
-    static constexpr int kThreads = (2 + kEpiWarps) * 32;
-    static constexpr int kBarBytes = (2 * kStages + 2 * kAccStages) * 8 + 16;
-    static constexpr int kSmem = kStages * STAGE + kBarBytes + 1024;
+    static constexpr int kEpiWarps = 16, kSfWarps = 2;
+    static constexpr int kThreads = (2 + kEpiWarps + kSfWarps) * 32;
+    static constexpr int kSfChunk = 8, kSfStages = 4;                       // k-blocks per ring slot, slots
+    static constexpr int kSfPitch = BM + 4;                                 // floats per k-block: 128 rows of A, 2 blocks of B
+    static constexpr int kSfBytes = kSfStages * kSfChunk * kSfPitch * 4;
+    static constexpr int kBarBytes = (2 * kStages + 2 * kAccStages + 2 * kSfStages) * 8 + 16;
+    static constexpr int kSmem = kStages * STAGE + kSfBytes + kBarBytes + 1024;
     static constexpr int kTmemCols = kAccStages * BN;
-    static constexpr int kColsPerThread = BN / 4;
+    // 640 threads are launched with 96 registers each (61440); the epilogue's four warpgroups take 104, the fifth keeps 64:
+    // 512 x 104 + 128 x 64 = 61440
+    static constexpr int kEpiRegs = 104, kOtherRegs = 64;
+    static constexpr int kTmaWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1, kSfWarp = kEpiWarps + 2;
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairFp8Cfg::kThreads, 1)
@@ -496,11 +548,14 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     using C = PairFp8Cfg;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kStages * C::STAGE);
+    float* sf_ring = reinterpret_cast<float*>(smem + C::kStages * C::STAGE);          // [slots][k-blocks][rows of A, 2 of B]
+    uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sf_ring) + C::kSfBytes);
     uint64_t* empty = full + C::kStages;
-    uint64_t* tmem_full = empty + C::kStages;
-    uint64_t* tmem_empty = tmem_full + C::kAccStages;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + C::kAccStages);
+    uint64_t* tmem_empty = empty + C::kStages;
+    uint64_t* tmem_drained = tmem_empty + C::kAccStages;       // the second CTA's own count of its epilogue warps
+    uint64_t* sf_full = tmem_drained + C::kAccStages;
+    uint64_t* sf_empty = sf_full + C::kSfStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sf_empty + C::kSfStages);
 
     const int warp = warp_id(), lane = lane_id();
     const uint32_t cta = cluster_ctarank();
@@ -509,7 +564,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int num_kb = p.K / C::BK;
     PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
 
-    if (warp == 0 && lane == 0) {
+    if (warp == C::kTmaWarp && lane == 0) {
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_b);
         for (int s = 0; s < C::kStages; ++s) {
@@ -517,12 +572,16 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             mbar_init(empty + s, 1);
         }
         for (int a = 0; a < C::kAccStages; ++a) {
-            mbar_init(tmem_full + a, 1);
-            mbar_init(tmem_empty + a, 2 * C::kEpiWarps);      // one arrival per epilogue warp of either CTA and k-block
+            mbar_init(tmem_empty + a, C::kEpiWarps + 1);      // the leader's epilogue warps and the second CTA's relay
+            mbar_init(tmem_drained + a, C::kEpiWarps);
+        }
+        for (int i = 0; i < C::kSfStages; ++i) {
+            mbar_init(sf_full + i, C::kSfWarps);
+            mbar_init(sf_empty + i, C::kEpiWarps);
         }
         fence_mbar_init();
     }
-    if (warp == 1) {
+    if (warp == C::kMmaWarp) {
         tmem_alloc_pair(tmem_slot, C::kTmemCols);
         tmem_relinquish_pair();
     }
@@ -531,105 +590,191 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
-            Scheduler sched(p, C::BN, 2 * BM, C::BK);
-            Tile t;
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
-                    uint8_t* sa = smem + s * C::STAGE;
-                    if (leader) mbar_arrive_expect_tx(full + s, 2 * C::STAGE);
-                    const uint32_t bar = map_to_cta(smem_u32(full + s), 0);
-                    tma_load_2d_pair(sa, &map_a, kb * C::BK, t.m0 + static_cast<int>(cta) * BM, bar);
-                    tma_load_2d_pair(sa + C::A_BYTES, &map_b, kb * C::BK, t.g * p.N + t.n0 + static_cast<int>(cta) * (C::BN / 2), bar);
-                    if (++s == C::kStages) { s = 0; ph ^= 1; }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer (leader only): one accumulator pass per k-block
-        if (leader && lane == 0) {
-            Scheduler sched(p, C::BN, 2 * BM, C::BK);
-            Tile t;
-            constexpr uint32_t idesc = make_idesc<true>(2 * BM, C::BN);
-            int s = 0, acc = 0;
-            uint32_t ph = 0, acc_ph = 0;
-            bool ok = true;
-            for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
-                    if (!(ok = pipe_wait(pc, full + s, ph))) break;
-                    tc_fence_after();
-                    const uint8_t* sa = smem + s * C::STAGE;
-                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + C::A_BYTES);
-                    const uint32_t d_addr = tmem_base + acc * C::BN;
+    if (warp < C::kEpiWarps) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kEpiRegs));
+        // ------------------------------------------------------------ epilogue warps (both CTAs, own 128 rows)
+        const int quarter = warp & 3;                  // the TMEM lanes this warp may read: [32 * quarter, +32)
+        const int part = warp >> 2;                    // which 64 of the 256 columns
+        Scheduler sched(p, C::BN, 2 * BM, C::BK);
+        Tile t;
+        int acc = 0, slot = 0, s = 0;
+        uint32_t sf_ph = 0, ph = 0;
+        bool ok = true, seen = false;
+        const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
+        uint64_t* my_empty = leader ? tmem_empty : tmem_drained;
+        static_assert(C::kAccStages <= C::kStages, "the stage barrier would lap the epilogue");
+        for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
+            uint64_t sum[32];
 #pragma unroll
-                    for (int k = 0; k < C::BK / C::UMMA_K; ++k) umma_pair_fp8(d_addr, da + 2 * k, db + 2 * k, idesc, k != 0);
-                    umma_commit_pair(empty + s);
-                    umma_commit_pair(tmem_full + acc);
+            for (int i = 0; i < 32; ++i) sum[i] = 0ull;
+            for (int kb0 = 0; ok && kb0 < num_kb; kb0 += C::kSfChunk) {
+                if (!(ok = pipe_wait(pc, sf_full + slot, sf_ph))) break;
+                const float* sf = sf_ring + slot * C::kSfChunk * C::kSfPitch;
+                const int n = min(C::kSfChunk, num_kb - kb0);
+                float scale = sf[quarter * 32 + lane] * sf[BM + (part >> 1)];
+                for (int j = 0; j < n; ++j) {
+                    if (!seen && !(ok = pipe_wait(pc, empty + s, ph))) break;      // the commit that frees stage s
+                    tc_fence_after();
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
-                    if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
+                    const uint32_t addr = lane_addr + acc * C::BN;
+                    uint32_t ra[16], rb[16];
+                    tmem_ld_32x16(addr, ra);
+                    tmem_ld_wait();
+                    tmem_ld_32x16(addr + 16, rb);
+                    fold(sum, ra, scale);
+                    tmem_ld_wait();
+                    tmem_ld_32x16(addr + 32, ra);
+                    fold(sum + 8, rb, scale);
+                    tmem_ld_wait();
+                    tmem_ld_32x16(addr + 48, rb);
+                    fold(sum + 16, ra, scale);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(my_empty + acc);      // the values are in registers: the accumulator can be reused
+                    acc ^= 1;
+                    seen = mbar_test_wait(empty + s, ph);
+                    sf += C::kSfPitch;
+                    float next = 0.f;
+                    if (j + 1 < n) next = sf[quarter * 32 + lane] * sf[BM + (part >> 1)];
+                    fold(sum + 24, rb, scale);
+                    scale = next;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sf_empty + slot);       // (the last scale of the slot has been used)
+                if (++slot == C::kSfStages) { slot = 0; sf_ph ^= 1; }
+            }
+            const int row = t.m0 + static_cast<int>(cta) * BM + quarter * 32 + lane;
+            const bool row_ok = row < t.m_end && row < p.M;
+            const bool zero_row = !row_ok && p.zero_gap && row < p.M && row < align_up(t.m_end, p.group_alignment);
+            if (ok && (row_ok || zero_row)) {
+                __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + part * 64;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t r[32];
+                    unpack_sums(sum + 16 * c, zero_row, r);
+                    store_row32(c_row + c * 32, r, p.c_wide != 0);
                 }
             }
         }
     } else {
-        // ------------------------------------------------------------ epilogue warps (both CTAs, own 128 rows)
-        const int quarter = warp & 3;                  // the TMEM lanes this warp may read: [32 * quarter, +32)
-        const int part = (warp - 2) / 4;               // which quarter of the 256 columns
-        constexpr int kCols = C::kColsPerThread;
-        Scheduler sched(p, C::BN, 2 * BM, C::BK);
-        Tile t;
-        int acc = 0;
-        uint32_t acc_ph = 0;
-        bool ok = true;
-        const int kblocks_b = p.K / 128;
-        for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
-            const int row = t.m0 + static_cast<int>(cta) * BM + quarter * 32 + lane;
-            const bool row_ok = row < t.m_end && row < p.M;
-            const bool zero_row = !row_ok && p.zero_gap && row < p.M && row < align_up(t.m_end, p.group_alignment);
-            const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-            __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + part * kCols;
-            float sum[kCols];
-#pragma unroll
-            for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
-            const float* sfb = p.sfb + (static_cast<int64_t>(t.g) * (p.N / 128) + (t.n0 + part * kCols) / 128) * kblocks_b;
-            const float* sfa = p.sfa + static_cast<int64_t>(row_ok ? row : 0) * p.sfa_row_stride;
-            float next_scale = sfa[0] * sfb[0];
-            for (int kb = 0; kb < num_kb; ++kb) {
-                const float scale = next_scale;
-                if (kb + 1 < num_kb) next_scale = sfa[static_cast<int64_t>(kb + 1) * p.sfa_k_stride] * sfb[kb + 1];
-                if (!(ok = pipe_wait(pc, tmem_full + acc, acc_ph))) break;
-                tc_fence_after();
-#pragma unroll
-                for (int c = 0; c < kCols / 16; ++c) {
-                    uint32_t r[16];
-                    tmem_ld_32x16(lane_addr + acc * C::BN + part * kCols + c * 16, r);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) sum[c * 16 + i] = fmaf(scale, __uint_as_float(r[i]), sum[c * 16 + i]);
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kOtherRegs));
+        if (warp == C::kTmaWarp) {
+            // ------------------------------------------------------------ TMA producer (both CTAs)
+            if (lane == 0) {
+                Scheduler sched(p, C::BN, 2 * BM, C::BK);
+                Tile t;
+                int s = 0;
+                uint32_t ph = 0;
+                bool ok = true;
+                for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
+                    for (int kb = 0; kb < num_kb; ++kb) {
+                        if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
+                        uint8_t* sa = smem + s * C::STAGE;
+                        if (leader) mbar_arrive_expect_tx(full + s, 2 * C::STAGE);
+                        const uint32_t bar = map_to_cta(smem_u32(full + s), 0);
+                        tma_load_2d_pair(sa, &map_a, kb * C::BK, t.m0 + static_cast<int>(cta) * BM, bar);
+                        tma_load_2d_pair(sa + C::A_BYTES, &map_b, kb * C::BK, t.g * p.N + t.n0 + static_cast<int>(cta) * (C::BN / 2), bar);
+                        if (++s == C::kStages) { s = 0; ph ^= 1; }
+                    }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty + acc), 0));
-                if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
             }
-            if (ok && zero_row) {
+        } else if (warp == C::kMmaWarp) {
+            // ------------------------------------------------------------ MMA issuer (leader only)
+            if (leader) {
+                Scheduler sched(p, C::BN, 2 * BM, C::BK);
+                Tile t;
+                constexpr uint32_t idesc = make_idesc<true>(2 * BM, C::BN);
+                const uint64_t da0 = make_smem_desc(smem), db0 = make_smem_desc(smem + C::A_BYTES);
+                int s = 0, acc = 0;
+                uint32_t ph = 0, acc_ph = 0;
+                bool ok = true, full_seen = false, empty_seen = false;
+                for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
+                    for (int kb = 0; kb < num_kb; ++kb) {
+                        if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
+                        if (!empty_seen && !(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
+                        tc_fence_after();
+                        const int s1 = s + 1 == C::kStages ? 0 : s + 1, acc1 = acc ^ 1;
+                        const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph, acc_ph1 = acc1 == 0 ? acc_ph ^ 1 : acc_ph;
+                        full_seen = mbar_test_wait(full + s1, ph1);
+                        empty_seen = mbar_test_wait(tmem_empty + acc1, acc_ph1 ^ 1);
+                        const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
+                        const uint32_t d_addr = tmem_base + acc * C::BN;
+                        if (elect_one()) {
 #pragma unroll
-                for (int v = 0; v < kCols / 8; ++v) *reinterpret_cast<int4*>(c_row + v * 8) = make_int4(0, 0, 0, 0);
+                            for (int k = 0; k < C::BK / C::UMMA_K; ++k) umma_pair_fp8(d_addr, da + 2 * k, db + 2 * k, idesc, k != 0);
+                            umma_commit_pair(empty + s);           // frees the stage and tells the epilogues that this pass is complete
+                        }
+                        s = s1;
+                        ph = ph1;
+                        acc = acc1;
+                        acc_ph = acc_ph1;
+                    }
+                }
+            } else if (!leader && lane == 0) {
+                // relay: sixteen arrivals of this CTA's warps become one across the cluster, where each costs tens of cycles
+                Scheduler sched(p, C::BN, 2 * BM, C::BK);
+                Tile t;
+                int acc = 0;
+                uint32_t acc_ph = 0;
+                bool ok = true;
+                const uint32_t empty_bar = map_to_cta(smem_u32(tmem_empty), 0);
+                for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs)
+                    for (int kb = 0; kb < num_kb; ++kb) {
+                        if (!(ok = pipe_wait(pc, tmem_drained + acc, acc_ph))) break;
+                        mbar_arrive_cluster_relaxed(empty_bar + acc * 8);
+                        if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
+                    }
             }
-            if (ok && row_ok) {
+        } else {
+            // ------------------------------------------------------------ scale warps (both CTAs, own 128 rows)
+            const int tid = (warp - C::kSfWarp) * 32 + lane;
+            const bool vec = p.sfa_k_stride == 1 && p.sfa_row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(p.sfa) & 15) == 0;
+            Scheduler sched(p, C::BN, 2 * BM, C::BK);
+            Tile t;
+            int slot = 0;
+            uint32_t sf_ph = 0;
+            bool ok = true;
+            for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
+                const int last = min(t.m_end, p.M) - 1;
+                const float* src[2];
 #pragma unroll
-                for (int v = 0; v < kCols / 8; ++v) {
-                    int4 out;
-                    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&out);
+                for (int i = 0; i < 2; ++i)      // (rows past the end repeat the last one: their sums are dropped)
+                    src[i] = p.sfa + static_cast<int64_t>(min(t.m0 + static_cast<int>(cta) * BM + tid + i * 64, last)) * p.sfa_row_stride;
+                const float* sfb = p.sfb + (static_cast<int64_t>(t.g) * (p.N / 128) + t.n0 / 128) * num_kb;
+                for (int kb0 = 0; kb0 < num_kb; kb0 += C::kSfChunk) {
+                    const int n = min(C::kSfChunk, num_kb - kb0);
+                    float v[2][C::kSfChunk];
+                    float vb = 0.f;
+                    if (vec && n == C::kSfChunk) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(sum[v * 8 + 2 * i], sum[v * 8 + 2 * i + 1]);
-                    *reinterpret_cast<int4*>(c_row + v * 8) = out;
+                        for (int i = 0; i < 2; ++i)
+#pragma unroll
+                            for (int j = 0; j < C::kSfChunk; j += 4) {
+                                const float4 f = *reinterpret_cast<const float4*>(src[i] + kb0 + j);
+                                v[i][j] = f.x;
+                                v[i][j + 1] = f.y;
+                                v[i][j + 2] = f.z;
+                                v[i][j + 3] = f.w;
+                            }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+#pragma unroll
+                            for (int j = 0; j < C::kSfChunk; ++j) v[i][j] = j < n ? src[i][static_cast<int64_t>(kb0 + j) * p.sfa_k_stride] : 0.f;
+                    }
+                    if (tid < 2 * C::kSfChunk && tid / 2 < n) vb = sfb[static_cast<int64_t>(tid & 1) * num_kb + kb0 + tid / 2];
+                    if (!(ok = pipe_wait(pc, sf_empty + slot, sf_ph ^ 1))) break;
+                    float* dst = sf_ring + slot * C::kSfChunk * C::kSfPitch;
+#pragma unroll
+                    for (int j = 0; j < C::kSfChunk; ++j) {
+                        dst[j * C::kSfPitch + tid] = v[0][j];
+                        dst[j * C::kSfPitch + tid + 64] = v[1][j];
+                    }
+                    if (tid < 2 * C::kSfChunk) dst[(tid / 2) * C::kSfPitch + BM + (tid & 1)] = vb;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sf_full + slot);
+                    if (++slot == C::kSfStages) { slot = 0; sf_ph ^= 1; }
                 }
             }
         }
@@ -637,31 +782,32 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
     tc_fence_before();
     cluster_sync_all();
-    if (warp == 1) {
+    if (warp == C::kMmaWarp) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, C::kTmemCols);
     }
 }
 
-// ---------------------------------------------------------------- host side
 // ==================================================================== e4m3 with hardware block scaling (128 x 256 tiles)
 // For scales that are exact powers of two the tensor core applies them itself (tcgen05.mma kind::mxf8f6f4.block_scale,
 // UE8M0 scale factors in tensor memory), so a tile accumulates over ALL of K in tensor memory and the epilogue runs once
-// per tile instead of once per k-block. Roles: TMA producer, MMA issuer, eight epilogue warps (two per lane quarter, 128
+// per tile instead of once per k-block. Roles: TMA producer, MMA issuer, sixteen epilogue warps (four per lane quarter, 64
 // columns each), four scale warps (one per lane quarter). Per k-block of 128 a scale warp writes the slot of that
 // pipeline stage in tensor memory: 4 columns for the rows of A (1x128 scales: all four 32-wide slices share the byte)
 // and 8 columns for the 256 columns of B (128x128 scales: two bytes per k-block, replicated); `full[s]` collects the
 // producer's bytes and the four scale warps, `empty[s]` (an MMA commit) frees both the shared-memory stage and its
 // scale slot. The scale bytes of a tile are staged in shared memory one tile ahead, so the feed never waits for memory.
 // The accumulator (256 columns) is single-buffered: tensor memory has 512 columns and the scale slots need their own.
+// (128 x 128 tiles with two accumulators were slower at every size, 1594 against 2200 TFLOP/s for long experts: 32 KB from L2
+// per k-block at the 45 to 55 bytes per cycle that an SM gets.)
 struct MxCfg {
     static constexpr int BN = 256, BK = 128, UMMA_K = 32;
-    static constexpr int kEpiWarps = 8, kSfWarps = 4;
+    static constexpr int kEpiWarps = 16, kSfWarps = 4;
     static constexpr int kThreads = (2 + kEpiWarps + kSfWarps) * 32;
     static constexpr int A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE = A_BYTES + B_BYTES;
-    static constexpr int kStages = 4;
+    static constexpr int kStages = 192 * 1024 / STAGE;
     static constexpr int kSfCols = 16;                 // columns per scale slot: 4 (A) + 8 (B), padded to a store of 16
-    static constexpr int kSfBase = BN;                 // first scale column behind the accumulator
+    static constexpr int kSfBase = 256;                // first scale column behind the accumulator
     static constexpr int kTmemCols = 512;
     static constexpr int kMaxKb = 64;                  // k-blocks whose scale bytes fit the staging area (K <= 8192)
     static constexpr int kSfPitch = BM + 16;           // per k-block: 128 bytes for the rows of A, 2 for B
@@ -673,7 +819,8 @@ struct MxCfg {
 __device__ __forceinline__ uint32_t ue8m0_of(float scale) { return (__float_as_uint(scale) >> 23) & 0xffu; }
 
 __global__ void __launch_bounds__(MxCfg::kThreads, 1)
-gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a32,
+               const GemmParams p) {
     using C = MxCfg;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -717,11 +864,13 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
                 const int b_row = t.g * p.N + t.n0;
+                const int boxes = small_boxes(t.m_end - t.m0);
+                const uint32_t bytes = boxes == 0 ? C::STAGE : boxes * (kSmallBox * 128) + C::B_BYTES;
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
                     if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
                     uint8_t* sa = smem + s * C::STAGE;
-                    mbar_arrive_expect_tx(full + s, C::STAGE);
-                    tma_load_2d(sa, &map_a, kb * C::BK, t.m0, full + s);
+                    mbar_arrive_expect_tx(full + s, bytes);
+                    load_rows(sa, &map_a, &map_a32, boxes, kb * C::BK, t.m0, full + s);
                     tma_load_2d(sa + C::A_BYTES, &map_b, kb * C::BK, b_row, full + s);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
@@ -729,37 +878,40 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            Scheduler sched(p, C::BN, BM, C::BK);
-            Tile t;
-            int s = 0;
-            uint32_t ph = 0, acc_ph = 0;
-            bool ok = true;
-            for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
-                if (!(ok = pipe_wait(pc, tmem_empty, acc_ph ^ 1))) break;
+        Scheduler sched(p, C::BN, BM, C::BK);
+        Tile t;
+        const uint64_t da0 = make_smem_desc(smem), db0 = make_smem_desc(smem + C::A_BYTES);
+        int s = 0;
+        uint32_t ph = 0, acc_ph = 0;
+        bool ok = true, full_seen = false;
+        for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
+            if (!(ok = pipe_wait(pc, tmem_empty, acc_ph ^ 1))) break;
+            for (int kb = t.kb0; kb < t.kb1; ++kb) {
+                if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
                 tc_fence_after();
-                for (int kb = t.kb0; kb < t.kb1; ++kb) {
-                    if (!(ok = pipe_wait(pc, full + s, ph))) break;
-                    tc_fence_after();
-                    const uint8_t* sa = smem + s * C::STAGE;
-                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + C::A_BYTES);
-                    const uint32_t sfa = tmem_base + C::kSfBase + s * C::kSfCols, sfb = sfa + 4;
+                const int s1 = s + 1 == C::kStages ? 0 : s + 1;
+                const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
+                full_seen = mbar_test_wait(full + s1, ph1);
+                const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
+                const uint32_t sfa = tmem_base + C::kSfBase + s * C::kSfCols, sfb = sfa + 4;
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < C::BK / C::UMMA_K; ++k)
-                        umma_mx(tmem_base, da + 2 * k, db + 2 * k, make_idesc_mx(BM, C::BN, static_cast<uint32_t>(k)),
-                                (kb != t.kb0 || k != 0) ? 1u : 0u, sfa, sfb);
+                        umma_mx(tmem_base, da + 2 * k, db + 2 * k, make_idesc_mx(BM, C::BN, static_cast<uint32_t>(k)), (kb != t.kb0 || k != 0) ? 1u : 0u, sfa, sfb);
                     umma_commit(empty + s);
-                    if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
-                if (!ok) break;
-                umma_commit(tmem_full);
-                acc_ph ^= 1;
+                s = s1;
+                ph = ph1;
             }
+            if (!ok) break;
+            if (elect_one()) umma_commit(tmem_full);
+            acc_ph ^= 1;
         }
     } else if (warp < 2 + C::kEpiWarps) {
         // ------------------------------------------------------------ epilogue warps: once per tile
         const int quarter = warp & 3;
-        const int half = (warp - 2) / 4;               // which 128 of the 256 columns
+        constexpr int kCols = C::BN / 4;               // columns per warp
+        const int part = (warp - 2) / 4;
         Scheduler sched(p, C::BN, BM, C::BK);
         Tile t;
         uint32_t acc_ph = 0;
@@ -768,24 +920,29 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int row = t.m0 + quarter * 32 + lane;
             const bool row_ok = row < t.m_end && row < p.M;
             const bool zero_row = !row_ok && p.zero_gap && row < p.M;
-            const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * 128;
-            __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + half * 128;
+            const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * kCols;
+            __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + part * kCols;
             if (!(ok = pipe_wait(pc, tmem_full, acc_ph))) break;
             tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                uint32_t r[32];
-                tmem_ld_32x32(lane_addr + c * 32, r);
-                tmem_ld_wait();
-                if (zero_row) {
+            // All of this warp's columns first: the accumulator is free for the next tile before anything is converted or
+            // stored, which costs as much as several k-blocks.
+            uint32_t r[kCols / 32][32];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = 0u;
-                }
-                if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
-            }
+            for (int c = 0; c < kCols / 32; ++c) tmem_ld_32x32(lane_addr + c * 32, r[c]);
+            tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tmem_empty);
+            if (row_ok || zero_row) {
+#pragma unroll
+                for (int c = 0; c < kCols / 32; ++c) {
+                    if (zero_row) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[c][i] = 0u;
+                    }
+                    store_row32(c_row + c * 32, r[c], p.c_wide != 0);
+                }
+            }
             acc_ph ^= 1;
         }
     } else {
@@ -793,14 +950,27 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int quarter = warp & 3;
         const int sf_tid = (warp - 2 - C::kEpiWarps) * 32 + lane;      // 0..127 = the row of the tile this thread stages
         const int kblocks = p.K / 128;
+        const bool vec = p.sfa_k_stride == 1 && kblocks % 4 == 0 && p.sfa_row_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(p.sfa) & 15) == 0;
         Scheduler sched(p, C::BN, BM, C::BK);
         Tile t, nxt;
         auto stage_tile = [&](const Tile& tt, uint8_t* dst) {
             const int row = tt.m0 + sf_tid;
             const bool valid = row < tt.m_end && row < p.M;
             const float* src = p.sfa + static_cast<int64_t>(valid ? row : 0) * p.sfa_row_stride;
-            for (int kb = tt.kb0; kb < tt.kb1; ++kb)
-                dst[(kb - tt.kb0) * C::kSfPitch + sf_tid] = static_cast<uint8_t>(valid ? ue8m0_of(src[static_cast<int64_t>(kb) * p.sfa_k_stride]) : 127u);
+            // (sixteen bytes at a time where they are contiguous: a lane has a row of its own, 32 lines per load)
+            if (vec) {
+#pragma unroll 4
+                for (int kb = 0; kb < kblocks; kb += 4) {
+                    const float4 f = *reinterpret_cast<const float4*>(src + kb);
+                    dst[kb * C::kSfPitch + sf_tid] = static_cast<uint8_t>(valid ? ue8m0_of(f.x) : 127u);
+                    dst[(kb + 1) * C::kSfPitch + sf_tid] = static_cast<uint8_t>(valid ? ue8m0_of(f.y) : 127u);
+                    dst[(kb + 2) * C::kSfPitch + sf_tid] = static_cast<uint8_t>(valid ? ue8m0_of(f.z) : 127u);
+                    dst[(kb + 3) * C::kSfPitch + sf_tid] = static_cast<uint8_t>(valid ? ue8m0_of(f.w) : 127u);
+                }
+            } else {
+                for (int kb = tt.kb0; kb < tt.kb1; ++kb)
+                    dst[(kb - tt.kb0) * C::kSfPitch + sf_tid] = static_cast<uint8_t>(valid ? ue8m0_of(src[static_cast<int64_t>(kb) * p.sfa_k_stride]) : 127u);
+            }
             const float* srcb = p.sfb + (static_cast<int64_t>(tt.g) * (p.N / 128) + tt.n0 / 128) * kblocks;
             for (int i = sf_tid; i < 2 * (tt.kb1 - tt.kb0); i += C::kSfWarps * 32) {
                 const int h = i & 1, kb = tt.kb0 + (i >> 1);
@@ -879,7 +1049,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // both CTAs; the leader's `tmem_empty` collects the epilogue warps of both.
 struct MxPairCfg {
     static constexpr int BN = 256, BK = 128, UMMA_K = 32;
-    static constexpr int kEpiWarps = 8, kSfWarps = 4;
+    static constexpr int kEpiWarps = 16, kSfWarps = 4;
     static constexpr int kThreads = (2 + kEpiWarps + kSfWarps) * 32;
     static constexpr int A_BYTES = BM * 128, B_BYTES = (BN / 2) * 128, STAGE = A_BYTES + B_BYTES;
     static constexpr int kStages = 6;
@@ -887,7 +1057,7 @@ struct MxPairCfg {
     static constexpr int kMaxKb = 64;
     static constexpr int kSfPitch = BM + 16;
     static constexpr int kSfStage = kMaxKb * kSfPitch;
-    static constexpr int kBarBytes = (2 * kStages + 2) * 8 + 16;
+    static constexpr int kBarBytes = (3 * kStages + 3) * 8 + 16;
     static constexpr int kSmem = kStages * STAGE + 2 * kSfStage + kBarBytes + 1024;
 };
 
@@ -901,7 +1071,8 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* empty = full + C::kStages;
     uint64_t* tmem_full = empty + C::kStages;
     uint64_t* tmem_empty = tmem_full + 1;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
+    uint64_t* sf_done = tmem_empty + 1;                  // the second CTA's own count of its scale warps
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sf_done + C::kStages);
 
     const int warp = warp_id(), lane = lane_id();
     const uint32_t cta = cluster_ctarank();
@@ -913,7 +1084,8 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_b);
         for (int s = 0; s < C::kStages; ++s) {
-            mbar_init(full + s, 1 + 2 * C::kSfWarps);
+            mbar_init(full + s, 1 + C::kSfWarps + 1);      // producer (+ bytes), the leader's scale warps, the second CTA's relay
+            mbar_init(sf_done + s, C::kSfWarps);
             mbar_init(empty + s, 1);
         }
         mbar_init(tmem_full, 1);
@@ -952,37 +1124,55 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (leader only)
-        if (leader && lane == 0) {
+        if (leader) {
+            Scheduler sched(p, C::BN, 2 * BM, C::BK);
+            Tile t;
+            const uint64_t da0 = make_smem_desc(smem), db0 = make_smem_desc(smem + C::A_BYTES);
+            int s = 0;
+            uint32_t ph = 0, acc_ph = 0;
+            bool ok = true, full_seen = false;
+            for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
+                if (!(ok = pipe_wait(pc, tmem_empty, acc_ph ^ 1))) break;
+                for (int kb = t.kb0; kb < t.kb1; ++kb) {
+                    if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
+                    tc_fence_after();
+                    const int s1 = s + 1 == C::kStages ? 0 : s + 1;
+                    const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
+                    full_seen = mbar_test_wait(full + s1, ph1);
+                    const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
+                    const uint32_t sfa = tmem_base + C::kSfBase + s * C::kSfCols, sfb = sfa + 4;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < C::BK / C::UMMA_K; ++k)
+                            umma_mx_pair(tmem_base, da + 2 * k, db + 2 * k, make_idesc_mx(2 * BM, C::BN, static_cast<uint32_t>(k)),
+                                         (kb != t.kb0 || k != 0) ? 1u : 0u, sfa, sfb);
+                        umma_commit_pair(empty + s);
+                    }
+                    s = s1;
+                    ph = ph1;
+                }
+                if (!ok) break;
+                if (elect_one()) umma_commit_pair(tmem_full);
+                acc_ph ^= 1;
+            }
+        } else if (!leader && lane == 0) {
+            // relay: the four arrivals of this CTA's scale warps become one across the cluster
             Scheduler sched(p, C::BN, 2 * BM, C::BK);
             Tile t;
             int s = 0;
-            uint32_t ph = 0, acc_ph = 0;
+            uint32_t ph = 0;
             bool ok = true;
-            for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
-                if (!(ok = pipe_wait(pc, tmem_empty, acc_ph ^ 1))) break;
-                tc_fence_after();
+            for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs)
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
-                    if (!(ok = pipe_wait(pc, full + s, ph))) break;
-                    tc_fence_after();
-                    const uint8_t* sa = smem + s * C::STAGE;
-                    const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + C::A_BYTES);
-                    const uint32_t sfa = tmem_base + C::kSfBase + s * C::kSfCols, sfb = sfa + 4;
-#pragma unroll
-                    for (int k = 0; k < C::BK / C::UMMA_K; ++k)
-                        umma_mx_pair(tmem_base, da + 2 * k, db + 2 * k, make_idesc_mx(2 * BM, C::BN, static_cast<uint32_t>(k)),
-                                     (kb != t.kb0 || k != 0) ? 1u : 0u, sfa, sfb);
-                    umma_commit_pair(empty + s);
+                    if (!(ok = pipe_wait(pc, sf_done + s, ph))) break;
+                    mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(full + s), 0));
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
-                if (!ok) break;
-                umma_commit_pair(tmem_full);
-                acc_ph ^= 1;
-            }
         }
     } else if (warp < 2 + C::kEpiWarps) {
         // ------------------------------------------------------------ epilogue warps (both CTAs, own 128 rows), once per tile
         const int quarter = warp & 3;
-        const int half = (warp - 2) / 4;
+        const int part = (warp - 2) / 4;               // which 64 of the 256 columns
         Scheduler sched(p, C::BN, 2 * BM, C::BK);
         Tile t;
         uint32_t acc_ph = 0;
@@ -991,24 +1181,29 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int row = t.m0 + static_cast<int>(cta) * BM + quarter * 32 + lane;
             const bool row_ok = row < t.m_end && row < p.M;
             const bool zero_row = !row_ok && p.zero_gap && row < p.M && row < align_up(t.m_end, p.group_alignment);
-            const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * 128;
-            __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + half * 128;
+            const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
+            __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + part * 64;
             if (!(ok = pipe_wait(pc, tmem_full, acc_ph))) break;
             tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                uint32_t r[32];
-                tmem_ld_32x32(lane_addr + c * 32, r);
-                tmem_ld_wait();
-                if (zero_row) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = 0u;
-                }
-                if (row_ok || zero_row) store_row32(c_row + c * 32, r, p.c_wide != 0);
-            }
+            // All of this warp's columns first: the (only) accumulator is free for the next tile before anything is converted
+            // or stored, which costs as much as several k-blocks.
+            uint32_t r[2][32];
+            tmem_ld_32x32(lane_addr, r[0]);
+            tmem_ld_32x32(lane_addr + 32, r[1]);
+            tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(tmem_empty), 0));
+            if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(tmem_empty), 0));
+            if (row_ok || zero_row) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    if (zero_row) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[c][i] = 0u;
+                    }
+                    store_row32(c_row + c * 32, r[c], p.c_wide != 0);
+                }
+            }
             acc_ph ^= 1;
         }
     } else {
@@ -1072,11 +1267,8 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    for (int j = 0; j < n; ++j) {
-                        // (the stores are complete: tcgen05.wait::st above; the arrival only has to get there)
-                        if (leader) mbar_arrive(full + sj[j]);
-                        else mbar_arrive_cluster_relaxed(map_to_cta(smem_u32(full + sj[j]), 0));
-                    }
+                    // (the stores are complete: tcgen05.wait::st above; the second CTA's relay passes its four arrivals on as one)
+                    for (int j = 0; j < n; ++j) mbar_arrive(leader ? full + sj[j] : sf_done + sj[j]);
                 }
             }
             sf_barrier();
@@ -1129,12 +1321,12 @@ bool make_kmajor_map(CUtensorMap* map, const void* base, int elem_bytes, uint64_
 
 namespace {
 
-template <auto kKernel, typename C>
-cudaError_t launch_tiles(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int grid, cudaStream_t stream) {
+template <auto kKernel, typename C, typename... Args>
+cudaError_t launch_tiles(int grid, cudaStream_t stream, const Args&... args) {
     static PreparedKernel prepared;
     const cudaError_t err = prepared.prepare(kKernel, C::kSmem);
     if (err != cudaSuccess) return err;
-    kKernel<<<grid, C::kThreads, C::kSmem, stream>>>(map_a, map_b, p);
+    kKernel<<<grid, C::kThreads, C::kSmem, stream>>>(args...);
     return cudaGetLastError();
 }
 
@@ -1145,22 +1337,28 @@ bool env_is(const char* name, char value) {
 
 }  // namespace
 
+// Which tiles a problem gets. What is known on the host: M rows in all (alignment gaps included), the number of groups, N, K.
+enum class Tiles { kPair256, kLone256, kLone128 };
+
+// Tiles of `bm` x `bn` over `units` at a time; about half of every group's last tile and of its alignment gap is padding.
+int num_waves(const GemmParams& p, int bm, int bn, int units) {
+    int64_t tiles_m;
+    if (p.k_grouped) tiles_m = static_cast<int64_t>(p.num_groups) * ceil_div(p.M, bm);
+    else if (p.group_end == nullptr) tiles_m = ceil_div(p.M, bm);
+    else {
+        const int64_t rows = std::max<int64_t>(p.M - static_cast<int64_t>(p.num_groups) * (std::min(p.group_alignment, 128) / 2), p.num_groups);
+        tiles_m = std::max<int64_t>(p.num_groups, rows / bm + p.num_groups / 2);
+    }
+    return static_cast<int>(ceil_div<int64_t>(tiles_m * (p.N / bn), units));
+}
+
 cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_stride_bytes, const void* b, int64_t b_row_stride_bytes,
                         bool fp8, int num_sms, cudaStream_t stream) {
     GemmParams p = params;
-    const int elem = fp8 ? 1 : 2;
+    const int elem = fp8 ? 1 : 2, bk = fp8 ? 128 : 64;
     p.c_wide = (reinterpret_cast<uintptr_t>(p.C) | static_cast<uint64_t>(p.ldc) * 2 | static_cast<uint64_t>(p.c_group_stride) * 2) % 32 == 0;
-    // bf16 with 256-wide tiles runs on CTA pairs (EP_GEMM_CTA_PAIR=0 keeps one CTA per tile); a pair needs two SMs.
-    // e4m3 on CTA pairs is opt-in (EP_GEMM_FP8_PAIR=1): with software block scaling the 256 x 256 tile halves the
-    // shared-memory fill per flop, but only two accumulator passes fit into tensor memory and the drain of a pass
-    // (64 columns per epilogue thread) then sets the pace: 0.94 PFLOP/s measured against 1.3 with 128 x 128 tiles and
-    // four passes in flight.
-    const bool pair_enabled = fp8 ? env_is("EP_GEMM_FP8_PAIR", '1') : !env_is("EP_GEMM_CTA_PAIR", '0');
-    const bool use_pair = p.N % 256 == 0 && pair_enabled && num_sms >= 2;
-    const int bn = fp8 ? (use_pair ? 256 : 128) : ((p.N % 256 == 0) ? 256 : 128);
-    const int bk = fp8 ? 128 : 64;
     const bool k_tail_ok = p.a_mn && p.b_mn && !p.k_grouped && p.num_groups == 1;     // rows past the end load as zeros
-    if (p.N % bn != 0 || (p.K % bk != 0 && !k_tail_ok) || p.M <= 0) return cudaErrorInvalidValue;
+    if (p.N % 128 != 0 || (p.K % bk != 0 && !k_tail_ok) || p.M <= 0) return cudaErrorInvalidValue;
     if (p.k_grouped && (fp8 || p.group_end == nullptr || p.group_alignment % bk != 0)) return cudaErrorInvalidValue;
     if ((p.a_mn || p.b_mn) && (fp8 || (p.a_mn && !p.b_mn))) return cudaErrorInvalidValue;
     const uint64_t K = static_cast<uint64_t>(p.K), a_stride = static_cast<uint64_t>(a_row_stride_bytes), b_stride = static_cast<uint64_t>(b_row_stride_bytes);
@@ -1169,36 +1367,57 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
     auto map_of = [&](CUtensorMap* map, const void* base, bool mn, uint64_t rows, uint64_t mats, uint64_t stride, uint32_t box) {
         return mn ? make_kmajor_map(map, base, elem, mats * K, rows, stride, 64) : make_kmajor_map(map, base, elem, mats * rows, K, stride, box);
     };
-    CUtensorMap map_a, map_b;
-    if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM)) return cudaErrorInvalidValue;
+    CUtensorMap map_a, map_a32, map_b;
+    if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM) ||
+        !map_of(&map_a32, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, kSmallBox))
+        return cudaErrorInvalidValue;
+    auto map_b_of = [&](uint32_t box) { return map_of(&map_b, b, p.b_mn != 0, static_cast<uint64_t>(p.N), b_mats, b_stride, box); };
+    const bool wide = p.N % 256 == 0, pairs = wide && num_sms >= 2;
+    const int pair_grid = num_sms & ~1;
+
     // e4m3 with power-of-two scales: the block-scaled instruction kind (EP_GEMM_FP8_MX=0 keeps the software scaling)
-    if (fp8 && p.scales_pow2 && !env_is("EP_GEMM_FP8_MX", '0') && !use_pair && p.N % 256 == 0 && p.K / 128 <= MxCfg::kMaxKb && !p.k_grouped) {
+    if (fp8 && p.scales_pow2 && !env_is("EP_GEMM_FP8_MX", '0') && !env_is("EP_GEMM_FP8_PAIR", '1') && wide && p.K / 128 <= MxCfg::kMaxKb) {
         // CTA pairs (EP_GEMM_FP8_MX_PAIR=1): 256 x 256 tiles, each CTA loads 128 rows of A and 128 of B. Opt-in: measured
         // no faster than lone CTAs (2.21 against 2.16 PFLOP/s), so the fill of shared memory from L2 is not what limits
         // the lone-CTA kernel; per k-block a CTA's shared memory takes 48 KB from TMA and hands 48 KB to the tensor
         // core in 541 tensor-pipe cycles either way, more than its 128 bytes per cycle.
-        const bool mx_pair = env_is("EP_GEMM_FP8_MX_PAIR", '1') && num_sms >= 2;
-        if (!map_of(&map_b, b, false, static_cast<uint64_t>(p.N), b_mats, b_stride, mx_pair ? 128 : 256)) return cudaErrorInvalidValue;
-        return mx_pair ? launch_tiles<gemm_mx_pair_kernel, MxPairCfg>(map_a, map_b, p, num_sms & ~1, stream)
-                       : launch_tiles<gemm_mx_kernel, MxCfg>(map_a, map_b, p, num_sms, stream);
+        if (env_is("EP_GEMM_FP8_MX_PAIR", '1') && pairs) {
+            if (!map_b_of(128)) return cudaErrorInvalidValue;
+            return launch_tiles<gemm_mx_pair_kernel, MxPairCfg>(pair_grid, stream, map_a, map_b, p);
+        }
+        if (!map_b_of(256)) return cudaErrorInvalidValue;
+        return launch_tiles<gemm_mx_kernel, MxCfg>(num_sms, stream, map_a, map_b, map_a32, p);
     }
-    if (!map_of(&map_b, b, p.b_mn != 0, static_cast<uint64_t>(p.N), b_mats, b_stride, static_cast<uint32_t>(use_pair ? bn / 2 : bn))) return cudaErrorInvalidValue;
-    if (fp8 && use_pair) return launch_tiles<gemm_pair_fp8_kernel, PairFp8Cfg>(map_a, map_b, p, num_sms & ~1, stream);
-    if (fp8) return launch_tiles<gemm_kernel<128, true>, Cfg<128, true>>(map_a, map_b, p, num_sms, stream);
-    if (bn == 256 && use_pair) {
-        const int grid = num_sms & ~1;
-        if (p.a_mn) return launch_tiles<gemm_pair_kernel<true, true>, PairCfg>(map_a, map_b, p, grid, stream);
-        return p.b_mn ? launch_tiles<gemm_pair_kernel<false, true>, PairCfg>(map_a, map_b, p, grid, stream)
-                      : launch_tiles<gemm_pair_kernel<false, false>, PairCfg>(map_a, map_b, p, grid, stream);
+    if (fp8) {
+        // Software scaling (EP_GEMM_FP8_PAIR=1 / 0 forces / forbids pairs): a pass takes about 1160 cycles on a pair (256 x 256)
+        // and 760 on a lone CTA (128 x 128), so pairs win unless their tiles are mostly padding or their last wave mostly
+        // empty (8 experts of 700 rows, 4096 x 4096: 143 against 168 us; 16 of 20 rows: 100 against 66 us).
+        const bool forced = env_is("EP_GEMM_FP8_PAIR", '1'), forbidden = env_is("EP_GEMM_FP8_PAIR", '0');
+        const bool use_pair = pairs && !forbidden && (forced || num_waves(p, 256, 256, num_sms / 2) * 1.5f < num_waves(p, 128, 128, num_sms));
+        if (!map_b_of(128)) return cudaErrorInvalidValue;
+        return use_pair ? launch_tiles<gemm_pair_fp8_kernel, PairFp8Cfg>(pair_grid, stream, map_a, map_b, p)
+                        : launch_tiles<gemm_kernel<128, true>, Cfg<128, true>>(num_sms, stream, map_a, map_b, map_a32, p);
     }
-    if (bn == 256) {
-        if (p.a_mn) return launch_tiles<gemm_kernel<256, false, true, true>, Cfg<256, false>>(map_a, map_b, p, num_sms, stream);
-        return p.b_mn ? launch_tiles<gemm_kernel<256, false, false, true>, Cfg<256, false>>(map_a, map_b, p, num_sms, stream)
-                      : launch_tiles<gemm_kernel<256, false>, Cfg<256, false>>(map_a, map_b, p, num_sms, stream);
+    // bf16: CTA pairs with 256 x 256 tiles (EP_GEMM_CTA_PAIR=0: never), or one CTA per 128 x 256 tile, which takes 1.13 times
+    // as long for its half but wastes less on ragged groups and in the last wave, and skips rows that do not exist (32 experts
+    // of 16 rows, 4096 x 7168: 302 against 390 us; 8 of 2000 rows: 345 against 310 us).
+    Tiles tiles = Tiles::kLone128;
+    if (wide) tiles = pairs && !env_is("EP_GEMM_CTA_PAIR", '0') && num_waves(p, 256, 256, num_sms / 2) <= num_waves(p, 128, 256, num_sms) * 1.13f
+                          ? Tiles::kPair256 : Tiles::kLone256;
+    if (!map_b_of(tiles == Tiles::kLone256 ? 256 : 128)) return cudaErrorInvalidValue;
+    if (tiles == Tiles::kPair256) {
+        if (p.a_mn) return launch_tiles<gemm_pair_kernel<true, true>, PairCfg>(pair_grid, stream, map_a, map_b, p);
+        return p.b_mn ? launch_tiles<gemm_pair_kernel<false, true>, PairCfg>(pair_grid, stream, map_a, map_b, p)
+                      : launch_tiles<gemm_pair_kernel<false, false>, PairCfg>(pair_grid, stream, map_a, map_b, p);
     }
-    if (p.a_mn) return launch_tiles<gemm_kernel<128, false, true, true>, Cfg<128, false>>(map_a, map_b, p, num_sms, stream);
-    return p.b_mn ? launch_tiles<gemm_kernel<128, false, false, true>, Cfg<128, false>>(map_a, map_b, p, num_sms, stream)
-                  : launch_tiles<gemm_kernel<128, false>, Cfg<128, false>>(map_a, map_b, p, num_sms, stream);
+    if (tiles == Tiles::kLone256) {
+        if (p.a_mn) return launch_tiles<gemm_kernel<256, false, true, true>, Cfg<256, false>>(num_sms, stream, map_a, map_b, map_a32, p);
+        return p.b_mn ? launch_tiles<gemm_kernel<256, false, false, true>, Cfg<256, false>>(num_sms, stream, map_a, map_b, map_a32, p)
+                      : launch_tiles<gemm_kernel<256, false>, Cfg<256, false>>(num_sms, stream, map_a, map_b, map_a32, p);
+    }
+    if (p.a_mn) return launch_tiles<gemm_kernel<128, false, true, true>, Cfg<128, false>>(num_sms, stream, map_a, map_b, map_a32, p);
+    return p.b_mn ? launch_tiles<gemm_kernel<128, false, false, true>, Cfg<128, false>>(num_sms, stream, map_a, map_b, map_a32, p)
+                  : launch_tiles<gemm_kernel<128, false>, Cfg<128, false>>(num_sms, stream, map_a, map_b, map_a32, p);
 }
 
 }  // namespace gemm

@@ -5,7 +5,7 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0        TMA producer: cp.async.bulk.tensor 2-D tiles (128B swizzle) of A (BM x BK) and
 //                 B (BN x BK) into a ring of shared-memory stages; never multicast
-//   warp 1        MMA issuer: one elected lane issues tcgen05.mma (M=128, N=BN, K=16 for bf16 /
+//   warp 1        MMA issuer: the warp walks the k-blocks, an elected lane issues tcgen05.mma (M=128, N=BN, K=16 for bf16 /
 //                 K=32 for e4m3) with the accumulator in tensor memory, tcgen05.commit releases the
 //                 stage and, after the last k-block, hands the accumulator to the epilogue
 //   warps 2..5    epilogue: tcgen05.ld (32 lanes x 32 columns per instruction), convert, store.

@@ -212,3 +212,43 @@ def test_gemm_k_grouped_mn_major(counts, N):
         want = a[s0:e].float().t() @ b[s0:e].float()
         assert torch.equal(out[i], torch.zeros_like(out[i])) if e == s0 else _rel_err(out[i], want) < 1e-2
         s0 = -(-e // align) * align
+
+
+@pytest.mark.parametrize('mode', ['bf16_lone', 'bf16_pair', 'fp8_lone', 'fp8_pair', 'fp8_hardware'])
+@pytest.mark.parametrize('counts', [[1, 32, 33, 96], [97, 0, 128, 129], [300, 1, 255, 31]])
+def test_grouped_tiles_with_few_rows(counts, mode, monkeypatch):
+    """Tiles of 1 to 128 rows around the edges of the 32-row boxes that the lone kernels load (a tile of at most 96 rows
+    loads only the boxes that hold rows), with a number of k-blocks (5, 10 for bf16) that divides by neither the stages of
+    the operand ring nor those of the scale ring. Scales are powers of two and the operands small whole numbers, so every
+    kernel's fp32 sums are exact: results equal the reference to half a bf16 step (7
+    fraction bits, so at most 2^-8 of the value)."""
+    import deepep_b200
+    monkeypatch.setenv('EP_GEMM_CTA_PAIR', '1' if mode.endswith('pair') else '0')
+    monkeypatch.setenv('EP_GEMM_FP8_PAIR', '1' if mode.endswith('pair') else '0')
+    G, N, K, align = len(counts), 512, 640, 128
+    g = torch.Generator(device='cuda').manual_seed(5)
+    ends, start = [], 0
+    for c in counts:
+        ends.append(start + c)
+        start = -(-(start + c) // align) * align
+    M = start
+    a = torch.randint(-3, 4, (M, K), device='cuda', generator=g).float()
+    b = torch.randint(-3, 4, (G, N, K), device='cuda', generator=g).float()
+    kwargs = dict(group_end=torch.tensor(ends, dtype=torch.int32, device='cuda'), group_alignment=align)
+    if mode.startswith('bf16'):
+        out = deepep_b200._C.gemm(a.bfloat16(), b.bfloat16(), **kwargs)
+        a_ref, b_ref = a, b
+    else:
+        sfa = torch.exp2(torch.randint(-2, 3, (M, K // 128), device='cuda', generator=g).float())
+        sfb = torch.exp2(torch.randint(-2, 3, (G, N // 128, K // 128), device='cuda', generator=g).float())
+        out = deepep_b200._C.gemm(a.to(torch.float8_e4m3fn), b.to(torch.float8_e4m3fn), sfa=sfa, sfb=sfb,
+                                  pow2_scales=mode == 'fp8_hardware', **kwargs)
+        a_ref = a * sfa.repeat_interleave(128, dim=1)
+        b_ref = b * sfb.repeat_interleave(128, dim=1).repeat_interleave(128, dim=2)
+    torch.cuda.synchronize()
+    assert deepep_b200._C.gemm_check_status() == 0
+    start = 0
+    for gi, c in enumerate(counts):
+        ref = (a_ref[start:start + c].double() @ b_ref[gi].double().t())
+        assert bool(((out[start:start + c].double() - ref).abs() <= ref.abs() * 2.0 ** -8).all())
+        start = -(-(start + c) // align) * align
