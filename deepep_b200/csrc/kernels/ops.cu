@@ -87,26 +87,6 @@ __global__ void __launch_bounds__(256) router_weights_kernel(const float* __rest
     }
 }
 
-// Gradient of the logits from the gradient of the top-k weights, one warp per token: the softmax Jacobian over the selected
-// experts, d logit_k = w_k (dw_k - sum_j w_j dw_j), zeros elsewhere (ten elementwise launches otherwise, bound by the host).
-__global__ void __launch_bounds__(256) router_backward_kernel(const int64_t* __restrict__ topk_idx, const float* __restrict__ w, const float* __restrict__ dw,
-                                                              int num_tokens, int num_topk, int num_experts, int padded, __nv_bfloat16* __restrict__ dlogits) {
-    const int t = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = lane_id();
-    if (t >= num_tokens) return;
-    __nv_bfloat16* row = dlogits + static_cast<int64_t>(t) * padded;
-    for (int i = lane * 8; i < padded; i += 256) *reinterpret_cast<int4*>(row + i) = make_int4(0, 0, 0, 0);
-    const int64_t o = static_cast<int64_t>(t) * num_topk + lane;
-    const float wv = lane < num_topk ? w[o] : 0.f, dv = lane < num_topk ? dw[o] : 0.f;
-    float inner = wv * dv;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) inner += __shfl_xor_sync(0xffffffffu, inner, s);
-    __syncwarp();           // the zeros of all lanes are in place
-    if (lane < num_topk) {
-        const int64_t e = topk_idx[o];
-        if (e >= 0 && e < num_experts) row[e] = __float2bfloat16_rn(wv * (dv - inner));
-    }
-}
-
 // ---------------------------------------------------------------- streaming kernels
 // One warp per (row, 512 channels) and nothing else, sixteen channels per lane: neighbouring warps have neighbouring bytes,
 // and a grid of many short blocks streams faster than a resident grid that loops over the same work (cast of 8192 x 7168:
@@ -120,6 +100,59 @@ __device__ __forceinline__ RowCol row_col(int columns) {
     const uint32_t w = blockIdx.x * (blockDim.x >> 5) + warp_id();
     const uint32_t row = w / static_cast<uint32_t>(columns);
     return {static_cast<int>(row), static_cast<int>(w - row * static_cast<uint32_t>(columns)) * kSpan + lane_id() * 16};
+}
+
+// Gradient of the router from the gradient of the top-k weights, one warp per (token, 512 channels): the softmax Jacobian
+// over the selected experts, d logit_k = w_k (dw_k - sum_j w_j dw_j), as the bf16 row that the weight gradient contracts
+// (zeros elsewhere), and dx += sum_k d logit_k * router[expert k] in fp32. Only the selected rows of the router weights are
+// read, from L1 and L2, and the sum is rounded once (a GEMM over all padded experts and an elementwise addition took 14 us
+// for 1000 x 2048 where this takes 4).
+__global__ void __launch_bounds__(256) router_backward_kernel(const int64_t* __restrict__ topk_idx, const float* __restrict__ w, const float* __restrict__ dw,
+                                                              int num_tokens, int num_topk, int num_experts, int padded, int hidden, int columns,
+                                                              const __nv_bfloat16* __restrict__ router, __nv_bfloat16* dx, __nv_bfloat16* __restrict__ dlogits) {
+    const RowCol rc = row_col(columns);
+    const int t = rc.row, lane = lane_id();
+    if (t >= num_tokens) return;
+    const int64_t o = static_cast<int64_t>(t) * num_topk + lane;
+    const float wv = lane < num_topk ? w[o] : 0.f, dv = lane < num_topk ? dw[o] : 0.f;
+    const int64_t sel = lane < num_topk ? topk_idx[o] : -1;
+    const int e = sel >= 0 && sel < num_experts ? static_cast<int>(sel) : -1;
+    float inner = wv * dv;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) inner += __shfl_xor_sync(0xffffffffu, inner, s);
+    const float g = wv * (dv - inner);
+    if (rc.ch == lane * 16) {       // the first column writes the row of the logits' gradient
+        __nv_bfloat16* row = dlogits + static_cast<int64_t>(t) * padded;
+        for (int i = lane * 8; i < padded; i += 256) *reinterpret_cast<int4*>(row + i) = make_int4(0, 0, 0, 0);
+        __syncwarp();               // the zeros of all lanes are in place
+        if (e >= 0) row[e] = __float2bfloat16_rn(g);
+    }
+    const int halves = min(2, (hidden - rc.ch) / 8);       // 16-byte pieces of this lane (hidden is a multiple of 8)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const bool in = h < halves;
+        __nv_bfloat16* at = dx + static_cast<int64_t>(t) * hidden + rc.ch + h * 8;
+        int4 v = in ? *reinterpret_cast<const int4*>(at) : make_int4(0, 0, 0, 0);
+        __nv_bfloat162* v2 = reinterpret_cast<__nv_bfloat162*>(&v);
+        float2 acc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = __bfloat1622float2(v2[i]);
+        for (int k = 0; k < num_topk; ++k) {
+            const int ek = __shfl_sync(0xffffffffu, e, k);
+            const float gk = __shfl_sync(0xffffffffu, g, k);
+            if (ek < 0 || !in) continue;
+            const int4 r = *reinterpret_cast<const int4*>(router + static_cast<int64_t>(ek) * hidden + rc.ch + h * 8);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&r)[i]);
+                acc[i].x = fmaf(gk, f.x, acc[i].x);
+                acc[i].y = fmaf(gk, f.y, acc[i].y);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v2[i] = __floats2bfloat162_rn(acc[i].x, acc[i].y);
+        if (in) *reinterpret_cast<int4*>(at) = v;
+    }
 }
 
 // Is the row in an alignment gap of the expanded layout (behind the rows of its expert)? Warp-collective, the same row on
@@ -438,11 +471,14 @@ cudaError_t router_weights(const float* w, int num_experts, int padded_experts, 
 }
 
 cudaError_t router_backward(const int64_t* topk_idx, const float* w, const float* dw, int num_tokens, int num_topk, int num_experts, int padded_experts,
-                            void* dlogits, cudaStream_t stream) {
+                            int hidden, const void* router, void* dx, void* dlogits, cudaStream_t stream) {
     if (num_tokens == 0) return cudaSuccess;
-    if (num_topk > 32 || padded_experts % 8 != 0) return cudaErrorInvalidValue;
-    router_backward_kernel<<<(num_tokens + 7) / 8, 256, 0, stream>>>(topk_idx, w, dw, num_tokens, num_topk, num_experts, padded_experts,
-                                                                     static_cast<__nv_bfloat16*>(dlogits));
+    const int columns = (hidden + kSpan - 1) / kSpan;
+    const int64_t warps = static_cast<int64_t>(num_tokens) * columns;
+    if (num_topk > 32 || padded_experts % 8 != 0 || hidden % 8 != 0 || warps >= (1ll << 31)) return cudaErrorInvalidValue;
+    router_backward_kernel<<<static_cast<int>((warps + 7) / 8), 256, 0, stream>>>(
+        topk_idx, w, dw, num_tokens, num_topk, num_experts, padded_experts, hidden, columns, static_cast<const __nv_bfloat16*>(router),
+        static_cast<__nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(dlogits));
     return cudaGetLastError();
 }
 

@@ -23,7 +23,7 @@ cudaError_t router_topk(const void* logits, bool bf16, int64_t row_stride, int n
 cudaError_t router_weights(const float* w, int num_experts, int padded_experts, int hidden, void* out, cudaStream_t stream);
 // bf16 dlogits [tokens, padded experts] from the top-k weights and their gradient
 cudaError_t router_backward(const int64_t* topk_idx, const float* w, const float* dw, int num_tokens, int num_topk, int num_experts, int padded_experts,
-                            void* dlogits, cudaStream_t stream);
+                            int hidden, const void* router, void* dx, void* dlogits, cudaStream_t stream);
 // bf16 [groups, rows, cols] -> e4m3 + one fp32 scale per 128 x 128 block
 cudaError_t quant_weights_128x128(const void* w, int groups, int rows, int cols, bool pow2, void* q, float* scales, cudaStream_t stream);
 // bf16 [rows, hidden] -> e4m3 [rows, hidden] + fp32 scales (element (row, block) at scales[row * row_stride + block * col_stride])

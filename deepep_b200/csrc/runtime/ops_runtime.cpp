@@ -16,6 +16,7 @@
 #include "../common/layout.hpp"
 #include "../kernels/gemm_api.hpp"
 #include "../kernels/ops_api.hpp"
+#include "ops_runtime.hpp"
 
 namespace py = pybind11;
 
@@ -27,6 +28,8 @@ namespace {
 at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, int device) {
     return at::detail::empty_cuda(sizes, dtype, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)), std::nullopt);
 }
+
+cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // one status word per device for the GEMM pipelines (0 = healthy)
 at::Tensor& gemm_status(int device) {
@@ -42,6 +45,8 @@ int gemm_check_status() {
     CUDA_RUNTIME_CHECK(cudaGetDevice(&device));
     return gemm_status(device).item<int>();
 }
+
+}  // namespace
 
 at::Tensor gemm_impl(const at::Tensor& a, const at::Tensor& b, const std::optional<at::Tensor>& sfa, const std::optional<at::Tensor>& sfb,
                      const std::optional<at::Tensor>& group_end, int group_alignment, std::optional<at::Tensor> out, int num_sms,
@@ -101,8 +106,6 @@ at::Tensor gemm_impl(const at::Tensor& a, const at::Tensor& b, const std::option
     return *out;
 }
 
-cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
-
 // out[g] = a[:, range g] @ b[:, range g]^T for all groups in one launch (bf16): the k range of group g is
 // [align(group_end[g-1], group_alignment), group_end[g]), read from the device array, no host synchronisation.
 // mn_major: the operands are given as [K, M] and [K, N] (the rows of an expert are the contraction dimension and lie in
@@ -143,7 +146,7 @@ at::Tensor gemm_k_grouped(const at::Tensor& a, const at::Tensor& b, const at::Te
 
 // bf16 a @ b with b as it lies in memory: b [K, N]; a [M, K], or a^T @ b with a [K, M] (any K then: the weight gradient of a
 // linear layer, rows of both being the tokens).
-at::Tensor gemm_mn(const at::Tensor& a, const at::Tensor& b, bool a_transposed) {
+static at::Tensor gemm_mn(const at::Tensor& a, const at::Tensor& b, bool a_transposed) {
     EP_HOST_ASSERT(a.is_cuda() && b.is_cuda() && a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1);
     EP_HOST_ASSERT(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16);
     const int M = static_cast<int>(a.size(a_transposed ? 1 : 0)), K = static_cast<int>(a.size(a_transposed ? 0 : 1)), N = static_cast<int>(b.size(1));
@@ -173,7 +176,7 @@ at::Tensor gemm_mn(const at::Tensor& a, const at::Tensor& b, bool a_transposed) 
     return out;
 }
 
-std::tuple<at::Tensor, at::Tensor> router_topk(const at::Tensor& logits, int num_topk) {
+static std::tuple<at::Tensor, at::Tensor> router_topk(const at::Tensor& logits, int num_topk) {
     const bool bf16 = logits.scalar_type() == at::kBFloat16;
     EP_HOST_ASSERT(logits.is_cuda() && logits.dim() == 2 && (bf16 || logits.scalar_type() == at::kFloat) && logits.stride(1) == 1);
     c10::cuda::CUDAGuard guard(logits.device());
@@ -202,21 +205,24 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> router_forward(const at::Tensor& 
     return {idx, tw, w};
 }
 
-// (dx [T, hidden], d_router [experts, hidden] bf16) from the gradient of the top-k weights
-std::tuple<at::Tensor, at::Tensor> router_backward(const at::Tensor& x, const at::Tensor& router_padded, const at::Tensor& topk_idx, const at::Tensor& w,
-                                                   const at::Tensor& dw, int num_experts) {
+// d_router [experts, hidden] in bf16 from the gradient of the top-k weights; the router's share of the input gradient is
+// added to dx [T, hidden] in place
+at::Tensor router_backward(const at::Tensor& x, const at::Tensor& router_padded, const at::Tensor& topk_idx, const at::Tensor& w,
+                           const at::Tensor& dw, int num_experts, const at::Tensor& dx) {
     EP_HOST_ASSERT(topk_idx.scalar_type() == at::kLong && topk_idx.is_contiguous() && w.is_contiguous() && w.scalar_type() == at::kFloat &&
                    dw.scalar_type() == at::kFloat && dw.is_contiguous() && dw.numel() == w.numel());
+    EP_HOST_ASSERT(dx.scalar_type() == at::kBFloat16 && dx.is_contiguous() && dx.sizes() == x.sizes() && router_padded.is_contiguous() &&
+                   router_padded.scalar_type() == at::kBFloat16 && router_padded.size(1) == dx.size(1) && dx.size(1) % 8 == 0);
     c10::cuda::CUDAGuard guard(x.device());
     const int T = static_cast<int>(topk_idx.size(0)), K = static_cast<int>(topk_idx.size(1)), padded = static_cast<int>(router_padded.size(0));
     at::Tensor dlogits = new_tensor({T, padded}, at::kBFloat16, x.get_device());
     CUDA_RUNTIME_CHECK(ops::router_backward(topk_idx.data_ptr<int64_t>(), w.data_ptr<float>(), dw.data_ptr<float>(), T, K, num_experts, padded,
-                                            dlogits.data_ptr(), cur_stream()));
-    return {gemm_mn(dlogits, router_padded, false), gemm_mn(dlogits, x, true).narrow(0, 0, num_experts)};
+                                            static_cast<int>(dx.size(1)), router_padded.data_ptr(), dx.data_ptr(), dlogits.data_ptr(), cur_stream()));
+    return gemm_mn(dlogits, x, true).narrow(0, 0, num_experts);
 }
 
 // bf16 [G, N, K] -> (e4m3 [G, N, K], fp32 scales [G, N / 128, K / 128])
-std::tuple<at::Tensor, at::Tensor> quant_weights_128x128(const at::Tensor& w, bool pow2) {
+static std::tuple<at::Tensor, at::Tensor> quant_weights_128x128(const at::Tensor& w, bool pow2) {
     EP_HOST_ASSERT(w.is_cuda() && w.dim() == 3 && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.size(1) % 128 == 0 && w.size(2) % 128 == 0);
     c10::cuda::CUDAGuard guard(w.device());
     const int G = static_cast<int>(w.size(0)), N = static_cast<int>(w.size(1)), K = static_cast<int>(w.size(2)), device = w.get_device();
@@ -225,7 +231,7 @@ std::tuple<at::Tensor, at::Tensor> quant_weights_128x128(const at::Tensor& w, bo
     return {q, sf};
 }
 
-std::tuple<at::Tensor, at::Tensor> quant_1x128(const at::Tensor& x, bool pow2, bool col_major_sf) {
+static std::tuple<at::Tensor, at::Tensor> quant_1x128(const at::Tensor& x, bool pow2, bool col_major_sf) {
     EP_HOST_ASSERT(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1 && (x.stride(0) * 2) % 16 == 0);
     c10::cuda::CUDAGuard guard(x.device());
     const int M = static_cast<int>(x.size(0)), H = static_cast<int>(x.size(1));
@@ -239,7 +245,7 @@ std::tuple<at::Tensor, at::Tensor> quant_1x128(const at::Tensor& x, bool pow2, b
 }
 
 // the row groups of an expanded dispatch (null = none)
-ops::RowGroups row_groups(const std::optional<at::Tensor>& group_end, int group_alignment) {
+static ops::RowGroups row_groups(const std::optional<at::Tensor>& group_end, int group_alignment) {
     ops::RowGroups g;
     if (!group_end.has_value()) return g;
     EP_HOST_ASSERT(group_end->is_cuda() && group_end->scalar_type() == at::kInt && group_end->is_contiguous() && group_alignment >= 1);
@@ -281,8 +287,7 @@ std::tuple<at::Tensor, std::optional<at::Tensor>> swiglu(const at::Tensor& x, co
     return {out, sf};
 }
 
-// returns dx, or with `with_byproducts` (dx, weighted activation [rows, inter] bf16, gradient of the row weight [rows] fp32)
-py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const std::optional<at::Tensor>& row_weight, bool with_byproducts,
+std::tuple<at::Tensor, at::Tensor, at::Tensor> swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const std::optional<at::Tensor>& row_weight, bool with_byproducts,
                            const std::optional<at::Tensor>& group_end, int group_alignment) {
     EP_HOST_ASSERT(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.is_contiguous() && dout.scalar_type() == at::kBFloat16 && dout.is_contiguous());
     c10::cuda::CUDAGuard guard(x.device());
@@ -298,12 +303,11 @@ py::object swiglu_backward(const at::Tensor& x, const at::Tensor& dout, const st
     CUDA_RUNTIME_CHECK(ops::swiglu_backward(x.data_ptr(), dout.data_ptr(), M, I, row_weight.has_value() ? row_weight->data_ptr<float>() : nullptr,
                                             row_groups(group_end, group_alignment), dx.data_ptr(), with_byproducts ? act.data_ptr() : nullptr,
                                             with_byproducts ? dweight.data_ptr<float>() : nullptr, cur_stream()));
-    if (with_byproducts) return py::make_tuple(dx, act, dweight);
-    return py::cast(dx);
+    return {dx, act, dweight};
 }
 
 // [rows, cols] -> [cols, rows], or the same for every matrix of a batch [n, rows, cols]
-at::Tensor transpose_bf16(const at::Tensor& x) {
+static at::Tensor transpose_bf16(const at::Tensor& x) {
     EP_HOST_ASSERT(x.is_cuda() && (x.dim() == 2 || x.dim() == 3) && x.scalar_type() == at::kBFloat16 && x.stride(-1) == 1);
     c10::cuda::CUDAGuard guard(x.device());
     const bool batched = x.dim() == 3;
@@ -315,18 +319,20 @@ at::Tensor transpose_bf16(const at::Tensor& x) {
     return out;
 }
 
-}  // namespace
-
 void register_ops_bindings(py::module_& m) {
     m.def("router_topk", &router_topk);
-    m.def("router_forward", &router_forward);
     m.def("router_backward", &router_backward);
     m.def("quant_weights_128x128", &quant_weights_128x128, py::arg("w"), py::arg("pow2") = false);
     m.def("quant_1x128", &quant_1x128, py::arg("x"), py::arg("pow2") = false, py::arg("col_major_sf") = false);
     m.def("dequant_1x128", &dequant_1x128, py::arg("q"), py::arg("sf"), py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
     m.def("swiglu", &swiglu, py::arg("x"), py::arg("row_weight") = py::none(), py::arg("num_valid_rows") = py::none(), py::arg("quant") = false,
           py::arg("pow2") = false, py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
-    m.def("swiglu_backward", &swiglu_backward, py::arg("x"), py::arg("dout"), py::arg("row_weight") = py::none(),
+    // returns dx, or with `with_byproducts` (dx, weighted activation [rows, inter] bf16, gradient of the row weight [rows] fp32)
+    m.def("swiglu_backward", [](const at::Tensor& x, const at::Tensor& dout, const std::optional<at::Tensor>& row_weight, bool with_byproducts,
+                                const std::optional<at::Tensor>& group_end, int group_alignment) -> py::object {
+        const auto [dx, act, dweight] = swiglu_backward(x, dout, row_weight, with_byproducts, group_end, group_alignment);
+        return with_byproducts ? py::object(py::make_tuple(dx, act, dweight)) : py::cast(dx);
+    }, py::arg("x"), py::arg("dout"), py::arg("row_weight") = py::none(),
           py::arg("with_byproducts") = false, py::arg("group_end") = py::none(), py::arg("group_alignment") = 1);
     m.def("transpose_bf16", &transpose_bf16);
     m.def("gemm", &gemm_impl, py::arg("a"), py::arg("b"), py::arg("sfa") = py::none(), py::arg("sfb") = py::none(),

@@ -13,8 +13,8 @@ kernel, which makes the combine a plain sum. Backward reverses the same pipeline
 the combine is a cached (replayed) dispatch, the gradient of the dispatch is a combine, the data
 gradients are grouped GEMMs with the transposed weights, the weight gradients are two GEMM launches
 grouped along the contraction dimension (all experts at once, segment bounds read on the device), and
-the gradient of the gate weights rides back with the combine. The router runs on the same tensor-core
-GEMM (``_RouterFunction``).
+the gradient of the gate weights rides back with the combine. ``FusedMoE`` runs all of it, router included, as one
+native call per direction (``_LayerFunction``).
 
 The reference library has no model code; this is the "fused MoE layer fwd+bwd" workload that its
 kernels exist to serve. Everything is written over LISTS of ranks so that the single-GPU emulation
@@ -72,6 +72,10 @@ class ExpertWeights:
         if self.use_fp8:
             self.w13_q, self.w13_sf = quantize_weight_128x128(self.w13, self.pow2_scales)
             self.w2_q, self.w2_sf = quantize_weight_128x128(self.w2, self.pow2_scales)
+
+    def forward_operands(self) -> List[torch.Tensor]:
+        """The tensors that the forward GEMMs read."""
+        return [self.w13_q, self.w13_sf, self.w2_q, self.w2_sf] if self.use_fp8 else [self.w13, self.w2]
 
 
 class _SingleRankComm:
@@ -171,40 +175,24 @@ def moe_backward(comm, weights: Sequence[ExpertWeights], ctxs, dys: Sequence[tor
     return [c[0] for c in comb], [c[1] for c in comb], dW13s, dW2s
 
 
-class _RouterFunction(torch.autograd.Function):
-    """Router of the layer on this library's kernels: logits = x @ W_r^T on the tcgen05 GEMM (bf16 operands, fp32
-    accumulation), top-k and softmax over the selected logits in ``router_topk``; the backward pass turns the gradient
-    of the top-k weights into the gradient of the logits (softmax Jacobian over the selected experts, zero elsewhere)
-    and into two more tensor-core GEMMs for dW_r and dx."""
+class _LayerFunction(torch.autograd.Function):
+    """The whole layer as one node, one native call in each direction. The router runs on this library's kernels: logits =
+    x @ W_r^T on the tcgen05 GEMM (bf16 operands, fp32 accumulation), top-k and softmax over the selected logits; its
+    backward pass turns the gradient of the top-k weights into the gradient of the logits (softmax Jacobian over the
+    selected experts, zero elsewhere), adds their share to dx and contracts them with x to dW_r."""
 
     @staticmethod
-    def forward(ctx, x, router, num_topk):
-        topk_idx, topk_weights, router_bf16 = _C.router_forward(x.detach().contiguous(), router.detach().contiguous(), num_topk)
-        ctx.save_for_backward(x, router_bf16, topk_idx, topk_weights)
-        ctx.router_dtype, ctx.num_experts = router.dtype, router.size(0)
-        ctx.mark_non_differentiable(topk_idx)
-        return topk_idx, topk_weights
-
-    @staticmethod
-    def backward(ctx, _d_idx, d_weights):
-        # d logit_k = w_k * (dw_k - sum_j w_j dw_j) on the selected experts; dx = dlogits @ W_r, dW_r = dlogits^T @ x
-        x, router_bf16, topk_idx, w = ctx.saved_tensors
-        dx, d_router = _C.router_backward(x.detach().contiguous(), router_bf16, topk_idx, w, d_weights.contiguous(), ctx.num_experts)
-        return dx, d_router.to(ctx.router_dtype), None
-
-
-class _MoEFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, topk_weights, w13, w2, layer, topk_idx):
-        ys, ctxs = moe_forward(layer.comm, [layer.weights], [x], [topk_idx], [topk_weights.detach()], layer.cfg)
-        ctx.layer, ctx.saved = layer, ctxs
-        return ys[0]
+    def forward(ctx, x, router, w13, w2, layer):
+        y, ctx.call = _C.moe_layer_forward(layer.buffer.runtime, layer._native_config(), x, router, layer.weights.forward_operands())
+        ctx.layer, ctx.router_dtype = layer, router.dtype
+        ctx.save_for_backward(x)
+        return y
 
     @staticmethod
     def backward(ctx, dy):
-        layer = ctx.layer
-        dxs, dws, dW13s, dW2s = moe_backward(layer.comm, [layer.weights], ctx.saved, [dy], layer.cfg)
-        return dxs[0], dws[0], dW13s[0], dW2s[0], None, None
+        w = ctx.layer.weights
+        dx, d_router, d13, d2 = _C.moe_layer_backward(ctx.layer.buffer.runtime, ctx.call, ctx.saved_tensors[0], dy, w.w13_t, w.w2_t)
+        return dx, d_router.to(ctx.router_dtype), d13, d2, None
 
 
 class FusedMoE(torch.nn.Module):
@@ -232,9 +220,14 @@ class FusedMoE(torch.nn.Module):
         """Call after an optimizer step: rebuilds the transposed / quantised weight copies."""
         self.weights = ExpertWeights(self.w13.data, self.w2.data, self.cfg.use_fp8, self.cfg.pow2_scales)
 
+    def _native_config(self):
+        c, b = self.cfg, self.buffer
+        num_sms = c.num_sms if c.num_sms > 0 else b.get_theoretical_num_sms(c.num_experts, c.num_topk)
+        return _C.MoELayerConfig(c.num_experts, c.num_topk, b.num_max_tokens_per_rank, c.expert_alignment, num_sms, c.use_fp8,
+                                 c.use_fp8 and c.pow2_scales and self.weights.pow2_scales, b.allow_multiple_reduction, b.fuse_combine_reduce)
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        topk_idx, topk_weights = _RouterFunction.apply(x, self.router, self.cfg.num_topk)
-        return _MoEFunction.apply(x, topk_weights, self.w13, self.w2, self, topk_idx)
+        return _LayerFunction.apply(x, self.router, self.w13, self.w2, self)
 
 
 def reference_moe(xs, topk_idx, topk_weights, w13_all: torch.Tensor, w2_all: torch.Tensor):

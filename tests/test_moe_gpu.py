@@ -74,3 +74,40 @@ def test_moe_module_single_rank_trains():
     for p in (x, layer.router, layer.w13, layer.w2):
         assert p.grad is not None and torch.isfinite(p.grad.float()).all() and p.grad.float().abs().sum() > 0
     buf.destroy()
+
+
+@pytest.mark.parametrize('T,H,I,E,K,use_fp8', [(1, 256, 128, 4, 1, False), (77, 640, 128, 8, 3, False), (300, 1024, 256, 16, 8, False),
+                                               (129, 512, 256, 8, 4, True)])
+def test_moe_module_gradients(T, H, I, E, K, use_fp8):
+    """All gradients of the layer (router's share of dx and the router weights included) against fp32 autograd over the
+    routing that the layer chose. bf16 intermediates bound the difference: every contraction sees operands rounded to 2^-9
+    and four roundings lie between an input and a gradient, 4 * 2^-9 < 1e-2 of the norm; e4m3 operands (2^-4) in the
+    forward products: the tolerance of the emulated-rank test above, plus its margins for gradients."""
+    import deepep_b200
+    from deepep_b200.models.moe import FusedMoE, MoEConfig, reference_moe
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    buf = deepep_b200.ElasticBuffer(SingleProcessGroup(), num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_gpu_timeout_secs=5)
+    layer = FusedMoE(buf, MoEConfig(hidden=H, intermediate=I, num_experts=E, num_topk=K, use_fp8=use_fp8, pow2_scales=use_fp8))
+    g = torch.Generator(device='cuda').manual_seed(6)
+    x = torch.randn((T, H), device='cuda', generator=g).bfloat16().requires_grad_(True)
+    dy = torch.randn((T, H), device='cuda', generator=g).bfloat16()
+    y = layer(x)
+    y.backward(dy)
+    buf.check_status()
+    xr = x.detach().float().requires_grad_(True)
+    wr, w13, w2 = (p.detach().bfloat16().float().requires_grad_(True) for p in (layer.router, layer.w13, layer.w2))
+    logits = xr @ wr.t()
+    idx = logits.bfloat16().float().topk(K, dim=1)[1]
+    w = torch.softmax(logits.gather(1, idx), dim=1)
+    ref = reference_moe([xr], [idx], [w], w13, w2)[0]
+    ref.backward(dy.float())
+    tol = 0.08 if use_fp8 else 0.02
+    assert _rel(y, ref.detach()) < tol
+    for got, want in ((x.grad, xr.grad), (layer.w13.grad, w13.grad), (layer.w2.grad, w2.grad)):
+        assert _rel(got, want) < tol + 0.03
+    if K > 1:
+        assert _rel(layer.router.grad, wr.grad) < tol + 0.05
+    else:
+        assert layer.router.grad.abs().max() == 0       # the softmax over one expert does not depend on its logit
+    assert layer.router.grad.dtype == layer.router.dtype
+    buf.destroy()
