@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(kEpiWarps * 32) combine_epilogue_kernel(const 
     bool flags_ok = true;
     // per source rank: first row of this rank's tokens in that rank's receive order, and how many rows it holds for us
     __shared__ int s_base[kMaxRanks], s_held[kMaxRanks];
+    if (!flagged) dependency_wait();        // the send kernel has completed, and with it all peers' sends (a no-op unless launched early)
     if (flagged && threadIdx.x < p.num_ranks) {
         const int src = threadIdx.x, me = p.c.rank;
         int base = 0;
@@ -397,9 +398,9 @@ __global__ void __launch_bounds__(1024, 1) combine_kernel(const __grid_constant_
         if (pend2 >= 0) row_landed(pend2);
         pend0 = pend1 = pend2 = -1;
     };
-    if (kFlags) {
-        // zero the counters the NEXT combine will count into (the other parity): no peer starts that combine before
-        // it has seen this rank's completion word, which is sent at the end of this kernel
+    {
+        // zero the counters the NEXT combine may count into (the other parity; whether this one counts or not): no peer
+        // starts that combine before it has seen this rank's completion word, which is sent at the end of this kernel
         uint32_t* next = reinterpret_cast<uint32_t*>(c.heap[c.rank] + p.off_comb_flag + static_cast<uint64_t>((p.epoch + 1) & 1) * R * p.flag_chunks * 4);
         for (int i = bid * blockDim.x + tid; i < R * p.flag_chunks; i += nb * blockDim.x) next[i] = 0u;
     }

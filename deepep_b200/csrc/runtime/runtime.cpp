@@ -218,7 +218,7 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
     const int device = rt0.heap_->device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
     if (rt0.num_ranks_ == 1 && V == 1) return {rt0.dispatch_single(args[0])};
-    StreamScope scope(args[0].sc, rt0);
+    StreamScope scope(args[0].sc, rt0, /*may_stay=*/true);
     const cudaStream_t stream = scope.comm.stream();
 
     const int R = rt0.num_ranks_;
@@ -310,12 +310,12 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
             r.num_unaligned = *a.h_num_unaligned;
             r.recv_src_metadata = *a.h_recv_src_metadata;
         } else {
-            r.token_slot = at::empty({T, R}, opts(at::kInt, device));
-            r.pair_row = at::empty({T, K}, opts(at::kInt, device));
-            r.psum_rank = at::empty({R}, opts(at::kInt, device));
-            r.psum_expert = at::empty({EL + 1}, opts(at::kInt, device));
-            r.num_unaligned = at::empty({EL}, opts(at::kInt, device));
-            r.count_matrix = at::empty({R, R}, opts(at::kInt, device));
+            r.token_slot = new_tensor({T, R}, at::kInt, device);
+            r.pair_row = new_tensor({T, K}, at::kInt, device);
+            r.psum_rank = new_tensor({R}, at::kInt, device);
+            r.psum_expert = new_tensor({EL + 1}, at::kInt, device);
+            r.num_unaligned = new_tensor({EL}, at::kInt, device);
+            r.count_matrix = new_tensor({R, R}, at::kInt, device);
         }
         p.token_slot = r.token_slot.data_ptr<int>();
         p.pair_row = r.pair_row.data_ptr<int>();
@@ -389,7 +389,7 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
             // payload (and row-major scales) are read where they landed: strided views of the receive region
             r.recv_x = at::from_blob(region, {N, H}, {rec_pitch / static_cast<int64_t>(c10::elementSize(out_dtype)), 1}, opts(out_dtype, device));
         } else {
-            r.recv_x = at::empty({rows, H}, opts(out_dtype, device));
+            r.recv_x = new_tensor({rows, H}, out_dtype, device);
         }
         if (has_sf) {
             const at::ScalarType sf_dtype = (!quant && a.sf->scalar_type() == at::kInt) ? at::kInt : at::kFloat;
@@ -399,16 +399,16 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
                 r.recv_sf = at::from_blob(region + x_row_bytes, {N, sf_packs}, {rec_pitch / 4, 1}, opts(sf_dtype, device));
                 sf_in_place = true;
             } else {
-                r.recv_sf = at::empty({rows, sf_packs}, opts(sf_dtype, device));
+                r.recv_sf = new_tensor({rows, sf_packs}, sf_dtype, device);
             }
         }
         if (!a.do_expand) {
-            r.recv_topk_idx = at::empty({N, K}, opts(idx_dtype, device));
-            if (a.topk_weights.has_value()) r.recv_topk_weights = at::empty({N, K}, opts(at::kFloat, device));
+            r.recv_topk_idx = new_tensor({N, K}, idx_dtype, device);
+            if (a.topk_weights.has_value()) r.recv_topk_weights = new_tensor({N, K}, at::kFloat, device);
         } else if (a.topk_weights.has_value()) {
-            r.recv_topk_weights = at::empty({rows}, opts(at::kFloat, device));
+            r.recv_topk_weights = new_tensor({rows}, at::kFloat, device);
         }
-        if (!cached) r.recv_src_metadata = at::empty({N, K + 2}, opts(at::kInt, device));
+        if (!cached) r.recv_src_metadata = new_tensor({N, K + 2}, at::kInt, device);
 
         DispatchEpilogueParams& q = ep[v];
         q.c = p.c;
@@ -442,7 +442,7 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
         q.num_idx_rows = static_cast<int>(r.recv_src_metadata.size(0));
         q.mask_weights = a.mask_weights ? 1 : 0;
         if (a.copy_topk_idx) {
-            r.topk_idx = at::empty({a.x.size(0), K}, opts(idx_dtype, device));
+            r.topk_idx = new_tensor({a.x.size(0), K}, idx_dtype, device);
             q.topk_idx = a.topk_idx->data_ptr();
             q.topk_idx_copy = r.topk_idx->data_ptr();
             q.topk_idx_bytes = static_cast<int64_t>(a.topk_idx->nbytes());
@@ -477,7 +477,7 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
     const int device = rt0.heap_->device();
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
     if (rt0.num_ranks_ == 1 && V == 1) return {rt0.combine_single(args[0])};
-    StreamScope scope(args[0].sc, rt0);
+    StreamScope scope(args[0].sc, rt0, /*may_stay=*/true);
     const cudaStream_t stream = scope.comm.stream();
 
     const int R = rt0.num_ranks_;
@@ -502,6 +502,11 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
     int mode = a0.fuse_reduce == 0 ? 0 : 1;
     for (const auto& a : args) if (!a.dst_slot.has_value() || !a.count_matrix.has_value()) mode = 0;
     if (gated) mode = 0;
+    // Without SMs of its own the reduce kernel starts when the send kernel ends, and the counters only cost (the senders'
+    // system-scope fences: 74 against 60 us for the sends of four ranks on one GPU). All ranks have to agree on the mode, so
+    // this is decided only where all of them are in this launch.
+    const int free_sms = rt0.num_device_sms_ / V - num_sms;
+    if (V == R && free_sms < 8) mode = 0;
     const int num_blocks = num_sms;
     const bool weighted = a0.weighted && a0.do_expand;
     if (weighted) EP_HOST_ASSERT_MSG(a0.topk_weights.has_value(), "a weighted combine needs the top-k weights of the expanded rows");
@@ -550,8 +555,8 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
         p.num_send_blocks = num_sms;
 
         auto& r = res[v];
-        r.combined_x = at::empty({T, H}, opts(at::kBFloat16, device));
-        if (a.topk_weights.has_value()) r.combined_topk_weights = at::empty({T, K}, opts(at::kFloat, device));
+        r.combined_x = new_tensor({T, H}, at::kBFloat16, device);
+        if (a.topk_weights.has_value()) r.combined_topk_weights = new_tensor({T, K}, at::kFloat, device);
         CombineEpilogueParams& q = ep[v];
         q.num_tokens = T;
         q.num_topk = K;
@@ -618,9 +623,8 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
     // Arrival-driven: the reduce runs beside the send kernel, on the SMs that kernel leaves free (it is launched as
     // a programmatic dependent, so all send blocks are resident before the first reduce block starts).
     const bool beside = mode == 1 && !split && rt0.use_pdl_;
-    const int free_sms = rt0.num_device_sms_ / V - num_sms;
     const int epi_sms = beside && free_sms >= 8 ? free_sms : std::max(1, rt0.num_device_sms_ / V);
-    CUDA_RUNTIME_CHECK(launch_combine_epilogue(ep.data(), V, epi_sms, stream, beside));
+    CUDA_RUNTIME_CHECK(launch_combine_epilogue(ep.data(), V, epi_sms, stream, !gated && !split && rt0.use_pdl_));
     ++rt0.num_launches_;
     rt0.prof_record(5, stream);
     rt0.prof_valid_[1] = rt0.profiling_ != 0;
