@@ -265,8 +265,8 @@ struct LocalMoveParams {
     int num_out_rows, num_idx_rows;
     uint64_t* timeline;
 };
-// `quant`: bf16 rows are cast to e4m3 with 1x128 scales. `programmatic`: behind the plan kernel, nothing in between.
-cudaError_t launch_local_move(const LocalMoveParams& p, bool quant, int num_sms, bool programmatic, cudaStream_t stream);
+// `quant`: bf16 rows are cast to e4m3 with 1x128 scales.
+cudaError_t launch_local_move(const LocalMoveParams& p, bool quant, int num_sms, cudaStream_t stream);
 
 struct LocalCombineParams {
     int num_tokens, num_topk, num_experts, row_bytes, do_expand, weighted, idx32;

@@ -12,6 +12,7 @@
 #include "api.hpp"
 #include "gemm_api.hpp"
 #include "gemm_sm100.cuh"
+#include "../common/launch.hpp"
 
 namespace ep {
 namespace gemm {
@@ -162,7 +163,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 
     const int warp = warp_id(), lane = lane_id();
     const int num_kb = p.K / C::BK;
-    PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
+    launch_dependents();
 
     if (warp == 0 && lane == 0) {
         prefetch_tensormap(&map_a);
@@ -183,6 +184,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         tmem_alloc(tmem_slot, C::kTmemCols);
         tmem_relinquish();
     }
+    dependency_wait();           // everything above may run while the kernel ahead of this one drains
+    const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -384,7 +387,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const uint32_t cta = cluster_ctarank();
     const bool leader = cta == 0;
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
+    launch_dependents();
 
     if (warp == 0 && lane == 0) {
         prefetch_tensormap(&map_a);
@@ -403,6 +406,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         tmem_alloc_pair(tmem_slot, C::kTmemCols);
         tmem_relinquish_pair();
     }
+    dependency_wait();
+    const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
     cluster_sync_all();          // barriers of both CTAs are initialised before anything arrives on them
     tc_fence_after();
@@ -562,7 +567,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const bool leader = cta == 0;
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     const int num_kb = p.K / C::BK;
-    PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
+    launch_dependents();
 
     if (warp == C::kTmaWarp && lane == 0) {
         prefetch_tensormap(&map_a);
@@ -585,6 +590,8 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         tmem_alloc_pair(tmem_slot, C::kTmemCols);
         tmem_relinquish_pair();
     }
+    dependency_wait();
+    const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
     cluster_sync_all();
     tc_fence_after();
@@ -832,7 +839,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
 
     const int warp = warp_id(), lane = lane_id();
-    PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
+    launch_dependents();
 
     if (warp == 0 && lane == 0) {
         prefetch_tensormap(&map_a);
@@ -849,6 +856,8 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tmem_alloc(tmem_slot, C::kTmemCols);
         tmem_relinquish();
     }
+    dependency_wait();           // everything above may run while the kernel ahead of this one drains
+    const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1078,7 +1087,7 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const uint32_t cta = cluster_ctarank();
     const bool leader = cta == 0;
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
+    launch_dependents();
 
     if (warp == 0 && lane == 0) {
         prefetch_tensormap(&map_a);
@@ -1096,6 +1105,8 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tmem_alloc_pair(tmem_slot, C::kTmemCols);
         tmem_relinquish_pair();
     }
+    dependency_wait();
+    const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
     cluster_sync_all();
     tc_fence_after();
@@ -1326,8 +1337,7 @@ cudaError_t launch_tiles(int grid, cudaStream_t stream, const Args&... args) {
     static PreparedKernel prepared;
     const cudaError_t err = prepared.prepare(kKernel, C::kSmem);
     if (err != cudaSuccess) return err;
-    kKernel<<<grid, C::kThreads, C::kSmem, stream>>>(args...);
-    return cudaGetLastError();
+    return launch_early(kKernel, dim3(grid), dim3(C::kThreads), C::kSmem, stream, args...);
 }
 
 bool env_is(const char* name, char value) {

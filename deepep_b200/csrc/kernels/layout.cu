@@ -8,6 +8,7 @@
 
 #include "api.hpp"
 #include "../common/device_utils.cuh"
+#include "../common/launch.hpp"
 
 namespace ep {
 
@@ -60,6 +61,8 @@ __global__ void __launch_bounds__(256) legacy_handle_kernel(const int* __restric
                                                             int num_tokens, int* rank_prefix, int* sent, int* received, int* send_head, bool* in_rank) {
     __shared__ int s_base[kMaxRanks];
     const int R = num_ranks;
+    launch_dependents();
+    dependency_wait();
     if (threadIdx.x < R) {
         const int d = threadIdx.x;
         int acc = 0;
@@ -106,9 +109,8 @@ cudaError_t launch_dispatch_layout(const void* topk_idx, bool idx32, int num_tok
 cudaError_t launch_legacy_handle(const int* count_matrix, const int* token_slot, int rank, int num_ranks, int num_tokens, int* rank_prefix,
                                  int* sent, int* received, int* send_head, bool* in_rank, cudaStream_t stream) {
     const int64_t want = ceil_div<int64_t>(static_cast<int64_t>(num_tokens) * num_ranks, 256);
-    legacy_handle_kernel<<<static_cast<int>(want < 1 ? 1 : (want > 148 ? 148 : want)), 256, 0, stream>>>(
-        count_matrix, token_slot, rank, num_ranks, num_tokens, rank_prefix, sent, received, send_head, in_rank);
-    return cudaGetLastError();
+    return launch_early(legacy_handle_kernel, dim3(static_cast<int>(want < 1 ? 1 : (want > 148 ? 148 : want))), dim3(256), 0, stream, count_matrix, token_slot,
+                        rank, num_ranks, num_tokens, rank_prefix, sent, received, send_head, in_rank);
 }
 
 }  // namespace ep

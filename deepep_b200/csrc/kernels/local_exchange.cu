@@ -21,6 +21,7 @@
 
 #include "api.hpp"
 #include "../common/device_utils.cuh"
+#include "../common/launch.hpp"
 
 namespace ep {
 
@@ -57,7 +58,9 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
         p.timeline[0] = now;
         p.stamps[0] = now;
     }
-    launch_dependents();            // the move kernel's blocks may become resident; they wait for this grid's end
+    // The move kernel reads its input before its own wait: it may become resident once everything ahead of this kernel is done.
+    dependency_wait();
+    launch_dependents();
     // (first half of the barrier after which the other CTAs' shared memory may be written)
     if (num_ctas > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 
@@ -260,6 +263,8 @@ __global__ void __launch_bounds__(kMoveThreads, kExpand ? 6 : 8) local_move_kern
     const int t = static_cast<int>(warp_global / static_cast<uint32_t>(p.columns)), col = static_cast<int>(warp_global % static_cast<uint32_t>(p.columns));
     const int off = col * kMoveSlice + lane * 32;
     int4 lo, hi;
+    launch_dependents();
+    if (!p.plan_ahead) dependency_wait();
     if (t < T) load_32(p.x + static_cast<int64_t>(t) * p.x_stride_bytes + off, p.src_row_bytes - off, wide_in, lo, hi);
     if (p.plan_ahead) dependency_wait();
     if (t < T) {
@@ -407,6 +412,8 @@ constexpr int kCombineThreads = 128;
 // kernel below, whose registers leave a third of the warps resident, the same copy took 45 instead of 39 us).
 __global__ void __launch_bounds__(256, 8) local_return_kernel(const __grid_constant__ LocalCombineParams p) {
     const int lane = lane_id(), K = p.num_topk;
+    launch_dependents();
+    dependency_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) p.timeline[0] = globaltimer_ns();
     const uint32_t warp_global = blockIdx.x * 8 + warp_id();
     const int t = static_cast<int>(warp_global / static_cast<uint32_t>(p.columns)), col = static_cast<int>(warp_global % static_cast<uint32_t>(p.columns));
@@ -436,6 +443,8 @@ __global__ void __launch_bounds__(kCombineThreads) local_combine_kernel(const __
     const int warp_global = blockIdx.x * (kCombineThreads / 32) + warp_id();
     const int col = warp_global % p.columns, step = p.warps / p.columns;
     const int v0 = col * 32 * NV + lane;
+    launch_dependents();
+    dependency_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) p.timeline[0] = globaltimer_ns();
     int t = warp_global < p.warps ? warp_global / p.columns : T;
     int next_row = -1, later_slot = -1;     // row of the next token (this lane's, when expanded), slot of the one after it
@@ -536,20 +545,6 @@ int balanced_warps(int tokens, int columns, int most) {
     return (per_column < 1 ? 1 : per_column) * columns;
 }
 
-template <typename Kernel, typename Params>
-cudaError_t launch_plain(Kernel kernel, const Params& p, int grid, int block, cudaStream_t stream, bool programmatic) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
 }  // namespace
 
 cudaError_t launch_local_plan(const LocalPlanParams& p, cudaStream_t stream) {
@@ -565,17 +560,19 @@ cudaError_t launch_local_plan(const LocalPlanParams& p, cudaStream_t stream) {
     cfg.blockDim = dim3(kPlanThreads);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = programmatic_launches() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, local_plan_kernel, p);
 }
 
 template <bool kQuant, bool kExpand>
-static cudaError_t launch_move_cfg(LocalMoveParams& p, int num_sms, bool programmatic, cudaStream_t stream) {
+static cudaError_t launch_move_cfg(LocalMoveParams& p, int num_sms, cudaStream_t stream) {
     static PreparedKernel prepared;
     cudaError_t err = prepared.prepare(local_move_kernel<kQuant, kExpand>, 0);
     if (err != cudaSuccess) return err;
@@ -586,17 +583,17 @@ static cudaError_t launch_move_cfg(LocalMoveParams& p, int num_sms, bool program
     if (kExpand && p.do_zero_padding)
         warps = std::max<int64_t>(warps, std::min<int64_t>(num_sms * 32, static_cast<int64_t>(p.num_experts) * ceil_div(p.expert_alignment, kPadRows)));
     const int grid = std::max(1, static_cast<int>(ceil_div<int64_t>(warps, kMoveThreads / 32)));
-    return launch_plain(local_move_kernel<kQuant, kExpand>, p, grid, kMoveThreads, stream, programmatic);
+    return launch_early(local_move_kernel<kQuant, kExpand>, dim3(grid), dim3(kMoveThreads), 0, stream, p);
 }
 
-cudaError_t launch_local_move(const LocalMoveParams& params, bool quant, int num_sms, bool programmatic, cudaStream_t stream) {
+cudaError_t launch_local_move(const LocalMoveParams& params, bool quant, int num_sms, cudaStream_t stream) {
     LocalMoveParams p = params;
     const uint64_t in_bits = reinterpret_cast<uintptr_t>(p.x) | static_cast<uint64_t>(p.x_stride_bytes);
     const uint64_t out_bits = reinterpret_cast<uintptr_t>(p.recv_x) | static_cast<uint64_t>(p.recv_x_pitch);
     p.wide_in = in_bits % 32 == 0;
     p.wide_out = out_bits % 32 == 0;
-    if (quant) return p.do_expand ? launch_move_cfg<true, true>(p, num_sms, programmatic, stream) : launch_move_cfg<true, false>(p, num_sms, programmatic, stream);
-    return p.do_expand ? launch_move_cfg<false, true>(p, num_sms, programmatic, stream) : launch_move_cfg<false, false>(p, num_sms, programmatic, stream);
+    if (quant) return p.do_expand ? launch_move_cfg<true, true>(p, num_sms, stream) : launch_move_cfg<true, false>(p, num_sms, stream);
+    return p.do_expand ? launch_move_cfg<false, true>(p, num_sms, stream) : launch_move_cfg<false, false>(p, num_sms, stream);
 }
 
 template <int NV, int NR, bool kExpand, bool kWeighted>
@@ -609,7 +606,7 @@ static cudaError_t launch_combine_cfg(LocalCombineParams& p, int num_sms, cudaSt
     const int warps_per_block = kCombineThreads / 32, most = num_sms * resident_blocks(kernel, kCombineThreads, per_sm) * warps_per_block;
     p.columns = ceil_div(p.row_bytes / 16, 32 * NV);
     p.warps = balanced_warps(p.num_tokens, p.columns, most);
-    return launch_plain(kernel, p, ceil_div(p.warps, warps_per_block), kCombineThreads, stream, false);
+    return launch_early(kernel, dim3(ceil_div(p.warps, warps_per_block)), dim3(kCombineThreads), 0, stream, p);
 }
 
 cudaError_t launch_local_combine(const LocalCombineParams& params, int num_sms, cudaStream_t stream) {
@@ -623,7 +620,7 @@ cudaError_t launch_local_combine(const LocalCombineParams& params, int num_sms, 
         p.wide = (reinterpret_cast<uintptr_t>(p.x) | static_cast<uint64_t>(p.x_stride_bytes) | reinterpret_cast<uintptr_t>(p.combined_x) | static_cast<uint64_t>(p.row_bytes)) % 32 == 0;
         const int64_t warps = static_cast<int64_t>(p.num_tokens) * p.columns;
         if (warps >= (1ll << 31)) return cudaErrorInvalidValue;
-        return launch_plain(local_return_kernel, p, static_cast<int>(ceil_div<int64_t>(warps, 8)), 256, stream, false);
+        return launch_early(local_return_kernel, dim3(static_cast<int>(ceil_div<int64_t>(warps, 8))), dim3(256), 0, stream, p);
     }
     // Otherwise a resident grid, since looking up the rows of a token is a chain of two loads that the loop hides; up to four
     // rows two vectors at a time, more than four one (128 bytes in flight per lane either way).

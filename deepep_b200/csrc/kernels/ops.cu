@@ -11,6 +11,7 @@
 
 #include "ops_api.hpp"
 #include "../common/device_utils.cuh"
+#include "../common/launch.hpp"
 
 namespace ep {
 namespace ops {
@@ -25,6 +26,8 @@ __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162f
 template <int kPerLane, typename Logit>
 __global__ void __launch_bounds__(256) router_topk_kernel(const Logit* __restrict__ logits, int64_t row_stride, int num_tokens, int num_experts, int num_topk,
                                                           int64_t* __restrict__ topk_idx, float* __restrict__ topk_weights) {
+    launch_dependents();
+    dependency_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = lane_id();
     if (warp >= num_tokens) return;
     const Logit* row = logits + static_cast<int64_t>(warp) * row_stride;
@@ -72,6 +75,8 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const Logit* __restric
 // Router weights fp32 [experts, hidden] -> bf16 [padded experts, hidden], zero rows behind the last expert (the GEMM tiles
 // its columns in multiples of 128).
 __global__ void __launch_bounds__(256) router_weights_kernel(const float* __restrict__ w, int num_experts, int padded, int hidden, __nv_bfloat16* __restrict__ out) {
+    launch_dependents();
+    dependency_wait();
     const int64_t n = static_cast<int64_t>(padded) * hidden / 8, real = static_cast<int64_t>(num_experts) * hidden / 8;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         int4 v = make_int4(0, 0, 0, 0);
@@ -110,6 +115,8 @@ __device__ __forceinline__ RowCol row_col(int columns) {
 __global__ void __launch_bounds__(256) router_backward_kernel(const int64_t* __restrict__ topk_idx, const float* __restrict__ w, const float* __restrict__ dw,
                                                               int num_tokens, int num_topk, int num_experts, int padded, int hidden, int columns,
                                                               const __nv_bfloat16* __restrict__ router, __nv_bfloat16* dx, __nv_bfloat16* __restrict__ dlogits) {
+    launch_dependents();
+    dependency_wait();
     const RowCol rc = row_col(columns);
     const int t = rc.row, lane = lane_id();
     if (t >= num_tokens) return;
@@ -202,6 +209,8 @@ __device__ __forceinline__ void pack16(const float (&f)[16], int4& lo, int4& hi)
 // is read once and held in registers between the two passes, instead of five passes over fp32 copies of the weights.
 __global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* __restrict__ w, int rows, int cols, int pow2, uint8_t* __restrict__ q,
                                                            float* __restrict__ scales) {
+    launch_dependents();
+    dependency_wait();
     __shared__ float s_max[8];
     const int64_t base = (static_cast<int64_t>(blockIdx.z) * rows + blockIdx.y * 128) * cols + blockIdx.x * 128;
     const int r0 = threadIdx.x >> 3, c = (threadIdx.x & 7) * 16;        // 32 rows per pass, 16 channels per thread
@@ -241,6 +250,8 @@ __global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* 
 __global__ void __launch_bounds__(256) quant_kernel(const uint8_t* __restrict__ x, int64_t x_stride_bytes, int rows, int hidden, int columns, int wide, int pow2,
                                                     uint8_t* __restrict__ out, float* __restrict__ scales, int64_t sf_row_stride,
                                                     int64_t sf_col_stride) {
+    launch_dependents();
+    dependency_wait();
     const RowCol rc = row_col(columns);
     if (rc.row >= rows) return;
     int4 lo, hi;
@@ -255,6 +266,8 @@ __global__ void __launch_bounds__(256) quant_kernel(const uint8_t* __restrict__ 
 
 __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scales, int64_t sf_row_stride,
                                                       int64_t sf_col_stride, int rows, int hidden, int columns, int wide, const RowGroups groups, uint8_t* __restrict__ out) {
+    launch_dependents();
+    dependency_wait();
     const RowCol rc = row_col(columns);
     if (rc.row >= rows) return;
     const bool in = rc.ch < hidden;
@@ -285,6 +298,8 @@ template <bool kQuant>
 __global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__ x, int rows, int inter, int columns, int wide, const float* __restrict__ row_weight,
                                                      const int* __restrict__ num_valid_rows, const RowGroups groups, uint8_t* __restrict__ out,
                                                      float* __restrict__ scales, int64_t sf_row_stride, int64_t sf_col_stride, int pow2) {
+    launch_dependents();
+    dependency_wait();
     const RowCol rc = row_col(columns);
     if (rc.row >= (num_valid_rows != nullptr ? min(*num_valid_rows, rows) : rows)) return;
     if (in_gap(groups, rc.row)) return;
@@ -321,6 +336,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__
 __global__ void __launch_bounds__(128) swiglu_bwd_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ dout, int inter, int wide,
                                                          const float* __restrict__ row_weight, const RowGroups groups, uint8_t* __restrict__ dx,
                                                          uint8_t* __restrict__ act_out, float* __restrict__ dweight) {
+    launch_dependents();
+    dependency_wait();
     __shared__ float s_part[4];
     const int row = blockIdx.x;
     const bool gap = in_gap(groups, row);
@@ -386,6 +403,8 @@ __global__ void __launch_bounds__(128) swiglu_bwd_kernel(const uint8_t* __restri
 // and stores them as one 16-byte vector. Edge tiles and unaligned tensors take the element-wise path.
 __global__ void __launch_bounds__(256) transpose_kernel(const __nv_bfloat16* __restrict__ in, int64_t in_stride, int64_t in_batch, int rows, int cols,
                                                         __nv_bfloat16* __restrict__ out, int64_t out_stride, int64_t out_batch, int aligned) {
+    launch_dependents();
+    dependency_wait();
     __shared__ uint32_t tile_t[64 * 33];      // [column][row pair]
     const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
     in += blockIdx.z * in_batch;
@@ -449,11 +468,10 @@ static cudaError_t router_topk_any(const Logit* logits, int64_t row_stride, int 
     if (num_experts > 2048 || num_topk > 32 || num_topk > num_experts) return cudaErrorInvalidValue;
     const int blocks = (num_tokens * 32 + 255) / 256;
     const int per_lane = (num_experts + 31) / 32;
-    if (per_lane <= 2) router_topk_kernel<2><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    else if (per_lane <= 8) router_topk_kernel<8><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    else if (per_lane <= 16) router_topk_kernel<16><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    else router_topk_kernel<64><<<blocks, 256, 0, stream>>>(logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
-    return cudaGetLastError();
+    if (per_lane <= 2) return launch_early(router_topk_kernel<2, Logit>, dim3(blocks), dim3(256), 0, stream, logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    if (per_lane <= 8) return launch_early(router_topk_kernel<8, Logit>, dim3(blocks), dim3(256), 0, stream, logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    if (per_lane <= 16) return launch_early(router_topk_kernel<16, Logit>, dim3(blocks), dim3(256), 0, stream, logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
+    return launch_early(router_topk_kernel<64, Logit>, dim3(blocks), dim3(256), 0, stream, logits, row_stride, num_tokens, num_experts, num_topk, topk_idx, topk_weights);
 }
 
 cudaError_t router_topk(const void* logits, bool bf16, int64_t row_stride, int num_tokens, int num_experts, int num_topk, int64_t* topk_idx,
@@ -465,9 +483,7 @@ cudaError_t router_topk(const void* logits, bool bf16, int64_t row_stride, int n
 cudaError_t router_weights(const float* w, int num_experts, int padded_experts, int hidden, void* out, cudaStream_t stream) {
     if (hidden % 8 != 0) return cudaErrorInvalidValue;
     const int64_t want = (static_cast<int64_t>(padded_experts) * hidden / 8 + 255) / 256;
-    router_weights_kernel<<<static_cast<int>(std::min<int64_t>(std::max<int64_t>(want, 1), 148 * 16)), 256, 0, stream>>>(
-        w, num_experts, padded_experts, hidden, static_cast<__nv_bfloat16*>(out));
-    return cudaGetLastError();
+    return launch_early(router_weights_kernel, dim3(static_cast<int>(std::min<int64_t>(std::max<int64_t>(want, 1), 148 * 16))), dim3(256), 0, stream, w, num_experts, padded_experts, hidden, static_cast<__nv_bfloat16*>(out));
 }
 
 cudaError_t router_backward(const int64_t* topk_idx, const float* w, const float* dw, int num_tokens, int num_topk, int num_experts, int padded_experts,
@@ -476,18 +492,15 @@ cudaError_t router_backward(const int64_t* topk_idx, const float* w, const float
     const int columns = (hidden + kSpan - 1) / kSpan;
     const int64_t warps = static_cast<int64_t>(num_tokens) * columns;
     if (num_topk > 32 || padded_experts % 8 != 0 || hidden % 8 != 0 || warps >= (1ll << 31)) return cudaErrorInvalidValue;
-    router_backward_kernel<<<static_cast<int>((warps + 7) / 8), 256, 0, stream>>>(
-        topk_idx, w, dw, num_tokens, num_topk, num_experts, padded_experts, hidden, columns, static_cast<const __nv_bfloat16*>(router),
+    return launch_early(router_backward_kernel, dim3(static_cast<int>((warps + 7) / 8)), dim3(256), 0, stream, topk_idx, w, dw, num_tokens, num_topk, num_experts, padded_experts, hidden, columns, static_cast<const __nv_bfloat16*>(router),
         static_cast<__nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(dlogits));
-    return cudaGetLastError();
 }
 
 cudaError_t quant_weights_128x128(const void* w, int groups, int rows, int cols, bool pow2, void* q, float* scales, cudaStream_t stream) {
     if (groups == 0 || rows == 0 || cols == 0) return cudaSuccess;
     if (rows % 128 != 0 || cols % 128 != 0 || groups > 65535 || rows / 128 > 65535) return cudaErrorInvalidValue;
-    weight_quant_kernel<<<dim3(cols / 128, rows / 128, groups), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(w), rows, cols, pow2 ? 1 : 0,
+    return launch_early(weight_quant_kernel, dim3(cols / 128, rows / 128, groups), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(w), rows, cols, pow2 ? 1 : 0,
                                                                                   static_cast<uint8_t*>(q), scales);
-    return cudaGetLastError();
 }
 
 cudaError_t quant_1x128(const void* x, int64_t x_stride_bytes, int rows, int hidden, bool pow2, void* out, float* scales,
@@ -495,10 +508,9 @@ cudaError_t quant_1x128(const void* x, int64_t x_stride_bytes, int rows, int hid
     if (rows == 0) return cudaSuccess;
     const int columns = ceil_div(hidden, kSpan), blocks = span_blocks(rows, columns);
     if (hidden % 128 != 0 || blocks == 0) return cudaErrorInvalidValue;
-    quant_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(x), x_stride_bytes, rows, hidden, columns,
+    return launch_early(quant_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), x_stride_bytes, rows, hidden, columns,
                                              is_wide({addr(x), static_cast<uint64_t>(x_stride_bytes)}), pow2, static_cast<uint8_t*>(out), scales,
                                              sf_row_stride, sf_col_stride);
-    return cudaGetLastError();
 }
 
 cudaError_t dequant_1x128(const void* q, const float* scales, int64_t sf_row_stride, int64_t sf_col_stride, int rows, int hidden,
@@ -506,9 +518,8 @@ cudaError_t dequant_1x128(const void* q, const float* scales, int64_t sf_row_str
     if (rows == 0) return cudaSuccess;
     const int columns = ceil_div(hidden, kSpan), blocks = span_blocks(rows, columns);
     if (hidden % 128 != 0 || blocks == 0) return cudaErrorInvalidValue;
-    dequant_kernel<<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(q), scales, sf_row_stride, sf_col_stride, rows, hidden, columns,
+    return launch_early(dequant_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(q), scales, sf_row_stride, sf_col_stride, rows, hidden, columns,
                                                is_wide({addr(out)}), groups, static_cast<uint8_t*>(out));
-    return cudaGetLastError();
 }
 
 cudaError_t swiglu(const void* x, int rows, int inter, const float* row_weight, const int* num_valid_rows, const RowGroups& groups, void* out, bool quant,
@@ -518,12 +529,11 @@ cudaError_t swiglu(const void* x, int rows, int inter, const float* row_weight, 
     if (inter % 8 != 0 || (quant && inter % 128 != 0) || blocks == 0) return cudaErrorInvalidValue;
     const int wide = is_wide({addr(x), addr(out), static_cast<uint64_t>(inter) * 2});
     if (quant)
-        swiglu_kernel<true><<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
+        return launch_early(swiglu_kernel<true>, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
                                                         static_cast<uint8_t*>(out), scales, sf_row_stride, sf_col_stride, pow2 ? 1 : 0);
     else
-        swiglu_kernel<false><<<blocks, 256, 0, stream>>>(static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
+        return launch_early(swiglu_kernel<false>, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
                                                          static_cast<uint8_t*>(out), nullptr, 0, 0, 0);
-    return cudaGetLastError();
 }
 
 cudaError_t swiglu_backward(const void* x, const void* dout, int rows, int inter, const float* row_weight, const RowGroups& groups, void* dx, void* act_out,
@@ -532,9 +542,8 @@ cudaError_t swiglu_backward(const void* x, const void* dout, int rows, int inter
     if (inter % 8 != 0) return cudaErrorInvalidValue;
     const int threads = std::min(128, align_up(ceil_div(inter, 16), 32));
     const int wide = is_wide({addr(x), addr(dout), addr(dx), addr(act_out), static_cast<uint64_t>(inter) * 2});
-    swiglu_bwd_kernel<<<rows, threads, 0, stream>>>(static_cast<const uint8_t*>(x), static_cast<const uint8_t*>(dout), inter, wide, row_weight, groups,
+    return launch_early(swiglu_bwd_kernel, dim3(rows), dim3(threads), 0, stream, static_cast<const uint8_t*>(x), static_cast<const uint8_t*>(dout), inter, wide, row_weight, groups,
                                                     static_cast<uint8_t*>(dx), static_cast<uint8_t*>(act_out), dweight);
-    return cudaGetLastError();
 }
 
 cudaError_t transpose_bf16(const void* in, int64_t in_stride, int64_t in_batch, int batch, int rows, int cols, void* out, int64_t out_stride,
@@ -542,9 +551,8 @@ cudaError_t transpose_bf16(const void* in, int64_t in_stride, int64_t in_batch, 
     if (rows == 0 || cols == 0 || batch == 0) return cudaSuccess;
     dim3 grid((cols + 63) / 64, (rows + 63) / 64, batch);
     const int aligned = in_stride % 8 == 0 && out_stride % 8 == 0 && in_batch % 8 == 0 && out_batch % 8 == 0 && addr(in) % 16 == 0 && addr(out) % 16 == 0;
-    transpose_kernel<<<grid, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(in), in_stride, in_batch, rows, cols, static_cast<__nv_bfloat16*>(out),
+    return launch_early(transpose_kernel, grid, dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(in), in_stride, in_batch, rows, cols, static_cast<__nv_bfloat16*>(out),
                                                out_stride, out_batch, aligned);
-    return cudaGetLastError();
 }
 
 }  // namespace ops

@@ -199,9 +199,8 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     q.timeline = timeline_of(local_ws_, kTlDispatch);
     const bool gated = a.sc.previous_event_before_epilogue.has_value();
     if (gated) a.sc.previous_event_before_epilogue->stream_wait(scope.comm);
-    const bool programmatic = !cached && !gated && use_pdl_;
-    q.plan_ahead = programmatic ? 1 : 0;
-    CUDA_RUNTIME_CHECK(launch_local_move(q, quant, num_device_sms_, programmatic, stream));
+    q.plan_ahead = !cached && !gated && use_pdl_ ? 1 : 0;
+    CUDA_RUNTIME_CHECK(launch_local_move(q, quant, num_device_sms_, stream));
     ++num_launches_;
     prof_record(1, stream);
     prof_record(2, stream);
