@@ -71,140 +71,42 @@ __device__ __forceinline__ int4 pack_bf16x8(const float (&acc)[8]) {
     return out;
 }
 
-// NV columns (16 bytes each) per lane and pass, rows taken NR at a time.
-template <int NV, int NR>
-__device__ __forceinline__ void reduce_columns(const CombineEpilogueParams& p, int t, uint32_t mask, int lane, const uint8_t* b0,
-                                               const uint8_t* b1) {
-    const int vec_per_row = p.hidden / 8;
-    const uint64_t row_bytes = static_cast<uint64_t>(p.hidden) * 2;
-    for (int v = lane; v < vec_per_row; v += 32 * NV) {
-        float acc[NV][8];
-#pragma unroll
-        for (int j = 0; j < NV; ++j)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
-        uint32_t todo = mask;
-        while (todo) {
-            int rows[NR];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                rows[r] = todo ? __ffs(todo) - 1 : -1;
-                todo &= todo - 1;       // 0 stays 0
-            }
-            int4 raw[NR][NV];
-            float wt[NR];
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                wt[r] = (p.weighted && rows[r] >= 0) ? row_weight(p, t, rows[r]) : 1.f;
-#pragma unroll
-                for (int j = 0; j < NV; ++j)
-                    if (rows[r] >= 0 && v + 32 * j < vec_per_row)
-                        raw[r][j] = ld_nc_int4(p.region_x + (static_cast<uint64_t>(rows[r]) * p.num_max_tokens + t) * row_bytes + (v + 32 * j) * 16);
-            }
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-#pragma unroll
-                for (int j = 0; j < NV; ++j)
-                    if (rows[r] >= 0 && v + 32 * j < vec_per_row) {
-                        if (p.weighted) accumulate_bf16x8_scaled(acc[j], raw[r][j], wt[r]);
-                        else accumulate_bf16x8(acc[j], raw[r][j]);
-                    }
-        }
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            if (v + 32 * j >= vec_per_row) break;
-            if (b0 != nullptr) accumulate_bf16x8(acc[j], ld_nc_int4(b0 + (v + 32 * j) * 16));
-            if (b1 != nullptr) accumulate_bf16x8(acc[j], ld_nc_int4(b1 + (v + 32 * j) * 16));
-            st_na_int4(p.combined_x + t * row_bytes + (v + 32 * j) * 16, pack_bf16x8(acc[j]));
-        }
-    }
-}
-
-// ==================================================================== reduce of one token (one warp)
-// combined_x[t] = sum over the lanes that hold a row for the token, ascending, fp32, + bias_0 + bias_1, one bf16 rounding.
-// `e` is the lane's expert (-1 = unused top-k lane), identical on both callers.
-__device__ __forceinline__ void reduce_token(const CombineEpilogueParams& p, int t, int e, int lane) {
-    const int K = p.num_topk, EL = p.num_local_experts;
-    const int vec_per_row = p.hidden / 8;
-    const uint64_t row_bytes = static_cast<uint64_t>(p.hidden) * 2;
-    const int slot_lane = e < 0 ? -1 : (p.use_rank_layout ? e / EL : lane);
-    uint32_t mask = slot_lane >= 0 ? (1u << slot_lane) : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mask |= __shfl_xor_sync(0xffffffffu, mask, o);
-    if (p.combined_topk_weights != nullptr && lane < K) {
-        float wv = 0.f;
-        if (slot_lane >= 0 && p.region_w != nullptr)
-            wv = p.region_w[(static_cast<uint64_t>(slot_lane) * p.num_max_tokens + t) * K + lane];
-        p.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = wv;
-    }
-    const uint8_t* b0 = p.bias0 != nullptr ? p.bias0 + t * row_bytes : nullptr;
-    const uint8_t* b1 = p.bias1 != nullptr ? p.bias1 + t * row_bytes : nullptr;
-    if (__popc(mask) == 1 && b0 == nullptr && b1 == nullptr && !p.weighted) {
-        // a single contribution (e.g. one rank): the sum is a copy; keep four loads in flight per lane
-        const uint8_t* src = p.region_x + (static_cast<uint64_t>(__ffs(mask) - 1) * p.num_max_tokens + t) * row_bytes;
-        uint8_t* dst = p.combined_x + t * row_bytes;
-        for (int v = lane; v < vec_per_row; v += 128) {
-            int4 raw[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (v + 32 * j < vec_per_row) raw[j] = ld_nc_int4(src + (v + 32 * j) * 16);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (v + 32 * j < vec_per_row) st_na_int4(dst + (v + 32 * j) * 16, raw[j]);
-        }
-        return;
-    }
-    // Eight 16-byte loads are in flight per lane before the first add: eight rows of one column, or (when at most
-    // four lanes contribute) four rows of two columns. The adds run in ascending lane order either way.
-    if (__popc(mask) <= 4)
-        reduce_columns<2, 4>(p, t, mask, lane, b0, b1);
-    else
-        reduce_columns<1, 8>(p, t, mask, lane, b0, b1);
-}
-
 __device__ __forceinline__ int token_expert(const CombineEpilogueParams& p, int t, int lane) {
     if (lane >= p.num_topk) return -1;
     return load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * p.num_topk + lane, p.num_local_experts * p.num_ranks);
 }
 
-__device__ __noinline__ void reduce_token_registers(const CombineEpilogueParams& p, int t, int e, int lane) {
-    reduce_token(p, t, e, lane);
+// ==================================================================== reduce epilogue (local, all SMs or those beside the send kernel)
+// combined_x[t] = sum over the lanes that hold a row for the token, ascending, fp32, + bias_0 + bias_1, one bf16 rounding.
+// A warp takes a part of a token's columns; per KB of the row it has four contributing rows in flight (32 bytes per lane and
+// row) and adds them from registers: 24 warps keep up to 96 KB per SM in flight, more than the bandwidth an SM reaches
+// needs. A token is cut into parts while there are fewer than four work items per warp, so that the last round of a small
+// batch is short. (Rows staged through shared memory with bulk copies and mbarriers by twelve warps spent 80 instructions
+// per 512 bytes of a row, half of them for rows that were not there: 49 us for 4 x 1024 tokens of 3.6 rows x 8 KB.)
+constexpr int kEpiWarps = 24, kEpiRows = 4, kEpiColumn = 1024;
+
+__device__ __forceinline__ void load_row32(const uint8_t* src, int bytes_left, bool wide, int4& lo, int4& hi) {
+    // (not the read-only path: with arrival counters the rows are written while this kernel runs)
+    if (wide && bytes_left >= 32) {
+        asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w) : "l"(src) : "memory");
+        return;
+    }
+    lo = hi = make_int4(0, 0, 0, 0);
+    if (bytes_left >= 16) lo = __ldcg(reinterpret_cast<const int4*>(src));
+    if (bytes_left >= 32) hi = __ldcg(reinterpret_cast<const int4*>(src + 16));
 }
 
-// ==================================================================== reduce epilogue (local, all SMs)
-// Rows are staged through shared memory with bulk copies: a warp owns a ring of kEpiSlots chunk slots of 1 KB and keeps
-// floor(kEpiSlots / n) chunks of each of a token's n contributing rows in flight (8 deep for two rows, 2 deep for
-// eight: the bytes in flight per SM, which set the bandwidth a reduce SM reaches, do not depend on the routing), then
-// every lane sums its two 16-byte pieces of the chunk over the rows in ascending lane order. The chunk size matters: every chunk costs a proxy fence, two
-// warp barriers and an mbarrier round, and with 512-byte chunks that fixed cost, not memory, set the pace (147 us
-// against 130 us for the EP8-shaped case). Tokens with at most one row, more than kEpiRows rows, or a row size that is
-// not a multiple of the chunk take the register path (reduce_token).
-constexpr int kEpiSlots = 16, kEpiMaxDepth = 8, kEpiRows = 8, kEpiChunk = 1024, kEpiWarps = 12;
-constexpr int kEpiWarpBytes = kEpiSlots * kEpiChunk;
-constexpr int kEpiSmem = kEpiWarps * kEpiWarpBytes + kEpiWarps * kEpiMaxDepth * 8;
-
-__global__ void __launch_bounds__(kEpiWarps * 32) combine_epilogue_kernel(const __grid_constant__ Multi<CombineEpilogueParams> m) {
-    extern __shared__ __align__(128) uint8_t epi_smem[];
+__global__ void __launch_bounds__(kEpiWarps * 32, 1) combine_epilogue_kernel(const __grid_constant__ Multi<CombineEpilogueParams> m) {
     const int vr = blockIdx.x / m.blocks_per_rank;
     const int bid = blockIdx.x % m.blocks_per_rank;
     const int nb = m.blocks_per_rank;
     const CombineEpilogueParams& p = m.r[vr];
     const int lane = lane_id(), warp = warp_id();
     const int num_warps = blockDim.x >> 5;
-    uint8_t* sbuf = epi_smem + static_cast<size_t>(warp) * kEpiWarpBytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + kEpiWarps * kEpiWarpBytes) + warp * kEpiMaxDepth;
-    if (lane == 0) {
-        for (int s = 0; s < kEpiMaxDepth; ++s) mbar_init(bars + s, 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    uint32_t parity = 0;                    // bit s = phase the next wait on stage s expects
-    bool staged_ok = true;                  // a wait that ever ran out sends the rest through the register path
     const int K = p.num_topk, EL = p.num_local_experts;
-    const uint64_t row_bytes = static_cast<uint64_t>(p.hidden) * 2;
-    const int nchunks = static_cast<int>(row_bytes / kEpiChunk);
-    const bool chunkable = row_bytes % kEpiChunk == 0;
-    const uint64_t deadline = globaltimer_ns() + 2000000000ull;
+    const int row_bytes = p.hidden * 2;
+    const int columns = ceil_div(row_bytes, kEpiColumn);
     uint64_t* timeline = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(p.local_ws) + kWsTimelineOffsetBytes) + 2 * kTlCombineReduce;
     if (bid == 0 && threadIdx.x == 0) timeline[0] = globaltimer_ns();
     // Flag-driven mode: this kernel runs beside the send kernel (it never waits for it as a whole); the tokens of
@@ -223,8 +125,14 @@ __global__ void __launch_bounds__(kEpiWarps * 32) combine_epilogue_kernel(const 
         s_held[src] = p.count_matrix[me * p.num_ranks + src];
     }
     __syncthreads();
+    const bool wide = ((reinterpret_cast<uintptr_t>(p.region_x) | reinterpret_cast<uintptr_t>(p.combined_x) | reinterpret_cast<uintptr_t>(p.bias0) |
+                        reinterpret_cast<uintptr_t>(p.bias1) | static_cast<uintptr_t>(row_bytes)) & 31) == 0;
+    int parts = 1;
+    while (parts * 2 <= columns && static_cast<int64_t>(p.num_tokens) * parts < 4 * nb * num_warps) parts *= 2;
+    const int per_part = ceil_div(columns, parts);
 
-    for (int t = bid * num_warps + warp; t < p.num_tokens && flags_ok; t += nb * num_warps) {
+    for (int64_t item = bid * num_warps + warp; item < static_cast<int64_t>(p.num_tokens) * parts && flags_ok; item += nb * num_warps) {
+        const int t = static_cast<int>(item / parts), part = static_cast<int>(item % parts);
         const int e = token_expert(p, t, lane);
         if (flagged) {
             bool ok = true;
@@ -242,73 +150,64 @@ __global__ void __launch_bounds__(kEpiWarps * 32) combine_epilogue_kernel(const 
             }
             flags_ok = __all_sync(0xffffffffu, ok);
             if (!flags_ok) break;
-            // (the rows are then read with bulk copies, which fetch from L2, where the senders' completed writes are;
-            // a full async-proxy fence per token would serialise the warps of the SM at microseconds apiece)
+            __syncwarp();
         }
         const int slot_lane = e < 0 ? -1 : (p.use_rank_layout ? e / EL : lane);
-        uint32_t mask = slot_lane >= 0 ? (1u << slot_lane) : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mask |= __shfl_xor_sync(0xffffffffu, mask, o);
-        const int n = __popc(mask);
-        if (!chunkable || !staged_ok || n < 2 || n > kEpiRows) {
-            reduce_token_registers(p, t, e, lane);
-            continue;
-        }
-        if (p.combined_topk_weights != nullptr && lane < K) {
+        uint32_t mask = __reduce_or_sync(0xffffffffu, slot_lane >= 0 ? (1u << slot_lane) : 0u);
+        if (part == 0 && p.combined_topk_weights != nullptr && lane < K) {
             float wv = 0.f;
             if (slot_lane >= 0 && p.region_w != nullptr)
                 wv = p.region_w[(static_cast<uint64_t>(slot_lane) * p.num_max_tokens + t) * K + lane];
             p.combined_topk_weights[static_cast<int64_t>(t) * K + lane] = wv;
         }
-        const uint8_t* b0 = p.bias0 != nullptr ? p.bias0 + t * row_bytes : nullptr;
-        const uint8_t* b1 = p.bias1 != nullptr ? p.bias1 + t * row_bytes : nullptr;
-        // lane r < n loads row r = the r-th contributing lane of the region (ascending)
+        const int n = __popc(mask);
+        // lane r < n knows row r = the r-th contributing lane of the region (ascending)
         const int my_slot = lane < n ? static_cast<int>(__fns(mask, 0, lane + 1)) : 0;
         const float my_wt = (p.weighted && lane < n) ? row_weight(p, t, my_slot) : 1.f;
-        const uint8_t* my_src = p.region_x + (static_cast<uint64_t>(my_slot) * p.num_max_tokens + t) * row_bytes;
-        uint8_t* dst = p.combined_x + t * row_bytes;
-        const int depth = min(kEpiMaxDepth, kEpiSlots / n);      // stage s of this token = slots [s * n, (s + 1) * n)
-        for (int c = 0; c < nchunks + depth - 1 && staged_ok; ++c) {
-            if (c < nchunks) {
-                const int s = c % depth;
-                fence_proxy_async_smem();       // this stage was read (generic proxy) one iteration ago
-                __syncwarp();
-                if (lane == 0) mbar_arrive_expect_tx(bars + s, static_cast<uint32_t>(n) * kEpiChunk);
-                __syncwarp();
-                if (lane < n) bulk_g2s(sbuf + (s * n + lane) * kEpiChunk, my_src + static_cast<uint64_t>(c) * kEpiChunk, kEpiChunk, bars + s);
-            }
-            if (c >= depth - 1) {
-                const int cc = c - (depth - 1), s = cc % depth;
-                uint32_t spins = 0;
-                bool ok = true;
-                while (!mbar_try_wait(bars + s, (parity >> s) & 1u)) {
-                    if ((++spins & 1023u) == 0 && globaltimer_ns() > deadline) { ok = false; break; }
+        const uint8_t* token_rows = p.region_x + static_cast<uint64_t>(t) * row_bytes + lane * 32;
+        const uint64_t lane_pitch = static_cast<uint64_t>(p.num_max_tokens) * row_bytes;
+        const uint64_t out = static_cast<uint64_t>(t) * row_bytes;
+        const bool copy = n == 1 && p.bias0 == nullptr && p.bias1 == nullptr && !p.weighted;       // the sum of one row is the row
+        for (int c = part * per_part; c < min(columns, (part + 1) * per_part); ++c) {
+            const int off = c * kEpiColumn, left = row_bytes - off - lane * 32;
+            float acc[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+            int4 lo[kEpiRows], hi[kEpiRows];
+            for (int r0 = 0; r0 < n; r0 += kEpiRows) {
+#pragma unroll
+                for (int j = 0; j < kEpiRows; ++j) {
+                    const int slot = __shfl_sync(0xffffffffu, my_slot, (r0 + j) & 31);
+                    if (r0 + j < n) load_row32(token_rows + slot * lane_pitch + off, left, wide, lo[j], hi[j]);
                 }
-                staged_ok = __all_sync(0xffffffffu, ok);
-                if (!staged_ok) break;
-                parity ^= 1u << s;
 #pragma unroll
-                for (int h = 0; h < kEpiChunk / 512; ++h) {
-                    float acc[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-#pragma unroll
-                    for (int r = 0; r < kEpiRows; ++r) {
-                        const float wt = p.weighted ? __shfl_sync(0xffffffffu, my_wt, r) : 1.f;
-                        if (r < n) {
-                            const int4 raw = *reinterpret_cast<const int4*>(sbuf + (s * n + r) * kEpiChunk + h * 512 + lane * 16);
-                            if (p.weighted) accumulate_bf16x8_scaled(acc, raw, wt);
-                            else accumulate_bf16x8(acc, raw);
-                        }
+                for (int j = 0; j < kEpiRows; ++j) {
+                    if (r0 + j >= n) break;
+                    float (&first)[8] = *reinterpret_cast<float (*)[8]>(acc);
+                    float (&second)[8] = *reinterpret_cast<float (*)[8]>(acc + 8);
+                    if (p.weighted) {
+                        const float wt = __shfl_sync(0xffffffffu, my_wt, r0 + j);
+                        accumulate_bf16x8_scaled(first, lo[j], wt);
+                        accumulate_bf16x8_scaled(second, hi[j], wt);
+                    } else {
+                        accumulate_bf16x8(first, lo[j]);
+                        accumulate_bf16x8(second, hi[j]);
                     }
-                    const int off = cc * kEpiChunk + h * 512 + lane * 16;
-                    if (b0 != nullptr) accumulate_bf16x8(acc, ld_nc_int4(b0 + off));
-                    if (b1 != nullptr) accumulate_bf16x8(acc, ld_nc_int4(b1 + off));
-                    st_na_int4(dst + off, pack_bf16x8(acc));
                 }
             }
+            float (&first)[8] = *reinterpret_cast<float (*)[8]>(acc);
+            float (&second)[8] = *reinterpret_cast<float (*)[8]>(acc + 8);
+            for (const uint8_t* bias : {p.bias0, p.bias1}) {
+                if (bias == nullptr) continue;
+                int4 blo, bhi;
+                load_32(bias + out + off + lane * 32, left, wide, blo, bhi);
+                accumulate_bf16x8(first, blo);
+                accumulate_bf16x8(second, bhi);
+            }
+            uint8_t* dst = p.combined_x + out + off + lane * 32;
+            if (copy) store_32(dst, left, wide, lo[0], hi[0]);
+            else store_32(dst, left, wide, pack_bf16x8(first), pack_bf16x8(second));
         }
-        if (!staged_ok) reduce_token_registers(p, t, e, lane);     // redo this token the slow way; later tokens skip the staging
     }
     __syncthreads();
     if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned long long*>(timeline + 1), static_cast<unsigned long long>(globaltimer_ns()));
@@ -648,12 +547,11 @@ cudaError_t launch_combine_epilogue(const CombineEpilogueParams* params, int num
     m.blocks_per_rank = num_sms;
     for (int v = 0; v < num_vranks; ++v) m.r[v] = params[v];
     static PreparedKernel prepared;
-    cudaError_t err = prepared.prepare(combine_epilogue_kernel, kEpiSmem);
+    cudaError_t err = prepared.prepare(combine_epilogue_kernel, 0);
     if (err != cudaSuccess) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_vranks * num_sms);
     cfg.blockDim = dim3(kEpiWarps * 32);
-    cfg.dynamicSmemBytes = kEpiSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

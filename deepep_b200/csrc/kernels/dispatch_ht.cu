@@ -69,38 +69,34 @@ __host__ __device__ inline int order_scratch_min_bytes(int num_experts, int num_
 // `src`: a step covers channels [base, base + 1024), reads bytes [2*base, 2*base + 2048) and
 // writes bytes [base, base + 1024), which only earlier steps have read, and the lanes of a step
 // have all loaded (the shuffles of the reduction are past) before any of them stores.
-// `scales` must not overlap the row.
+// `scales` must not overlap the row. Eight lanes share a group of 128 channels, lane j takes its 16-byte pieces j and j + 8
+// (every second group the other way round, which keeps the eight-byte stores of neighbouring groups in different banks).
 __device__ __forceinline__ void quantize_row(const uint8_t* src, uint8_t* out, float* scales, int hidden, bool pow2, int lane) {
-    constexpr int kUnroll = 4;   // independent 256-channel steps in flight per lane (hides shuffle / divide latency)
-    for (int base = 0; base < hidden; base += 256 * kUnroll) {
-        int4 raw[kUnroll];
-        float amax[kUnroll];
+    constexpr int kUnroll = 2;   // independent 512-channel steps in flight per lane (hides shuffle / divide latency)
+    const int group = lane >> 3, first = (lane & 7) + 8 * (group & 1), second = first ^ 8;
+    for (int base = 0; base < hidden; base += 512 * kUnroll) {
+        int4 lo[kUnroll], hi[kUnroll];
+        float scale[kUnroll];
+        int4 q[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int ch = base + u * 256 + lane * 8;
-            raw[u] = ch < hidden ? *reinterpret_cast<const int4*>(src + ch * 2) : make_int4(0, 0, 0, 0);
-            amax[u] = amax_bf16x8(raw[u]);
+            const int g0 = base + u * 512 + group * 128;
+            lo[u] = hi[u] = make_int4(0, 0, 0, 0);
+            if (g0 < hidden) {
+                lo[u] = *reinterpret_cast<const int4*>(src + g0 * 2 + first * 16);
+                hi[u] = *reinterpret_cast<const int4*>(src + g0 * 2 + second * 16);
+            }
         }
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) amax[u] = fmaxf(amax[u], __shfl_xor_sync(0xffffffffu, amax[u], o));
-        }
+        for (int u = 0; u < kUnroll; ++u) q[u] = cast16_e4m3(lo[u], hi[u], pow2, scale[u]);
         __syncwarp();
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
-            const int ch = base + u * 256 + lane * 8;
-            float scale, inv;
-            fp8_scale_from_amax(amax[u], pow2, scale, inv);
-            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
-            const float2 a = __bfloat1622float2(h2[0]), b = __bfloat1622float2(h2[1]);
-            const float2 c = __bfloat1622float2(h2[2]), d = __bfloat1622float2(h2[3]);
-            uint2 packed;
-            packed.x = pack4_e4m3(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
-            packed.y = pack4_e4m3(c.x * inv, c.y * inv, d.x * inv, d.y * inv);
-            if (ch < hidden) {
-                *reinterpret_cast<uint2*>(out + ch) = packed;
-                if ((lane & 15) == 0) scales[ch >> 7] = scale;
+            const int g0 = base + u * 512 + group * 128;
+            if (g0 < hidden) {
+                *reinterpret_cast<int2*>(out + g0 + first * 8) = make_int2(q[u].x, q[u].y);
+                *reinterpret_cast<int2*>(out + g0 + second * 8) = make_int2(q[u].z, q[u].w);
+                if ((lane & 7) == 0) scales[g0 >> 7] = scale[u];
             }
         }
     }
@@ -215,9 +211,10 @@ __global__ void __launch_bounds__(1024, 1) dispatch_kernel(const __grid_constant
         // warps turns that into positions inside the block. Everything is in token order, so the
         // result does not depend on timing.
         const int scratch_bytes = p.smem_scratch_bytes;
-        int cw = num_warps;
+        // A lane works on one token: more counting warps than 32-token batches only lengthen the prefix over the warps.
+        int cw = min(num_warps, max(1, ceil_div(t1 - t0, 32)));
         const int per_warp = (2 * E + kMaxRanks) * 4;
-        // a lane works on one token: odd row pitches keep the lanes' words of a column in different banks
+        // odd row pitches keep the lanes' words of a column in different banks
         const int Kp = K | 1, Rp = R | 1;
         while (cw > 1 && (cw * per_warp > scratch_bytes / 2 || scratch_bytes - cw * per_warp < 32 * (Kp + Rp) * 4)) --cw;
         int* s_wcnt = reinterpret_cast<int*>(s_bufs);          // [cw][E]  per-warp expert counters, then bases
@@ -817,7 +814,7 @@ cudaError_t launch_dispatch_epilogue(const DispatchEpilogueParams* params, int n
     const bool move_rows = params[0].copy_x || params[0].do_expand;
     const int stage = align_up(params[0].x_row_bytes, 128) + 16;
     int warps = move_rows ? smem_optin / stage : 32;
-    if (warps > (move_rows ? 16 : 32)) warps = move_rows ? 16 : 32;
+    if (warps > 32) warps = 32;
     if (warps < 1) return cudaErrorInvalidValue;
     const int smem_bytes = move_rows ? warps * stage : 0;
     static PreparedKernel prepared;
