@@ -6,6 +6,7 @@
 #include <torch/extension.h>
 
 #include "runtime.hpp"
+#include "tensors.hpp"
 
 namespace py = pybind11;
 using namespace ep;
@@ -75,7 +76,7 @@ py::list dispatch_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const 
         DispatchResult& r = res[v];
         py::object count_matrix = py::none(), per_expert = py::none();
         if (r.count_matrix.defined()) count_matrix = py::cast(r.count_matrix);
-        if (!args[v].cached) per_expert = py::cast(r.psum_expert.narrow(0, 0, r.psum_expert.size(0) - 1));    // the last word is the number of expanded rows
+        if (!args[v].cached) per_expert = py::cast(first_rows(r.psum_expert, r.psum_expert.size(0) - 1));    // the last word is the number of expanded rows
         out.append(py::make_tuple(r.recv_x, r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert,
                                   per_expert, r.num_unaligned, r.recv_src_metadata, count_matrix, r.topk_idx, r.num_recv_tokens,
                                   r.num_expanded_tokens, r.num_sms, r.num_recv_tokens_per_expert_list, r.event, r.counts_pending));

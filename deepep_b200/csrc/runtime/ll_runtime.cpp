@@ -81,12 +81,14 @@ std::optional<EventHandle> ll_dispatch(const std::vector<std::shared_ptr<Runtime
         EP_HOST_ASSERT((io.topk_idx.scalar_type() == at::kLong || io.topk_idx.scalar_type() == at::kInt) && io.topk_idx.is_contiguous() && io.topk_idx.size(0) == io.x.size(0) && io.topk_idx.size(1) == K);
         if (!io.packed_recv_x.defined()) {
             io.packed_recv_x = new_tensor({EL, R * Tm, H}, use_fp8 ? at::kFloat8_e4m3fn : at::kBFloat16, device);
-            io.packed_recv_count = new_tensor({EL}, at::kInt, device);
-            io.src_info = new_tensor({EL, R * Tm}, at::kInt, device);
-            io.layout_range = new_tensor({EL, R}, at::kLong, device);
+            const int64_t rows = static_cast<int64_t>(R) * Tm;
+            TensorPack pack(TensorPack::room(EL, 4) + TensorPack::room(EL * rows, 4) + TensorPack::room(EL * R, 8), device);
+            io.packed_recv_count = pack.take({EL}, at::kInt);
+            io.src_info = pack.take({EL, rows}, at::kInt);
+            io.layout_range = pack.take({EL, R}, at::kLong);
             if (use_fp8) {
-                if (use_ue8m0) io.packed_recv_sf = new_tensor({EL, H / 512, R * Tm}, at::kInt, device).transpose(1, 2);
-                else io.packed_recv_sf = new_tensor({EL, H / 128, R * Tm}, at::kFloat, device).transpose(1, 2);
+                const int64_t packs = use_ue8m0 ? H / 512 : H / 128;
+                io.packed_recv_sf = new_strided({EL, rows, packs}, {packs * rows, 1, rows}, use_ue8m0 ? at::kInt : at::kFloat, device);
             }
         }
         LLDispatchParams& p = m.r[v];
@@ -262,9 +264,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, std::optional<EventHandle>> get_d
     if (previous_event.has_value()) previous_event->stream_wait(comm);
     else if (!stay) stream_wait(comm, compute);
     const int T = static_cast<int>(topk_idx.size(0)), K = static_cast<int>(topk_idx.size(1)), R = rt.num_ranks();
-    auto per_rank = new_tensor({R}, at::kInt, device);
-    auto per_expert = new_tensor({num_experts}, at::kInt, device);
-    auto in_rank = new_tensor({T, R}, at::kBool, device);
+    TensorPack pack(TensorPack::room(R, 4) + TensorPack::room(num_experts, 4) + TensorPack::room(static_cast<int64_t>(T) * R, 1), device);
+    auto per_rank = pack.take({R}, at::kInt), per_expert = pack.take({num_experts}, at::kInt), in_rank = pack.take({T, R}, at::kBool);
     CUDA_RUNTIME_CHECK(launch_dispatch_layout(topk_idx.data_ptr(), topk_idx.scalar_type() == at::kInt, T, K, R, num_experts, per_rank.data_ptr<int>(),
                                               per_expert.data_ptr<int>(), in_rank.data_ptr<bool>(), launch.stream()));
     std::optional<EventHandle> event;
@@ -288,10 +289,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, std::optional<at::Ten
     const int R = rt.num_ranks(), T = static_cast<int>(token_slot.size(0)), device = rt.heap().device();
     EP_HOST_ASSERT(count_matrix.is_contiguous() && count_matrix.numel() == R * R && token_slot.is_contiguous() && token_slot.size(1) == R);
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
-    auto prefix = new_tensor({R, R}, at::kInt, device), sent = new_tensor({R, 1}, at::kInt, device), received = new_tensor({R, 1}, at::kInt, device);
-    auto send_head = new_tensor({T, R}, at::kInt, device);
+    const int64_t slots = static_cast<int64_t>(T) * R;
+    TensorPack pack(TensorPack::room(R * R, 4) + 2 * TensorPack::room(R, 4) + TensorPack::room(slots, 4) + TensorPack::room(slots, 1), device);
+    auto prefix = pack.take({R, R}, at::kInt), sent = pack.take({R, 1}, at::kInt), received = pack.take({R, 1}, at::kInt), send_head = pack.take({T, R}, at::kInt);
     std::optional<at::Tensor> in_rank;
-    if (with_in_rank) in_rank = new_tensor({T, R}, at::kBool, device);
+    if (with_in_rank) in_rank = pack.take({T, R}, at::kBool);
     CUDA_RUNTIME_CHECK(launch_legacy_handle(count_matrix.data_ptr<int>(), token_slot.data_ptr<int>(), rt.rank(), R, T, prefix.data_ptr<int>(),
                                             sent.data_ptr<int>(), received.data_ptr<int>(), send_head.data_ptr<int>(),
                                             with_in_rank ? in_rank->data_ptr<bool>() : nullptr, at::cuda::getCurrentCUDAStream().stream()));

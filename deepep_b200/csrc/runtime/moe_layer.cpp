@@ -8,6 +8,7 @@
 
 #include "ops_runtime.hpp"
 #include "runtime.hpp"
+#include "tensors.hpp"
 
 namespace py = pybind11;
 
@@ -72,7 +73,7 @@ std::tuple<at::Tensor, std::shared_ptr<LayerCall>> layer_forward(const std::shar
     c->d = std::move(Runtime::dispatch({rt}, args)[0]);
     DispatchResult& d = c->d;
     const int el = static_cast<int>(d.num_unaligned.size(0));
-    c->ends = d.psum_expert.narrow(0, 0, el);
+    c->ends = first_rows(d.psum_expert, el);
 
     auto gemm = [&](const at::Tensor& rows, const OptTensor& sf, int w) {
         const OptTensor wsf = cfg.fp8 ? OptTensor(weights[w + 1]) : std::nullopt;
@@ -87,11 +88,11 @@ std::tuple<at::Tensor, std::shared_ptr<LayerCall>> layer_forward(const std::shar
         std::tie(d.num_recv_tokens, d.num_expanded_tokens, d.num_recv_tokens_per_expert_list) = rt->take_counts(el);
         d.counts_pending = false;
         const int64_t rows = d.num_expanded_tokens;
-        d.recv_x = d.recv_x.narrow(0, 0, rows);
-        if (d.recv_sf.has_value()) d.recv_sf = d.recv_sf->narrow(0, 0, rows);
-        d.recv_topk_weights = d.recv_topk_weights->narrow(0, 0, rows);
-        c->h1 = c->h1.narrow(0, 0, rows);
-        d.recv_src_metadata = d.recv_src_metadata.narrow(0, 0, d.num_recv_tokens);
+        d.recv_x = first_rows(d.recv_x, rows);
+        if (d.recv_sf.has_value()) d.recv_sf = first_rows(*d.recv_sf, rows);
+        d.recv_topk_weights = first_rows(*d.recv_topk_weights, rows);
+        c->h1 = first_rows(c->h1, rows);
+        d.recv_src_metadata = first_rows(d.recv_src_metadata, d.num_recv_tokens);
     }
     return {y, c};
 }

@@ -2,7 +2,6 @@
 // The reference library has no compute kernels; these exist for the fused MoE layer and the
 // tensor-parallel fused operators built on the same runtime.
 #include <ATen/cuda/CUDAContext.h>
-#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -17,17 +16,13 @@
 #include "../kernels/gemm_api.hpp"
 #include "../kernels/ops_api.hpp"
 #include "ops_runtime.hpp"
+#include "tensors.hpp"
 
 namespace py = pybind11;
 
 namespace ep {
 
 namespace {
-
-// A new tensor from the caching allocator, without the trip through the operator dispatcher (as long as the allocation).
-at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, int device) {
-    return at::detail::empty_cuda(sizes, dtype, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)), std::nullopt);
-}
 
 cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
@@ -218,7 +213,7 @@ at::Tensor router_backward(const at::Tensor& x, const at::Tensor& router_padded,
     at::Tensor dlogits = new_tensor({T, padded}, at::kBFloat16, x.get_device());
     CUDA_RUNTIME_CHECK(ops::router_backward(topk_idx.data_ptr<int64_t>(), w.data_ptr<float>(), dw.data_ptr<float>(), T, K, num_experts, padded,
                                             static_cast<int>(dx.size(1)), router_padded.data_ptr(), dx.data_ptr(), dlogits.data_ptr(), cur_stream()));
-    return gemm_mn(dlogits, x, true).narrow(0, 0, num_experts);
+    return first_rows(gemm_mn(dlogits, x, true), num_experts);
 }
 
 // bf16 [G, N, K] -> (e4m3 [G, N, K], fp32 scales [G, N / 128, K / 128])

@@ -310,12 +310,16 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
             r.num_unaligned = *a.h_num_unaligned;
             r.recv_src_metadata = *a.h_recv_src_metadata;
         } else {
-            r.token_slot = new_tensor({T, R}, at::kInt, device);
-            r.pair_row = new_tensor({T, K}, at::kInt, device);
-            r.psum_rank = new_tensor({R}, at::kInt, device);
-            r.psum_expert = new_tensor({EL + 1}, at::kInt, device);
-            r.num_unaligned = new_tensor({EL}, at::kInt, device);
-            r.count_matrix = new_tensor({R, R}, at::kInt, device);
+            const int64_t pairs = static_cast<int64_t>(T) * K, slots = static_cast<int64_t>(T) * R;
+            TensorPack pack(TensorPack::room(slots, 4) + TensorPack::room(pairs, 4) + TensorPack::room(R, 4) + TensorPack::room(EL + 1, 4) + TensorPack::room(EL, 4) +
+                            TensorPack::room(R * R, 4) + (a.copy_topk_idx ? TensorPack::room(pairs, static_cast<int64_t>(c10::elementSize(idx_dtype))) : 0), device);
+            r.token_slot = pack.take({T, R}, at::kInt);
+            r.pair_row = pack.take({T, K}, at::kInt);
+            r.psum_rank = pack.take({R}, at::kInt);
+            r.psum_expert = pack.take({EL + 1}, at::kInt);
+            r.num_unaligned = pack.take({EL}, at::kInt);
+            r.count_matrix = pack.take({R, R}, at::kInt);
+            if (a.copy_topk_idx) r.topk_idx = pack.take({T, K}, idx_dtype);
         }
         p.token_slot = r.token_slot.data_ptr<int>();
         p.pair_row = r.pair_row.data_ptr<int>();
@@ -394,7 +398,7 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
         if (has_sf) {
             const at::ScalarType sf_dtype = (!quant && a.sf->scalar_type() == at::kInt) ? at::kInt : at::kFloat;
             if (a.col_major_sf) {
-                r.recv_sf = at::empty_strided({rows, sf_packs}, {1, align_up(std::max(rows, 1), 4)}, opts(sf_dtype, device));
+                r.recv_sf = new_strided({rows, sf_packs}, {1, align_up(std::max(rows, 1), 4)}, sf_dtype, device);
             } else if (zero_copy) {
                 r.recv_sf = at::from_blob(region + x_row_bytes, {N, sf_packs}, {rec_pitch / 4, 1}, opts(sf_dtype, device));
                 sf_in_place = true;
@@ -442,11 +446,12 @@ std::vector<DispatchResult> Runtime::dispatch(const std::vector<std::shared_ptr<
         q.num_idx_rows = static_cast<int>(r.recv_src_metadata.size(0));
         q.mask_weights = a.mask_weights ? 1 : 0;
         if (a.copy_topk_idx) {
-            r.topk_idx = new_tensor({a.x.size(0), K}, idx_dtype, device);
+            if (!r.topk_idx.has_value()) r.topk_idx = new_tensor({a.x.size(0), K}, idx_dtype, device);
             q.topk_idx = a.topk_idx->data_ptr();
             q.topk_idx_copy = r.topk_idx->data_ptr();
             q.topk_idx_bytes = static_cast<int64_t>(a.topk_idx->nbytes());
         }
+        if (!a0.sc.async_with_compute_stream) continue;
         for (const at::Tensor& t : {r.recv_x, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert, r.num_unaligned, r.recv_src_metadata,
                                     a.x, *a.topk_idx})
             touched.push_back(t);
@@ -598,15 +603,14 @@ std::vector<CombineResult> Runtime::combine(const std::vector<std::shared_ptr<Ru
             EP_HOST_ASSERT(a.dst_slot->scalar_type() == at::kInt && a.dst_slot->is_contiguous() && a.dst_slot->dim() == 2 &&
                            a.dst_slot->size(0) == T && a.dst_slot->size(1) == R);
             EP_HOST_ASSERT(a.count_matrix->scalar_type() == at::kInt && a.count_matrix->is_contiguous() && a.count_matrix->numel() == R * R);
-            touched.push_back(*a.dst_slot);
-            touched.push_back(*a.count_matrix);
             q.arrivals = reinterpret_cast<const uint32_t*>(rt.heap_->base() + lay.combine_flag) +
                          static_cast<size_t>(p.epoch & 1) * R * lay.combine_flag_chunks;
             q.dst_slot = a.dst_slot->data_ptr<int>();
             q.count_matrix = a.count_matrix->data_ptr<int>();
         }
+        if (!a0.sc.async_with_compute_stream) continue;
         for (const at::Tensor& t : {r.combined_x, a.x, a.recv_src_metadata, a.topk_idx, a.psum_rank}) touched.push_back(t);
-        for (const auto& t : {r.combined_topk_weights, a.topk_weights, a.bias0, a.bias1})
+        for (const auto& t : {r.combined_topk_weights, a.topk_weights, a.bias0, a.bias1, a.dst_slot, a.count_matrix})
             if (t.has_value()) touched.push_back(*t);
     }
     CombineLaunch launch;

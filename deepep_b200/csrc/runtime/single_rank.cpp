@@ -1,6 +1,5 @@
 // Dispatch and combine drivers of a group of one rank (kernels/local_exchange.cu): the same arguments, checks and results
 // as the multi-rank drivers (runtime.cpp), without the heap.
-#include <ATen/ops/empty_strided.h>
 #include <ATen/ops/from_blob.h>
 
 #include "runtime.hpp"
@@ -70,12 +69,16 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
         r.num_unaligned = *a.h_num_unaligned;
         r.recv_src_metadata = *a.h_recv_src_metadata;
     } else {
-        r.token_slot = new_tensor({T, 1}, at::kInt, device);
-        r.pair_row = new_tensor({T, K}, at::kInt, device);
-        r.psum_rank = new_tensor({1}, at::kInt, device);
-        r.psum_expert = new_tensor({E + 1}, at::kInt, device);
-        r.num_unaligned = new_tensor({E}, at::kInt, device);
-        r.count_matrix = new_tensor({1, 1}, at::kInt, device);
+        const int64_t idx_size = static_cast<int64_t>(c10::elementSize(idx_dtype)), pairs = static_cast<int64_t>(T) * K;
+        TensorPack pack(2 * TensorPack::room(1, 4) + TensorPack::room(T, 4) + TensorPack::room(pairs, 4) + TensorPack::room(E + 1, 4) + TensorPack::room(E, 4) +
+                        (a.copy_topk_idx ? TensorPack::room(pairs, idx_size) : 0), device);
+        r.token_slot = pack.take({T, 1}, at::kInt);
+        r.pair_row = pack.take({T, K}, at::kInt);
+        r.psum_rank = pack.take({1}, at::kInt);
+        r.psum_expert = pack.take({E + 1}, at::kInt);
+        r.num_unaligned = pack.take({E}, at::kInt);
+        r.count_matrix = pack.take({1, 1}, at::kInt);
+        if (a.copy_topk_idx) r.topk_idx = pack.take({T, K}, idx_dtype);
         LocalPlanParams p = {};
         p.num_tokens = T;
         p.num_topk = K;
@@ -143,7 +146,7 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     if (has_sf) {
         const at::ScalarType sf_dtype = (!quant && a.sf->scalar_type() == at::kInt) ? at::kInt : at::kFloat;
         if (a.col_major_sf) {
-            r.recv_sf = at::empty_strided({rows_bound, sf_packs}, {1, align_up(std::max(rows_bound, 1), 4)}, opts(sf_dtype, device));
+            r.recv_sf = new_strided({rows_bound, sf_packs}, {1, align_up(std::max(rows_bound, 1), 4)}, sf_dtype, device);
         } else if (zero_copy) {
             r.recv_sf = at::from_blob(region + x_row_bytes, {rows_bound, sf_packs}, {rec_pitch / 4, 1}, opts(sf_dtype, device));
         } else {
@@ -157,7 +160,6 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
         r.recv_topk_weights = new_tensor({rows_bound}, at::kFloat, device);
     }
     if (!cached) r.recv_src_metadata = new_tensor({idx_bound, K + 2}, at::kInt, device);
-    if (a.copy_topk_idx && !cached) r.topk_idx = new_tensor({T, K}, idx_dtype, device);
 
     LocalMoveParams q = {};
     q.num_tokens = T;
@@ -208,9 +210,12 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     prof_split_[0] = profiling_ == 2;
 
     // the full-length tensors are what the streams have to know about; the views below share their memory
-    std::vector<at::Tensor> touched = {r.recv_x, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert, r.num_unaligned, r.recv_src_metadata, a.x, topk_idx};
-    for (const auto& t : {r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.topk_idx, a.sf, a.topk_weights, a.cumulative_stats})
-        if (t.has_value()) touched.push_back(*t);
+    std::vector<at::Tensor> touched;
+    if (a.sc.async_with_compute_stream) {
+        touched = {r.recv_x, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert, r.num_unaligned, r.recv_src_metadata, a.x, topk_idx};
+        for (const auto& t : {r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.topk_idx, a.sf, a.topk_weights, a.cumulative_stats})
+            if (t.has_value()) touched.push_back(*t);
+    }
     if (cut && a.defer_counts) {
         r.counts_pending = true;
         r.num_recv_tokens = idx_bound;
@@ -218,7 +223,7 @@ DispatchResult Runtime::dispatch_single(DispatchArgs& a) {
     } else if (cut) {
         read_counts();
         const int rows = a.do_expand ? r.num_expanded_tokens : r.num_recv_tokens;
-        auto shorten = [](at::Tensor& t, int n) { if (t.size(0) != n) t = t.narrow(0, 0, n); };
+        auto shorten = [](at::Tensor& t, int n) { t = first_rows(t, n); };
         shorten(r.recv_x, rows);
         if (r.recv_sf.has_value()) shorten(*r.recv_sf, rows);
         if (r.recv_topk_idx.has_value()) shorten(*r.recv_topk_idx, r.num_recv_tokens);
@@ -301,9 +306,12 @@ CombineResult Runtime::combine_single(CombineArgs& a) {
     prof_record(5, stream);
     prof_valid_[1] = profiling_ != 0;
     prof_split_[1] = profiling_ == 2;
-    std::vector<at::Tensor> touched = {r.combined_x, a.x, a.recv_src_metadata, a.topk_idx, a.psum_rank, *a.dst_slot};
-    for (const auto& t : {r.combined_topk_weights, a.topk_weights, a.bias0, a.bias1})
-        if (t.has_value()) touched.push_back(*t);
+    std::vector<at::Tensor> touched;
+    if (a.sc.async_with_compute_stream) {
+        touched = {r.combined_x, a.x, a.recv_src_metadata, a.topk_idx, a.psum_rank, *a.dst_slot};
+        for (const auto& t : {r.combined_topk_weights, a.topk_weights, a.bias0, a.bias1})
+            if (t.has_value()) touched.push_back(*t);
+    }
     r.event = scope.finish(a.sc, touched);
     return r;
 }

@@ -4,9 +4,8 @@
 
 #include <cstdlib>
 
-#include <ATen/cuda/EmptyTensor.h>
-
 #include "runtime.hpp"
+#include "tensors.hpp"
 
 namespace ep {
 
@@ -17,12 +16,6 @@ inline bool env_flag(const char* name) {
 
 inline at::TensorOptions opts(at::ScalarType dtype, int device) {
     return at::TensorOptions().dtype(dtype).device(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
-}
-
-// A new tensor from the caching allocator. (at::empty goes through the operator dispatcher, which costs as much as the
-// allocation: a dispatch makes ten small tensors, and at small sizes the host is what bounds it.)
-inline at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, int device) {
-    return at::detail::empty_cuda(sizes, dtype, at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device)), std::nullopt);
 }
 
 // Everything the stream-control arguments ask for before the first launch.
