@@ -259,8 +259,8 @@ class Buffer:
         args = (num_max_dispatch_tokens_per_rank, num_experts, use_fp8, round_scale, use_ue8m0)
         hook: Optional[Callable] = None
         if not return_recv_hook:
-            packed, sf, count, src_info, layout_range, event = _C.ll_dispatch_one(self.runtime, x, topk_idx, cumulative_local_expert_recv_stats,
-                                                                                  wait_stats, *args, num_sms, self.enable_shrink, async_finish)
+            packed, sf, count, src_info, layout_range, event = _C.ll_dispatch_one(self.runtime, (
+                x, topk_idx, cumulative_local_expert_recv_stats, wait_stats, *args, num_sms, self.enable_shrink, async_finish))
         else:
             io = _C.LLDispatchIO()
             io.x, io.topk_idx = x, topk_idx
@@ -293,8 +293,8 @@ class Buffer:
             wait_stats = wait_stats[self.rank]
         hook: Optional[Callable] = None
         if not return_recv_hook:
-            out, event = _C.ll_combine_one(self.runtime, x, topk_idx, topk_weights, src_info, layout_range, out, wait_stats,
-                                           num_max_dispatch_tokens_per_rank, num_experts, use_logfmt, num_sms, self.enable_shrink, async_finish)
+            out, event = _C.ll_combine_one(self.runtime, (x, topk_idx, topk_weights, src_info, layout_range, out, wait_stats,
+                                                          num_max_dispatch_tokens_per_rank, num_experts, use_logfmt, num_sms, self.enable_shrink, async_finish))
             return out, EventOverlap(event), hook
         io = _C.LLCombineIO()
         io.x, io.topk_idx, io.topk_weights = x, topk_idx, topk_weights

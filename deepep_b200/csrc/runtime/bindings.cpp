@@ -5,6 +5,7 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include "py_tuples.hpp"
 #include "runtime.hpp"
 #include "tensors.hpp"
 
@@ -13,57 +14,53 @@ using namespace ep;
 
 namespace {
 
-using OptTensor = std::optional<at::Tensor>;
-
-template <typename T>
-T item(const py::tuple& t, int i) { return t[i].cast<T>(); }
-
 // A call of one rank arrives as one tuple and its results leave as one tuple: filling an argument block and reading a
 // result block attribute by attribute from Python cost about 15 us per call, which bounded small calls. The orders are
 // those of ElasticBuffer._dispatch_call / _dispatch_result / _combine_call.
-DispatchArgs dispatch_args(const py::tuple& t) {
+DispatchArgs dispatch_args(PyObject* call) {
+    const TupleReader t(call, 24);
     DispatchArgs a;
-    a.x = item<at::Tensor>(t, 0);
-    a.sf = item<OptTensor>(t, 1);
-    a.topk_idx = item<OptTensor>(t, 2);
-    a.topk_weights = item<OptTensor>(t, 3);
-    a.cumulative_stats = item<OptTensor>(t, 4);
-    a.num_experts = item<int>(t, 5);
-    a.num_max_tokens = item<int>(t, 6);
-    a.expert_alignment = item<int>(t, 7);
-    a.num_sms = item<int>(t, 8);
-    a.quant_mode = item<int>(t, 9);
-    a.do_expand = item<bool>(t, 10);
-    a.do_zero_padding = item<bool>(t, 11);
-    a.do_cpu_sync = item<bool>(t, 12);
-    a.zero_copy = item<bool>(t, 13);
-    a.num_worst_tokens = item<int>(t, 14);
-    a.col_major_sf = item<bool>(t, 15);
-    a.copy_topk_idx = item<bool>(t, 16);
-    a.sc.previous_event = item<std::optional<EventHandle>>(t, 17);
-    a.sc.previous_event_before_epilogue = item<std::optional<EventHandle>>(t, 18);
-    a.sc.async_with_compute_stream = item<bool>(t, 19);
-    a.sc.allocate_on_comm_stream = item<bool>(t, 20);
-    a.mask_weights = item<bool>(t, 22);
-    a.defer_counts = item<bool>(t, 23);
-    if (!t[21].is_none()) {        // the routing of an earlier dispatch
-        const auto h = item<py::tuple>(t, 21);
+    a.x = t.tensor(0);
+    a.sf = t.maybe_tensor(1);
+    a.topk_idx = t.maybe_tensor(2);
+    a.topk_weights = t.maybe_tensor(3);
+    a.cumulative_stats = t.maybe_tensor(4);
+    a.num_experts = t.integer(5);
+    a.num_max_tokens = t.integer(6);
+    a.expert_alignment = t.integer(7);
+    a.num_sms = t.integer(8);
+    a.quant_mode = t.integer(9);
+    a.do_expand = t.flag(10);
+    a.do_zero_padding = t.flag(11);
+    a.do_cpu_sync = t.flag(12);
+    a.zero_copy = t.flag(13);
+    a.num_worst_tokens = t.integer(14);
+    a.col_major_sf = t.flag(15);
+    a.copy_topk_idx = t.flag(16);
+    a.sc.previous_event = t.event(17);
+    a.sc.previous_event_before_epilogue = t.event(18);
+    a.sc.async_with_compute_stream = t.flag(19);
+    a.sc.allocate_on_comm_stream = t.flag(20);
+    a.mask_weights = t.flag(22);
+    a.defer_counts = t.flag(23);
+    if (!t.none(21)) {        // the routing of an earlier dispatch
+        const TupleReader h(t.item(21), 8);
         a.cached = true;
-        a.h_token_slot = item<OptTensor>(h, 0);
-        a.h_pair_row = item<OptTensor>(h, 1);
-        a.h_psum_rank = item<OptTensor>(h, 2);
-        a.h_psum_expert = item<OptTensor>(h, 3);
-        a.h_num_unaligned = item<OptTensor>(h, 4);
-        a.h_recv_src_metadata = item<OptTensor>(h, 5);
-        a.h_num_recv_tokens = item<int>(h, 6);
-        a.h_num_expanded_tokens = item<int>(h, 7);
+        a.h_token_slot = h.maybe_tensor(0);
+        a.h_pair_row = h.maybe_tensor(1);
+        a.h_psum_rank = h.maybe_tensor(2);
+        a.h_psum_expert = h.maybe_tensor(3);
+        a.h_num_unaligned = h.maybe_tensor(4);
+        a.h_recv_src_metadata = h.maybe_tensor(5);
+        a.h_num_recv_tokens = h.integer(6);
+        a.h_num_expanded_tokens = h.integer(7);
     }
     return a;
 }
 
 py::list dispatch_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const py::list& calls) {
     std::vector<DispatchArgs> args;
-    for (const auto& c : calls) args.push_back(dispatch_args(c.cast<py::tuple>()));
+    for (const auto& c : calls) args.push_back(dispatch_args(c.ptr()));
     std::vector<DispatchResult> res;
     {
         // The drivers may block on the host for a long time (the wait for the received counts): they run without the GIL
@@ -74,12 +71,13 @@ py::list dispatch_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const 
     py::list out;
     for (size_t v = 0; v < res.size(); ++v) {
         DispatchResult& r = res[v];
-        py::object count_matrix = py::none(), per_expert = py::none();
-        if (r.count_matrix.defined()) count_matrix = py::cast(r.count_matrix);
-        if (!args[v].cached) per_expert = py::cast(first_rows(r.psum_expert, r.psum_expert.size(0) - 1));    // the last word is the number of expanded rows
-        out.append(py::make_tuple(r.recv_x, r.recv_sf, r.recv_topk_idx, r.recv_topk_weights, r.token_slot, r.pair_row, r.psum_rank, r.psum_expert,
-                                  per_expert, r.num_unaligned, r.recv_src_metadata, count_matrix, r.topk_idx, r.num_recv_tokens,
-                                  r.num_expanded_tokens, r.num_sms, r.num_recv_tokens_per_expert_list, r.event, r.counts_pending));
+        std::optional<at::Tensor> per_expert;
+        if (!args[v].cached) per_expert = first_rows(r.psum_expert, r.psum_expert.size(0) - 1);    // the last word is the number of expanded rows
+        TupleWriter t(19);
+        t.put(r.recv_x).put(r.recv_sf).put(r.recv_topk_idx).put(r.recv_topk_weights).put(r.token_slot).put(r.pair_row).put(r.psum_rank).put(r.psum_expert)
+            .put(per_expert).put(r.num_unaligned).put(r.recv_src_metadata).put(r.count_matrix).put(r.topk_idx).put(r.num_recv_tokens)
+            .put(r.num_expanded_tokens).put(r.num_sms).put(r.num_recv_tokens_per_expert_list).put(r.event).put(r.counts_pending);
+        out.append(t.take());
     }
     return out;
 }
@@ -87,28 +85,28 @@ py::list dispatch_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const 
 py::list combine_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const py::list& calls) {
     std::vector<CombineArgs> args;
     for (const auto& c : calls) {
-        const auto t = c.cast<py::tuple>();
+        const TupleReader t(c.ptr(), 20);
         CombineArgs a;
-        a.x = item<at::Tensor>(t, 0);
-        a.topk_weights = item<OptTensor>(t, 1);
-        a.bias0 = item<OptTensor>(t, 2);
-        a.bias1 = item<OptTensor>(t, 3);
-        a.recv_src_metadata = item<at::Tensor>(t, 4);
-        a.topk_idx = item<at::Tensor>(t, 5);
-        a.psum_rank = item<at::Tensor>(t, 6);
-        a.dst_slot = item<OptTensor>(t, 7);
-        a.count_matrix = item<OptTensor>(t, 8);
-        a.num_experts = item<int>(t, 9);
-        a.num_max_tokens = item<int>(t, 10);
-        a.num_sms = item<int>(t, 11);
-        a.do_expand = item<bool>(t, 12);
-        a.weighted = item<bool>(t, 13);
-        a.allow_multiple_reduction = item<bool>(t, 14);
-        a.fuse_reduce = item<int>(t, 15);
-        a.sc.previous_event = item<std::optional<EventHandle>>(t, 16);
-        a.sc.previous_event_before_epilogue = item<std::optional<EventHandle>>(t, 17);
-        a.sc.async_with_compute_stream = item<bool>(t, 18);
-        a.sc.allocate_on_comm_stream = item<bool>(t, 19);
+        a.x = t.tensor(0);
+        a.topk_weights = t.maybe_tensor(1);
+        a.bias0 = t.maybe_tensor(2);
+        a.bias1 = t.maybe_tensor(3);
+        a.recv_src_metadata = t.tensor(4);
+        a.topk_idx = t.tensor(5);
+        a.psum_rank = t.tensor(6);
+        a.dst_slot = t.maybe_tensor(7);
+        a.count_matrix = t.maybe_tensor(8);
+        a.num_experts = t.integer(9);
+        a.num_max_tokens = t.integer(10);
+        a.num_sms = t.integer(11);
+        a.do_expand = t.flag(12);
+        a.weighted = t.flag(13);
+        a.allow_multiple_reduction = t.flag(14);
+        a.fuse_reduce = t.integer(15);
+        a.sc.previous_event = t.event(16);
+        a.sc.previous_event_before_epilogue = t.event(17);
+        a.sc.async_with_compute_stream = t.flag(18);
+        a.sc.allocate_on_comm_stream = t.flag(19);
         args.push_back(std::move(a));
     }
     std::vector<CombineResult> res;
@@ -117,7 +115,11 @@ py::list combine_calls(const std::vector<std::shared_ptr<Runtime>>& rts, const p
         res = Runtime::combine(rts, args);
     }
     py::list out;
-    for (auto& r : res) out.append(py::make_tuple(r.combined_x, r.combined_topk_weights, r.event));
+    for (auto& r : res) {
+        TupleWriter t(3);
+        t.put(r.combined_x).put(r.combined_topk_weights).put(r.event);
+        out.append(t.take());
+    }
     return out;
 }
 

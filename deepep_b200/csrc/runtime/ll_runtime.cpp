@@ -8,6 +8,7 @@
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
+#include "py_tuples.hpp"
 #include "runtime.hpp"
 #include "stream_scope.hpp"
 
@@ -194,35 +195,36 @@ std::optional<EventHandle> ll_combine(const std::vector<std::shared_ptr<Runtime>
 }
 
 // The calls of one process (one rank) without an IO object on the Python side: one trip into native code.
-py::tuple ll_dispatch_one(const std::shared_ptr<Runtime>& rt, const at::Tensor& x, const at::Tensor& topk_idx, std::optional<at::Tensor> cumulative_stats,
-                          std::optional<at::Tensor> wait_stats, int num_max_tokens, int num_experts, bool use_fp8, bool round_scale, bool use_ue8m0,
-                          int num_sms, bool shrink, bool async_finish) {
+py::tuple ll_dispatch_one(const std::shared_ptr<Runtime>& rt, py::tuple call) {
+    const TupleReader t(call.ptr(), 12);
     LLDispatchIO io;
-    io.x = x;
-    io.topk_idx = topk_idx;
-    io.cumulative_stats = std::move(cumulative_stats);
-    io.wait_stats = std::move(wait_stats);
+    io.x = t.tensor(0);
+    io.topk_idx = t.tensor(1);
+    io.cumulative_stats = t.maybe_tensor(2);
+    io.wait_stats = t.maybe_tensor(3);
     std::vector<LLDispatchIO*> ios = {&io};
-    auto event = ll_dispatch({rt}, ios, num_max_tokens, num_experts, use_fp8, round_scale, use_ue8m0, kLLSend | kLLRecv, num_sms, shrink, async_finish, false);
-    return py::make_tuple(std::move(io.packed_recv_x), std::move(io.packed_recv_sf), std::move(io.packed_recv_count), std::move(io.src_info),
-                          std::move(io.layout_range), std::move(event));
+    const auto event = ll_dispatch({rt}, ios, t.integer(4), t.integer(5), t.flag(6), t.flag(7), t.flag(8), kLLSend | kLLRecv, t.integer(9), t.flag(10), t.flag(11), false);
+    TupleWriter out(6);
+    out.put(io.packed_recv_x).put(io.packed_recv_sf).put(io.packed_recv_count).put(io.src_info).put(io.layout_range).put(event);
+    return out.take();
 }
 
-py::tuple ll_combine_one(const std::shared_ptr<Runtime>& rt, const at::Tensor& x, const at::Tensor& topk_idx, const at::Tensor& topk_weights,
-                         const at::Tensor& src_info, const at::Tensor& layout_range, std::optional<at::Tensor> out, std::optional<at::Tensor> wait_stats,
-                         int num_max_tokens, int num_experts, bool use_logfmt, int num_sms, bool shrink, bool async_finish) {
+py::tuple ll_combine_one(const std::shared_ptr<Runtime>& rt, py::tuple call) {
+    const TupleReader t(call.ptr(), 13);
     LLCombineIO io;
-    io.x = x;
-    io.topk_idx = topk_idx;
-    io.topk_weights = topk_weights;
-    io.src_info = src_info;
-    io.layout_range = layout_range;
-    io.use_logfmt = use_logfmt;
-    if (out.has_value()) io.combined_x = std::move(*out);
-    io.wait_stats = std::move(wait_stats);
+    io.x = t.tensor(0);
+    io.topk_idx = t.tensor(1);
+    io.topk_weights = t.tensor(2);
+    io.src_info = t.tensor(3);
+    io.layout_range = t.tensor(4);
+    if (!t.none(5)) io.combined_x = t.tensor(5);
+    io.wait_stats = t.maybe_tensor(6);
+    io.use_logfmt = t.flag(9);
     std::vector<LLCombineIO*> ios = {&io};
-    auto event = ll_combine({rt}, ios, num_max_tokens, num_experts, kLLSend | kLLRecv, num_sms, shrink, async_finish, false);
-    return py::make_tuple(std::move(io.combined_x), std::move(event));
+    const auto event = ll_combine({rt}, ios, t.integer(7), t.integer(8), kLLSend | kLLRecv, t.integer(10), t.flag(11), t.flag(12), false);
+    TupleWriter out(2);
+    out.put(io.combined_x).put(event);
+    return out.take();
 }
 
 // bf16 [EL, R * T_max, H] view of the staging half that the NEXT combine send may read from
