@@ -30,33 +30,40 @@ __global__ void __launch_bounds__(kLLLocalThreads) ll_local_dispatch_kernel(cons
     const int bid = blockIdx.x, nb = gridDim.x;
     dependency_wait();
     launch_dependents();
-    const bool masked = *reinterpret_cast<volatile int*>(ll_mask_words(p.c.local_ws)) != 0;     // this rank has masked itself
+    const int row_bytes = H * 2, slices = ceil_div(row_bytes, 1024);
+    // The chain of dependent loads is what these few microseconds are made of: the mask word, the routing and the first
+    // slices of the block's first row are requested together.
+    const int mask_word = *reinterpret_cast<volatile int*>(ll_mask_words(p.c.local_ws));
+    int4 lo = make_int4(0, 0, 0, 0), hi = lo;
+    auto load = [&](int t, int s) {
+        const int off = s * 1024 + lane * 32;
+        lo = hi = make_int4(0, 0, 0, 0);
+        if (t < T && off < row_bytes) {                             // rows are multiples of 256 bytes: 32 bytes are in or out
+            const uint8_t* src = p.x + static_cast<int64_t>(t) * row_bytes + off;
+            lo = *reinterpret_cast<const int4*>(src);
+            hi = *reinterpret_cast<const int4*>(src + 16);
+        }
+    };
+    load(bid, warp);
     for (int e = tid; e < E; e += kLLLocalThreads) s_hist[e] = 0;
-    for (int i = tid; i < T * K; i += kLLLocalThreads) s_idx[i] = masked ? -1 : load_topk_idx(p.topk_idx, p.idx32 != 0, i, E);
+    for (int i = tid; i < T * K; i += kLLLocalThreads) {
+        const int e = load_topk_idx(p.topk_idx, p.idx32 != 0, i, E);
+        s_idx[i] = mask_word != 0 ? -1 : e;                         // this rank has masked itself
+    }
     __syncthreads();
     for (int i = tid; i < T * K; i += kLLLocalThreads)
         if (s_idx[i] >= 0) atomicAdd(s_hist + s_idx[i], 1);
-    const int row_bytes = H * 2, slices = ceil_div(row_bytes, 1024);
     const int sf_per_row = p.use_fp8 ? (p.use_ue8m0 ? H / 512 : H / 128) : 0;
     const int64_t out_row_bytes = p.use_fp8 ? H : row_bytes;
     for (int t = bid; t < T; t += nb) {
-        // the first slice of every warp is requested before the positions are known
-        const uint8_t* src = p.x + static_cast<int64_t>(t) * row_bytes;
-        int4 lo = make_int4(0, 0, 0, 0), hi = lo;
-        auto load = [&](int s) {
-            const int off = s * 1024 + lane * 32;
-            lo = hi = make_int4(0, 0, 0, 0);
-            if (off < row_bytes) {                                  // rows are multiples of 256 bytes: 32 bytes are in or out
-                lo = *reinterpret_cast<const int4*>(src + off);
-                hi = *reinterpret_cast<const int4*>(src + off + 16);
-            }
-        };
-        if (warp < slices) load(warp);
+        if (t != bid) load(t, warp);        // (the first slice of every warp: before the positions are known)
         if (warp < K) {
             const int e = s_idx[t * K + warp];
             int before = 0;
-            if (e >= 0)
+            if (e >= 0) {
+#pragma unroll 8
                 for (int i = lane; i < t * K; i += 32) before += s_idx[i] == e;
+            }
             before = warp_reduce_sum(before);
             if (lane == 0) {
                 s_exp[warp] = e;
@@ -66,7 +73,7 @@ __global__ void __launch_bounds__(kLLLocalThreads) ll_local_dispatch_kernel(cons
         }
         __syncthreads();
         for (int s = warp; s < slices; s += kLLLocalWarps) {
-            if (s != warp) load(s);
+            if (s != warp) load(t, s);
             const int off = s * 1024 + lane * 32;
             if (!p.use_fp8) {
                 if (off < row_bytes)
@@ -122,23 +129,28 @@ __global__ void __launch_bounds__(kLLCombineThreads) ll_local_combine_kernel(con
     const int tid = threadIdx.x, lane = lane_id(), warp = warp_id();
     dependency_wait();
     launch_dependents();
-    const bool masked = *reinterpret_cast<volatile int*>(ll_mask_words(p.c.local_ws)) != 0;
+    const int mask_word = *reinterpret_cast<volatile int*>(ll_mask_words(p.c.local_ws));
     const int parts = ceil_div(H, kLLCombineCols);
     for (int item = blockIdx.x; item < T * parts; item += gridDim.x) {
         const int t = item / parts, ch = (item % parts) * kLLCombineCols + tid * 8;
         for (int k = warp; k < K; k += kLLCombineThreads / 32) {
-            const int e = masked ? -1 : load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + k, E);
+            const int e = load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + k, E);
+            const float weight = p.topk_weights[static_cast<int64_t>(t) * K + k];
             int row = -1;
-            if (e >= 0) {
+            if (e >= 0 && mask_word == 0) {
+                // the first rows are looked at before it is known how many there are (one step less in the chain of loads)
+                const int* info = p.src_info + static_cast<int64_t>(e) * Tm;
+                const int first = lane < Tm ? info[lane] : -1;
                 const int n = min(static_cast<int>(p.layout_range[e] & 0xffffffff), Tm);
                 const int want = t | (k << 16);
-                for (int j = lane; j < n; j += 32)
-                    if (p.src_info[static_cast<int64_t>(e) * Tm + j] == want) row = j;
+                if (lane < n && first == want) row = lane;
+                for (int j = lane + 32; j < n; j += 32)
+                    if (info[j] == want) row = j;
             }
             row = __reduce_max_sync(0xffffffffu, row);
             if (lane == 0) {
                 s_row[k] = row < 0 ? -1 : e * Tm + row;
-                s_w[k] = p.topk_weights[static_cast<int64_t>(t) * K + k];
+                s_w[k] = weight;
             }
         }
         __syncthreads();
