@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
         for (int i = 0; i < kPlanRegTopk; ++i)
             e_reg[i] = (i < K && lane + 32 * i < pairs) ? load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(a) * K + lane + 32 * i, E) : -1;
     }
-    for (int i = tid; i < kPlanWarps * (E + 1) + kPlanWarps * E; i += kPlanThreads) s_cnt[i] = 0;     // counters and masks
+    for (int i = tid; i < kPlanWarps * (2 * E + 1) / 4; i += kPlanThreads) reinterpret_cast<int4*>(s_cnt)[i] = make_int4(0, 0, 0, 0);     // counters and masks
     __syncthreads();
 
     int* mine = s_cnt + warp * (E + 1);
@@ -87,10 +87,13 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     int tokens_before = 0;
     if (in_regs) {
         uint32_t taken = 0;         // tokens of the warp with a valid expert
+        // token of pair i: i / K for i < 256, as a product (sixteen divisions a lane were a fifth of this kernel's issue slots)
+        const uint32_t inv_k = 65536u / static_cast<uint32_t>(K) + 1u;
+        auto token_of = [&](int i) { return (static_cast<uint32_t>(i) * inv_k) >> 16; };
 #pragma unroll
         for (int i = 0; i < kPlanRegTopk; ++i)
             if (e_reg[i] >= 0) {
-                const uint32_t bit = 1u << ((lane + 32 * i) / K);
+                const uint32_t bit = 1u << token_of(lane + 32 * i);
                 atomicOr(mask_of + e_reg[i], bit);
                 taken |= bit;
             }
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
             pos_reg[i] = 0;
             if (e_reg[i] >= 0) {
                 const uint32_t m = mask_of[e_reg[i]];
-                pos_reg[i] = __popc(m & ((1u << ((lane + 32 * i) / K)) - 1u));
+                pos_reg[i] = __popc(m & ((1u << token_of(lane + 32 * i)) - 1u));
                 if (pos_reg[i] == 0) mine[e_reg[i]] = __popc(m);      // the first token of a mask writes the count
             }
         }
@@ -202,8 +205,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     __syncthreads();
     if (tid < E) {
         int start = incl - aligned;
-#pragma unroll
-        for (int w = 0; w < kMaxLocalExperts / 32; ++w) start += w < warp ? s_warp_sum[w] : 0;
+        for (int w = 0; w < warp; ++w) start += s_warp_sum[w];
         s_base[tid] = start + before;
         if (cta == 0) {
             if (p.host_counts != nullptr) {
