@@ -25,7 +25,6 @@ struct GemmParams {
     // MN-major operands (bf16): A is given as [K, M], B as [num_groups * K, N] (k_grouped: [K, N]), both row-major. A may only
     // be MN-major together with B. A plain problem with both may have any K.
     int a_mn, b_mn;
-    int b_ahead;                 // k-blocks of its first tile's weights that a CTA asks into L2 before its turn (filled in by the launcher)
     int c_wide;                  // rows of C start on 32-byte boundaries (filled in by the launcher)
     __nv_bfloat16* C;
     int64_t ldc;                 // elements between rows of C

@@ -86,20 +86,6 @@ struct Scheduler {
     }
 };
 
-// A decode batch is bound by the weights it streams, and HBM idles while the kernels ahead of its first GEMM sort out a few
-// rows. Where about every group has one row tile, CTA i begins with the i-th block of weight rows: it asks for them before it
-// waits for the kernel ahead (into L2 only, so a wrong guess, or weights that are still being written, cost nothing but the
-// traffic). 12 k-blocks of 148 CTAs are 57 MB, what HBM delivers meanwhile (64 tokens through 32 experts, 4096 x 7168 and
-// 7168 x 2048 e4m3, the whole layer: 268.4 us without, 267.6 / 265.1 / 264.7 / 266.9 with 4 / 12 / 16 / 24). Staying ahead like
-// this during the main loop was much slower (365 us).
-constexpr int kBlocksAhead = 12;
-__device__ __forceinline__ void weights_ahead(const GemmParams& p, const CUtensorMap* map_b, int bn, int bk) {
-    if (p.b_ahead == 0 || lane_id() != 0) return;
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * bn;
-    if (row >= static_cast<int64_t>(p.num_groups) * p.N) return;
-    for (int kb = 0; kb < p.b_ahead; ++kb) tma_prefetch_2d(map_b, kb * bk, static_cast<int>(row));
-}
-
 template <int BN, bool kFp8>
 struct Cfg {
     static constexpr int kEpiWarps = kFp8 ? 16 : 4;     // FP8: 4 lane quarters x 4 column quarters, so that many passes overlap
@@ -198,7 +184,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         tmem_alloc(tmem_slot, C::kTmemCols);
         tmem_relinquish();
     }
-    if (warp == 0) weights_ahead(p, &map_b, BN, C::BK);
     dependency_wait();           // everything above may run while the kernel ahead of this one drains
     const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
@@ -871,7 +856,6 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         tmem_alloc(tmem_slot, C::kTmemCols);
         tmem_relinquish();
     }
-    if (warp == 0) weights_ahead(p, &map_b, C::BN, C::BK);
     dependency_wait();           // everything above may run while the kernel ahead of this one drains
     const PipeCtx pc{p.error, globaltimer_ns() + p.timeout_ns};
     tc_fence_before();
@@ -1397,8 +1381,6 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
     if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM) ||
         !map_of(&map_a32, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, kSmallBox))
         return cudaErrorInvalidValue;
-    if (p.group_end != nullptr && !p.k_grouped && !p.b_mn && p.M <= p.num_groups * 2 * BM)
-        p.b_ahead = std::min(p.K / bk, kBlocksAhead);
     auto map_b_of = [&](uint32_t box) { return map_of(&map_b, b, p.b_mn != 0, static_cast<uint64_t>(p.N), b_mats, b_stride, box); };
     const bool wide = p.N % 256 == 0, pairs = wide && num_sms >= 2;
     const int pair_grid = num_sms & ~1;
