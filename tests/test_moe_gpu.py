@@ -76,7 +76,7 @@ def test_moe_module_single_rank_trains():
     buf.destroy()
 
 
-@pytest.mark.parametrize('T,H,I,E,K,use_fp8', [(1, 256, 128, 4, 1, False), (77, 640, 128, 8, 3, False), (300, 1024, 256, 16, 8, False),
+@pytest.mark.parametrize('T,H,I,E,K,use_fp8', [(1, 256, 128, 4, 1, False), (77, 640, 128, 8, 3, False), (300, 1024, 256, 16, 8, False), (40, 256, 128, 120, 4, False),
                                                (129, 512, 256, 8, 4, True)])
 def test_moe_module_gradients(T, H, I, E, K, use_fp8):
     """All gradients of the layer (router's share of dx and the router weights included) against fp32 autograd over the
