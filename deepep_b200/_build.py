@@ -1,6 +1,6 @@
 """In-tree build of the native extension ``deepep_b200._C`` for sm_100a.
 
-``python -m deepep_b200._build`` compiles every ``csrc/kernels/*.cu`` with nvcc
+``python deepep_b200/_build.py`` (by its path: importing the package needs what this builds) compiles every ``csrc/kernels/*.cu`` with nvcc
 (``-gencode arch=compute_100a,code=sm_100a``), every ``csrc/runtime/*.cpp`` with g++ against
 the PyTorch headers, and links them into ``deepep_b200/_C.<abi>.so`` next to this file.
 Objects are cached under ``build/`` keyed by a hash of the source, the headers and the flags,

@@ -9,8 +9,8 @@ Build-time switches (read from the environment, like the reference's setup.py:70
 
 Parity: setup.py:92-218 of the reference (CUDAExtension + persistent environment variables baked at build time).
 """
+import importlib.util
 import os
-import sys
 from pathlib import Path
 
 from setuptools import Extension, find_packages, setup
@@ -25,9 +25,11 @@ class BuildNative(build_ext):
     """Runs the in-tree builder and copies the shared object to where setuptools expects it."""
 
     def run(self):
-        sys.path.insert(0, str(ROOT))
-        from deepep_b200 import _build
-        target = _build.build()
+        # by its path: importing the package needs the extension that is built here
+        spec = importlib.util.spec_from_file_location('_deepep_b200_builder', ROOT / 'deepep_b200' / '_build.py')
+        builder = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(builder)
+        target = builder.build()
         for ext in self.extensions:
             dest = Path(self.get_ext_fullpath(ext.name))
             dest.parent.mkdir(parents=True, exist_ok=True)
