@@ -19,6 +19,8 @@ inline bool programmatic_launches() {
 // memory and descriptors can go before), and launch_dependents() so that its own successor can do the same. The gap between
 // dependent kernels of 2 to 3 us and the set-up of a GEMM (2 us) go away; a layer has six to twenty of them.
 // (A kernel whose successor reads inputs before its own wait has to wait first and announce afterwards.)
+// Every kernel launched like this calls dependency_wait() in every block before it ends, also where it needs nothing of the
+// kernel ahead: the wait of the kernel behind it covers this one only, and through it what this one has waited for.
 template <typename... Params, typename... Args>
 cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream, const Args&... args) {
     cudaLaunchConfig_t cfg = {};

@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(kEpiWarps * 32, 1) combine_epilogue_kernel(con
     const int columns = ceil_div(row_bytes, kEpiColumn);
     uint64_t* timeline = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(p.local_ws) + kWsTimelineOffsetBytes) + 2 * kTlCombineReduce;
     if (bid == 0 && threadIdx.x == 0) timeline[0] = globaltimer_ns();
-    // Flag-driven mode: this kernel runs beside the send kernel (it never waits for it as a whole); the tokens of
-    // a warp are visited in ascending order, which is also the order in which their rows arrive.
+    // Flag-driven mode: this kernel runs beside the send kernel (it waits for it as a whole only when its own work is done);
+    // the tokens of a warp are visited in ascending order, which is also the order in which their rows arrive.
     const bool flagged = p.arrivals != nullptr;
     const WaitCtx w = make_wait_ctx(p.c);
     bool flags_ok = true;
@@ -209,6 +209,10 @@ __global__ void __launch_bounds__(kEpiWarps * 32, 1) combine_epilogue_kernel(con
             else store_32(dst, left, wide, pack_bf16x8(first), pack_bf16x8(second));
         }
     }
+    // Beside the send kernel: this rank's rows are in, but the send kernel may still be reading the caller's rows for a slower
+    // peer. Whatever follows in the stream waits for this kernel and, launched early itself, for nothing else: it has to be
+    // able to rely on both being over (the caller's rows may be freed and written again by then).
+    if (flagged) dependency_wait();
     __syncthreads();
     if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned long long*>(timeline + 1), static_cast<unsigned long long>(globaltimer_ns()));
 }

@@ -353,3 +353,21 @@ def test_barrier_and_repeat():
     for _ in range(5):
         cl.barrier(with_cpu_sync=True)
     cl.destroy()
+
+
+def test_reduce_beside_the_send_kernel_ends_after_it():
+    """Kernels launched early behind a combine wait for the reduce kernel only. It runs beside the send kernel and has its
+    rows before that kernel is done with the caller's, so it may not end first."""
+    R, T, H, E, K = 4, 256, 1024, 32, 4
+    cl = _cluster(R, T, H, K, fuse_reduce=1)
+    xs, idxs, ws = make_routed_inputs(R, T, H, E, K, seed=8, device='cuda')
+    out = cl.dispatch([dict(x=xs[r], topk_idx=idxs[r], topk_weights=ws[r], num_experts=E, num_sms=4) for r in range(R)])
+    for _ in range(5):
+        cl.combine([dict(x=out[r][0], handle=out[r][3]) for r in range(R)])
+        torch.cuda.synchronize()
+        cl.check_status()
+        for r in range(R):
+            _, _, _, _, send_start, send_end, reduce_start, reduce_end = cl.runtimes[r].last_timeline()[:8]
+            assert send_start < reduce_start < send_end, 'the reduce kernel did not run beside the send kernel'
+            assert reduce_end >= send_end
+    cl.destroy()
