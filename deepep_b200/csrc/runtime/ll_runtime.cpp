@@ -41,12 +41,14 @@ int64_t ll_buffer_size(int num_ranks, int num_max_tokens, int hidden, int num_ex
 // only go over the communication stream and back).
 struct LLStreams {
     at::cuda::CUDAStream compute, launch;
+    Runtime& runtime;
     LLStreams(Runtime& rt, bool async_finish, bool use_compute)
-        : compute(at::cuda::getCurrentCUDAStream()), launch(async_finish && !use_compute ? rt.comm_stream() : compute) {
+        : compute(at::cuda::getCurrentCUDAStream()), launch(async_finish && !use_compute ? rt.comm_stream() : compute), runtime(rt) {
         if (launch != compute) stream_wait(launch, compute);
-        rt.order_behind_last_call(launch);
+        rt.order_behind_last_call(launch, compute);
     }
     std::optional<EventHandle> finish(bool async_finish) {
+        runtime.call_ended(launch, std::nullopt);
         if (async_finish) return EventHandle(launch);
         return std::nullopt;
     }

@@ -111,17 +111,53 @@ std::vector<int64_t> Runtime::last_timeline() {
     return out;
 }
 
-// A call's kernels share the workspace and the regions of the calls before it. Calls on one stream are ordered by it;
-// when the stream changes, the new one waits for the old one. Inside a graph capture only streams of the capture can be
-// waited for (and work from before the capture is the caller's to order, as ever).
-void Runtime::order_behind_last_call(const at::cuda::CUDAStream& stream) {
-    if (last_stream_.has_value() && *last_stream_ != stream) {
-        cudaStreamCaptureStatus now = cudaStreamCaptureStatusNone, before = cudaStreamCaptureStatusNone;
-        CUDA_RUNTIME_CHECK(cudaStreamIsCapturing(stream.stream(), &now));
-        CUDA_RUNTIME_CHECK(cudaStreamIsCapturing(last_stream_->stream(), &before));
-        if (now == before) stream_wait(stream, *last_stream_);
+// A call's kernels share the workspace and the regions with the calls before it. Calls on one stream are ordered by it; when
+// the stream changes, the new one waits for the last call: for the event at its end, or, the first time, for all that its
+// stream holds (recording an event behind every call costs host time and keeps the next kernel from starting early, which
+// programs that stay on one stream need not pay). A caller's own stream may be gone by the next call: it is never looked at
+// again, the event stands for it. Inside a graph capture only streams of that capture can be waited for: work from before the
+// capture is the caller's to order, and calls of the capture leave the order of the others as it is.
+static bool is_callers_own(const at::cuda::CUDAStream& s) { return s.stream() != nullptr && s.id() == reinterpret_cast<int64_t>(s.stream()); }
+
+static unsigned long long capture_of(const at::cuda::CUDAStream& s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    CUDA_RUNTIME_CHECK(cudaStreamGetCaptureInfo(s.stream(), &status, &id));
+    return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
+void Runtime::order_behind_last_call(const at::cuda::CUDAStream& stream, const at::cuda::CUDAStream& behind) {
+    const unsigned long long capture = capture_of(stream);
+    in_capture_ = capture != 0;
+    if (in_capture_) {
+        if (capture == capture_id_ && *capture_stream_ != stream && *capture_stream_ != behind) stream_wait(stream, *capture_stream_);
+        capture_id_ = capture;
+        capture_stream_ = stream;
+        return;
     }
-    last_stream_ = stream;
+    auto is = [&](const std::optional<at::cuda::CUDAStream>& s) { return s.has_value() && (*s == stream || *s == behind); };
+    if ((last_.stream.has_value() || last_.has_event) && !is(last_.stream) && !is(last_.joined)) {
+        streams_change_ = true;
+        if (last_.has_event) {
+            last_.event.block(stream);
+        } else {
+            EP_HOST_ASSERT_MSG(capture_of(*last_.stream) == 0, "the stream of the previous call is being captured: this call cannot be ordered behind that one");
+            stream_wait(stream, *last_.stream);
+        }
+    }
+    last_.has_event = false;
+    last_.joined.reset();
+    last_.stream.reset();
+    if (!is_callers_own(stream)) last_.stream = stream;
+}
+
+void Runtime::call_ended(const at::cuda::CUDAStream& stream, const std::optional<at::cuda::CUDAStream>& joined) {
+    if (in_capture_) return;
+    if (streams_change_ || is_callers_own(stream)) {
+        last_.event.record(stream);
+        last_.has_event = true;
+    }
+    if (joined.has_value() && !is_callers_own(*joined) && last_.stream.has_value()) last_.joined = joined;
 }
 
 void Runtime::connect_local(const std::vector<std::shared_ptr<Runtime>>& runtimes) {
@@ -176,7 +212,7 @@ void Runtime::barrier(const std::vector<std::shared_ptr<Runtime>>& rts, bool use
     const auto compute = at::cuda::getCurrentCUDAStream();
     const auto stream = use_comm_stream ? rt0.comm_stream_ : compute;
     if (use_comm_stream) stream_wait(stream, compute);
-    rt0.order_behind_last_call(stream);
+    rt0.order_behind_last_call(stream, compute);
     Multi<BarrierParams> m;
     m.num_vranks = static_cast<int>(rts.size());
     m.blocks_per_rank = 1;
@@ -188,6 +224,7 @@ void Runtime::barrier(const std::vector<std::shared_ptr<Runtime>>& rts, bool use
     CUDA_RUNTIME_CHECK(launch_barrier(m, stream));
     ++rt0.num_launches_;
     if (use_comm_stream) stream_wait(compute, stream);
+    rt0.call_ended(stream, compute);
     if (with_cpu_sync) {
         CUDA_RUNTIME_CHECK(cudaStreamSynchronize(stream));
         for (const auto& rt : rts) rt->check_status();

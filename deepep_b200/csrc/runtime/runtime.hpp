@@ -168,8 +168,10 @@ public:
     CombineResult combine_single(CombineArgs& a);
     // (received tokens, expanded rows, aligned counts per expert) of the last dispatch with host counts
     std::tuple<int, int, std::vector<int>> take_counts(int num_local_experts);
-    // orders the kernels of a call on `stream` behind those of this runtime's previous call
-    void order_behind_last_call(const at::cuda::CUDAStream& stream);
+    // Before the first launch of a call: orders its kernels on `stream`, which is behind `behind` already, after those of this
+    // runtime's previous call. After the last launch: `call_ended` with the stream that has waited for the call since, if any.
+    void order_behind_last_call(const at::cuda::CUDAStream& stream, const at::cuda::CUDAStream& behind);
+    void call_ended(const at::cuda::CUDAStream& stream, const std::optional<at::cuda::CUDAStream>& joined);
 
     // sizing
     static int64_t ht_buffer_size(int num_ranks, int num_max_tokens, int hidden, int num_topk) {
@@ -200,7 +202,15 @@ private:
     uint64_t gpu_timeout_ns_;
     double cpu_timeout_secs_;
     at::cuda::CUDAStream comm_stream_;
-    std::optional<at::cuda::CUDAStream> last_stream_;      // of the last call
+    struct LastCall {
+        std::optional<at::cuda::CUDAStream> stream, joined;     // where it ran and who has waited for it (streams of PyTorch's only)
+        at::cuda::CUDAEvent event;                              // recorded at its end, where `has_event`
+        bool has_event = false;
+    } last_;
+    bool streams_change_ = false;                               // some call ran on another stream than the call before it
+    bool in_capture_ = false;                                   // the call that is being queued is part of a graph capture
+    unsigned long long capture_id_ = 0;                         // the graph capture that `capture_stream_` belongs to, 0 = none
+    std::optional<at::cuda::CUDAStream> capture_stream_;        // of the last call inside it
     int num_device_sms_ = 0, smem_optin_ = 0;
     bool destroyed_ = false;
     int profiling_ = 0;

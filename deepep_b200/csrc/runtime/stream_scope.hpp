@@ -21,15 +21,16 @@ inline at::TensorOptions opts(at::ScalarType dtype, int device) {
 // Everything the stream-control arguments ask for before the first launch.
 struct StreamScope {
     at::cuda::CUDAStream compute, comm;     // `comm`: where the kernels of the call go
+    Runtime& runtime;
     bool switched = false;
     // `may_stay`: a call that hands back nothing asynchronous and waits for nothing but the caller's stream may run on
     // that stream itself. That is the same order of work without the four event calls of the round trip over the
     // communication stream (about 5 us of host time and a few microseconds between dependent kernels on the GPU).
     StreamScope(const StreamControl& sc, Runtime& rt, bool may_stay = false)
-        : compute(at::cuda::getCurrentCUDAStream()), comm(rt.comm_stream()) {
+        : compute(at::cuda::getCurrentCUDAStream()), comm(rt.comm_stream()), runtime(rt) {
         if (may_stay && !sc.async_with_compute_stream && !sc.allocate_on_comm_stream && !sc.previous_event.has_value()) {
             comm = compute;
-            rt.order_behind_last_call(comm);
+            rt.order_behind_last_call(comm, compute);
             return;
         }
         if (sc.allocate_on_comm_stream) {
@@ -38,7 +39,7 @@ struct StreamScope {
         }
         if (sc.previous_event.has_value()) sc.previous_event->stream_wait(comm);
         else stream_wait(comm, compute);
-        rt.order_behind_last_call(comm);
+        rt.order_behind_last_call(comm, sc.previous_event.has_value() ? comm : compute);
     }
     // Either hands back an event (async) or makes the compute stream wait for the comm stream.
     std::optional<EventHandle> finish(const StreamControl& sc, const std::vector<at::Tensor>& tensors) {
@@ -63,6 +64,8 @@ struct StreamScope {
             stream_wait(compute, comm);
         }
         if (switched) at::cuda::setCurrentCUDAStream(compute);
+        if (sc.async_with_compute_stream) runtime.call_ended(comm, std::nullopt);
+        else runtime.call_ended(comm, compute);
         return event;
     }
 };

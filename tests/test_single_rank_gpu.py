@@ -112,23 +112,83 @@ def test_dispatch_combine_against_the_oracle(T, H, E, K, expand, mode):
     buf.destroy()
 
 
-def test_calls_that_change_streams_stay_in_order():
-    """A synchronous call runs on the caller's stream, an asynchronous one on the communication stream: both use the
-    buffer's regions and must not overtake one another."""
-    T, H, E, K = 512, 2048, 16, 4
-    buf = _buffer(T, H, K)
-    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=3, device='cuda')
-    side = torch.cuda.Stream()
-    for it in range(8):
-        xi = (x.float() * (it + 1)).bfloat16()
-        recv, _, _, h, ev = buf.dispatch(xi, topk_idx=idx, num_experts=E, zero_copy=True, async_with_compute_stream=True)
-        ev.current_stream_wait()
-        side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):
-            out = buf.combine(recv, h)[0]
-        torch.cuda.current_stream().wait_stream(side)
-        assert torch.equal(out, xi)
+def _zero_copy_dispatch(buf, x, idx, **kw):
+    return buf.dispatch(x, topk_idx=idx, num_experts=16, zero_copy=True, do_cpu_sync=False, **kw)
+
+
+@pytest.mark.parametrize('capture_between', [False, True])
+@pytest.mark.parametrize('first', ['comm', 'side', 'external'])
+def test_calls_that_change_streams_stay_in_order(first, capture_between):
+    """A synchronous call runs on the caller's stream, an asynchronous one on the communication stream. All use the buffer's
+    regions and must not overtake one another, whatever the caller does about its streams: here it orders nothing. A call that
+    is held up on its stream is followed by calls on another one; the second of them writes the same half of the receive
+    region and has to be the one that stays."""
+    T, H = 512, 2048
+    buf = _buffer(T, H, 4)
+    (x,), (idx,), _ = make_routed_inputs(1, T, H, 16, 4, seed=3, device='cuda')
+    xs = [(x.float() * (i + 1)).bfloat16() for i in range(4)]
+    late, other = torch.cuda.Stream(), torch.cuda.Stream()
+    if first == 'external':
+        late, raw = _external_stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(late):
+        torch.cuda._sleep(200_000_000)                       # about a tenth of a second
+        _zero_copy_dispatch(buf, xs[1], idx, async_with_compute_stream=first == 'comm')
+    if capture_between:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            _zero_copy_dispatch(buf, xs[2], idx)             # (never replayed: it only takes its turn in the double buffer)
+    with torch.cuda.stream(other):
+        if not capture_between:
+            _zero_copy_dispatch(buf, xs[2], idx)
+        recv, _, _, handle, _ = _zero_copy_dispatch(buf, xs[3], idx)
+        combined = buf.combine(recv, handle)[0]
+    torch.cuda.synchronize()
+    buf.check_status()
+    assert torch.equal(recv[:handle.psum_num_recv_tokens_per_scaleup_rank[0]], xs[3][(idx >= 0).any(dim=1)])
+    assert torch.equal(combined, xs[3])
+    if capture_between:
+        graph.reset()
+    if first == 'external':
+        _destroy_stream(raw)
     buf.destroy()
+
+
+def _external_stream():
+    import ctypes
+    lib = ctypes.CDLL('libcudart.so.12')
+    raw = ctypes.c_void_p()
+    assert lib.cudaStreamCreateWithFlags(ctypes.byref(raw), 1) == 0          # non-blocking, like PyTorch's own
+    return torch.cuda.ExternalStream(raw.value), raw
+
+
+def _destroy_stream(raw):
+    import ctypes
+    assert ctypes.CDLL('libcudart.so.12').cudaStreamDestroy(raw) == 0
+
+
+def test_a_stream_of_the_caller_may_be_gone_by_the_next_call():
+    import deepep_b200
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    T, H, E, K = 64, 1024, 16, 4
+    buf = _buffer(T, H, K)
+    ll = deepep_b200.Buffer(SingleProcessGroup(), num_rdma_bytes=deepep_b200.Buffer.get_low_latency_rdma_size_hint(T, H, 1, E), low_latency_mode=True,
+                            num_gpu_timeout_secs=5)
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=4, device='cuda')
+    for _ in range(3):
+        stream, raw = _external_stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            recv, _, _, handle, _ = buf.dispatch(x, topk_idx=idx, num_experts=E)
+            rows, _, lh, _, _ = ll.low_latency_dispatch(x, idx, T, E, use_fp8=False)
+        stream.synchronize()
+        _destroy_stream(raw)
+        assert torch.equal(buf.combine(recv, handle)[0], x)
+        out = ll.low_latency_combine(rows, idx, w, lh)[0]
+        assert (out.float() - x.float() * w.sum(dim=1, keepdim=True)).abs().max() <= 2 ** -7 * x.float().abs().max()
+    torch.cuda.synchronize()
+    buf.destroy()
+    ll.destroy()
 
 
 @pytest.mark.parametrize('T,H,E,K', [
