@@ -271,7 +271,7 @@ cudaError_t launch_local_move(const LocalMoveParams& p, bool quant, int num_sms,
 struct LocalCombineParams {
     int num_tokens, num_topk, num_experts, row_bytes, do_expand, weighted, idx32;
     int round_partial;        // the sum of a token's rows is rounded to bf16 before the biases are added
-    int num_x_rows;
+    int num_x_rows, num_meta_rows;
     int columns, warps, wide; // columns of a row, warps, rows on 32-byte boundaries (filled in by the launcher)
     const uint8_t* x;
     int64_t x_stride_bytes;

@@ -288,6 +288,8 @@ __global__ void __launch_bounds__(kMoveThreads, kExpand ? 6 : 8) local_move_kern
             }
             const uint32_t valid = __ballot_sync(0xffffffffu, e >= 0);
             const int slot = p.token_slot[t];
+            // (the weights of an expanded row go with the row, also where the token has no place in the routing outputs)
+            if (kExpand && row >= 0 && p.recv_topk_weights != nullptr) p.recv_topk_weights[row] = p.topk_weights[static_cast<int64_t>(t) * K + lane];
             if (slot >= 0 && slot < p.num_idx_rows && lane < K) {
                 const int64_t o = static_cast<int64_t>(slot) * K + lane;
                 if (!kExpand) {
@@ -297,8 +299,6 @@ __global__ void __launch_bounds__(kMoveThreads, kExpand ? 6 : 8) local_move_kern
                     }
                     if (p.recv_topk_weights != nullptr)
                         p.recv_topk_weights[o] = p.mask_weights && e < 0 ? 0.f : p.topk_weights[static_cast<int64_t>(t) * K + lane];
-                } else if (row >= 0 && p.recv_topk_weights != nullptr) {
-                    p.recv_topk_weights[row] = p.topk_weights[static_cast<int64_t>(t) * K + lane];
                 }
                 if (p.write_metadata) {
                     int* md = p.recv_src_metadata + static_cast<int64_t>(slot) * (K + 2);
@@ -451,7 +451,8 @@ __global__ void __launch_bounds__(kCombineThreads) local_combine_kernel(const __
     int t = warp_global < p.warps ? warp_global / p.columns : T;
     int next_row = -1, later_slot = -1;     // row of the next token (this lane's, when expanded), slot of the one after it
     auto request_row = [&](int slot) {
-        if (kExpand) next_row = lane < K && slot >= 0 ? p.recv_src_metadata[static_cast<int64_t>(slot) * (K + 2) + 2 + lane] : -1;
+        // (a token beyond the rows that the caller made room for has no metadata)
+        if (kExpand) next_row = lane < K && slot >= 0 && slot < p.num_meta_rows ? p.recv_src_metadata[static_cast<int64_t>(slot) * (K + 2) + 2 + lane] : -1;
         else next_row = slot;
     };
     if (t < T) request_row(p.token_slot[t]);

@@ -280,6 +280,7 @@ CombineResult Runtime::combine_single(CombineArgs& a) {
     p.idx32 = idx_dtype == at::kInt ? 1 : 0;
     p.round_partial = (!a.do_expand || a.allow_multiple_reduction) ? 1 : 0;
     p.num_x_rows = static_cast<int>(a.x.size(0));
+    p.num_meta_rows = static_cast<int>(a.recv_src_metadata.size(0));
     p.x = static_cast<const uint8_t*>(a.x.data_ptr());
     p.x_stride_bytes = a.x.stride(0) * 2;
     p.topk_weights = a.topk_weights.has_value() ? a.topk_weights->data_ptr<float>() : nullptr;

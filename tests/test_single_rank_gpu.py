@@ -112,6 +112,25 @@ def test_dispatch_combine_against_the_oracle(T, H, E, K, expand, mode):
     buf.destroy()
 
 
+def test_expanded_dispatch_with_less_room_than_tokens():
+    """`num_worst_tokens` below the received count: the routing outputs end there, and so do the tokens that a combine finds.
+    Expanded rows have room of their own: all of them arrive, with their weights."""
+    T, H, E, K, room = 300, 256, 8, 3, 171
+    buf = _buffer(T, H, K)
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=12, device='cuda')
+    recv, _, rw, handle, _ = buf.dispatch(x, topk_idx=idx, topk_weights=w, num_experts=E, do_expand=True, do_cpu_sync=False, num_worst_tokens=room)
+    assert handle.recv_src_metadata.size(0) == room
+    rows = handle.dst_expanded_row_idx.long()
+    assert torch.equal(recv[rows.flatten()].view(T, K, H), x[:, None].expand(T, K, H)) and torch.equal(rw[rows], w)
+    out, ow, _ = buf.combine(recv, handle, topk_weights=rw)
+    ref, wref = (x.float() * K).bfloat16(), w.clone()
+    ref[room:], wref[room:] = 0, 0
+    assert torch.equal(out, ref) and torch.equal(ow, wref)
+    torch.cuda.synchronize()
+    buf.check_status()
+    buf.destroy()
+
+
 def _zero_copy_dispatch(buf, x, idx, **kw):
     return buf.dispatch(x, topk_idx=idx, num_experts=16, zero_copy=True, do_cpu_sync=False, **kw)
 
