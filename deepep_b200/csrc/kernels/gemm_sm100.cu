@@ -226,28 +226,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         uint32_t ph = 0, acc_ph = 0;
         bool ok = true, full_seen = false, empty_seen = false;
         for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
-            if constexpr (!kFp8) {
-                if (!(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
-            }
+            if constexpr (!kFp8) pipe_wait_lane(pc, false, tmem_empty + acc, acc_ph ^ 1, ok);
             for (int kb = t.kb0; kb < t.kb1; ++kb) {
                 if constexpr (kFp8) {
-                    if (!empty_seen && !(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
+                    if (!(ok = pipe_wait_warp(pc, empty_seen, tmem_empty + acc, acc_ph ^ 1))) break;
+                    if (!(ok = pipe_wait_warp(pc, full_seen, full + s, ph))) break;
+                } else {
+                    pipe_wait_lane(pc, full_seen, full + s, ph, ok);
                 }
-                if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
                 tc_fence_after();
                 const int s1 = s + 1 == C::kStages ? 0 : s + 1;
                 const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
-                full_seen = mbar_test_wait(full + s1, ph1);
+                full_seen = kFp8 ? pipe_test_warp(full + s1, ph1) : mbar_test_wait(full + s1, ph1);
                 int acc1 = acc;
                 uint32_t acc_ph1 = acc_ph;
                 if constexpr (kFp8) {
                     acc1 = acc + 1 == C::kAccStages ? 0 : acc + 1;
                     acc_ph1 = acc1 == 0 ? acc_ph ^ 1 : acc_ph;
-                    empty_seen = mbar_test_wait(tmem_empty + acc1, acc_ph1 ^ 1);
+                    empty_seen = pipe_test_warp(tmem_empty + acc1, acc_ph1 ^ 1);
                 }
                 const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
                 const uint32_t d_addr = tmem_base + acc * BN;
-                if (elect_one()) {
+                if (elect_one() && ok) {
 #pragma unroll
                     for (int k = 0; k < C::BK / C::UMMA_K; ++k) {
                         const uint32_t accumulate = kFp8 ? (k != 0) : (kb != t.kb0 || k != 0);
@@ -261,13 +261,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                 acc_ph = acc_ph1;
             }
             if constexpr (!kFp8) {
-                if (!ok) break;
-                if (elect_one()) {
+                if (elect_one() && ok) {
                     if (t.kb1 > t.kb0) umma_commit(tmem_full + acc);
                     else mbar_arrive(tmem_full + acc);        // an empty k range: nothing was issued, the epilogue writes zeros
                 }
                 if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
             }
+            if constexpr (!kFp8) ok = pipe_alive_warp(ok);
         }
     } else {
         // ------------------------------------------------------------ epilogue warps
@@ -287,7 +287,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             __nv_bfloat16* c_row = p.C + (p.k_grouped ? static_cast<int64_t>(t.g) * p.c_group_stride : 0) +
                                    static_cast<int64_t>(row) * p.ldc + t.n0 + part * kCols;
             if constexpr (!kFp8) {
-                if (!(ok = pipe_wait(pc, tmem_full + acc, acc_ph))) break;
+                pipe_wait_lane(pc, false, tmem_full + acc, acc_ph, ok);
+                if (!(ok = pipe_alive_warp(ok))) break;
                 tc_fence_after();
                 const bool empty_k = t.kb1 <= t.kb0;
 #pragma unroll 1
@@ -322,7 +323,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     // The commit that frees stage s of the ring. (At most kAccStages <= kStages passes are ahead of this warp: the
                     // barrier cannot have completed another phase meanwhile.)
                     static_assert(C::kAccStages <= C::kStages, "the stage barrier would lap the epilogue");
-                    if (!seen && !(ok = pipe_wait(pc, empty + s, ph))) break;
+                    if (!(ok = pipe_wait_warp(pc, seen, empty + s, ph))) break;
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                     tc_fence_after();
                     uint32_t r0[32];
@@ -332,7 +333,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tmem_empty + acc);      // the values are in registers: the accumulator can be reused
                     if (++acc == C::kAccStages) { acc = 0; acc_ph ^= 1; }
-                    seen = mbar_test_wait(empty + s, ph);              // (asked before the sums, needed after them)
+                    seen = pipe_test_warp(empty + s, ph);              // (asked before the sums, needed after them)
                     fold(sum, r0, scale);
                 }
                 if (ok && (row_ok || zero_row)) {
@@ -484,7 +485,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const bool zero_row = !row_ok && p.zero_gap && row < p.M && row < align_up(t.m_end, p.group_alignment);
             const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
             __nv_bfloat16* c_row = p.C + (p.k_grouped ? static_cast<int64_t>(t.g) * p.c_group_stride : 0) + static_cast<int64_t>(row) * p.ldc + t.n0;
-            if (!(ok = pipe_wait(pc, tmem_full + acc, acc_ph))) break;
+            pipe_wait_lane(pc, false, tmem_full + acc, acc_ph, ok);
+            if (!(ok = pipe_alive_warp(ok))) break;
             tc_fence_after();
             const bool empty_k = t.kb1 <= t.kb0;
 #pragma unroll 1
@@ -614,13 +616,13 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             uint64_t sum[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) sum[i] = 0ull;
-            for (int kb0 = 0; ok && kb0 < num_kb; kb0 += C::kSfChunk) {
-                if (!(ok = pipe_wait(pc, sf_full + slot, sf_ph))) break;
+            for (int kb0 = 0; kb0 < num_kb; kb0 += C::kSfChunk) {
+                pipe_wait_lane(pc, false, sf_full + slot, sf_ph, ok);
                 const float* sf = sf_ring + slot * C::kSfChunk * C::kSfPitch;
                 const int n = min(C::kSfChunk, num_kb - kb0);
                 float scale = sf[quarter * 32 + lane] * sf[BM + (part >> 1)];
                 for (int j = 0; j < n; ++j) {
-                    if (!seen && !(ok = pipe_wait(pc, empty + s, ph))) break;      // the commit that frees stage s
+                    pipe_wait_lane(pc, seen, empty + s, ph, ok);      // the commit that frees stage s
                     tc_fence_after();
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                     const uint32_t addr = lane_addr + acc * C::BN;
@@ -651,6 +653,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 if (lane == 0) mbar_arrive(sf_empty + slot);       // (the last scale of the slot has been used)
                 if (++slot == C::kSfStages) { slot = 0; sf_ph ^= 1; }
             }
+            ok = pipe_alive_warp(ok);
             const int row = t.m0 + static_cast<int>(cta) * BM + quarter * 32 + lane;
             const bool row_ok = row < t.m_end && row < p.M;
             const bool zero_row = !row_ok && p.zero_gap && row < p.M && row < align_up(t.m_end, p.group_alignment);
@@ -698,8 +701,8 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 bool ok = true, full_seen = false, empty_seen = false;
                 for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
                     for (int kb = 0; kb < num_kb; ++kb) {
-                        if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
-                        if (!empty_seen && !(ok = pipe_wait(pc, tmem_empty + acc, acc_ph ^ 1))) break;
+                        pipe_wait_lane(pc, full_seen, full + s, ph, ok);
+                        pipe_wait_lane(pc, empty_seen, tmem_empty + acc, acc_ph ^ 1, ok);
                         tc_fence_after();
                         const int s1 = s + 1 == C::kStages ? 0 : s + 1, acc1 = acc ^ 1;
                         const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph, acc_ph1 = acc1 == 0 ? acc_ph ^ 1 : acc_ph;
@@ -707,7 +710,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         empty_seen = mbar_test_wait(tmem_empty + acc1, acc_ph1 ^ 1);
                         const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
                         const uint32_t d_addr = tmem_base + acc * C::BN;
-                        if (elect_one()) {
+                        if (elect_one() && ok) {
 #pragma unroll
                             for (int k = 0; k < C::BK / C::UMMA_K; ++k) umma_pair_fp8(d_addr, da + 2 * k, db + 2 * k, idesc, k != 0);
                             umma_commit_pair(empty + s);           // frees the stage and tells the epilogues that this pass is complete
@@ -717,6 +720,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         acc = acc1;
                         acc_ph = acc_ph1;
                     }
+                    ok = pipe_alive_warp(ok);
                 }
             } else if (!leader && lane == 0) {
                 // relay: sixteen arrivals of this CTA's warps become one across the cluster, where each costs tens of cycles
@@ -771,7 +775,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                             for (int j = 0; j < C::kSfChunk; ++j) v[i][j] = j < n ? src[i][static_cast<int64_t>(kb0 + j) * p.sfa_k_stride] : 0.f;
                     }
                     if (tid < 2 * C::kSfChunk && tid / 2 < n) vb = sfb[static_cast<int64_t>(tid & 1) * num_kb + kb0 + tid / 2];
-                    if (!(ok = pipe_wait(pc, sf_empty + slot, sf_ph ^ 1))) break;
+                    pipe_wait_lane(pc, false, sf_empty + slot, sf_ph ^ 1, ok);
                     float* dst = sf_ring + slot * C::kSfChunk * C::kSfPitch;
 #pragma unroll
                     for (int j = 0; j < C::kSfChunk; ++j) {
@@ -783,6 +787,7 @@ gemm_pair_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     if (lane == 0) mbar_arrive(sf_full + slot);
                     if (++slot == C::kSfStages) { slot = 0; sf_ph ^= 1; }
                 }
+                ok = pipe_alive_warp(ok);
             }
         }
     }
@@ -822,6 +827,20 @@ struct MxCfg {
     static constexpr int kBarBytes = (2 * kStages + 2) * 8 + 16;
     static constexpr int kSmem = kStages * STAGE + 2 * kSfStage + kBarBytes + 1024;
 };
+
+// Barrier of the scale warps of a CTA: true where all of them are `up`.
+__device__ __forceinline__ bool scale_warps_meet(bool up, int threads) {
+    uint32_t all;
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.u32 p, %1, 0;\n"
+        "barrier.cta.red.and.aligned.pred q, 3, %2, p;\n"
+        "selp.u32 %0, 1, 0, q;\n"
+        "}\n"
+        : "=r"(all) : "r"(up ? 1u : 0u), "r"(threads) : "memory");
+    return all != 0;
+}
 
 __device__ __forceinline__ uint32_t ue8m0_of(float scale) { return (__float_as_uint(scale) >> 23) & 0xffu; }
 
@@ -894,16 +913,16 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         uint32_t ph = 0, acc_ph = 0;
         bool ok = true, full_seen = false;
         for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
-            if (!(ok = pipe_wait(pc, tmem_empty, acc_ph ^ 1))) break;
+            pipe_wait_lane(pc, false, tmem_empty, acc_ph ^ 1, ok);
             for (int kb = t.kb0; kb < t.kb1; ++kb) {
-                if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
+                pipe_wait_lane(pc, full_seen, full + s, ph, ok);
                 tc_fence_after();
                 const int s1 = s + 1 == C::kStages ? 0 : s + 1;
                 const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
                 full_seen = mbar_test_wait(full + s1, ph1);
                 const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
                 const uint32_t sfa = tmem_base + C::kSfBase + s * C::kSfCols, sfb = sfa + 4;
-                if (elect_one()) {
+                if (elect_one() && ok) {
 #pragma unroll
                     for (int k = 0; k < C::BK / C::UMMA_K; ++k)
                         umma_mx(tmem_base, da + 2 * k, db + 2 * k, make_idesc_mx(BM, C::BN, static_cast<uint32_t>(k)), (kb != t.kb0 || k != 0) ? 1u : 0u, sfa, sfb);
@@ -912,9 +931,9 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 s = s1;
                 ph = ph1;
             }
-            if (!ok) break;
-            if (elect_one()) umma_commit(tmem_full);
+            if (elect_one() && ok) umma_commit(tmem_full);
             acc_ph ^= 1;
+            ok = pipe_alive_warp(ok);
         }
     } else if (warp < 2 + C::kEpiWarps) {
         // ------------------------------------------------------------ epilogue warps: once per tile
@@ -931,7 +950,8 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const bool zero_row = !row_ok && p.zero_gap && row < p.M;
             const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * kCols;
             __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + part * kCols;
-            if (!(ok = pipe_wait(pc, tmem_full, acc_ph))) break;
+            pipe_wait_lane(pc, false, tmem_full, acc_ph, ok);
+            if (!(ok = pipe_alive_warp(ok))) break;
             tc_fence_after();
             // All of this warp's columns first: the accumulator is free for the next tile before anything is converted or
             // stored, which costs as much as several k-blocks.
@@ -986,28 +1006,28 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 dst[(kb - tt.kb0) * C::kSfPitch + BM + h] = static_cast<uint8_t>(ue8m0_of(srcb[static_cast<int64_t>(h) * kblocks + kb]));
             }
         };
-        auto sf_barrier = [&]() { asm volatile("bar.sync 3, %0;" ::"r"(C::kSfWarps * 32) : "memory"); };
+        // (a warp that has given up still comes to the barrier and takes the other scale warps with it)
+        auto sf_barrier = [&](bool up) { return scale_warps_meet(up, C::kSfWarps * 32); };
         int s = 0, buf = 0;
         uint32_t ph = 0;
         bool ok = true;
         bool have = sched.get(blockIdx.x, t);
         if (have) stage_tile(t, sf_stage);
-        sf_barrier();
+        sf_barrier(true);
         for (int ti = blockIdx.x; ok && have; ti += gridDim.x) {
             const bool have_next = sched.get(ti + gridDim.x, nxt);
             if (have_next) stage_tile(nxt, sf_stage + (buf ^ 1) * C::kSfStage);      // one tile ahead
             const uint8_t* mine = sf_stage + buf * C::kSfStage;
             // two k-blocks per round: the wait for the tensor-memory stores (a few hundred cycles) is paid once per round,
             // otherwise a scale warp, which sees every k-block, could not keep up with the tensor pipe
-            for (int kb = t.kb0; ok && kb < t.kb1; kb += 2) {
+            for (int kb = t.kb0; kb < t.kb1; kb += 2) {
                 const int n = min(2, t.kb1 - kb);
                 int sj[2];
                 for (int j = 0; j < n; ++j) {
                     sj[j] = s;
-                    if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
+                    pipe_wait_lane(pc, false, empty + s, ph ^ 1, ok);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
-                if (!ok) break;
                 tc_fence_after();
                 for (int j = 0; j < n; ++j) {
                     const uint8_t* src = mine + (kb + j - t.kb0) * C::kSfPitch;
@@ -1033,7 +1053,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
             }
-            sf_barrier();       // the next tile's bytes are complete; nobody reads this tile's any more
+            ok = sf_barrier(ok);       // the next tile's bytes are complete; nobody reads this tile's any more
             buf ^= 1;
             t = nxt;
             have = have_next;
@@ -1143,16 +1163,16 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             uint32_t ph = 0, acc_ph = 0;
             bool ok = true, full_seen = false;
             for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
-                if (!(ok = pipe_wait(pc, tmem_empty, acc_ph ^ 1))) break;
+                pipe_wait_lane(pc, false, tmem_empty, acc_ph ^ 1, ok);
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
-                    if (!full_seen && !(ok = pipe_wait(pc, full + s, ph))) break;
+                    pipe_wait_lane(pc, full_seen, full + s, ph, ok);
                     tc_fence_after();
                     const int s1 = s + 1 == C::kStages ? 0 : s + 1;
                     const uint32_t ph1 = s1 == 0 ? ph ^ 1 : ph;
                     full_seen = mbar_test_wait(full + s1, ph1);
                     const uint64_t da = da0 + s * (C::STAGE >> 4), db = db0 + s * (C::STAGE >> 4);
                     const uint32_t sfa = tmem_base + C::kSfBase + s * C::kSfCols, sfb = sfa + 4;
-                    if (elect_one()) {
+                    if (elect_one() && ok) {
 #pragma unroll
                         for (int k = 0; k < C::BK / C::UMMA_K; ++k)
                             umma_mx_pair(tmem_base, da + 2 * k, db + 2 * k, make_idesc_mx(2 * BM, C::BN, static_cast<uint32_t>(k)),
@@ -1162,9 +1182,9 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     s = s1;
                     ph = ph1;
                 }
-                if (!ok) break;
-                if (elect_one()) umma_commit_pair(tmem_full);
+                if (elect_one() && ok) umma_commit_pair(tmem_full);
                 acc_ph ^= 1;
+                ok = pipe_alive_warp(ok);
             }
         } else if (!leader && lane == 0) {
             // relay: the four arrivals of this CTA's scale warps become one across the cluster
@@ -1194,7 +1214,8 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const bool zero_row = !row_ok && p.zero_gap && row < p.M && row < align_up(t.m_end, p.group_alignment);
             const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + part * 64;
             __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + t.n0 + part * 64;
-            if (!(ok = pipe_wait(pc, tmem_full, acc_ph))) break;
+            pipe_wait_lane(pc, false, tmem_full, acc_ph, ok);
+            if (!(ok = pipe_alive_warp(ok))) break;
             tc_fence_after();
             // All of this warp's columns first: the (only) accumulator is free for the next tile before anything is converted
             // or stored, which costs as much as several k-blocks.
@@ -1236,28 +1257,28 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 dst[(kb - tt.kb0) * C::kSfPitch + BM + h] = static_cast<uint8_t>(ue8m0_of(srcb[static_cast<int64_t>(h) * kblocks + kb]));
             }
         };
-        auto sf_barrier = [&]() { asm volatile("bar.sync 3, %0;" ::"r"(C::kSfWarps * 32) : "memory"); };
+        // (a warp that has given up still comes to the barrier and takes the other scale warps with it)
+        auto sf_barrier = [&](bool up) { return scale_warps_meet(up, C::kSfWarps * 32); };
         int s = 0, buf = 0;
         uint32_t ph = 0;
         bool ok = true;
         bool have = sched.get(pair, t);
         if (have) stage_tile(t, sf_stage);
-        sf_barrier();
+        sf_barrier(true);
         for (int ti = pair; ok && have; ti += num_pairs) {
             const bool have_next = sched.get(ti + num_pairs, nxt);
             if (have_next) stage_tile(nxt, sf_stage + (buf ^ 1) * C::kSfStage);
             const uint8_t* mine = sf_stage + buf * C::kSfStage;
             // two k-blocks per round: the wait for the tensor-memory stores (a few hundred cycles) is paid once per round,
             // otherwise a scale warp, which sees every k-block, could not keep up with the tensor pipe
-            for (int kb = t.kb0; ok && kb < t.kb1; kb += 2) {
+            for (int kb = t.kb0; kb < t.kb1; kb += 2) {
                 const int n = min(2, t.kb1 - kb);
                 int sj[2];
                 for (int j = 0; j < n; ++j) {
                     sj[j] = s;
-                    if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
+                    pipe_wait_lane(pc, false, empty + s, ph ^ 1, ok);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
-                if (!ok) break;
                 tc_fence_after();
                 for (int j = 0; j < n; ++j) {
                     const uint8_t* src = mine + (kb + j - t.kb0) * C::kSfPitch;
@@ -1282,7 +1303,7 @@ gemm_mx_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     for (int j = 0; j < n; ++j) mbar_arrive(leader ? full + sj[j] : sf_done + sj[j]);
                 }
             }
-            sf_barrier();
+            ok = sf_barrier(ok);
             buf ^= 1;
             t = nxt;
             have = have_next;

@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kAgThreads, 1) ag_gemm_kernel(const __grid_con
             int src, chunk, n0;
             decode(t, src, chunk, n0);
             const int row = src * Ml + chunk * BM + quarter * 32 + lane;
-            if (!pipe_wait(pc, tmem_full + acc, acc_ph)) break;
+            if (!pipe_alive_warp(pipe_wait(pc, tmem_full + acc, acc_ph))) break;
             tc_fence_after();
             __nv_bfloat16* c_row = p.C + static_cast<int64_t>(row) * p.ldc + n0;
 #pragma unroll 1
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kRsThreads, 1) gemm_rs_kernel(const __grid_con
                 if (!__all_sync(0xffffffffu, arrived) && lane == 0) atomicExch(p.error, static_cast<int>(kStatusTileFlag));
                 __syncwarp();
             }
-            if (!pipe_wait(pc, tmem_full + acc, acc_ph)) break;
+            if (!pipe_alive_warp(pipe_wait(pc, tmem_full + acc, acc_ph))) break;
             tc_fence_after();
             // (the previous tile's bulk store of this lane has completed: it is waited for right after it is issued)
             const int r_in_tile = quarter * 32 + lane;
