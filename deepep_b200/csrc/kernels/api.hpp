@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 
 #include "../common/layout.hpp"
 
@@ -19,8 +20,8 @@ namespace ep {
 // use: an SM has to drain and reconfigure when consecutive kernels prefer different ones, which costs microseconds
 // between the back-to-back kernels of a dispatch / combine step.
 // One static object per kernel remembers, per device, what the attributes were set to: the two driver calls cost a
-// microsecond or two of host time, which every launch used to pay. (The limit only ever grows; two threads that race
-// set the same attributes twice.)
+// microsecond or two of host time, which every launch used to pay. The limit only ever grows: it is set under a lock, or a
+// thread with a smaller launch could lower it again between another thread's preparation and its launch.
 class PreparedKernel {
 public:
     template <typename Kernel>
@@ -30,6 +31,8 @@ public:
         if (err != cudaSuccess) return err;
         const bool known = device >= 0 && device < kDevices;
         if (known && granted_[device].load(std::memory_order_acquire) > dynamic_smem_bytes) return cudaSuccess;
+        const std::lock_guard<std::mutex> lock(mutex_);
+        if (known && granted_[device].load(std::memory_order_relaxed) > dynamic_smem_bytes) return cudaSuccess;
         err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic_smem_bytes);
         if (err != cudaSuccess) return err;
         err = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -41,6 +44,7 @@ public:
 private:
     static constexpr int kDevices = 64;
     std::atomic<int> granted_[kDevices] = {};      // granted bytes + 1, 0 = never set
+    std::mutex mutex_;
 };
 
 // ---------------------------------------------------------------- cross-rank barrier
