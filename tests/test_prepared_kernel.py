@@ -25,8 +25,8 @@ extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute attr,
     limit = value;
     return cudaSuccess;
 }
-static void kernel(int) {}
 int main() {
+    const void* kernel = nullptr;       // (any handle: only the stand-ins see it)
     ep::PreparedKernel prepared;
     std::thread small([&] { prepared.prepare(kernel, 1000); });
     while (small_inside == 0) std::this_thread::yield();
