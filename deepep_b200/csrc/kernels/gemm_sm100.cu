@@ -1323,14 +1323,12 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeFn get_encode_fn() {
-    static EncodeFn fn = nullptr;
-    if (fn == nullptr) {
+    static const EncodeFn fn = [] {
         void* ptr = nullptr;
         cudaDriverEntryPointQueryResult res;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &res) == cudaSuccess &&
-            res == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeFn>(ptr);
-    }
+        const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &res) == cudaSuccess && res == cudaDriverEntryPointSuccess;
+        return found ? reinterpret_cast<EncodeFn>(ptr) : nullptr;
+    }();
     return fn;
 }
 

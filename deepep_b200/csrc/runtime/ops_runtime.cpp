@@ -9,6 +9,7 @@
 #include <torch/extension.h>
 
 #include <map>
+#include <mutex>
 #include <optional>
 
 #include "../common/exception.hpp"
@@ -26,9 +27,11 @@ namespace {
 
 cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
-// one status word per device for the GEMM pipelines (0 = healthy)
+// one status word per device for the GEMM pipelines (0 = healthy); the calls of a layer come here without the GIL
 at::Tensor& gemm_status(int device) {
+    static std::mutex mutex;
     static std::map<int, at::Tensor> words;
+    const std::lock_guard<std::mutex> lock(mutex);
     auto it = words.find(device);
     if (it == words.end())
         it = words.emplace(device, at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device))))).first;

@@ -1,5 +1,9 @@
 """Fused MoE layer forward + backward (bf16 and FP8 forward) with emulated ranks, against a dense
 fp32 PyTorch reference with autograd; plus the single-rank nn.Module path."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -111,3 +115,38 @@ def test_moe_module_gradients(T, H, I, E, K, use_fp8):
         assert layer.router.grad.abs().max() == 0       # the softmax over one expert does not depend on its logit
     assert layer.router.grad.dtype == layer.router.dtype
     buf.destroy()
+
+
+def test_layers_of_several_threads():
+    """Each thread has a buffer, a layer and a stream of its own; what the layers share (the launch set-up and the status word
+    of the tensor-core kernels) is reached without the GIL. In a process of its own: the first calls are the ones that matter."""
+    code = """
+import threading, torch, deepep_b200
+from deepep_b200.models.moe import FusedMoE, MoEConfig
+from deepep_b200.parallel.local_cluster import SingleProcessGroup
+N, T, H, I, E, K = 6, 100, 256, 128, 4, 2
+layers = [FusedMoE(deepep_b200.ElasticBuffer(SingleProcessGroup(), num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_gpu_timeout_secs=5),
+                   MoEConfig(hidden=H, intermediate=I, num_experts=E, num_topk=K)) for _ in range(N)]
+x = torch.randn((T, H), device='cuda').bfloat16()
+streams, start, out = [torch.cuda.Stream() for _ in range(N)], threading.Barrier(N), [None] * N
+torch.cuda.synchronize()
+def work(i):
+    with torch.cuda.stream(streams[i]):
+        xi = x.clone().requires_grad_(True)
+        start.wait()
+        for _ in range(20):
+            xi.grad = None
+            y = layers[i](xi)
+            y.backward(x)
+        out[i] = (y.detach(), xi.grad)
+        streams[i].synchronize()
+threads = [threading.Thread(target=work, args=(i,)) for i in range(N)]
+for t in threads: t.start()
+for t in threads: t.join()
+xi = x.clone().requires_grad_(True)
+y = layers[0](xi)
+y.backward(x)
+assert all(torch.equal(a, y) and torch.equal(b, xi.grad) for a, b in out)
+"""
+    done = subprocess.run([sys.executable, '-c', code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
