@@ -25,6 +25,9 @@ namespace ep {
 
 namespace {
 
+// A contiguous tensor that starts on a 16-byte boundary (the wide loads of the kernels); a view into a flat buffer may not.
+at::Tensor on_16_bytes(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(); }
+
 cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // one status word per device for the GEMM pipelines (0 = healthy); the calls of a layer come here without the GIL
@@ -193,7 +196,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> router_forward(const at::Tensor& 
     at::Tensor w = router;
     if (router.scalar_type() != at::kBFloat16 || padded != E) {
         w = new_tensor({padded, H}, at::kBFloat16, device);
-        const at::Tensor f = router.scalar_type() == at::kFloat ? router : router.to(at::kFloat);
+        const at::Tensor f = on_16_bytes(router.scalar_type() == at::kFloat ? router : router.to(at::kFloat));
         CUDA_RUNTIME_CHECK(ops::router_weights(f.data_ptr<float>(), E, padded, H, w.data_ptr(), cur_stream()));
     }
     const at::Tensor logits = gemm_impl(x, w, std::nullopt, std::nullopt, std::nullopt, 1, std::nullopt, 0, false, true);
@@ -225,7 +228,8 @@ static std::tuple<at::Tensor, at::Tensor> quant_weights_128x128(const at::Tensor
     c10::cuda::CUDAGuard guard(w.device());
     const int G = static_cast<int>(w.size(0)), N = static_cast<int>(w.size(1)), K = static_cast<int>(w.size(2)), device = w.get_device();
     auto q = new_tensor({G, N, K}, at::kFloat8_e4m3fn, device), sf = new_tensor({G, N / 128, K / 128}, at::kFloat, device);
-    CUDA_RUNTIME_CHECK(ops::quant_weights_128x128(w.data_ptr(), G, N, K, pow2, q.data_ptr(), sf.data_ptr<float>(), cur_stream()));
+    const at::Tensor aligned = on_16_bytes(w);
+    CUDA_RUNTIME_CHECK(ops::quant_weights_128x128(aligned.data_ptr(), G, N, K, pow2, q.data_ptr(), sf.data_ptr<float>(), cur_stream()));
     return {q, sf};
 }
 
@@ -259,7 +263,8 @@ at::Tensor dequant_1x128(const at::Tensor& q, const at::Tensor& sf, const std::o
     const int M = static_cast<int>(q.size(0)), H = static_cast<int>(q.size(1));
     EP_HOST_ASSERT(H % 128 == 0 && sf.size(0) == M && sf.size(1) == H / 128);
     auto out = new_tensor({M, H}, at::kBFloat16, q.get_device());
-    CUDA_RUNTIME_CHECK(ops::dequant_1x128(q.data_ptr(), sf.data_ptr<float>(), sf.stride(0), sf.stride(1), M, H, row_groups(group_end, group_alignment),
+    const at::Tensor aligned = on_16_bytes(q);
+    CUDA_RUNTIME_CHECK(ops::dequant_1x128(aligned.data_ptr(), sf.data_ptr<float>(), sf.stride(0), sf.stride(1), M, H, row_groups(group_end, group_alignment),
                                           out.data_ptr(), cur_stream()));
     return out;
 }

@@ -127,3 +127,32 @@ def test_streaming_ops_skip_or_zero_alignment_gaps(I):
         q.view(torch.uint8)[~valid] = 0x7f          # NaN
         back = C.dequant_1x128(q, sf, group_end=ends, group_alignment=align)
         assert torch.equal(back[valid], C.dequant_1x128(*C.quant_1x128(dout))[valid]) and (back[~valid] == 0).all()
+
+
+@pytest.mark.parametrize('offset', [1, 8, 16])
+def test_inputs_that_start_anywhere(offset):
+    """Contiguous views into flat buffers, as parameter buckets and received messages are: they start on no 16-byte boundary."""
+    from deepep_b200 import ops
+    from deepep_b200.models.moe import FusedMoE, MoEConfig, quantize_weight_128x128
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    import deepep_b200
+    g = torch.Generator(device='cuda').manual_seed(offset)
+
+    def view(t):
+        flat = torch.empty(t.numel() + offset, dtype=t.dtype, device='cuda')
+        flat[offset:].view(t.shape).copy_(t)
+        return flat[offset:].view(t.shape)
+
+    q, sf = ops.quant_1x128(torch.randn((5, 384), device='cuda', generator=g).bfloat16())
+    assert torch.equal(ops.dequant_1x128(view(q), sf), ops.dequant_1x128(q, sf))
+    w = torch.randn((2, 256, 128), device='cuda', generator=g).bfloat16()
+    for a, b in zip(quantize_weight_128x128(view(w)), quantize_weight_128x128(w)):
+        assert torch.equal(a.float(), b.float())
+    buf = deepep_b200.ElasticBuffer(SingleProcessGroup(), num_max_tokens_per_rank=32, hidden=256, num_topk=2, num_gpu_timeout_secs=5)
+    layer = FusedMoE(buf, MoEConfig(hidden=256, intermediate=128, num_experts=4, num_topk=2))
+    x = torch.randn((32, 256), device='cuda', generator=g).bfloat16()
+    y = layer(x)
+    layer.router.data = view(layer.router.data)
+    assert torch.equal(layer(x), y)
+    torch.cuda.synchronize()
+    buf.destroy()
