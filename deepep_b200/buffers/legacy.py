@@ -175,6 +175,7 @@ class Buffer:
         num_recv_tokens_per_expert_list, handle, event)``; with a cached ``handle`` only ``recv_x`` and the
         event are meaningful. ``num_worst_tokens > 0`` skips the CPU sync and returns worst-case shapes.
         ``num_experts`` is inferred from ``num_tokens_per_expert`` when not given."""
+        check_torch_deterministic()
         config = config or self.get_dispatch_config(self.group_size)
         hidden = (x[0] if isinstance(x, tuple) else x).size(1)
         prev = getattr(previous_event, 'event', None)

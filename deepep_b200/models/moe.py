@@ -28,6 +28,7 @@ from typing import Any, List, Optional, Sequence, Tuple
 import torch
 
 from .._native import _C, require_native
+from ..utils.envs import check_torch_deterministic
 
 
 @dataclass
@@ -85,6 +86,7 @@ class _SingleRankComm:
         self.buffers = [buffer]
 
     def dispatch(self, per_rank_kwargs):
+        check_torch_deterministic()
         buf, kw = self.buffers[0], per_rank_kwargs[0]
         call = buf._dispatch_call(**kw)
         return [buf._dispatch_result(_C.Runtime.dispatch([buf.runtime], [call])[0], call, kw.get('handle'))]
@@ -190,6 +192,7 @@ class _LayerFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
+        check_torch_deterministic()
         w = ctx.layer.weights
         dx, d_router, d13, d2 = _C.moe_layer_backward(ctx.layer.buffer.runtime, ctx.call, ctx.saved_tensors[0], dy, w.w13_t, w.w2_t)
         return dx, d_router.to(ctx.router_dtype), d13, d2, None
@@ -227,6 +230,7 @@ class FusedMoE(torch.nn.Module):
                                  c.use_fp8 and c.pow2_scales and self.weights.pow2_scales, b.allow_multiple_reduction, b.fuse_combine_reduce)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        check_torch_deterministic()
         return _LayerFunction.apply(x, self.router, self.w13, self.w2, self)
 
 

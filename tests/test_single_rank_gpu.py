@@ -302,3 +302,29 @@ def test_engram_fetch_from_local_memory(hidden, fp8):
     torch.cuda.synchronize()
     buf.check_status()
     buf.destroy()
+
+
+def test_calls_refuse_to_run_under_filled_uninitialised_memory():
+    """PyTorch's deterministic mode with filled memory would write over what arrives: every entry point says so."""
+    import deepep_b200
+    from deepep_b200.models.moe import FusedMoE, MoEConfig
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    T, H, E, K = 32, 256, 4, 2
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=1, device='cuda')
+    buf = _buffer(T, H, K)
+    old = deepep_b200.Buffer(SingleProcessGroup(), num_nvl_bytes=deepep_b200.Buffer.get_dispatch_config(1).get_nvl_buffer_size_hint(2 * H, 1, T, K),
+                             num_gpu_timeout_secs=5)
+    layer = FusedMoE(buf, MoEConfig(hidden=H, intermediate=128, num_experts=E, num_topk=K))
+    y = layer(x.requires_grad_(True))
+    recv, _, _, handle, _ = buf.dispatch(x.detach(), topk_idx=idx, topk_weights=w, num_experts=E)
+    calls = [lambda: buf.dispatch(x.detach(), topk_idx=idx, num_experts=E), lambda: buf.combine(recv, handle), lambda: layer(x), lambda: y.sum().backward(),
+             lambda: old.dispatch(x.detach(), topk_idx=idx, topk_weights=w, num_experts=E)]
+    torch.use_deterministic_algorithms(True)
+    try:
+        for call in calls:
+            with pytest.raises(AssertionError, match='fill_uninitialized_memory'):
+                call()
+    finally:
+        torch.use_deterministic_algorithms(False)
+    buf.destroy()
+    old.destroy()
