@@ -213,7 +213,7 @@ class Buffer:
             rank_prefix, sent, received, send_head, in_rank = _C.legacy_handle(self.runtime, ep_handle.num_tokens_per_rank_matrix,
                                                                                ep_handle.dst_buffer_slot_idx, is_token_in_rank is None)
             if async_finish:
-                event = EventOverlap(_C.EventHandle())
+                event.event.record_again()
         legacy = LegacyHandle((rank_prefix, sent, received, ep_handle.recv_src_metadata[:, 0],
                                in_rank if is_token_in_rank is None else is_token_in_rank, send_head), ep_handle)
         return recv_x, recv_topk_idx, recv_topk_weights, ep_handle.num_recv_tokens_per_expert_list, legacy, event

@@ -151,6 +151,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
     py::class_<EventHandle>(m, "EventHandle")
         .def(py::init<>())
+        .def("record_again", &EventHandle::record_again)
         .def("current_stream_wait", &EventHandle::current_stream_wait);
 
     py::class_<Runtime, std::shared_ptr<Runtime>>(m, "Runtime")

@@ -33,6 +33,8 @@ struct EventHandle {
 
     EventHandle() : event(std::make_shared<at::cuda::CUDAEvent>()) { event->record(at::cuda::getCurrentCUDAStream()); }
     explicit EventHandle(const at::cuda::CUDAStream& stream) : event(std::make_shared<at::cuda::CUDAEvent>()) { event->record(stream); }
+    // moves the event behind what the current stream holds by now; the tensors that it keeps alive stay
+    void record_again() const { event->record(at::cuda::getCurrentCUDAStream()); }
     void current_stream_wait() const { event->block(at::cuda::getCurrentCUDAStream()); }
     void stream_wait(const at::cuda::CUDAStream& stream) const { event->block(stream); }
 };

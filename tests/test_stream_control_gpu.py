@@ -2,6 +2,9 @@
 asynchronous completion, allocation on the communication stream, handle copies, zero / one / two biases, and a
 double run that must give identical bytes. One rank, so the expected values are closed-form."""
 import itertools
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -98,3 +101,31 @@ def test_double_run_is_bit_identical():
         hashes.append(h)
         cl.destroy()
     assert hashes[0] == hashes[1]
+
+
+def test_an_asynchronous_event_keeps_the_tensors_alive():
+    """EP_AVOID_RECORD_STREAM=1: the event of an asynchronous call holds the call's tensors until it is dropped (the switch is
+    read once per process). The first generation's dispatch moves its event behind the kernel that fills its handle."""
+    code = """
+import torch, deepep_b200
+from deepep_b200.parallel.local_cluster import SingleProcessGroup
+T, H, E, K = 512, 2048, 16, 4
+buf = deepep_b200.Buffer(SingleProcessGroup(), num_nvl_bytes=deepep_b200.Buffer.get_dispatch_config(1).get_nvl_buffer_size_hint(2 * H, 1, T, K))
+idx = torch.randint(0, E, (T, K), device='cuda')
+for weights in (None, torch.rand((T, K), device='cuda')):
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    x = torch.randn((T, H), device='cuda').bfloat16()
+    out = buf.dispatch(x, topk_idx=idx, topk_weights=weights, num_experts=E, async_finish=True)
+    event = out[5]
+    del x, out
+    assert torch.cuda.memory_allocated() >= before + 2 * T * H * 2, 'rows and input are free while the kernels may still run'
+    event.current_stream_wait()
+    torch.cuda.synchronize()
+    del event
+    assert torch.cuda.memory_allocated() == before
+buf.destroy()
+"""
+    done = subprocess.run([sys.executable, '-c', code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300,
+                          env=dict(os.environ, EP_AVOID_RECORD_STREAM='1'))
+    assert done.returncode == 0, done.stderr[-2000:]
