@@ -187,7 +187,9 @@ class _LayerFunction(torch.autograd.Function):
     def forward(ctx, x, router, w13, w2, layer):
         y, ctx.call = _C.moe_layer_forward(layer.buffer.runtime, layer._native_config(), x, router, layer.weights.forward_operands())
         ctx.layer, ctx.router_dtype = layer, router.dtype
-        ctx.save_for_backward(x)
+        # where the kernels read the router as it is (no converted copy), autograd has to notice a change before the backward pass
+        as_it_is = router.dtype == torch.bfloat16 and router.size(0) % 128 == 0 and router.is_contiguous()
+        ctx.save_for_backward(x, *([router] if as_it_is else []))
         return y
 
     @staticmethod

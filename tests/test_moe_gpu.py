@@ -150,3 +150,29 @@ assert all(torch.equal(a, y) and torch.equal(b, xi.grad) for a, b in out)
 """
     done = subprocess.run([sys.executable, '-c', code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+def test_a_router_that_changes_before_the_backward_pass_is_noticed():
+    """A bf16 router over a multiple of 128 experts is read where it lies; any other one is converted into a copy, which a
+    change does not reach."""
+    import deepep_b200
+    from deepep_b200.models.moe import FusedMoE, MoEConfig
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    T, H, I, K = 64, 256, 128, 2
+    for E, dtype in ((128, torch.bfloat16), (128, torch.float32), (8, torch.bfloat16)):
+        buf = deepep_b200.ElasticBuffer(SingleProcessGroup(), num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_gpu_timeout_secs=5)
+        layer = FusedMoE(buf, MoEConfig(hidden=H, intermediate=I, num_experts=E, num_topk=K))
+        layer.router = torch.nn.Parameter(layer.router.detach().to(dtype))
+        x = torch.randn((T, H), device='cuda', generator=torch.Generator(device='cuda').manual_seed(2)).bfloat16().requires_grad_(True)
+        layer(x).sum().backward()
+        kept, x.grad = x.grad, None
+        y = layer(x)
+        with torch.no_grad():
+            layer.router.mul_(2)
+        if E == 128 and dtype == torch.bfloat16:
+            with pytest.raises(RuntimeError, match='modified by an inplace operation'):
+                y.sum().backward()
+        else:
+            y.sum().backward()
+            assert torch.equal(x.grad, kept)
+        buf.destroy()
