@@ -58,6 +58,13 @@ def quantize_weight_128x128(w: torch.Tensor, pow2: bool = False) -> Tuple[torch.
     return q, scale.contiguous()
 
 
+def _transposed(w: torch.Tensor) -> torch.Tensor:
+    """``[G, N, K]`` -> contiguous ``[G, K, N]``."""
+    if w.is_cuda and w.dtype == torch.bfloat16 and _C is not None and w.size(0) <= 65535:      # (the kernel's grid)
+        return _C.transpose_bf16(w)
+    return w.transpose(1, 2).contiguous()
+
+
 class ExpertWeights:
     """This rank's experts: ``w13 [local experts, 2 * intermediate, hidden]`` (gate rows first, then up) and
     ``w2 [local experts, hidden, intermediate]`` in bf16, plus the derived copies the kernels read."""
@@ -68,8 +75,8 @@ class ExpertWeights:
 
     def refresh(self) -> None:
         """Rebuilds the transposed (for data gradients) and quantised (for FP8 forward) copies after an update."""
-        self.w13_t = _C.transpose_bf16(self.w13)               # [EL, hidden, 2I]
-        self.w2_t = _C.transpose_bf16(self.w2)                 # [EL, I, hidden]
+        self.w13_t = _transposed(self.w13)                     # [EL, hidden, 2I]
+        self.w2_t = _transposed(self.w2)                       # [EL, I, hidden]
         if self.use_fp8:
             self.w13_q, self.w13_sf = quantize_weight_128x128(self.w13, self.pow2_scales)
             self.w2_q, self.w2_sf = quantize_weight_128x128(self.w2, self.pow2_scales)

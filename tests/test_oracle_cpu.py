@@ -206,3 +206,18 @@ def test_bench_reference_arm_reports_unavailable():
     assert res.returncode == 0
     line = json.loads(res.stdout.strip().splitlines()[-1])
     assert line['impl'] == 'reference' and isinstance(line.get('unavailable'), str) and line['unavailable']
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('pow2', [False, True])
+def test_expert_weights_on_the_cpu(dtype, pow2):
+    """A checkpoint's experts can be prepared anywhere, in any floating type."""
+    from deepep_b200.models.moe import ExpertWeights
+    g = torch.Generator().manual_seed(1)
+    w13, w2 = torch.randn((2, 256, 128), generator=g).to(dtype), torch.randn((2, 128, 128), generator=g).to(dtype)
+    e = ExpertWeights(w13, w2, True, pow2)
+    assert torch.equal(e.w13_t, w13.transpose(1, 2)) and e.w13_t.is_contiguous() and torch.equal(e.w2_t, w2.transpose(1, 2))
+    back = e.w13_q.float().view(2, 2, 128, 1, 128) * e.w13_sf.view(2, 2, 1, 1, 1)
+    # e4m3 rounds to a sixteenth of a value, and to half of 2^-9 scales below its normal range
+    want = w13.float().view(2, 2, 128, 1, 128)
+    assert ((back - want).abs() <= want.abs() / 16 + e.w13_sf.view(2, 2, 1, 1, 1) * 2 ** -10).all()
