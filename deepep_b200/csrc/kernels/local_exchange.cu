@@ -85,11 +85,25 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     int* mine = s_cnt + warp * (E + 1);
     uint32_t* mask_of = s_mask + warp * E;
     int tokens_before = 0;
+    // token of pair i: i / K for i < 32 K <= 1024, as a product (sixteen divisions a lane were a fifth of this kernel's issue slots)
+    const uint32_t inv_k = 65536u / static_cast<uint32_t>(K) + 1u;
+    auto token_of = [&](int i) { return (static_cast<uint32_t>(i) * inv_k) >> 16; };
+    // All pairs of the 32 tokens from `base` on, in the same contiguous order, eight loads in flight (a lane that walked along
+    // its own token's row waited for one load at a time: 239 against 101 us for a dispatch of 8192 tokens with top-32).
+    auto walk_pairs = [&](int base, auto&& visit) {
+        const int64_t first = static_cast<int64_t>(base) * K;
+        const int n = min(32, b - base) * K;
+        for (int i0 = lane; i0 - lane < n; i0 += 256) {
+            int e[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) e[u] = i0 + 32 * u < n ? load_topk_idx(p.topk_idx, p.idx32 != 0, first + i0 + 32 * u, E) : -1;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i0 + 32 * u < n) visit(first + i0 + 32 * u, i0 + 32 * u, e[u]);
+        }
+    };
     if (in_regs) {
         uint32_t taken = 0;         // tokens of the warp with a valid expert
-        // token of pair i: i / K for i < 256, as a product (sixteen divisions a lane were a fifth of this kernel's issue slots)
-        const uint32_t inv_k = 65536u / static_cast<uint32_t>(K) + 1u;
-        auto token_of = [&](int i) { return (static_cast<uint32_t>(i) * inv_k) >> 16; };
 #pragma unroll
         for (int i = 0; i < kPlanRegTopk; ++i)
             if (e_reg[i] >= 0) {
@@ -113,40 +127,23 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
     } else {
         // any number of batches per warp, any top-k: relative positions go to global memory and are completed below
         for (int base = a; base < b; base += 32) {
-            const int t = base + lane;
-            bool any = false;
-            if (t < b) {
-                for (int k = 0; k < K; ++k) {
-                    const int e = load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + k, E);
-                    if (e >= 0) {
-                        atomicOr(mask_of + e, 1u << lane);
-                        any = true;
-                    }
-                }
-            }
+            uint32_t taken = 0;
+            walk_pairs(base, [&](int64_t, int i, int e) {
+                if (e < 0) return;
+                const uint32_t bit = 1u << token_of(i);
+                atomicOr(mask_of + e, bit);
+                taken |= bit;
+            });
             __syncwarp();
-            const uint32_t bal = __ballot_sync(0xffffffffu, any);
-            if (t < b) {
-                p.token_slot[t] = any ? tokens_before + __popc(bal & lanemask_lt()) : -1;
-                for (int k = 0; k < K; ++k) {
-                    const int64_t i = static_cast<int64_t>(t) * K + k;
-                    const int e = load_topk_idx(p.topk_idx, p.idx32 != 0, i, E);
-                    p.pair_row[i] = e >= 0 ? mine[e] + __popc(mask_of[e] & lanemask_lt()) : -1;
-                }
-            }
-            tokens_before += __popc(bal);
+            taken = __reduce_or_sync(0xffffffffu, taken);
+            if (base + lane < b) p.token_slot[base + lane] = (taken >> lane) & 1u ? tokens_before + __popc(taken & lanemask_lt()) : -1;
+            tokens_before += __popc(taken);
+            walk_pairs(base, [&](int64_t at, int i, int e) { p.pair_row[at] = e >= 0 ? mine[e] + __popc(mask_of[e] & ((1u << token_of(i)) - 1u)) : -1; });
             __syncwarp();
-            if (t < b) {
-                for (int k = 0; k < K; ++k) {
-                    const int e = load_topk_idx(p.topk_idx, p.idx32 != 0, static_cast<int64_t>(t) * K + k, E);
-                    if (e < 0) continue;
-                    const uint32_t m = mask_of[e];
-                    if (m != 0 && (m & lanemask_lt()) == 0) {
-                        mine[e] += __popc(m);
-                        mask_of[e] = 0;
-                    }
-                }
-            }
+            walk_pairs(base, [&](int64_t, int i, int e) {       // the first token of a mask adds the count and clears it
+                const uint32_t m = e >= 0 ? mask_of[e] : 0u;
+                if (m != 0 && (m & ((1u << token_of(i)) - 1u)) == 0 && atomicExch(mask_of + e, 0u) != 0) mine[e] += __popc(m);
+            });
             __syncwarp();
         }
     }
@@ -234,13 +231,11 @@ __global__ void __launch_bounds__(kPlanThreads, 1) local_plan_kernel(const __gri
             if (i < K && lane + 32 * i < pairs)
                 p.pair_row[static_cast<int64_t>(a) * K + lane + 32 * i] = e_reg[i] < 0 ? -1 : s_base[e_reg[i]] + mine[e_reg[i]] + pos_reg[i];
     } else {
-        for (int t = a + lane; t < b; t += 32) {        // (every lane wrote the positions of the same tokens itself)
-            if (p.token_slot[t] >= 0) p.token_slot[t] += slot_base;
-            for (int k = 0; k < K; ++k) {
-                const int64_t i = static_cast<int64_t>(t) * K + k;
-                const int e = load_topk_idx(p.topk_idx, p.idx32 != 0, i, E);
-                if (e >= 0) p.pair_row[i] += s_base[e] + mine[e];
-            }
+        for (int base = a; base < b; base += 32) {      // (every lane completes what it wrote itself)
+            if (base + lane < b && p.token_slot[base + lane] >= 0) p.token_slot[base + lane] += slot_base;
+            walk_pairs(base, [&](int64_t at, int, int e) {
+                if (e >= 0) p.pair_row[at] += s_base[e] + mine[e];
+            });
         }
     }
     if (cta == 0 && tid < 7) p.stamps[1 + tid] = globaltimer_ns();

@@ -21,6 +21,8 @@ def _buffer(T, H, K, **kw):
     (1025, 256, 256, 8),     # two planning blocks, the second with one token more than the first leaves
     (8300, 128, 64, 2),      # more than one batch of 32 tokens per warp
     (70, 512, 32, 9),        # more top-k lanes than a planning lane keeps in registers
+    (1100, 128, 64, 32),     # the largest top-k, two planning blocks
+    (9000, 128, 40, 17),     # an odd large top-k and two batches per warp
 ])
 @pytest.mark.parametrize('expand', [False, True])
 @pytest.mark.parametrize('mode', ['bf16', 'fused', 'fused_col_major', 'prequantised'])
