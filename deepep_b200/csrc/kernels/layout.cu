@@ -3,7 +3,8 @@
 //
 // Parity: csrc/kernels/legacy/layout.cu:10-122 (get_dispatch_layout) of the reference,
 // which splits experts and ranks over separate SM groups; here every block histograms its
-// own slice of tokens in shared memory and merges with one atomic per non-zero bin.
+// own slice of tokens in shared memory and merges with one atomic per non-zero bin (into the first block of a cluster, or
+// into global memory).
 #include <cooperative_groups.h>
 
 #include "api.hpp"
@@ -15,18 +16,11 @@ namespace ep {
 namespace {
 
 constexpr int kLayoutThreads = 1024, kLayoutMaxCtas = 8;
+constexpr int kLayoutWideThreads = 256;
 
-// One thread-block cluster counts everything: a histogram per CTA in shared memory, summed into the first CTA's through
-// distributed shared memory. Counting with global atomics wanted two cleared arrays first, i.e. three launches.
-__global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const void* __restrict__ topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks,
-                                                     int num_experts, int* num_tokens_per_rank, int* num_tokens_per_expert,
-                                                     bool* is_token_in_rank) {
-    extern __shared__ int s_hist[];   // [num_experts + num_ranks]
-    int* s_expert = s_hist;
-    int* s_rank = s_hist + num_experts;
-    for (int i = threadIdx.x; i < num_experts + num_ranks; i += blockDim.x) s_hist[i] = 0;
-    auto cluster = cooperative_groups::this_cluster();
-    cluster.sync();                   // every CTA's histogram is cleared, and every CTA is there
+// This block's share of the tokens (grid-strided): histogram in shared memory, one row of the mask per token.
+__device__ __forceinline__ void count_tokens(const void* __restrict__ topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks, int num_experts,
+                                             int* s_expert, int* s_rank, bool* is_token_in_rank) {
     const int experts_per_rank = num_experts / num_ranks;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < num_tokens; t += gridDim.x * blockDim.x) {
         uint32_t mask = 0;
@@ -43,6 +37,20 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const void* __re
             if (in) atomicAdd(s_rank + r, 1);
         }
     }
+}
+
+// One thread-block cluster counts everything: a histogram per CTA in shared memory, summed into the first CTA's through
+// distributed shared memory. Counting with global atomics wants two cleared arrays first, i.e. three launches.
+__global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const void* __restrict__ topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks,
+                                                     int num_experts, int* num_tokens_per_rank, int* num_tokens_per_expert,
+                                                     bool* is_token_in_rank) {
+    extern __shared__ int s_hist[];   // [num_experts + num_ranks]
+    int* s_expert = s_hist;
+    int* s_rank = s_hist + num_experts;
+    for (int i = threadIdx.x; i < num_experts + num_ranks; i += blockDim.x) s_hist[i] = 0;
+    auto cluster = cooperative_groups::this_cluster();
+    cluster.sync();                   // every CTA's histogram is cleared, and every CTA is there
+    count_tokens(topk_idx, idx32, num_tokens, num_topk, num_ranks, num_experts, s_expert, s_rank, is_token_in_rank);
     __syncthreads();
     if (blockIdx.x != 0) {
         int* first = cluster.map_shared_rank(s_hist, 0);
@@ -54,6 +62,23 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(const void* __re
         for (int i = threadIdx.x; i < num_experts; i += blockDim.x) num_tokens_per_expert[i] = s_expert[i];
         for (int i = threadIdx.x; i < num_ranks; i += blockDim.x) num_tokens_per_rank[i] = s_rank[i];
     }
+}
+
+// The same on all SMs, added up in global memory (cleared before).
+__global__ void __launch_bounds__(kLayoutWideThreads) layout_wide_kernel(const void* __restrict__ topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks,
+                                                                         int num_experts, int* num_tokens_per_rank, int* num_tokens_per_expert,
+                                                                         bool* is_token_in_rank) {
+    extern __shared__ int s_hist[];
+    int* s_expert = s_hist;
+    int* s_rank = s_hist + num_experts;
+    for (int i = threadIdx.x; i < num_experts + num_ranks; i += blockDim.x) s_hist[i] = 0;
+    __syncthreads();
+    count_tokens(topk_idx, idx32, num_tokens, num_topk, num_ranks, num_experts, s_expert, s_rank, is_token_in_rank);
+    __syncthreads();
+    for (int i = threadIdx.x; i < num_experts; i += blockDim.x)
+        if (s_expert[i] != 0) atomicAdd(num_tokens_per_expert + i, s_expert[i]);
+    for (int i = threadIdx.x; i < num_ranks; i += blockDim.x)
+        if (s_rank[i] != 0) atomicAdd(num_tokens_per_rank + i, s_rank[i]);
 }
 
 // A thousand small words: one launch instead of the ten elementwise launches that the same takes in PyTorch.
@@ -89,12 +114,26 @@ __global__ void __launch_bounds__(256) legacy_handle_kernel(const int* __restric
 cudaError_t launch_dispatch_layout(const void* topk_idx, bool idx32, int num_tokens, int num_topk, int num_ranks, int num_experts,
                                    int* num_tokens_per_rank, int* num_tokens_per_expert, bool* is_token_in_rank,
                                    cudaStream_t stream) {
+    // Up to 64k pairs one cluster is the shorter way (one launch; 8.4 us for 8192 x 8), above that its eight SMs are the longer
+    // one (16384 x 8: 10.4 us, 8192 x 16: 14.4, 32768 x 8: 16.2, 131072 x 8: 47; on all SMs 32768 x 8 takes 9.2 us with the two
+    // memsets, 131072 x 8 13.5).
+    const size_t smem_bytes = static_cast<size_t>(num_experts + num_ranks) * sizeof(int);
+    if (static_cast<int64_t>(num_tokens) * num_topk > (1 << 16)) {
+        cudaError_t err = cudaMemsetAsync(num_tokens_per_rank, 0, sizeof(int) * num_ranks, stream);
+        if (err != cudaSuccess) return err;
+        err = cudaMemsetAsync(num_tokens_per_expert, 0, sizeof(int) * num_experts, stream);
+        if (err != cudaSuccess) return err;
+        const int blocks = ceil_div(num_tokens, kLayoutWideThreads);
+        layout_wide_kernel<<<blocks < 148 ? blocks : 148, kLayoutWideThreads, smem_bytes, stream>>>(
+            topk_idx, idx32, num_tokens, num_topk, num_ranks, num_experts, num_tokens_per_rank, num_tokens_per_expert, is_token_in_rank);
+        return cudaGetLastError();
+    }
     int ctas = 1;
     while (ctas < kLayoutMaxCtas && ctas * kLayoutThreads < num_tokens) ctas *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(kLayoutThreads);
-    cfg.dynamicSmemBytes = static_cast<size_t>(num_experts + num_ranks) * sizeof(int);
+    cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

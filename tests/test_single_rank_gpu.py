@@ -330,3 +330,19 @@ def test_calls_refuse_to_run_under_filled_uninitialised_memory():
         torch.use_deterministic_algorithms(False)
     buf.destroy()
     old.destroy()
+
+
+@pytest.mark.parametrize('T,K', [(0, 2), (1, 8), (1025, 3), (8192, 8), (8193, 8), (65536, 1), (65537, 1), (5000, 32)])
+def test_layout_query_on_both_sides_of_its_line(T, K):
+    """One cluster up to 64k pairs, all SMs above."""
+    import deepep_b200
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    E = 96
+    buf = deepep_b200.Buffer(SingleProcessGroup(), num_nvl_bytes=1 << 24, num_gpu_timeout_secs=5)
+    g = torch.Generator(device='cuda').manual_seed(T)
+    idx = torch.randint(-1, E, (T, K), device='cuda', generator=g)
+    for dtype in (torch.int64, torch.int32):
+        per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx.to(dtype), E)
+        assert torch.equal(per_expert.long(), torch.bincount(idx[idx >= 0], minlength=E))
+        assert torch.equal(in_rank[:, 0], (idx >= 0).any(dim=1)) and per_rank.item() == int(in_rank.sum())
+    buf.destroy()
