@@ -93,14 +93,21 @@ __global__ void __launch_bounds__(256) router_weights_kernel(const float* __rest
 }
 
 // ---------------------------------------------------------------- streaming kernels
-// One warp per (row, 512 channels) and nothing else, sixteen channels per lane: neighbouring warps have neighbouring bytes,
-// and a grid of many short blocks streams faster than a resident grid that loops over the same work (cast of 8192 x 7168:
-// 29 against 31-34 us). All of them are bound by HBM once the arithmetic per channel is short enough to hide.
-constexpr int kSpan = 512;
+// One piece of sixteen channels per lane and nothing else: neighbouring lanes have neighbouring pieces, and a grid of many
+// short blocks streams faster than a resident grid that loops over the same work (cast of 8192 x 7168: 29 against 31-34 us).
+// All of them are bound by HBM once the arithmetic per channel is short enough to hide. The pieces are numbered through the
+// whole tensor: with a warp per (row, 512 channels) narrow rows left most lanes without work (SwiGLU of 200000 x 8 took 66
+// us, the cast of 300000 x 128 58). Widths of casts are multiples of 128, so the eight lanes of a scale group are one row's.
+constexpr int kPiece = 16, kSpan = 512;
 
 struct RowCol {
     int row, ch;        // first channel of this lane
 };
+__device__ __forceinline__ RowCol row_piece(int pieces) {       // pieces of a row; the last rows' warps may reach past the tensor
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, row = i / static_cast<uint32_t>(pieces);
+    return {static_cast<int>(row), static_cast<int>(i - row * static_cast<uint32_t>(pieces)) * kPiece};
+}
+// A warp per (row, 512 channels), for kernels whose lanes work on a row together.
 __device__ __forceinline__ RowCol row_col(int columns) {
     const uint32_t w = blockIdx.x * (blockDim.x >> 5) + warp_id();
     const uint32_t row = w / static_cast<uint32_t>(columns);
@@ -162,8 +169,8 @@ __global__ void __launch_bounds__(256) router_backward_kernel(const int64_t* __r
     }
 }
 
-// Is the row in an alignment gap of the expanded layout (behind the rows of its expert)? Warp-collective, the same row on
-// every lane: the row belongs to the first group whose aligned end lies behind it.
+// Is the row in an alignment gap of the expanded layout (behind the rows of its expert)? The row belongs to the first group
+// whose aligned end lies behind it. Warp-collective, the same row on every lane:
 __device__ __forceinline__ bool in_gap(const RowGroups& g, int row) {
     if (g.ends == nullptr) return false;
     for (int base = 0; base < g.num; base += 32) {
@@ -176,6 +183,18 @@ __device__ __forceinline__ bool in_gap(const RowGroups& g, int row) {
         }
     }
     return true;
+}
+// ... and any row on any lane of a whole warp.
+__device__ __forceinline__ bool in_gap_of_lane(const RowGroups& g, int row) {
+    if (g.ends == nullptr) return false;
+    if (__all_sync(0xffffffffu, row == __shfl_sync(0xffffffffu, row, 0))) return in_gap(g, row);
+    int lo = 0, hi = g.num;
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (align_up(g.ends[mid], g.alignment) > row) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo == g.num || row >= g.ends[lo];
 }
 
 // 1 / (1 + e^-x) with the hardware's exponential and reciprocal (a few units in the last place of fp32, where the results
@@ -247,37 +266,36 @@ __global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* 
 }
 
 // ---------------------------------------------------------------- 1x128 quantisation
-__global__ void __launch_bounds__(256) quant_kernel(const uint8_t* __restrict__ x, int64_t x_stride_bytes, int rows, int hidden, int columns, int wide, int pow2,
+__global__ void __launch_bounds__(256) quant_kernel(const uint8_t* __restrict__ x, int64_t x_stride_bytes, int rows, int hidden, int wide, int pow2,
                                                     uint8_t* __restrict__ out, float* __restrict__ scales, int64_t sf_row_stride,
                                                     int64_t sf_col_stride) {
     launch_dependents();
     dependency_wait();
-    const RowCol rc = row_col(columns);
-    if (rc.row >= rows) return;
+    const RowCol rc = row_piece(hidden / kPiece);
+    const bool in = rc.row < rows;
     int4 lo, hi;
-    load_32(x + rc.row * x_stride_bytes + rc.ch * 2, (hidden - rc.ch) * 2, wide != 0, lo, hi);
+    load_32(x + rc.row * x_stride_bytes + rc.ch * 2, in ? kPiece * 2 : 0, wide != 0, lo, hi);
     float scale;
     const int4 q = cast16_e4m3(lo, hi, pow2 != 0, scale);       // hidden % 128 == 0: a scale group is all in or all out
-    if (rc.ch < hidden) {
+    if (in) {
         st_na_int4(out + static_cast<int64_t>(rc.row) * hidden + rc.ch, q);
         if ((lane_id() & 7) == 0) scales[rc.row * sf_row_stride + (rc.ch >> 7) * sf_col_stride] = scale;
     }
 }
 
 __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scales, int64_t sf_row_stride,
-                                                      int64_t sf_col_stride, int rows, int hidden, int columns, int wide, const RowGroups groups, uint8_t* __restrict__ out) {
+                                                      int64_t sf_col_stride, int rows, int hidden, int wide, const RowGroups groups, uint8_t* __restrict__ out) {
     launch_dependents();
     dependency_wait();
-    const RowCol rc = row_col(columns);
-    if (rc.row >= rows) return;
-    const bool in = rc.ch < hidden;
+    const RowCol rc = row_piece(hidden / kPiece);
+    const bool in = rc.row < rows;
     int4 raw = make_int4(0, 0, 0, 0);
     float s = 0.f;
     if (in) {
         raw = ld_nc_int4(q + static_cast<int64_t>(rc.row) * hidden + rc.ch);
         s = scales[rc.row * sf_row_stride + (rc.ch >> 7) * sf_col_stride];
     }
-    const bool gap = in_gap(groups, rc.row);
+    const bool gap = in_gap_of_lane(groups, rc.row);
     const __nv_fp8x2_storage_t* p2 = reinterpret_cast<const __nv_fp8x2_storage_t*>(&raw);
     float f[16];
 #pragma unroll
@@ -289,26 +307,27 @@ __global__ void __launch_bounds__(256) dequant_kernel(const uint8_t* __restrict_
     }
     int4 lo, hi;
     pack16(f, lo, hi);
-    store_32(out + (static_cast<int64_t>(rc.row) * hidden + rc.ch) * 2, (hidden - rc.ch) * 2, wide != 0, lo, hi);
+    store_32(out + (static_cast<int64_t>(rc.row) * hidden + rc.ch) * 2, in ? kPiece * 2 : 0, wide != 0, lo, hi);
 }
 
 // ---------------------------------------------------------------- SwiGLU: out = silu(gate) * up (* row weight), optional fused 1x128 cast
 // Rows in alignment gaps are left alone (a decode batch over 32 experts has 4096 rows, of which 512 mean something).
 template <bool kQuant>
-__global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__ x, int rows, int inter, int columns, int wide, const float* __restrict__ row_weight,
+__global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__ x, int rows, int inter, int wide, const float* __restrict__ row_weight,
                                                      const int* __restrict__ num_valid_rows, const RowGroups groups, uint8_t* __restrict__ out,
                                                      float* __restrict__ scales, int64_t sf_row_stride, int64_t sf_col_stride, int pow2) {
     launch_dependents();
     dependency_wait();
-    const RowCol rc = row_col(columns);
-    if (rc.row >= (num_valid_rows != nullptr ? min(*num_valid_rows, rows) : rows)) return;
-    if (in_gap(groups, rc.row)) return;
-    const int left = (inter - rc.ch) * 2;
+    const RowCol rc = row_piece(ceil_div(inter, kPiece));
+    const bool gap = in_gap_of_lane(groups, rc.row);
+    const bool in = !gap && rc.row < (num_valid_rows != nullptr ? min(*num_valid_rows, rows) : rows);
+    if (!__any_sync(0xffffffffu, in)) return;
+    const int left = in ? (inter - rc.ch) * 2 : 0;
     const uint8_t* src = x + (static_cast<int64_t>(rc.row) * 2 * inter + rc.ch) * 2;
     int4 glo, ghi, ulo, uhi;
     load_32(src, left, wide != 0, glo, ghi);
     load_32(src + static_cast<int64_t>(inter) * 2, left, wide != 0, ulo, uhi);
-    const float wr = row_weight != nullptr ? row_weight[rc.row] : 1.f;
+    const float wr = row_weight != nullptr && in ? row_weight[rc.row] : 1.f;
     float g[16], u[16];
     unpack16(glo, ghi, g);
     unpack16(ulo, uhi, u);
@@ -333,12 +352,12 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const uint8_t* __restrict__
 // row's gate weight. One block per row, so that the two by-products of the MoE backward pass come out of the same read of
 // (gate, up, dout): the weighted activation silu(gate) * up * w (the operand of the W2 weight gradient) and the gradient
 // of the gate weight, sum_i dout_i * silu(gate_i) * up_i (a row dot product). Rows in alignment gaps give zeros.
-__global__ void __launch_bounds__(128) swiglu_bwd_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ dout, int inter, int wide,
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const uint8_t* __restrict__ x, const uint8_t* __restrict__ dout, int inter, int wide,
                                                          const float* __restrict__ row_weight, const RowGroups groups, uint8_t* __restrict__ dx,
                                                          uint8_t* __restrict__ act_out, float* __restrict__ dweight) {
     launch_dependents();
     dependency_wait();
-    __shared__ float s_part[4];
+    __shared__ float s_part[8];
     const int row = blockIdx.x;
     const bool gap = in_gap(groups, row);
     const float wr = row_weight != nullptr && !gap ? row_weight[row] : 1.f;
@@ -447,10 +466,10 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __nv_bfloat16* __r
     }
 }
 
-// blocks of eight warps for one warp per (row, kSpan channels); 0 = too many for one grid
-int span_blocks(int rows, int columns) {
-    const int64_t warps = static_cast<int64_t>(rows) * columns;
-    return warps < (1ll << 32) - 8 ? static_cast<int>((warps + 7) / 8) : 0;
+// blocks of 256 threads for one thread per piece; 0 = too many to be numbered
+int piece_blocks(int rows, int width) {
+    const int64_t pieces = static_cast<int64_t>(rows) * ceil_div(width, kPiece);
+    return pieces < (1ll << 32) - 256 ? static_cast<int>((pieces + 255) / 256) : 0;
 }
 int is_wide(std::initializer_list<uint64_t> parts) {
     uint64_t bits = 0;
@@ -506,9 +525,9 @@ cudaError_t quant_weights_128x128(const void* w, int groups, int rows, int cols,
 cudaError_t quant_1x128(const void* x, int64_t x_stride_bytes, int rows, int hidden, bool pow2, void* out, float* scales,
                         int64_t sf_row_stride, int64_t sf_col_stride, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
-    const int columns = ceil_div(hidden, kSpan), blocks = span_blocks(rows, columns);
+    const int blocks = piece_blocks(rows, hidden);
     if (hidden % 128 != 0 || blocks == 0) return cudaErrorInvalidValue;
-    return launch_early(quant_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), x_stride_bytes, rows, hidden, columns,
+    return launch_early(quant_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), x_stride_bytes, rows, hidden,
                                              is_wide({addr(x), static_cast<uint64_t>(x_stride_bytes)}), pow2, static_cast<uint8_t*>(out), scales,
                                              sf_row_stride, sf_col_stride);
 }
@@ -516,23 +535,23 @@ cudaError_t quant_1x128(const void* x, int64_t x_stride_bytes, int rows, int hid
 cudaError_t dequant_1x128(const void* q, const float* scales, int64_t sf_row_stride, int64_t sf_col_stride, int rows, int hidden,
                           const RowGroups& groups, void* out, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
-    const int columns = ceil_div(hidden, kSpan), blocks = span_blocks(rows, columns);
+    const int blocks = piece_blocks(rows, hidden);
     if (hidden % 128 != 0 || blocks == 0) return cudaErrorInvalidValue;
-    return launch_early(dequant_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(q), scales, sf_row_stride, sf_col_stride, rows, hidden, columns,
+    return launch_early(dequant_kernel, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(q), scales, sf_row_stride, sf_col_stride, rows, hidden,
                                                is_wide({addr(out)}), groups, static_cast<uint8_t*>(out));
 }
 
 cudaError_t swiglu(const void* x, int rows, int inter, const float* row_weight, const int* num_valid_rows, const RowGroups& groups, void* out, bool quant,
                    float* scales, int64_t sf_row_stride, int64_t sf_col_stride, bool pow2, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
-    const int columns = ceil_div(inter, kSpan), blocks = span_blocks(rows, columns);
+    const int blocks = piece_blocks(rows, inter);
     if (inter % 8 != 0 || (quant && inter % 128 != 0) || blocks == 0) return cudaErrorInvalidValue;
     const int wide = is_wide({addr(x), addr(out), static_cast<uint64_t>(inter) * 2});
     if (quant)
-        return launch_early(swiglu_kernel<true>, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
+        return launch_early(swiglu_kernel<true>, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), rows, inter, wide, row_weight, num_valid_rows, groups,
                                                         static_cast<uint8_t*>(out), scales, sf_row_stride, sf_col_stride, pow2 ? 1 : 0);
     else
-        return launch_early(swiglu_kernel<false>, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), rows, inter, columns, wide, row_weight, num_valid_rows, groups,
+        return launch_early(swiglu_kernel<false>, dim3(blocks), dim3(256), 0, stream, static_cast<const uint8_t*>(x), rows, inter, wide, row_weight, num_valid_rows, groups,
                                                          static_cast<uint8_t*>(out), nullptr, 0, 0, 0);
 }
 
@@ -540,7 +559,9 @@ cudaError_t swiglu_backward(const void* x, const void* dout, int rows, int inter
                             float* dweight, cudaStream_t stream) {
     if (rows == 0) return cudaSuccess;
     if (inter % 8 != 0) return cudaErrorInvalidValue;
-    const int threads = std::min(128, align_up(ceil_div(inter, 16), 32));
+    // (more than 128 threads lengthen the blocks' ends; where the rows alone do not fill the GPU they shorten the rows: 8 x 16384
+    // 11.4 us with 128)
+    const int threads = std::min(rows < 296 ? 256 : 128, align_up(ceil_div(inter, 16), 32));
     const int wide = is_wide({addr(x), addr(dout), addr(dx), addr(act_out), static_cast<uint64_t>(inter) * 2});
     return launch_early(swiglu_bwd_kernel, dim3(rows), dim3(threads), 0, stream, static_cast<const uint8_t*>(x), static_cast<const uint8_t*>(dout), inter, wide, row_weight, groups,
                                                     static_cast<uint8_t*>(dx), static_cast<uint8_t*>(act_out), dweight);

@@ -95,7 +95,8 @@ def test_transpose_interior_edge_and_unaligned(rows, cols):
         assert torch.equal(C.transpose_bf16(v), v.t().contiguous())
 
 
-@pytest.mark.parametrize('I', [24, 384, 640])       # one lane with half its channels, a partial column, a column and a quarter
+# rows of half a piece, of two pieces (the last one half), of four and eight: many rows in a warp; more than a warp, not whole warps
+@pytest.mark.parametrize('I', [8, 24, 64, 128, 384, 640])
 def test_streaming_ops_skip_or_zero_alignment_gaps(I):
     """Rows of the expanded layout behind their expert's end: the forward kernel leaves them alone, the backward kernels
     write zeros there, whatever the inputs hold in them."""
@@ -156,3 +157,38 @@ def test_inputs_that_start_anywhere(offset):
     assert torch.equal(layer(x), y)
     torch.cuda.synchronize()
     buf.destroy()
+
+
+@pytest.mark.parametrize('M,I', [(1, 8), (37, 8), (333, 128), (100, 384), (7, 16384)])
+def test_streaming_ops_on_narrow_and_long_rows(M, I):
+    """Rows that share a warp, and rows that a block of twice the threads walks; row counts that leave lanes without work."""
+    from deepep_b200 import ops
+    from deepep_b200.utils.math import per_token_cast_back, per_token_cast_to_fp8
+    import deepep_b200
+    g = torch.Generator(device='cuda').manual_seed(M + I)
+    x = torch.randn((M, 2 * I), device='cuda', generator=g).bfloat16()
+    rw = torch.rand((M,), device='cuda', generator=g)
+    dout = torch.randn((M, I), device='cuda', generator=g).bfloat16()
+    xf, wf = x.double().requires_grad_(True), rw.double().requires_grad_(True)
+    ref = torch.nn.functional.silu(xf[:, :I]) * xf[:, I:] * wf[:, None]
+    ref.backward(dout.double())
+    half = max(1, M // 2)
+    out, _ = ops.swiglu(x, rw)
+    part, _ = ops.swiglu(x, rw, num_valid_rows=torch.tensor([half], dtype=torch.int32, device='cuda'))
+    assert torch.equal(part[:half], out[:half])
+    # one bf16 rounding (2^-9 of a value) and a few fp32 ones
+    assert ((out.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-30).all()
+    dx, act, dw = deepep_b200._C.swiglu_backward(x, dout, rw, True)
+    assert ((dx.double() - xf.grad).abs() <= 2 ** -7 * xf.grad.abs() + 1e-4).all()
+    assert ((act.double() - ref).abs() <= 2 ** -7 * ref.abs() + 1e-30).all()
+    # the activation that the gradient of the weight sees is rounded to bf16: 2^-9 of every term
+    terms = (dout.double() * ref.detach() / wf[:, None].detach()).abs().sum(dim=1)
+    assert ((dw.double() - wf.grad).abs() <= 2 ** -8 * terms + 1e-6).all()
+    if I % 128 == 0:
+        q, sf = ops.swiglu(x, rw, quant=True)
+        rq, rsf = per_token_cast_to_fp8(out)
+        assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(sf, rsf)
+        q, sf = ops.quant_1x128(x)
+        rq, rsf = per_token_cast_to_fp8(x)
+        assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(sf, rsf)
+        assert torch.equal(ops.dequant_1x128(q, sf), per_token_cast_back(rq, rsf))
