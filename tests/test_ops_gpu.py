@@ -192,3 +192,24 @@ def test_streaming_ops_on_narrow_and_long_rows(M, I):
         rq, rsf = per_token_cast_to_fp8(x)
         assert torch.equal(q.view(torch.uint8), rq.view(torch.uint8)) and torch.equal(sf, rsf)
         assert torch.equal(ops.dequant_1x128(q, sf), per_token_cast_back(rq, rsf))
+
+
+def test_swiglu_far_from_zero():
+    """Gates whose sigmoid is about 1e-38, infinities and NaN: as the formula in fp32 gives them, also beside ordinary values."""
+    from deepep_b200 import ops
+    gates = torch.tensor([float('-inf'), float('inf'), float('nan'), -87.0, -87.5, -88.0, -88.5, 87.5, 100.0, 3e38, 0.0, -0.0, 1e-38, 5.0, -86.5, -1.0], device='cuda').bfloat16()
+    up = torch.full((16,), 2.0 ** 60, device='cuda').bfloat16()
+    up[9] = 0.5
+    x = torch.cat([gates, up]).view(1, 32)
+    gf, uf = gates.double(), up.double()
+    s = torch.sigmoid(gf)
+    ref, out = gf * s * uf, ops.swiglu(x)[0][0].double()
+    dx = ops.swiglu_backward(x, torch.ones((1, 16), device='cuda').bfloat16())[0].double()
+    dg, du = uf * s * (1 + gf * (1 - s)), gf * s
+    tiny = 2.0 ** -126                                   # the smallest normal fp32 number: fewer bits are left below it
+    for got, want in ((out, ref), (dx[:16], dg), (dx[16:], du)):
+        ok = want.isfinite()
+        # the exponential's error grows with its argument: 88 * 2^-23 of the result, then bf16 roundings; a sigmoid below the normal range
+        # has an error of up to 2^-149 itself, times the factors behind it
+        assert ((got[ok] - want[ok]).abs() <= 2 ** -7 * want[ok].abs() + tiny).all()
+        assert (got[want.isnan()].isnan()).all()
