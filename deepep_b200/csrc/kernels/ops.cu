@@ -231,29 +231,36 @@ __device__ __forceinline__ void pack16(const float (&f)[16], int4& lo, int4& hi)
 
 // ---------------------------------------------------------------- 128x128 weight quantisation: one block per weight block
 // The arithmetic is that of the elementwise definition (scale = max(amax, 1e-4) / 448, correctly rounded divisions); the block
-// is read once and held in registers between the two passes, instead of five passes over fp32 copies of the weights.
+// is read once and held in registers between the two passes, instead of five passes over fp32 copies of the weights. A NaN
+// anywhere in the block is its maximum, so that the whole block becomes NaN: weights that have gone wrong stay visible.
+__device__ __forceinline__ uint32_t magnitude_bits(const int4& raw) {      // of the largest magnitude; NaN above infinity
+    auto mag = [](int w) { return static_cast<uint32_t>(w) & 0x7fff7fffu; };
+    const uint32_t m = __vmaxu2(__vmaxu2(mag(raw.x), mag(raw.y)), __vmaxu2(mag(raw.z), mag(raw.w)));
+    return max(m >> 16, m & 0xffffu);
+}
 __global__ void __launch_bounds__(256) weight_quant_kernel(const __nv_bfloat16* __restrict__ w, int rows, int cols, int pow2, uint8_t* __restrict__ q,
                                                            float* __restrict__ scales) {
     launch_dependents();
     dependency_wait();
-    __shared__ float s_max[8];
+    __shared__ uint32_t s_max[8];
     const int64_t base = (static_cast<int64_t>(blockIdx.z) * rows + blockIdx.y * 128) * cols + blockIdx.x * 128;
     const int r0 = threadIdx.x >> 3, c = (threadIdx.x & 7) * 16;        // 32 rows per pass, 16 channels per thread
     int4 lo[4], hi[4];
-    float amax = 0.f;
+    uint32_t bits = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const uint8_t* src = reinterpret_cast<const uint8_t*>(w + base + static_cast<int64_t>(r0 + 32 * i) * cols + c);
         lo[i] = ld_nc_int4(src);
         hi[i] = ld_nc_int4(src + 16);
-        amax = fmaxf(amax, fmaxf(amax_bf16x8(lo[i]), amax_bf16x8(hi[i])));
+        bits = max(bits, max(magnitude_bits(lo[i]), magnitude_bits(hi[i])));
     }
-    amax = warp_reduce_max_width(amax, 32);
-    if (lane_id() == 0) s_max[warp_id()] = amax;
+    bits = __reduce_max_sync(0xffffffffu, bits);
+    if (lane_id() == 0) s_max[warp_id()] = bits;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, s_max[i]);
-    float scale = __fdiv_rn(fmaxf(amax, 1e-4f), 448.f);
+    for (int i = 0; i < 8; ++i) bits = max(bits, s_max[i]);
+    const float amax = __uint_as_float(bits << 16);
+    float scale = __fdiv_rn(amax < 1e-4f ? 1e-4f : amax, 448.f);
     if (pow2) scale = exp2f(ceilf(log2f(scale)));
     if (threadIdx.x == 0) scales[(static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = scale;
     const float inv = pow2 ? 1.f / scale : 0.f;                         // exact for a power of two

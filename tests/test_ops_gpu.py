@@ -213,3 +213,18 @@ def test_swiglu_far_from_zero():
         # has an error of up to 2^-149 itself, times the factors behind it
         assert ((got[ok] - want[ok]).abs() <= 2 ** -7 * want[ok].abs() + tiny).all()
         assert (got[want.isnan()].isnan()).all()
+
+
+@pytest.mark.parametrize('pow2', [False, True])
+def test_weight_quantisation_of_blocks_that_are_not_finite(pow2):
+    """A NaN makes its whole 128 x 128 block NaN, an infinity leaves zeros beside a NaN, as the elementwise definition has it;
+    an all-zero block and one of the smallest values keep the floor of the scale."""
+    from deepep_b200.models.moe import quantize_weight_128x128
+    w = (torch.randn((2, 256, 384), device='cuda', generator=torch.Generator(device='cuda').manual_seed(9)) * 0.02).bfloat16()
+    w[0, 5, 7], w[0, 130, 300], w[1, 255, 0], w[1, :128, :128] = float('nan'), float('-inf'), float('-nan'), 0
+    w[1, :128, 128:256] = 1e-30
+    (q, sf), (rq, rsf) = quantize_weight_128x128(w, pow2), quantize_weight_128x128(w.cpu(), pow2)
+    q, rq = q.float().cpu(), rq.float()
+    assert torch.equal(sf.cpu().isnan(), rsf.isnan()) and torch.equal(sf.cpu().nan_to_num(0), rsf.nan_to_num(0))
+    assert torch.equal(q.isnan(), rq.isnan()) and torch.equal(q.nan_to_num(0), rq.nan_to_num(0))
+    assert q[0, :128, :128].isnan().all() and rsf[0, 0, 0].isnan()
