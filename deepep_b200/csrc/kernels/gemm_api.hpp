@@ -22,8 +22,8 @@ struct GemmParams {
     // beyond its end up to the next multiple of 64 must be zero. A group without rows gives zeros.
     int k_grouped;
     int64_t c_group_stride;      // elements between C[g] and C[g + 1]
-    // MN-major operands (bf16): A is given as [K, M], B as [num_groups * K, N] (k_grouped: [K, N]), both row-major. A may only
-    // be MN-major together with B. A plain problem with both may have any K.
+    // MN-major operands (bf16, plain or k_grouped problems): A is given as [K, M], B as [K, N], both row-major. A may only be
+    // MN-major together with B. A plain problem with both may have any K.
     int a_mn, b_mn;
     int c_wide;                  // rows of C start on 32-byte boundaries (filled in by the launcher)
     __nv_bfloat16* C;
@@ -40,7 +40,7 @@ struct GemmParams {
 bool make_kmajor_map(CUtensorMap* map, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t row_stride_bytes,
                      uint32_t box_rows);
 
-// A: [M, K] (MN-major: [K, M]) with row pitch `a_row_stride_bytes`; B: [num_groups * N, K] (MN-major: [num_groups * K, N]) with row pitch `b_row_stride_bytes`;
+// A: [M, K] (MN-major: [K, M]) with row pitch `a_row_stride_bytes`; B: [num_groups * N, K] (MN-major: [K, N]) with row pitch `b_row_stride_bytes`;
 // both bf16 (fp8 = false) or e4m3.
 cudaError_t launch_gemm(const GemmParams& p, const void* a, int64_t a_row_stride_bytes, const void* b, int64_t b_row_stride_bytes,
                         bool fp8, int num_sms, cudaStream_t stream);

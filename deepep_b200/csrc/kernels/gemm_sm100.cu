@@ -201,7 +201,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             bool ok = true;
             for (int ti = blockIdx.x; ok && sched.get(ti, t); ti += gridDim.x) {
                 // (an MN-major B of a plain problem; group g of a grouped one starts at row g * K of the stacked [K, N] matrices)
-                const int b_row = (p.k_grouped || kBMN ? 0 : t.g * p.N) + t.n0, b_k = kBMN && !p.k_grouped ? t.g * p.K : 0;
+                const int b_row = (p.k_grouped || kBMN ? 0 : t.g * p.N) + t.n0;
                 const int boxes = kAMN ? 0 : small_boxes(t.m_end - t.m0);
                 const uint32_t bytes = boxes == 0 ? C::STAGE : boxes * (kSmallBox * 128) + C::B_BYTES;
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
@@ -210,7 +210,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
                     mbar_arrive_expect_tx(full + s, bytes);
                     if constexpr (kAMN) load_operand<kAMN>(sa, &map_a, kb * C::BK, t.m0, BM, full + s);
                     else load_rows(sa, &map_a, &map_a32, boxes, kb * C::BK, t.m0, full + s);
-                    load_operand<kBMN>(sa + C::A_BYTES, &map_b, b_k + kb * C::BK, b_row, BN, full + s);
+                    load_operand<kBMN>(sa + C::A_BYTES, &map_b, kb * C::BK, b_row, BN, full + s);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
             }
@@ -424,14 +424,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             bool ok = true;
             for (int ti = pair; ok && sched.get(ti, t); ti += num_pairs) {
                 const int b_row = (p.k_grouped || kBMN ? 0 : t.g * p.N) + t.n0 + static_cast<int>(cta) * (C::BN / 2);
-                const int b_k = kBMN && !p.k_grouped ? t.g * p.K : 0;
                 for (int kb = t.kb0; kb < t.kb1; ++kb) {
                     if (!(ok = pipe_wait(pc, empty + s, ph ^ 1))) break;
                     uint8_t* sa = smem + s * C::STAGE;
                     if (leader) mbar_arrive_expect_tx(full + s, 2 * C::STAGE);
                     const uint32_t bar = map_to_cta(smem_u32(full + s), 0);
                     load_operand_pair<kAMN>(sa, &map_a, kb * C::BK, t.m0 + static_cast<int>(cta) * BM, BM, bar);
-                    load_operand_pair<kBMN>(sa + C::A_BYTES, &map_b, b_k + kb * C::BK, b_row, C::BN / 2, bar);
+                    load_operand_pair<kBMN>(sa + C::A_BYTES, &map_b, kb * C::BK, b_row, C::BN / 2, bar);
                     if (++s == C::kStages) { s = 0; ph ^= 1; }
                 }
             }
@@ -1389,17 +1388,17 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
     const bool k_tail_ok = p.a_mn && p.b_mn && !p.k_grouped && p.num_groups == 1;     // rows past the end load as zeros
     if (p.N % 128 != 0 || (p.K % bk != 0 && !k_tail_ok) || p.M <= 0) return cudaErrorInvalidValue;
     if (p.k_grouped && (fp8 || p.group_end == nullptr || p.group_alignment % bk != 0)) return cudaErrorInvalidValue;
-    if ((p.a_mn || p.b_mn) && (fp8 || (p.a_mn && !p.b_mn))) return cudaErrorInvalidValue;
+    if ((p.a_mn || p.b_mn) && (fp8 || (p.a_mn && !p.b_mn) || (!p.k_grouped && p.num_groups != 1))) return cudaErrorInvalidValue;
     const uint64_t K = static_cast<uint64_t>(p.K), a_stride = static_cast<uint64_t>(a_row_stride_bytes), b_stride = static_cast<uint64_t>(b_row_stride_bytes);
     const uint64_t b_mats = p.k_grouped ? 1 : static_cast<uint64_t>(p.num_groups);
     // operand maps: K-major [rows, K] in boxes of `box` rows, or MN-major [K, columns] in boxes of 64 x 64
     auto map_of = [&](CUtensorMap* map, const void* base, bool mn, uint64_t rows, uint64_t mats, uint64_t stride, uint32_t box) {
         return mn ? make_kmajor_map(map, base, elem, mats * K, rows, stride, 64) : make_kmajor_map(map, base, elem, mats * rows, K, stride, box);
     };
-    CUtensorMap map_a, map_a32, map_b;
-    if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM) ||
-        !map_of(&map_a32, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, kSmallBox))
-        return cudaErrorInvalidValue;
+    CUtensorMap map_a, map_a32 = {}, map_b;
+    if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM)) return cudaErrorInvalidValue;
+    // (only the kernels of lone CTAs read it, and only for K-major rows: an encoding costs the host a third of a microsecond)
+    auto small_a_map = [&]() { return p.a_mn != 0 || map_of(&map_a32, a, false, static_cast<uint64_t>(p.M), 1, a_stride, kSmallBox); };
     auto map_b_of = [&](uint32_t box) { return map_of(&map_b, b, p.b_mn != 0, static_cast<uint64_t>(p.N), b_mats, b_stride, box); };
     const bool wide = p.N % 256 == 0, pairs = wide && num_sms >= 2;
     const int pair_grid = num_sms & ~1;
@@ -1414,7 +1413,7 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
             if (!map_b_of(128)) return cudaErrorInvalidValue;
             return launch_tiles<gemm_mx_pair_kernel, MxPairCfg>(pair_grid, stream, map_a, map_b, p);
         }
-        if (!map_b_of(256)) return cudaErrorInvalidValue;
+        if (!map_b_of(256) || !small_a_map()) return cudaErrorInvalidValue;
         return launch_tiles<gemm_mx_kernel, MxCfg>(num_sms, stream, map_a, map_b, map_a32, p);
     }
     if (fp8) {
@@ -1423,7 +1422,7 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
         // empty (8 experts of 700 rows, 4096 x 4096: 143 against 168 us; 16 of 20 rows: 100 against 66 us).
         const bool forced = env_is("EP_GEMM_FP8_PAIR", '1'), forbidden = env_is("EP_GEMM_FP8_PAIR", '0');
         const bool use_pair = pairs && !forbidden && (forced || num_waves(p, 256, 256, num_sms / 2) * 1.5f < num_waves(p, 128, 128, num_sms));
-        if (!map_b_of(128)) return cudaErrorInvalidValue;
+        if (!map_b_of(128) || (!use_pair && !small_a_map())) return cudaErrorInvalidValue;
         return use_pair ? launch_tiles<gemm_pair_fp8_kernel, PairFp8Cfg>(pair_grid, stream, map_a, map_b, p)
                         : launch_tiles<gemm_kernel<128, true>, Cfg<128, true>>(num_sms, stream, map_a, map_b, map_a32, p);
     }
@@ -1439,6 +1438,7 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
         return p.b_mn ? launch_tiles<gemm_pair_kernel<false, true>, PairCfg>(pair_grid, stream, map_a, map_b, p)
                       : launch_tiles<gemm_pair_kernel<false, false>, PairCfg>(pair_grid, stream, map_a, map_b, p);
     }
+    if (!small_a_map()) return cudaErrorInvalidValue;
     if (tiles == Tiles::kLone256) {
         if (p.a_mn) return launch_tiles<gemm_kernel<256, false, true, true>, Cfg<256, false>>(num_sms, stream, map_a, map_b, map_a32, p);
         return p.b_mn ? launch_tiles<gemm_kernel<256, false, false, true>, Cfg<256, false>>(num_sms, stream, map_a, map_b, map_a32, p)
