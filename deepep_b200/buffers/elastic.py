@@ -494,7 +494,9 @@ class ElasticBuffer:
         ``zero_copy`` returns ``recv_x`` (and row-major scales) as strided views of the receive region: they stay
         valid until the second next dispatch of any rank of the group, which overwrites that half of the region;
         ``num_worst_tokens`` (with ``do_cpu_sync=False``) sets the row count of the outputs, whose routing rows
-        past the received count are filled with -1 / 0.
+        past the received count are filled with -1 / 0. ``num_sms`` is how many SMs the communication kernels hold while
+        rows travel (0: the SM model's value). A group of one rank has none of these kernels: its rows are moved by short
+        blocks that run wherever the GPU has room, and ``num_sms`` is only noted in the handle.
 
         Returns ``(recv_x | (recv_x, recv_sf), recv_topk_idx, recv_topk_weights, handle, event)``.
         In the expanded layout ``recv_topk_idx`` is ``None`` and ``recv_topk_weights`` is 1-D.
@@ -539,7 +541,7 @@ class ElasticBuffer:
         expanded layout and ``allow_multiple_reduction`` each rank's partial sum is rounded once
         more). ``topk_weights`` are carried back to ``combined_topk_weights``; with ``weighted=True`` (expanded
         layout only) every expanded row is also multiplied by its weight before it is added, i.e. the result is
-        ``sum_k w_k * x_k`` as the low-latency combine computes it.
+        ``sum_k w_k * x_k`` as the low-latency combine computes it. ``num_sms``: as in :meth:`dispatch` (0: the handle's).
 
         Returns ``(combined_x, combined_topk_weights, event)``.
         """

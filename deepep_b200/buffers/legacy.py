@@ -25,8 +25,9 @@ from .elastic import ElasticBuffer, EPHandle
 
 
 class Config:
-    """Tuning knobs of the normal-mode kernels. Only ``num_sms`` has an effect here; the chunk sizes of
-    the reference's queue-based kernels are kept as attributes for compatibility."""
+    """Tuning knobs of the normal-mode kernels. Only ``num_sms`` has an effect here, in groups of more than one rank
+    (:meth:`ElasticBuffer.dispatch`); the chunk sizes of the reference's queue-based kernels are kept as attributes for
+    compatibility."""
 
     def __init__(self, num_sms: int = 24, num_max_nvl_chunked_send_tokens: int = 6, num_max_nvl_chunked_recv_tokens: int = 256,
                  num_max_rdma_chunked_send_tokens: int = 6, num_max_rdma_chunked_recv_tokens: int = 256):
@@ -252,6 +253,8 @@ class Buffer:
         dimensions, ``recv_count [local experts]`` and
         ``handle = (src_info, layout_range, num_max_dispatch_tokens_per_rank, hidden, num_experts)``.
         With ``return_recv_hook`` only the sends are issued; ``hook()`` launches the receive part.
+        ``dispatch_wait_recv_cost_stats`` (int64 ``[ranks]``) is increased by the nanoseconds that this rank has waited for
+        each source's messages; a group of one rank has no messages, nothing is waited for and nothing is added.
         """
         check_torch_deterministic()
         wait_stats = dispatch_wait_recv_cost_stats
@@ -283,7 +286,9 @@ class Buffer:
         ``x`` is ``[local experts, ranks * max tokens, hidden]`` bf16 (with ``zero_copy`` it is the tensor
         from :meth:`get_next_low_latency_combine_buffer`). With ``use_logfmt`` every group of 128 channels whose
         largest magnitude is below 1 travels as 10-bit log-format values (160 instead of 256 bytes), the other
-        groups stay bf16; ``deepep_b200.utils.math.logfmt_roundtrip`` restates the rounding. Returns
+        groups stay bf16; ``deepep_b200.utils.math.logfmt_roundtrip`` restates the rounding.
+        ``combine_wait_recv_cost_stats``: as in :meth:`low_latency_dispatch` (with LogFMT a group of one rank sends messages
+        too). Returns
         ``(combined_x, event, hook)``. Reference: ``deep_ep/buffers/legacy.py:640-700``.
         """
         check_torch_deterministic()

@@ -1397,7 +1397,7 @@ cudaError_t launch_gemm(const GemmParams& params, const void* a, int64_t a_row_s
     };
     CUtensorMap map_a, map_a32 = {}, map_b;
     if (!map_of(&map_a, a, p.a_mn != 0, static_cast<uint64_t>(p.M), 1, a_stride, BM)) return cudaErrorInvalidValue;
-    // (only the kernels of lone CTAs read it, and only for K-major rows: an encoding costs the host a third of a microsecond)
+    // (encoded on the host for every call: only the kernels of lone CTAs read it, and only for K-major rows)
     auto small_a_map = [&]() { return p.a_mn != 0 || map_of(&map_a32, a, false, static_cast<uint64_t>(p.M), 1, a_stride, kSmallBox); };
     auto map_b_of = [&](uint32_t box) { return map_of(&map_b, b, p.b_mn != 0, static_cast<uint64_t>(p.N), b_mats, b_stride, box); };
     const bool wide = p.N % 256 == 0, pairs = wide && num_sms >= 2;

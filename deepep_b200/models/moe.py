@@ -17,8 +17,9 @@ the gradient of the gate weights rides back with the combine. ``FusedMoE`` runs 
 native call per direction (``_LayerFunction``).
 
 The reference library has no model code; this is the "fused MoE layer fwd+bwd" workload that its
-kernels exist to serve. Everything is written over LISTS of ranks so that the single-GPU emulation
-(``LocalCluster``) and the real one-rank-per-process case share one code path.
+kernels exist to serve. ``moe_forward`` and ``moe_backward`` are written over LISTS of ranks, for the single-GPU emulation
+(``LocalCluster``) and for layers put together by hand; the native calls of ``FusedMoE`` (``csrc/runtime/moe_layer.cpp``) take
+the same steps in the same order for the rank of a process and give the same bits.
 """
 from __future__ import annotations
 
@@ -87,7 +88,8 @@ class ExpertWeights:
 
 
 class _SingleRankComm:
-    """Gives one ``ElasticBuffer`` the list interface of ``LocalCluster``."""
+    """Gives one ``ElasticBuffer`` the list interface of ``LocalCluster``: the ``comm`` of ``moe_forward`` and ``moe_backward``
+    for the rank of a process."""
 
     def __init__(self, buffer):
         self.buffers = [buffer]
@@ -220,7 +222,7 @@ class FusedMoE(torch.nn.Module):
         super().__init__()
         require_native()
         self.cfg, self.buffer = cfg, buffer
-        self.comm = _SingleRankComm(buffer)
+        self.comm = _SingleRankComm(buffer)      # for moe_forward / moe_backward with this layer's weights
         el = cfg.num_experts // buffer.num_ranks
         g = torch.Generator(device='cpu').manual_seed(seed + buffer.rank_idx)
         self.router = torch.nn.Parameter((torch.randn((cfg.num_experts, cfg.hidden), generator=g) * 0.02).to(device))

@@ -176,3 +176,30 @@ def test_a_router_that_changes_before_the_backward_pass_is_noticed():
             y.sum().backward()
             assert torch.equal(x.grad, kept)
         buf.destroy()
+
+
+@pytest.mark.parametrize('T,E,K,use_fp8,pow2', [(77, 8, 3, False, False), (1, 4, 1, False, False), (130, 16, 4, True, True), (64, 8, 2, True, False)])
+def test_module_and_list_functions_give_the_same_bits(T, E, K, use_fp8, pow2):
+    """The native calls of the module against moe_forward / moe_backward on the same routing."""
+    import deepep_b200
+    from deepep_b200 import ops
+    from deepep_b200.models.moe import FusedMoE, MoEConfig, moe_backward, moe_forward, route
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    H, I = 512, 256
+    buf = deepep_b200.ElasticBuffer(SingleProcessGroup(), num_max_tokens_per_rank=T, hidden=H, num_topk=K, num_gpu_timeout_secs=5)
+    layer = FusedMoE(buf, MoEConfig(hidden=H, intermediate=I, num_experts=E, num_topk=K, use_fp8=use_fp8, pow2_scales=pow2))
+    g = torch.Generator(device='cuda').manual_seed(T)
+    x = torch.randn((T, H), device='cuda', generator=g).bfloat16().requires_grad_(True)
+    dy = torch.randn((T, H), device='cuda', generator=g).bfloat16()
+    y = layer(x)
+    y.backward(dy)
+    padded = torch.nn.functional.pad(layer.router.detach().bfloat16(), (0, 0, 0, -E % 128))
+    idx, w = route(ops.gemm(x.detach(), padded)[:, :E], K)
+    ys, ctxs = moe_forward(layer.comm, [layer.weights], [x.detach()], [idx], [w], layer.cfg)
+    assert torch.equal(ys[0], y)
+    dx, dw, d13, d2 = (t[0] for t in moe_backward(layer.comm, [layer.weights], ctxs, [dy], layer.cfg))
+    d_router = deepep_b200._C.router_backward(x.detach(), padded, idx, w, dw, E, dx)       # (adds its share to dx)
+    assert torch.equal(d13, layer.w13.grad) and torch.equal(d2, layer.w2.grad)
+    assert torch.equal(dx, x.grad) and torch.equal(d_router.float(), layer.router.grad)
+    buf.check_status()
+    buf.destroy()

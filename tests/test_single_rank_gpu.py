@@ -264,8 +264,6 @@ def test_low_latency_against_the_oracle(T, H, E, K, mode, hook):
                     j = int(((idx[:t] == e).any(dim=1)).sum())
                     ref[t] += w[t, k] * rows[e, j].float()
         for logfmt in (False, True):        # LogFMT takes the message path of the multi-rank kernels, on the same handle
-            if logfmt and H % 128 != 0:
-                continue
             out, _, h = buf.low_latency_combine(rows, idx, w, handle, use_logfmt=logfmt, return_recv_hook=hook)
             if hook:
                 h()
@@ -345,4 +343,25 @@ def test_layout_query_on_both_sides_of_its_line(T, K):
         per_rank, _, per_expert, in_rank, _ = buf.get_dispatch_layout(idx.to(dtype), E)
         assert torch.equal(per_expert.long(), torch.bincount(idx[idx >= 0], minlength=E))
         assert torch.equal(in_rank[:, 0], (idx >= 0).any(dim=1)) and per_rank.item() == int(in_rank.sum())
+    buf.destroy()
+
+
+@pytest.mark.parametrize('hook', [False, True])
+def test_one_rank_waits_for_nobody(hook):
+    """The statistics of the time spent waiting for each source stay as they are."""
+    import deepep_b200
+    from deepep_b200.parallel.local_cluster import SingleProcessGroup
+    T, H, E, K = 16, 512, 8, 2
+    buf = deepep_b200.Buffer(SingleProcessGroup(), num_rdma_bytes=deepep_b200.Buffer.get_low_latency_rdma_size_hint(T, H, 1, E), low_latency_mode=True,
+                             num_gpu_timeout_secs=5)
+    (x,), (idx,), (w,) = make_routed_inputs(1, T, H, E, K, seed=2, device='cuda')
+    for shape in ((1,), (1, 1)):
+        a, b = torch.full(shape, 7, dtype=torch.int64, device='cuda'), torch.full(shape, 9, dtype=torch.int64, device='cuda')
+        rows, _, handle, _, recv = buf.low_latency_dispatch(x, idx, T, E, use_fp8=False, dispatch_wait_recv_cost_stats=a, return_recv_hook=hook)
+        if hook:
+            recv()
+        _, _, recv = buf.low_latency_combine(rows, idx, w, handle, combine_wait_recv_cost_stats=b, return_recv_hook=hook)
+        if hook:
+            recv()
+        assert (a == 7).all() and (b == 9).all()
     buf.destroy()
