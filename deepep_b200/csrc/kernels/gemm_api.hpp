@@ -37,6 +37,10 @@ struct GemmParams {
     uint64_t timeout_ns;
 };
 
+// The current device's status word for `error` above: part of the module, so it is zero before the first launch on any stream,
+// also where that launch is part of a graph capture, and there is nothing to set up once.
+cudaError_t status_word(int** word);
+
 bool make_kmajor_map(CUtensorMap* map, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t row_stride_bytes,
                      uint32_t box_rows);
 

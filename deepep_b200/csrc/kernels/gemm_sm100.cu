@@ -7,6 +7,7 @@
 // The reference library contains no GEMM; this is the compute half of the fused MoE layer and of
 // the all-gather -> GEMM / GEMM -> reduce-scatter operators (tp_fused.cu).
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 
 #include "api.hpp"
@@ -16,6 +17,8 @@
 
 namespace ep {
 namespace gemm {
+
+__device__ int pipe_status;         // see status_word
 
 namespace {
 
@@ -1332,6 +1335,19 @@ EncodeFn get_encode_fn() {
 }
 
 }  // namespace
+
+cudaError_t status_word(int** word) {
+    constexpr int kDevices = 64;
+    static std::atomic<int*> known[kDevices] = {};
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    const bool cached = device >= 0 && device < kDevices;
+    if (cached && (*word = known[device].load(std::memory_order_relaxed)) != nullptr) return cudaSuccess;
+    err = cudaGetSymbolAddress(reinterpret_cast<void**>(word), pipe_status);
+    if (err == cudaSuccess && cached) known[device].store(*word, std::memory_order_relaxed);
+    return err;
+}
 
 // 2-D K-major tensor map: `rows` x `cols` elements of `elem_bytes`, row pitch `row_stride_bytes`,
 // box = `box_rows` x (128 / elem_bytes) elements, 128-byte swizzle.

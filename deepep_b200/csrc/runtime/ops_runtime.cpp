@@ -3,13 +3,10 @@
 // tensor-parallel fused operators built on the same runtime.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/ops/empty.h>
-#include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
 #include <torch/extension.h>
 
-#include <map>
-#include <mutex>
 #include <optional>
 
 #include "../common/exception.hpp"
@@ -30,21 +27,18 @@ at::Tensor on_16_bytes(const at::Tensor& t) { return reinterpret_cast<uintptr_t>
 
 cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
-// one status word per device for the GEMM pipelines (0 = healthy); the calls of a layer come here without the GIL
-at::Tensor& gemm_status(int device) {
-    static std::mutex mutex;
-    static std::map<int, at::Tensor> words;
-    const std::lock_guard<std::mutex> lock(mutex);
-    auto it = words.find(device);
-    if (it == words.end())
-        it = words.emplace(device, at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, static_cast<c10::DeviceIndex>(device))))).first;
-    return it->second;
+// the status word of the GEMM pipelines on the current device (0 = healthy)
+int* gemm_status() {
+    int* word = nullptr;
+    CUDA_RUNTIME_CHECK(gemm::status_word(&word));
+    return word;
 }
 
 int gemm_check_status() {
-    int device = 0;
-    CUDA_RUNTIME_CHECK(cudaGetDevice(&device));
-    return gemm_status(device).item<int>();
+    int value = 0;
+    CUDA_RUNTIME_CHECK(cudaMemcpyAsync(&value, gemm_status(), sizeof(value), cudaMemcpyDeviceToHost, cur_stream()));
+    CUDA_RUNTIME_CHECK(cudaStreamSynchronize(cur_stream()));
+    return value;
 }
 
 }  // namespace
@@ -97,7 +91,7 @@ at::Tensor gemm_impl(const at::Tensor& a, const at::Tensor& b, const std::option
         p.sfb = sfb->data_ptr<float>();
         p.scales_pow2 = pow2_scales ? 1 : 0;
     }
-    p.error = gemm_status(device).data_ptr<int>();
+    p.error = gemm_status();
     p.timeout_ns = 10ull * 1000 * 1000 * 1000;
     const int sms = num_sms > 0 ? num_sms : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     const int64_t b_stride = (grouped ? b.stride(1) : b.stride(0)) * elem;
@@ -138,7 +132,7 @@ at::Tensor gemm_k_grouped(const at::Tensor& a, const at::Tensor& b, const at::Te
     p.c_group_stride = static_cast<int64_t>(M) * N;
     p.C = reinterpret_cast<__nv_bfloat16*>(out->data_ptr());
     p.ldc = N;
-    p.error = gemm_status(device).data_ptr<int>();
+    p.error = gemm_status();
     p.timeout_ns = 10ull * 1000 * 1000 * 1000;
     const int sms = num_sms > 0 ? num_sms : at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
     CUDA_RUNTIME_CHECK(gemm::launch_gemm(p, a.data_ptr(), a.stride(0) * 2, b.data_ptr(), b.stride(0) * 2, false, sms, cur_stream()));
@@ -170,7 +164,7 @@ static at::Tensor gemm_mn(const at::Tensor& a, const at::Tensor& b, bool a_trans
     p.b_mn = 1;
     p.C = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
     p.ldc = N;
-    p.error = gemm_status(device).data_ptr<int>();
+    p.error = gemm_status();
     p.timeout_ns = 10ull * 1000 * 1000 * 1000;
     CUDA_RUNTIME_CHECK(gemm::launch_gemm(p, a.data_ptr(), a.stride(0) * 2, b.data_ptr(), b.stride(0) * 2, false,
                                          at::cuda::getCurrentDeviceProperties()->multiProcessorCount, cur_stream()));

@@ -252,3 +252,28 @@ def test_grouped_tiles_with_few_rows(counts, mode, monkeypatch):
         ref = (a_ref[start:start + c].double() @ b_ref[gi].double().t())
         assert bool(((out[start:start + c].double() - ref).abs() <= ref.abs() * 2.0 ** -8).all())
         start = -(-(start + c) // align) * align
+
+
+def test_first_gemm_of_a_process_inside_a_capture():
+    """The status word of the pipelines is there, and zero, before anything has run: the first call may be part of a graph that
+    is replayed later or never. (A process of its own.)"""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch, deepep_b200
+C = deepep_b200._C
+a, b = torch.ones((128, 256), device='cuda').bfloat16(), torch.ones((128, 256), device='cuda').bfloat16()
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    captured = C.gemm(a, b)
+eager = C.gemm(a, b)
+assert (eager == 256).all() and C.gemm_check_status() == 0
+graph.replay()
+torch.cuda.synchronize()
+assert (captured == 256).all() and C.gemm_check_status() == 0
+graph.reset()
+"""
+    done = subprocess.run([sys.executable, '-c', code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
